@@ -1,18 +1,10 @@
-// fillflags.cuh -- the pit fill's per-cell flags and their set-up, shared by
-// the fill (pitfill.cu) and the fused front, which sets them up as it writes
-// the quantized grid.
+// fillflags.cuh -- the pit fill's passability test.
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
 #include "stage_math.cuh"
 
 namespace cageo {
-
-// Per-cell flag bits.  FCLEAN (flood A with clean marks): the cell's level
-// is reached by a path of passable relays from an outlet, so flood B, whose
-// walls are non-passable cells only, gives it the same value.
-constexpr uint8_t FNODATA = 0x01, FOUTLET = 0x02, FNONPASS = 0x04, FCONF = 0x08,
-                  FBELOW = 0x10, FBELOWA = 0x20, FCLEAN = 0x40, FUNSURE = 0x80;
 
 // fill_passable() of a quantized value q = RN(k / 1000) (k an integer, as
 // fill_quantize makes every value the fill sees).  With minE = 0 and
@@ -29,17 +21,6 @@ __device__ __forceinline__ bool passable_quantized(float q, float minE) {
     return p >= rintf(p);
   }
   return fill_passable(q, minE);
-}
-
-// Flags of a cell before the floods: NODATA; otherwise non-passable when
-// its quantized value q fails the round trip at minE, and an outlet (clean
-// from the start: outlets keep q in both floods) on the border or at 0.
-__device__ __forceinline__ uint8_t fill_init_flags(float q, float nodata, float minE,
-                                                   bool border) {
-  if (q == nodata) return FNODATA;
-  uint8_t f = passable_quantized(q, minE) ? 0 : FNONPASS;
-  if (border || q == 0.0f) f |= FOUTLET | FCLEAN;
-  return f;
 }
 
 }  // namespace cageo

@@ -14,27 +14,40 @@
 // on cells with a strictly lower q, so the solution is unique, and it is
 // computed here by monotone relaxations:
 //
-//   1. flood A: every reached cell relays (non-passable outlets do not):
-//      gives L_A <= L everywhere (a lower bound);
-//   2. non-passable cells with L_A >= q are certainly expanding ("confirmed");
-//      the other non-passable cells are walls for now;
-//   3. flood B from +inf with walls: an upper bound L_B >= L;
-//   4. phases: M = min L_B over unconfirmed non-passable cells with
-//      L_B >= q; every such cell with q <= M is confirmed (no later change
-//      can take its level below M >= q); relax again; repeat until none.
+//   1. walled flood: only passable cells relay.  Every level is a path the
+//      reference's fill may take, so the result S is an upper bound; a
+//      non-passable cell with S == q was reached below q (its incoming level
+//      is a passable value, never q itself) and is a wall for good.  On
+//      terrain rounded to 1 mm about 1% of the cells are non-passable, and S
+//      differs from the answer on 0.1-0.2% of the cells: pockets of lakes cut
+//      off by non-passable cells under water (S > q), which do expand.
+//   2. lower bound A: from S, the non-passable cells with S > q relay as well
+//      (and go on relaying when they fall below q): the cells that truly
+//      expand are among them, so A <= answer <= S.  If no such cell ends at
+//      or below its q, A solves the fill's equation, whose solution is
+//      unique: A is the answer.
+//   3. otherwise the cells with A != S form 8-connected components that no
+//      change can leave.  A component without a cell of the kind just named
+//      is settled at A.  In the others the cells restart at S, those
+//      non-passable cells with A > q are confirmed (they certainly expand),
+//      and phases follow: relax; M = the component's least level among
+//      unconfirmed non-passable cells above their q; every such cell with
+//      q <= M is confirmed (no later change can take its level below M);
+//      until none is left.
 //
-// Each flood is a persistent cooperative kernel.  One warp owns a 32x32
-// tile at a time, stages W, q, flags and the relay values of a one-cell
-// halo in shared memory and sweeps it down, up, right and left (Gauss-Seidel)
-// until it stops changing; a tile whose border changed queues the
-// neighbouring tiles on an asynchronous work queue (no pass barriers; see
-// the queue below).  A flood ends when no tile is queued or in process.
-// Every wait and every loop is bounded; exceeding a bound sets an error
-// flag that the host turns into CAGEO_ERR_NO_CONVERGENCE.
+// Steps 2 and 3 work on lists of cells (fill_resolve_kernel); the flood of
+// step 1 -- and the exact fill, which is that flood without walls -- is a
+// persistent cooperative kernel over 32x32 tiles (levelflood.cuh): one warp
+// owns a tile at a time and sweeps it until it is a fixed point for its
+// neighbours' rims; a tile whose rim changed queues the neighbouring tiles on
+// an asynchronous work queue (no pass barriers; tilequeue.cuh).  The flood
+// ends when no tile is queued or in process.  Every wait and every loop is
+// bounded; exceeding a bound sets an error flag that the host turns into
+// CAGEO_ERR_NO_CONVERGENCE.
 #include <algorithm>
-#include <type_traits>
 #include "common.cuh"
 #include "fillflags.cuh"
+#include "levelflood.cuh"
 #include "pitfill.cuh"
 #include "stage_math.cuh"
 #include "tilequeue.cuh"
@@ -45,35 +58,37 @@ namespace cageo {
 enum : int {
   S_MIN = 0,       // ordered min of q (minE)
   S_ERR = 3,       // 0 ok; 1 barrier wait; 2 idle wait; 3 queue state; 4 visits; 5 phases; 6 union
-  S_M = 7,         // 3 slots: ordered phase minima
-  S_CAND = 10,     // number of undecided cells
-  S_PASS = 11,     // drains run so far in this fill (a drain empties the work queue)
+  S_FLAG = 7,      // resolution: something happened in this round
+  S_RESULT = 8,    // ... and its value at the last barrier
+  S_MORE_AT = 9,   // S_MORE at the last barrier
+  S_CAND = 10,     // walls on the list of the resolution
+  S_MORE = 22,     // cells listed by the resolution itself
+  S_OPEN = 23,     // cells of the reopened components
+  S_PASS = 11,     // floods and relaxations run so far in this fill
   S_PHASES = 12,
-  S_PASSES_A = 13, // drains of flood A (1)
-  S_PASSES_B = 14, // drains of flood B before the first phase (1)
-  S_US_A = 15,     // microseconds of flood A
-  S_US_B = 16,     // microseconds of flood B up to its first convergence
-  S_US_P = 17,     // microseconds of the phase loop
-  S_PEND = 18,     // 3 slots: pending cells seen by a phase
+  S_PASSES_A = 13, // drains of the flood (1)
+  S_STEPS = 14,    // relaxation steps of the resolution's longest front, before the phases
+  S_US_A = 15,     // microseconds of the flood
+  S_US_B = 16,     // microseconds of the lower bound (or of a repair flood)
+  S_US_P = 17,     // microseconds of the phases
   S_RESET = 21,    // warm-started exact fill: cells restarted from +inf (unsupported)
-  S_DBG = 24,      // 8 slots: the phase loop's state when it passed its limit (see below)
   // Per-visit statistics, updated by every tile visit: a line of their own
   // (96..127), away from the error flag that idle warps poll.
-  S_TILES_A = 96,   // tiles processed by flood A
-  S_ROUNDS_A = 97,  // sweep rounds run by flood A
-  S_TILES_B = 98,   // tiles processed by flood B (phases included)
-  S_ROUNDS_B = 99,  // sweep rounds run by flood B
+  S_TILES_A = 96,   // tiles processed by the flood
+  S_ROUNDS_A = 97,  // sweep rounds run by the flood
+  S_TILES_B = 98,   // tiles processed by a repair flood
+  S_ROUNDS_B = 99,  // sweep rounds run by a repair flood
   S_KCYC_LOAD = 100,   // kilo-cycles (summed over tile visits) staging tiles
   S_KCYC_SWEEP = 101,  // kilo-cycles sweeping
   S_KCYC_STORE = 102,  // kilo-cycles writing back and queueing
-  S_KCYC_IDLE_A = 103, // kilo-cycles warps of flood A waited for a tile (tail included)
-  S_KCYC_IDLE_B = 104, // the same for flood B's drains
+  S_KCYC_IDLE_A = 103, // kilo-cycles warps of the flood waited for a tile (tail included)
+  S_KCYC_IDLE_B = 104, // the same for a repair flood
   S_HEAD = 128,      // work-queue tickets handed out (own 128-byte line)
   S_TAIL = 160,      // work-queue entries pushed (own line)
   S_PENDING = 192,   // tiles queued or being processed (own line)
   S_BAR_COUNT = kBarCountSlot,
   S_BAR_GEN = kBarGenSlot,
-  S_SIZE = 224
+  S_SIZE = kFillScalars
 };
 
 __device__ __forceinline__ unsigned long long global_ns() {
@@ -82,56 +97,22 @@ __device__ __forceinline__ unsigned long long global_ns() {
   return t;
 }
 
-constexpr int kTile = 32;
-constexpr int kRS = 35;           // relay row stride (34 used)
-constexpr int kWS = 33;           // W/q row stride
-constexpr int kFS = 36;           // flag row stride (bytes)
+// Per-cell flag bits of the resolution.
+constexpr unsigned int kActive = 1, kConfirmed = 2, kMember = 4, kReopened = 8;
 
-// Per-warp staged tile.  R: relay values of the tile and its one-cell halo.
-// In flood A (modes 0 and 2) every cell that can change relays its own W,
-// so W lives in R and only q is kept beside it (Q); flood B keeps (W, q)
-// pairs (WQ), since its walls relay +inf whatever their W.  F: flags of the
-// tile's own cells.  HC: clean relays of the halo (mode 2): [0] the row
-// above and [1] the row below the tile (halo x 0..33), [2] the column left
-// and [3] the column right of it (halo y 0..33); 1 = clean and passable.
-struct SmemA {
-  float R[34 * kRS];
-  float Q[kTile * kWS];
-  uint8_t F[kTile * kFS];
-  uint8_t HC[4][34];
-};
-struct SmemB {
-  float R[34 * kRS];
-  float2 WQ[kTile * kWS];
-  uint8_t F[kTile * kFS];
-};
-template <int MODE>
-using WarpSmem = typename std::conditional<MODE == 1, SmemB, SmemA>::type;
-
-// Warps per block (one block per SM) of the flood launches.  Flood B runs
-// 16 (14.0 KB of shared memory each); flood A runs 16, 20 or 22 (10.0 KB
-// each), chosen by FillWork::flood_warps (the autotuner picks it), with the
-// register budget the launch bounds give each.
-constexpr int kWarpsB = 16;
-
-__device__ __forceinline__ float staged_w(const SmemA& s, int x, int y) {
-  return s.R[(y + 1) * kRS + x + 1];
-}
-__device__ __forceinline__ float staged_w(const SmemB& s, int x, int y) {
-  return s.WQ[y * kWS + x].x;
-}
-__device__ __forceinline__ float staged_q(const SmemA& s, int x, int y) {
-  return s.Q[y * kWS + x];
-}
-__device__ __forceinline__ float staged_q(const SmemB& s, int x, int y) {
-  return s.WQ[y * kWS + x].y;
+// The space that the flood's rims and masks share with the component labels
+// of the resolution: the labels are the larger part except on grids only a
+// few cells wide.
+static size_t shared_bytes(size_t n, size_t nt) {
+  return std::max(align_up(n * 4, 256), align_up(nt * kRimCells * sizeof(uint2), 256) +
+                                            3 * align_up(nt * kTile * 4, 256));
 }
 
 size_t fill_workspace_bytes(int W, int H) {
   size_t n = (size_t)W * H;
   size_t nt = (size_t)((W + kTile - 1) / kTile) * ((H + kTile - 1) / kTile);
   return align_up(n, 256) + align_up(nt * 4, 256) + align_up((2 * nt + kRingSlack) * 4, 256) +
-         2 * align_up(nt, 256) + 3 * align_up(n * 4, 256) + 1024;
+         2 * align_up(nt, 256) + 2 * align_up(n * 4, 256) + shared_bytes(n, nt) + 1024;
 }
 
 FillWork fill_carve(void* base, int W, int H) {
@@ -150,50 +131,27 @@ FillWork fill_carve(void* base, int W, int H) {
   p += align_up((2 * nt + kRingSlack) * 4, 256);
   w.tseed = (uint8_t*)p;
   p += align_up(nt, 256);
-  w.tconv = (uint8_t*)p;
+  w.tvis = (uint8_t*)p;
   p += align_up(nt, 256);
-  w.cand = (uint32_t*)p;
-  p += align_up(n * 4, 256);
   w.aux = (uint32_t*)p;
   p += align_up(n * 4, 256);
-  w.cmin = (uint32_t*)p;
+  w.cand = (uint32_t*)p;
   p += align_up(n * 4, 256);
+  w.label = (uint32_t*)p;
+  char* r = p;
+  w.rim = (uint2*)r;
+  r += align_up(nt * kRimCells * sizeof(uint2), 256);
+  w.mclean = (uint32_t*)r;
+  r += align_up(nt * kTile * 4, 256);
+  w.mdead = (uint32_t*)r;
+  r += align_up(nt * kTile * 4, 256);
+  w.mwall = (uint32_t*)r;
+  p += shared_bytes(n, nt);
   w.scal = (unsigned int*)p;
   return w;
 }
 
 unsigned int* fill_min_slot(const FillWork& w) { return w.scal + S_MIN; }
-
-// Flood modes: 0 = flood A (every reached cell relays), 2 = flood A that
-// also keeps the clean marks (FCLEAN), 1 = flood B (non-passable cells that
-// are not confirmed are walls).
-template <int MODE>
-__device__ __forceinline__ float relay(float w, uint8_t f, float q) {
-  if (f & FNODATA) return kInf;
-  if (f & FOUTLET) return (f & FNONPASS) ? kInf : q;
-  if (MODE != 1 || !(f & FNONPASS)) return w;
-  // A clean cell kept flood A's level, which is finite; it is confirmed
-  // exactly when it is not below its q (what FCONF records for the others).
-  // Every level flood B relays is a passable value (it starts at a passable
-  // outlet's q and is only carried or raised to a passable cell's q), never
-  // a non-passable q, so a non-passable cell whose level equals its q was
-  // reached below it and is a wall: the store that lowered it to q also set
-  // FBELOW.  Testing w != q keeps a halo read that sees the new level but
-  // not yet the new flags (another SM's write-back stores the two with no
-  // order between them) from relaying q.
-  return ((f & (FCONF | FCLEAN)) && !(f & FBELOW) && w != q) ? w : kInf;
-}
-
-struct FloodArgs {
-  const float* q;
-  float* Wg;
-  FillWork w;
-  // Flood B runs as two launches: 1 = seeding and the main drain, 2 = the
-  // confirmation phases (the undecided cells found and labelled by plain
-  // kernels in between).  3 = the repair flood of a warm-started exact fill
-  // (its statistics go to flood B's slots).  Flood A ignores 1 and 2.
-  int stage = 0;
-};
 
 // ---- asynchronous tile work queue (tilequeue.cuh) --------------------------
 // The fill's queue: tile states in w.queued, the ring in w.lists
@@ -210,67 +168,8 @@ __device__ __forceinline__ TileQueue fill_queue(const FillWork& w) {
 
 __device__ __forceinline__ void enqueue(const FillWork& w, int t) { tq_enqueue(fill_queue(w), t); }
 
-// Relaxation of staged cell (x, y) given m, the least relay among the
-// neighbours it reads, split into its loads (cell_load) and its update
-// (cell_store, true if the cell changed) so that the two cells of a sweep
-// step are both loaded before either is written.  A cell whose incoming
-// level has dropped below its own q (FBELOW) is final in both floods: its
-// value is q and its relay can no longer change.
-struct CellEval {
-  float w, q, m;
-  uint8_t f;
-};
-
-template <class S>
-__device__ __forceinline__ CellEval cell_load(const S& s, int x, int y, float m) {
-  return CellEval{staged_w(s, x, y), staged_q(s, x, y), m, s.F[y * kFS + x]};
-}
-
-template <int MODE>
-__device__ __forceinline__ bool cell_store(WarpSmem<MODE>& s, int x, int y, const CellEval& e) {
-  if (e.f & (FNODATA | FOUTLET | FBELOW)) return false;
-  const float nw = fminf(e.w, fmaxf(e.q, e.m));
-  const bool below = e.m < e.q;  // sets FBELOW, which the cell does not have yet
-  if (nw == e.w && !below) return false;
-  if constexpr (MODE == 1) s.WQ[y * kWS + x].x = nw;  // in flood A, R below holds W
-  // A fall of W withdraws the cell's clean mark (its clean path may not
-  // reach the new level); the clean pass after the sweeps derives it again.
-  if (MODE == 2 && nw != e.w) s.F[y * kFS + x] = (e.f | (below ? FBELOW : 0)) & (uint8_t)~FCLEAN;
-  else if (below) s.F[y * kFS + x] = e.f | FBELOW;
-  // relay<MODE>() of a cell that is neither NODATA nor an outlet
-  const bool wall = MODE == 1 && (e.f & FNONPASS) && (below || !(e.f & (FCONF | FCLEAN)));
-  s.R[(y + 1) * kRS + (x + 1)] = wall ? kInf : nw;
-  return true;
-}
-
-// Least relay of the three staged cells in relay row ry (tile row ry - 1),
-// tile columns x-1..x+1: the neighbours of (x, ry - 2) below it or of
-// (x, ry) above it.
-template <class S>
-__device__ __forceinline__ float row3_min(const S& s, int x, int ry) {
-  const float* r = &s.R[ry * kRS + x];
-  return fminf(fminf(r[0], r[1]), r[2]);
-}
-
-// Least relay of the three staged cells in relay column rx (tile column
-// rx - 1), tile rows y-1..y+1.
-template <class S>
-__device__ __forceinline__ float col3_min(const S& s, int rx, int y) {
-  const float* r = &s.R[y * kRS + rx];
-  return fminf(fminf(r[0], r[kRS]), r[2 * kRS]);
-}
-
-// Per-warp visit statistics (lane 0), added to the scalar block every 64
-// visits and when a drain ends: one atomic per counter and flush instead of
-// five atomics on one cache line per visit.
-struct VisitStats {
-  unsigned int tiles = 0, rounds = 0, kload = 0, ksweep = 0, kstore = 0, kidle = 0;
-};
-
-template <int MODE>
 __device__ __forceinline__ void flush_stats(const FillWork& w, VisitStats& st, bool b_slots) {
   if (!st.tiles && !st.kidle) return;
-  b_slots = b_slots || MODE == 1;
   atomicAdd(&w.scal[b_slots ? S_TILES_B : S_TILES_A], st.tiles);
   atomicAdd(&w.scal[b_slots ? S_ROUNDS_B : S_ROUNDS_A], st.rounds);
   atomicAdd(&w.scal[S_KCYC_LOAD], st.kload);
@@ -280,359 +179,7 @@ __device__ __forceinline__ void flush_stats(const FillWork& w, VisitStats& st, b
   st = VisitStats{};
 }
 
-// Clean marks of a tile whose W has converged for its halo (flood A with
-// clean marks).  A cell turns clean when a neighbour that is clean and
-// passable (a relay flood B keeps) offers a level <= its W: that
-// neighbour's clean path, extended by the cell, reaches the cell at no more
-// than W, and flood B, which never undershoots flood A, then gives it W
-// too.  The rule is sound whatever W is, so a cell keeps its mark until its
-// W falls (cell_store withdraws it).  Lane = tile column x; per-lane masks
-// hold bit y for tile row y.  The eight "offers <= W" tests are made once
-// per cell; the marks then spread by bit operations on the column masks
-// (neighbour columns by shuffles) until no lane changes, at most
-// `max_iter` times.  Returns this lane's column of newly clean cells.
-__device__ __forceinline__ unsigned int clean_pass(SmemA& s, int lane, int max_iter) {
-  unsigned int qN = 0, qS = 0, qW = 0, qE = 0, qNW = 0, qNE = 0, qSW = 0, qSE = 0;
-  unsigned int cl = 0, pas = 0;
-  // Relay rows y, y+1, y+2 (tile rows y-1, y, y+1) at columns lane..lane+2.
-  float a0 = s.R[lane], a1 = s.R[lane + 1], a2 = s.R[lane + 2];
-  float b0 = s.R[kRS + lane], b1 = s.R[kRS + lane + 1], b2 = s.R[kRS + lane + 2];
-#pragma unroll 4
-  for (int y = 0; y < kTile; y++) {
-    const float* rc = &s.R[(y + 2) * kRS + lane];
-    const float c0 = rc[0], c1 = rc[1], c2 = rc[2];
-    const uint8_t f = s.F[y * kFS + lane];
-    const unsigned int bit = 1u << y;
-    // b1 is the cell's own relay: its W (every non-outlet cell relays in flood A).
-    const float wv = b1;
-    if (f & FCLEAN) cl |= bit;
-    if (!(f & (FNONPASS | FNODATA))) pas |= bit;
-    if (!(f & (FCLEAN | FNODATA)) && wv < kInf) {
-      if (a0 <= wv) qNW |= bit;
-      if (a1 <= wv) qN |= bit;
-      if (a2 <= wv) qNE |= bit;
-      if (b0 <= wv) qW |= bit;
-      if (b2 <= wv) qE |= bit;
-      if (c0 <= wv) qSW |= bit;
-      if (c1 <= wv) qS |= bit;
-      if (c2 <= wv) qSE |= bit;
-    }
-    a0 = b0; a1 = b1; a2 = b2;
-    b0 = c0; b1 = c1; b2 = c2;
-  }
-  const unsigned int cl0 = cl;
-  if (!__any_sync(0xffffffffu, (qN | qS | qW | qE | qNW | qNE | qSW | qSE) != 0)) return 0u;
-  // Clean relays of the halo: this lane's cells of the rows above and below
-  // the tile, and the halo columns as 34-bit masks (bit = halo row 0..33).
-  const unsigned long long top = s.HC[0][lane + 1], bot = s.HC[1][lane + 1];
-  unsigned long long lcol = __ballot_sync(0xffffffffu, s.HC[2][lane] != 0);
-  unsigned long long rcol = __ballot_sync(0xffffffffu, s.HC[3][lane] != 0);
-  lcol |= ((unsigned long long)s.HC[2][32] << 32) | ((unsigned long long)s.HC[2][33] << 33);
-  rcol |= ((unsigned long long)s.HC[3][32] << 32) | ((unsigned long long)s.HC[3][33] << 33);
-  for (int it = 0; it < max_iter; it++) {
-    // Column mask of clean relays, bit = halo row (tile row + 1).
-    const unsigned long long own = ((unsigned long long)(cl & pas) << 1) | top | (bot << 33);
-    unsigned long long L = __shfl_up_sync(0xffffffffu, own, 1);
-    unsigned long long R = __shfl_down_sync(0xffffffffu, own, 1);
-    if (lane == 0) L = lcol;
-    if (lane == 31) R = rcol;
-    const unsigned int nc =
-        cl | (qN & (unsigned int)own) | (qS & (unsigned int)(own >> 2)) |
-        (qW & (unsigned int)(L >> 1)) | (qE & (unsigned int)(R >> 1)) | (qNW & (unsigned int)L) |
-        (qNE & (unsigned int)R) | (qSW & (unsigned int)(L >> 2)) | (qSE & (unsigned int)(R >> 2));
-    const bool changed = nc != cl;
-    cl = nc;
-    if (!__any_sync(0xffffffffu, changed)) break;
-  }
-  const unsigned int turned = cl & ~cl0;
-  for (unsigned int m = turned; m; m &= m - 1) {
-    const int y = __ffs(m) - 1;
-    s.F[y * kFS + lane] |= FCLEAN;
-  }
-  __syncwarp();
-  return turned;
-}
-
-// Returns whether every cell of the tile is final (NODATA, outlet or FBELOW;
-// with clean marks also clean).
-template <int MODE>
-__device__ bool process_tile(WarpSmem<MODE>& s, const FloodArgs& a, int t, int lane, VisitStats& st) {
-  const FillWork& w = a.w;
-  const int W = w.W, H = w.H;
-  const int tx = t % w.tiles_x, ty = t / w.tiles_x;
-  const int x0 = tx * kTile, y0 = ty * kTile;
-  const long long c0 = clock64();
-  if constexpr (MODE != 1) {
-    // Flood A needs q only for the tile's own cells (an outlet's W is its q,
-    // which is all its relay needs), and q never changes: asynchronous
-    // copies, all in flight while the loop below loads W and the flags.
-    for (int idx = lane; idx < kTile * kTile; idx += 32) {
-      const int ty_ = idx >> 5, tx_ = idx & 31;
-      const int gx = x0 + tx_, gy = y0 + ty_;
-      float* dq = &s.Q[ty_ * kWS + tx_];
-      if (gx < W && gy < H) cp_async4(dq, a.q + (int64_t)gy * W + gx);
-      else *dq = 0.0f;
-    }
-  }
-  // Flood A on a tile whose 32 columns lie inside the grid, with 16-byte
-  // aligned rows: its columns' levels and flags by 16-byte and 4-byte loads
-  // (8 chunks of 4 cells per staged row, 8.5 per lane, all in flight at
-  // once), the two halo columns by scalar loads: about 21 loads per lane
-  // instead of 72.  Every load lies inside the grid.
-  const bool vec = MODE != 1 && x0 + kTile <= W && (W & 3) == 0 &&
-                   ((reinterpret_cast<uintptr_t>(a.Wg) | reinterpret_cast<uintptr_t>(w.flags)) &
-                    15u) == 0;
-  if (vec) {
-    constexpr int kChunks = 34 * (kTile / 4);  // 272
-#pragma unroll
-    for (int it = 0; it < (kChunks + 31) / 32; it++) {
-      const int k = lane + 32 * it;
-      if (k < kChunks) {
-        const int hy = k >> 3, c = k & 7;
-        const int gy = y0 - 1 + hy;
-        float4 wv = make_float4(kInf, kInf, kInf, kInf);
-        unsigned int f4 = 0x01010101u * FNODATA;
-        if (gy >= 0 && gy < H) {
-          const int64_t i = (int64_t)gy * W + x0 + 4 * c;
-          wv = __ldcg(reinterpret_cast<const float4*>(a.Wg + i));
-          f4 = __ldcg(reinterpret_cast<const unsigned int*>(w.flags + i));
-        }
-        float* r = &s.R[hy * kRS + 1 + 4 * c];
-        r[0] = relay<MODE>(wv.x, (uint8_t)f4, wv.x);
-        r[1] = relay<MODE>(wv.y, (uint8_t)(f4 >> 8), wv.y);
-        r[2] = relay<MODE>(wv.z, (uint8_t)(f4 >> 16), wv.z);
-        r[3] = relay<MODE>(wv.w, (uint8_t)(f4 >> 24), wv.w);
-        if (hy >= 1 && hy <= kTile)
-          *reinterpret_cast<unsigned int*>(&s.F[(hy - 1) * kFS + 4 * c]) = f4;
-      }
-    }
-#pragma unroll
-    for (int it = 0; it < 3; it++) {
-      const int k = lane + 32 * it;
-      if (k < 2 * 34) {
-        const int side = k >= 34 ? 1 : 0, hy = k - 34 * side;
-        const int hx = side ? kTile + 1 : 0;
-        const int gx = x0 - 1 + hx, gy = y0 - 1 + hy;
-        float wv = kInf;
-        uint8_t fv = FNODATA;
-        if (gx >= 0 && gx < W && gy >= 0 && gy < H) {
-          const int64_t i = (int64_t)gy * W + gx;
-          wv = __ldcg(a.Wg + i);
-          fv = __ldcg(w.flags + i);
-        }
-        s.R[hy * kRS + hx] = relay<MODE>(wv, fv, wv);
-      }
-    }
-  }
-#pragma unroll 12
-  for (int idx = vec ? 34 * 34 : lane; idx < 34 * 34; idx += 32) {
-    int hy = idx / 34, hx = idx - hy * 34;
-    int gx = x0 - 1 + hx, gy = y0 - 1 + hy;
-    float wv = kInf, qv = 0.0f;
-    uint8_t fv = FNODATA;
-    if (gx >= 0 && gx < W && gy >= 0 && gy < H) {
-      int64_t i = (int64_t)gy * W + gx;
-      wv = __ldcg(a.Wg + i);  // L2: written by other SMs with no barrier in between
-      if constexpr (MODE == 1) qv = a.q[i];
-      fv = __ldcg(w.flags + i);
-    }
-    s.R[hy * kRS + hx] = relay<MODE>(wv, fv, MODE == 1 ? qv : wv);
-    if (hx >= 1 && hx <= kTile && hy >= 1 && hy <= kTile) {
-      if constexpr (MODE == 1) s.WQ[(hy - 1) * kWS + hx - 1] = make_float2(wv, qv);
-      s.F[(hy - 1) * kFS + hx - 1] = fv;
-    }
-  }
-  if constexpr (MODE != 1) cp_async_wait();
-  unsigned int clean0 = 0;  // MODE 2: this lane's column, rows clean when staged
-  if constexpr (MODE == 2) {
-    // Clean relays of the halo: strips of 34 cells (row above, row below,
-    // column left, column right), flags read again from L2, after the
-    // levels and a fence.  A clean mark holds for the level it was derived
-    // at; a write-back that lowers a clean cell's level (withdrawing or
-    // re-deriving its mark) stores the flags, fences, then stores the level.
-    // So a halo level read above that is already the new one comes with a
-    // flag read here that is at least as new: never a stale clean mark with
-    // a lower level, which could mark a neighbour clean too low.
-    __threadfence();
-    for (int k = lane; k < 4 * 34; k += 32) {
-      const int strip = k / 34, j = k - strip * 34;
-      const int hx = strip < 2 ? j : (strip == 2 ? 0 : 33);
-      const int hy = strip < 2 ? (strip == 0 ? 0 : 33) : j;
-      const int gx = x0 - 1 + hx, gy = y0 - 1 + hy;
-      uint8_t fv = FNODATA;
-      if (gx >= 0 && gx < W && gy >= 0 && gy < H) fv = __ldcg(w.flags + (int64_t)gy * W + gx);
-      s.HC[strip][j] = (fv & (FCLEAN | FNONPASS | FNODATA)) == FCLEAN;
-    }
-    __syncwarp();
-#pragma unroll 8
-    for (int y = 0; y < kTile; y++)
-      clean0 |= (s.F[y * kFS + lane] & FCLEAN) ? (1u << y) : 0u;
-  }
-  __syncwarp();
-  const long long c1 = clock64();
-  // Sweeps.  Each of the four directions reads only the three neighbours on
-  // the side it comes from: down (row by row from the top) the row above,
-  // up the row below, right the column to the left, left the column to the
-  // right; a round is a vertical phase (down and up interleaved) and a
-  // horizontal phase (right and left interleaved).  Together the four read
-  // all 8 neighbours.  Warp-uniform masks hold the rows (pd, pu) and
-  // columns (pr, pl) each direction still has to evaluate; a bit is cleared
-  // when its row or column is evaluated.  A change at (x, y) sets the
-  // directions that read it: row y+1 down, y-1 up, column x+1 right, x-1
-  // left.  A bit set for a row or column its sweep has already passed stays
-  // set into the next round.  When all four masks are empty, every cell has
-  // been evaluated against each neighbour since that neighbour last changed:
-  // the tile is at a fixpoint for its halo.
-  // A tile that converged on an earlier visit is a fixpoint for its old halo:
-  // only the rows and columns that read the halo need evaluating first.
-  // (written by whichever warp processed the tile last, maybe on another SM)
-  const bool revisit = ((volatile uint8_t*)w.tconv)[t] != 0;
-  const int max_rounds = w.max_rounds;
-  unsigned int pd = revisit ? 1u : ~0u, pu = revisit ? 0x80000000u : ~0u;
-  unsigned int pr = pd, pl = pu;
-  unsigned int dc = 0;  // this lane's column: rows of the cells changed on this visit
-  int rounds = 0;
-  // A step evaluates both of its rows (columns) when either is pending: the
-  // two cells are loaded before either is stored, so their dependency chains
-  // overlap.  Extra evaluations are harmless (any relaxation step is), and
-  // at the crossing (k = 16) a cell that reads the other's old value is
-  // re-evaluated through the masks like any other.
-  for (; rounds < max_rounds && (pd | pu | pr | pl); rounds++) {
-    // Step k evaluates row k (down) and row 31 - k (up); steps with neither
-    // pending are skipped by a find-first-set over both masks.
-    for (int k = 0; k < kTile; k++) {
-      const unsigned int m = (pd | __brev(pu)) >> k;
-      if (!m) break;
-      k += __ffs(m) - 1;
-      const int d = k, u = kTile - 1 - k;
-      const unsigned int bd = 1u << d, bu = 1u << u;
-      pd &= ~bd;
-      pu &= ~bu;
-      const CellEval ed = cell_load(s, lane, d, row3_min(s, lane, d));
-      const CellEval eu = cell_load(s, lane, u, row3_min(s, lane, u + 2));
-      const bool cd = cell_store<MODE>(s, lane, d, ed);
-      const bool cu = cell_store<MODE>(s, lane, u, eu);
-      dc |= (cd ? bd : 0u) | (cu ? bu : 0u);
-      const unsigned int b1 = __ballot_sync(0xffffffffu, cd), b2 = __ballot_sync(0xffffffffu, cu);
-      if (b1 | b2) {
-        const unsigned int rows = (b1 ? bd : 0u) | (b2 ? bu : 0u), cols = b1 | b2;
-        pd |= rows << 1;
-        pu |= rows >> 1;
-        pr |= cols << 1;
-        pl |= cols >> 1;
-      }
-      __syncwarp();
-    }
-    for (int k = 0; k < kTile; k++) {
-      const unsigned int m = (pr | __brev(pl)) >> k;
-      if (!m) break;
-      k += __ffs(m) - 1;
-      const int l = k, r = kTile - 1 - k;
-      const unsigned int bl = 1u << l, br = 1u << r;
-      pr &= ~bl;
-      pl &= ~br;
-      const CellEval el = cell_load(s, l, lane, col3_min(s, l, lane));
-      const CellEval er = cell_load(s, r, lane, col3_min(s, r + 2, lane));
-      const bool cl = cell_store<MODE>(s, l, lane, el);
-      const bool cr = cell_store<MODE>(s, r, lane, er);
-      const unsigned int b1 = __ballot_sync(0xffffffffu, cl), b2 = __ballot_sync(0xffffffffu, cr);
-      if (b1 | b2) {
-        const unsigned int cols = (b1 ? bl : 0u) | (b2 ? br : 0u), rows = b1 | b2;
-        pr |= cols << 1;
-        pl |= cols >> 1;
-        pd |= rows << 1;
-        pu |= rows >> 1;
-        dc |= (lane == l ? b1 : 0u) | (lane == r ? b2 : 0u);
-      }
-      __syncwarp();
-    }
-  }
-  const bool capped = (pd | pu | pr | pl) != 0;
-  // Each round of the clean pass marks at least one more cell, so 1024
-  // rounds always reach its fixpoint.
-  if constexpr (MODE == 2) dc |= clean_pass(s, lane, kTile * kTile);
-  const long long c2 = clock64();
-  if (lane == 0) {
-    w.tconv[t] = capped ? 0 : 1;
-    st.tiles++;
-    st.rounds += (unsigned int)rounds;
-  }
-  // Write back the changed cells, row by row (coalesced); note which
-  // borders changed.  Cells outside the grid are NODATA and never change.
-  // With clean marks, a changed cell that was clean when staged may have a
-  // lower level and a withdrawn or re-derived mark: flags first, a fence,
-  // then the levels (the readers' side is in the staging above).
-  const unsigned int rows_changed = __reduce_or_sync(0xffffffffu, dc);
-  bool flags_first = false;
-  if constexpr (MODE == 2) flags_first = __any_sync(0xffffffffu, (dc & clean0) != 0u);
-  if (flags_first) {
-    for (unsigned int rows = rows_changed; rows; rows &= rows - 1) {
-      const int y = __ffs(rows) - 1;
-      if ((dc >> y) & 1u) w.flags[(int64_t)(y0 + y) * W + (x0 + lane)] = s.F[y * kFS + lane];
-    }
-    __threadfence();
-  }
-  for (unsigned int rows = rows_changed; rows; rows &= rows - 1) {
-    const int y = __ffs(rows) - 1;
-    if ((dc >> y) & 1u) {
-      const int64_t i = (int64_t)(y0 + y) * W + (x0 + lane);
-      a.Wg[i] = staged_w(s, lane, y);
-      if (!flags_first) w.flags[i] = s.F[y * kFS + lane];
-    }
-  }
-  // The write-back (and a "not converged" mark) is visible before any
-  // neighbour is queued or the tile's state changes.  A visit that changed
-  // nothing wrote nothing and queues no one.
-  if (rows_changed) __threadfence();
-  const unsigned int dl = __shfl_sync(0xffffffffu, dc, 0), dr = __shfl_sync(0xffffffffu, dc, 31);
-  // 1 L, 2 R, 4 T, 8 B, 16 TL, 32 TR, 64 BL, 128 BR
-  const unsigned int sides = (dl ? 1u : 0u) | (dr ? 2u : 0u) | ((rows_changed & 1u) ? 4u : 0u) |
-                             ((rows_changed >> 31) ? 8u : 0u) | ((dl & 1u) ? 16u : 0u) |
-                             ((dr & 1u) ? 32u : 0u) | ((dl >> 31) ? 64u : 0u) |
-                             ((dr >> 31) ? 128u : 0u);
-  // Every cell final?  Only a change can make it so after the first visit: a
-  // later visit that changed nothing leaves the answer of the visit before.
-  bool done = false;
-  if (rows_changed || !revisit) {
-    bool fin = true;
-    for (int idx = lane; idx < kTile * kTile; idx += 32) {
-      const uint8_t f = s.F[(idx >> 5) * kFS + (idx & 31)];
-      fin &= (f & (FNODATA | FOUTLET | FBELOW)) != 0;
-      // With clean marks, a cell that may still turn clean is not final.
-      if (MODE == 2) fin &= (f & (FNODATA | FCLEAN)) != 0;
-    }
-    done = __all_sync(0xffffffffu, fin);
-  }
-  // Lanes 0..8 queue self (if capped) and the 8 neighbours whose halo changed.
-  if (lane < 9) {
-    int dx = 0, dy = 0;
-    bool want = false;
-    switch (lane) {
-      case 0: want = capped; break;
-      case 1: dx = -1; want = sides & 1; break;
-      case 2: dx = 1; want = sides & 2; break;
-      case 3: dy = -1; want = sides & 4; break;
-      case 4: dy = 1; want = sides & 8; break;
-      case 5: dx = -1; dy = -1; want = sides & 16; break;
-      case 6: dx = 1; dy = -1; want = sides & 32; break;
-      case 7: dx = -1; dy = 1; want = sides & 64; break;
-      case 8: dx = 1; dy = 1; want = sides & 128; break;
-    }
-    int nx = tx + dx, ny = ty + dy;
-    if (want && nx >= 0 && ny >= 0 && nx < w.tiles_x && ny < w.tiles_y)
-      enqueue(w, ny * w.tiles_x + nx);
-  }
-  __syncwarp();
-  if (lane == 0) {
-    const long long c3 = clock64();
-    st.kload += (unsigned int)((c1 - c0) >> 10);
-    st.ksweep += (unsigned int)((c2 - c1) >> 10);
-    st.kstore += (unsigned int)((c3 - c2) >> 10);
-  }
-  return done;
-}
-
-// Lock-free union-find over the undecided cells (labels in w.aux): links
+// Lock-free union-find over the cells of the resolution (w.label): links
 // always point to a smaller cell index, so no cycle can form; roots are
 // hooked with CAS, paths halved with plain stores.  Bounded loops.
 __device__ __forceinline__ uint32_t uf_find(uint32_t* lab, uint32_t x) {
@@ -670,14 +217,15 @@ __device__ __forceinline__ bool uf_unite(uint32_t* lab, uint32_t a, uint32_t b) 
   return false;
 }
 
-// One warp: process queued tiles until no tile is queued or being processed
-// anywhere.  During a drain only a warp processing a tile can queue one,
-// and that tile keeps `pending` above 0, so pending == 0 means no push can
-// come: a ticket still waiting then is abandoned (head and tail are reset
-// after the drain).  False on an error or a wait limit.
-template <int MODE>
-__device__ bool drain(WarpSmem<MODE>& s, const FloodArgs& a, int lane, int ntiles) {
-  const FillWork& w = a.w;
+// One warp: process queued tiles (visit(t, stats), which returns whether the
+// tile can never change again) until no tile is queued or being processed
+// anywhere.  During a drain only a warp processing a tile can queue one, and
+// that tile keeps `pending` above 0, so pending == 0 means no push can come: a
+// ticket still waiting then is abandoned (head and tail are reset after the
+// drain).  b_slots: the statistics go to flood B's counters.  False on an
+// error or a wait limit.
+template <class Visit>
+__device__ bool drain(const FillWork& w, int lane, int ntiles, bool b_slots, Visit visit) {
   volatile unsigned int* vs = w.scal;
   const unsigned int visit_cap = 1000u * (unsigned int)min(ntiles, 4000000);
   long long ticket = -1;
@@ -692,10 +240,10 @@ __device__ bool drain(WarpSmem<MODE>& s, const FloodArgs& a, int lane, int ntile
     if (t >= 0) {
       if (lane == 0 && idle_from >= 0) st.kidle += (unsigned int)((clock64() - idle_from) >> 10);
       idle_from = -1;
-      const bool done = process_tile<MODE>(s, a, t, lane, st);
+      const bool done = visit(t, st);
       if (lane == 0) {
         tq_finish(fill_queue(w), t, done);
-        if (st.tiles >= 64) flush_stats<MODE>(w, st, a.stage == 3);
+        if (st.tiles >= 64) flush_stats(w, st, b_slots);
       }
       __syncwarp();
       idle = 0;
@@ -707,235 +255,129 @@ __device__ bool drain(WarpSmem<MODE>& s, const FloodArgs& a, int lane, int ntile
       break;
     }
     if (vs[S_PENDING] == 0u) break;
-    const bool idle_limit = ++idle > (1LL << 24);
-    if (idle_limit || vs[(MODE == 1 || a.stage == 3) ? S_TILES_B : S_TILES_A] > visit_cap) {
+    const bool idle_limit = ++idle > (1LL << 25);
+    if (idle_limit || vs[b_slots ? S_TILES_B : S_TILES_A] > visit_cap) {
       if (lane == 0) atomicCAS((int*)(w.scal + S_ERR), 0, idle_limit ? 2 : 4);
       ok = false;
       break;
     }
     if (idle_from < 0) idle_from = clock64();
     __nanosleep(ns);
-    if (ns < 1024) ns <<= 1;
+    if (ns < 512) ns <<= 1;
   }
   if (lane == 0) {
     if (idle_from >= 0) st.kidle += (unsigned int)((clock64() - idle_from) >> 10);
-    flush_stats<MODE>(w, st, a.stage == 3);
+    flush_stats(w, st, b_slots);
   }
   __syncwarp();
   return ok;
 }
 
-template <int MODE, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, 1)
-fill_flood_kernel(FloodArgs a) {
+// Seed the queue with the marked tiles (a tile without an outlet, or without
+// a cell to repair, cannot change before a neighbour does, which queues it),
+// one 2x2 parity class of tiles after another with a grid barrier in
+// between, so the ring holds them class by class.  Tiles taken at the same
+// time are then rarely neighbours, and each class starts from the finished
+// borders of the classes before it: in a CPU simulation of the queue (2048^2
+// realization, 1/29 of the tiles in flight) this took the visits per tile
+// from 3.19 in plain tile order to 2.68.
+__device__ __forceinline__ bool seed_queue(const FillWork& w, const GridSync& gs, int gwarp,
+                                           int nwarps, int lane, int ntiles) {
+  bool go = true;
+  const int gthread = gwarp * 32 + lane, nthreads = nwarps * 32;
+  for (int c = 0; c < 4 && go; c++) {
+    for (int i = gthread; i < ntiles; i += nthreads) {
+      const int tx = i % w.tiles_x, ty = i / w.tiles_x;
+      if (((tx & 1) | ((ty & 1) << 1)) == c && w.tseed[i]) enqueue(w, i);
+    }
+    go = grid_barrier(gs, gridDim.x);
+  }
+  return go;
+}
+
+// The walled flood, the exact fill (no walls), the warm-started exact fill
+// (MARKS: with clean marks) and its repair flood.  Blocks of at most WARPS warps, one per SM; a
+// small grid's tiles are spread over all SMs with fewer warps each.
+template <bool MARKS, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 1) level_flood_kernel(LevelArgs a) {
   extern __shared__ __align__(16) unsigned char smraw[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  WarpSmem<MODE>& s = reinterpret_cast<WarpSmem<MODE>*>(smraw)[warp];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  LevelSmem& s = reinterpret_cast<LevelSmem*>(smraw)[warp];
   const FillWork& w = a.w;
-  const unsigned int nblocks = gridDim.x;
-  const int gwarp = blockIdx.x * WARPS + warp, nwarps = gridDim.x * WARPS;
+  const int gwarp = blockIdx.x * warps + warp, nwarps = gridDim.x * warps;
   const int ntiles = w.tiles_x * w.tiles_y;
   GridSync gs{w.scal + S_BAR_COUNT, w.scal + S_BAR_GEN, (int*)(w.scal + S_ERR)};
-  volatile unsigned int* vs = w.scal;
-  const int p0 = (int)vs[S_PASS] + 2;
-  int p = p0;
-  int ph = 0;
-  const bool phases = MODE == 1 && a.stage == 2;
   const unsigned long long t_start = global_ns();
-  // Seed the queue with the tiles that hold a relaying outlet (a tile
-  // without one cannot change before a neighbour does, which queues it),
-  // one 2x2 parity class of tiles after another with a grid barrier in
-  // between, so the ring holds them class by class.  Tiles taken at the
-  // same time are then rarely neighbours, and each class starts from the
-  // finished borders of the classes before it: in a CPU simulation of the
-  // queue (2048^2 realization, 1/29 of the tiles in flight) this took the
-  // visits per tile from 3.19 in plain tile order to 2.68.
-  bool go = true;
-  for (int c = 0; c < 4 && go && !phases; c++) {
-    for (int i = gwarp; i < ntiles; i += nwarps) {
-      const int tx = i % w.tiles_x, ty = i / w.tiles_x;
-      if (lane == 0 && ((tx & 1) | ((ty & 1) << 1)) == c && w.tseed[i]) enqueue(w, i);
-    }
-    go = grid_barrier(gs, nblocks);
-  }
-  while (go) {
-    const bool drained = drain<MODE>(s, a, lane, ntiles);
-    if (!grid_barrier(gs, nblocks) || !drained) break;
-    {
-      if (!phases) break;  // flood A, or flood B's main drain
-      // The queue is empty (abandoned tickets aside): restart its positions.
-      // No push comes before the next grid barrier.
-      if (blockIdx.x == 0 && threadIdx.x == 0) {
-        vs[S_HEAD] = 0u;
-        vs[S_TAIL] = 0u;
-      }
-      // ---- confirmation phase ----
-      // Flood A gave a lower bound (W_A in aux, FBELOWA), flood B an upper
-      // bound (Wg, FBELOW).  Where they agree the cell is final; the
-      // undecided cells (listed in cand, labelled by component in aux by
-      // the kernels between the two flood B launches) form 8-connected
-      // components that no later change can leave, so each component takes
-      // its own phase minimum.
-      const int64_t tid0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-      const int64_t tstride = (int64_t)gridDim.x * blockDim.x;
-      const unsigned int nu = vs[S_CAND];
-      if (blockIdx.x == 0 && threadIdx.x == 0) vs[S_PEND + (ph + 1) % 3] = 0u;
-      for (int64_t j = tid0; j < nu; j += tstride) {
-        const uint32_t c = w.cand[j], r = w.aux[c];
-        if (r == c) w.cmin[c] = 0xffffffffu;
-        // Every label is a root: a cell labelled otherwise would take a
-        // minimum nothing resets.
-        if (ph == 0 && w.aux[r] != r) atomicCAS((int*)(w.scal + S_ERR), 0, 6);
-      }
-      if (!grid_barrier(gs, nblocks)) break;
-      // Flags and levels were written by other SMs' drains, the minima by
-      // atomics: all are read from L2 (an L1 line could hold an older value
-      // across the grid barrier).
-      unsigned int pend = 0, npend = 0;
-      for (int64_t j = tid0; j < nu; j += tstride) {
-        uint32_t c = w.cand[j];
-        uint8_t f = __ldcg(w.flags + c);
-        if ((f & FNONPASS) && !(f & (FCONF | FBELOW))) {
-          float wv = __ldcg(a.Wg + c);
-          if (wv < kInf) {
-            atomicMin(&w.cmin[w.aux[c]], float_to_ordered(wv));
-            pend = 1;
-            npend++;
-          }
-        }
-      }
-      npend = __reduce_add_sync(0xffffffffu, npend);
-      if (lane == 0 && npend) atomicAdd(&w.scal[S_DBG], npend);
-      pend = __reduce_or_sync(0xffffffffu, pend);
-      if (lane == 0 && pend) atomicOr(&w.scal[S_PEND + ph % 3], 1u);
-      if (!grid_barrier(gs, nblocks)) break;
-      if (vs[S_PEND + ph % 3] == 0u) break;
-      // Each phase confirms at least one cell of every component with a
-      // pending cell (the one holding its minimum level), so there are at
-      // most as many phases as undecided cells.
-      if (ph > (int)min(nu, 0x7fffff00u) + 8) {
-        // Record one pending cell whose level is its component's recorded
-        // minimum: [26] cell, [27] level, [28] q, [29] the minimum read
-        // back, [30] its label, [31] the label's own label ([24] pending
-        // cells counted over the phases, [25] confirmations of the last).
-        for (int64_t j = tid0; j < nu; j += tstride) {
-          const uint32_t c = w.cand[j];
-          const uint8_t f = __ldcg(w.flags + c);
-          if (!(f & FNONPASS) || (f & (FCONF | FBELOW))) continue;
-          const float wv = __ldcg(a.Wg + c);
-          const uint32_t r = w.aux[c];
-          const unsigned int mo = __ldcg(w.cmin + r);
-          if (wv < kInf && float_to_ordered(wv) == mo &&
-              atomicCAS(&w.scal[S_DBG + 2], 0u, c + 1u) == 0u) {
-            w.scal[S_DBG + 3] = __float_as_uint(wv);
-            w.scal[S_DBG + 4] = __float_as_uint(a.q[c]);
-            w.scal[S_DBG + 5] = mo;
-            w.scal[S_DBG + 6] = r;
-            w.scal[S_DBG + 7] = w.aux[r];
-          }
-        }
-        if (threadIdx.x == 0) atomicCAS((int*)(w.scal + S_ERR), 0, 5);
-        break;
-      }
-      if (blockIdx.x == 0 && threadIdx.x == 0) w.scal[S_DBG + 1] = 0u;
-      if (!grid_barrier(gs, nblocks)) break;
-      unsigned int nconf = 0;
-      for (int64_t j = tid0; j < nu; j += tstride) {
-        uint32_t c = w.cand[j];
-        uint8_t f = __ldcg(w.flags + c);
-        if (!(f & FNONPASS) || (f & (FCONF | FBELOW))) continue;
-        const unsigned int mo = __ldcg(w.cmin + w.aux[c]);
-        if (mo == 0xffffffffu || !(a.q[c] <= ordered_to_float(mo))) continue;
-        nconf++;
-        w.flags[c] = f | FCONF;
-        if (__ldcg(a.Wg + c) < kInf) {
-          // The cell now relays: every tile whose halo holds it must rerun.
-          int cx = (int)(c % (uint32_t)w.W), cy = (int)(c / (uint32_t)w.W);
-          w.tconv[(cy / kTile) * w.tiles_x + cx / kTile] = 0;  // its neighbours inside must rerun
-          int tx0 = max(cx - 1, 0) / kTile, tx1 = min(cx + 1, w.W - 1) / kTile;
-          int ty0 = max(cy - 1, 0) / kTile, ty1 = min(cy + 1, w.H - 1) / kTile;
-          for (int ty = ty0; ty <= ty1; ty++)
-            for (int tx = tx0; tx <= tx1; tx++) enqueue(w, ty * w.tiles_x + tx);
-        }
-      }
-      nconf = __reduce_add_sync(0xffffffffu, nconf);
-      if (lane == 0 && nconf) atomicAdd(&w.scal[S_DBG + 1], nconf);
-      ph++;
-      if (!grid_barrier(gs, nblocks)) break;
-    }
-    p++;
-  }
+  bool go = seed_queue(w, gs, gwarp, nwarps, lane, ntiles);
+  const bool repair = a.stage == 3;
+  if (go)
+    go = drain(w, lane, ntiles, repair, [&](int t, VisitStats& st) {
+      level_visit<MARKS>(s, a, t, lane, st, [&](int n) { enqueue(w, n); });
+      return false;
+    });
+  grid_barrier(gs, gridDim.x);
+  // Tiles no outlet reaches were never queued: their masks and start levels
+  // are written here, so that every tile holds them.
+  for (int t = gwarp; t < ntiles && !repair; t += nwarps)
+    if (__ldcg(w.tvis + t) == 0) level_untouched(a, t, lane);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    vs[S_PASS] = (unsigned int)p;
+    volatile unsigned int* vs = w.scal;
+    vs[S_PASS] = vs[S_PASS] + 2;
     const unsigned int us = (unsigned int)((global_ns() - t_start) / 1000);
-    if (MODE != 1 && a.stage == 3) {
-      vs[S_US_B] = us;
-    } else if (MODE != 1) {
-      vs[S_PASSES_A] = (unsigned int)(p - p0 + 1);
-      vs[S_US_A] = us;
-    } else if (!phases) {
-      vs[S_PASSES_B] = (unsigned int)(p - p0 + 1);
-      vs[S_US_B] = us;
-    } else {
-      vs[S_PHASES] = (unsigned int)ph;
-      vs[S_US_P] = us;
+    if (!repair) vs[S_PASSES_A] = 1;
+    vs[repair ? S_US_B : S_US_A] = us;
+  }
+}
+
+// Start of a fill: the scalar block, the seeds, the tile states, the work
+// queue (no tile queued, the ring empty), the rims (no level, no flag) and the
+// cell flags, in
+// one launch instead of a kernel and six memsets (2 us each).
+__global__ void fill_begin_kernel(FillWork w, int ntiles) {
+  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = tid; i < S_SIZE; i += nthreads)
+    w.scal[i] = i == S_MIN ? 0xffffffffu : 0u;
+  const int64_t ring = 2 * (int64_t)ntiles + kRingSlack;
+  for (int64_t i = tid; i < ring; i += nthreads) {
+    w.lists[i] = kEmptySlot;
+    if (i < ntiles) {
+      w.queued[i] = kIdle;
+      w.tseed[i] = 0;
+      w.tvis[i] = 0;
     }
   }
+  const uint4 none = make_uint4(0x7f800000u, 0u, 0x7f800000u, 0u);  // two entries (+inf, 0)
+  uint4* rim = reinterpret_cast<uint4*>(w.rim);
+  for (int64_t i = tid; i < (int64_t)ntiles * (kRimCells / 2); i += nthreads) rim[i] = none;
+  uint4* f = reinterpret_cast<uint4*>(w.flags);  // (its space is a multiple of 256 bytes)
+  const int64_t fw = ((int64_t)w.W * w.H + 15) / 16;
+  for (int64_t i = tid; i < fw; i += nthreads) f[i] = make_uint4(0u, 0u, 0u, 0u);
 }
 
-// Cells per thread of the elementwise fill kernels (fewer, longer blocks).
-constexpr int kCellsPerThread = 4;
-
-__global__ void fill_init_kernel(const float* __restrict__ q, float* __restrict__ Wg,
-                                 uint8_t* __restrict__ F, const unsigned int* minslot,
-                                 uint8_t* __restrict__ tseed, int tiles_x, int W, int H,
-                                 int slab_h, float nodata, int check_only) {
-  // Block rows step over the grid's rows (no division to find a cell's x
-  // and y); kCellsPerThread cells a block-width apart per thread
-  // (coalesced).  A stack of realizations takes each slab's borders and
-  // minimum.
-  for (int y = blockIdx.y; y < H; y += gridDim.y) {
-  const int slab = y / slab_h, ys = y - slab * slab_h;
-  const float minE = ordered_to_float(minslot[slab]);
-  // After a fused front: its set-up assumed minE = 0.
-  if (check_only && minE == 0.0f) continue;
-#pragma unroll
-  for (int k = 0; k < kCellsPerThread; k++) {
-    const int x = (blockIdx.x * kCellsPerThread + k) * blockDim.x + threadIdx.x;
-    if (x >= W) break;
-    const int64_t i = (int64_t)y * W + x;
-    const float qv = q[i];
-    const uint8_t f =
-        fill_init_flags(qv, nodata, minE, x == 0 || ys == 0 || x == W - 1 || ys == slab_h - 1);
-    F[i] = f;
-    Wg[i] = (f & (FNODATA | FOUTLET)) ? qv : kInf;
-    if ((f & FOUTLET) && !(f & FNONPASS)) tseed[(y / kTile) * tiles_x + x / kTile] = 1;
+// The seeds of a grid no other kernel has marked: tiles holding an outlet (a
+// border cell of its slab, or a cell at 0).  One warp per tile.
+__global__ void __launch_bounds__(256) fill_seed_kernel(const float* __restrict__ q, FillWork w) {
+  const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (t >= w.tiles_x * w.tiles_y) return;
+  const int x = (t % w.tiles_x) * kTile + lane, y0 = (t / w.tiles_x) * kTile;
+  const int slab_h = w.slab_h ? w.slab_h : w.H;
+  bool any = false;
+#pragma unroll 8
+  for (int y = y0; y < y0 + kTile; y++) {
+    if (x >= w.W || y >= w.H) break;
+    const int ys = y % slab_h;
+    any |= x == 0 || x == w.W - 1 || ys == 0 || ys == slab_h - 1 ||
+           q[(int64_t)y * w.W + x] == 0.0f;
   }
-  }
+  if (__any_sync(0xffffffffu, any) && lane == 0) w.tseed[t] = 1;
 }
 
-// Exact mode (the reference's GPU fill, src/pitfilling/PitFillingAlgorithmGPUCUDA.cu:201-231):
-// NODATA cells keep NODATA and never relay; border cells and cells equal to
-// 0 are outlets that keep their elevation and relay it; every other cell
-// starts at +inf, or at a warm-start value no lower than its elevation.
-__global__ void fill_init_exact_kernel(const float* __restrict__ v, float* __restrict__ Wg,
-                                       uint8_t* __restrict__ F, const float* __restrict__ warm,
-                                       uint8_t* __restrict__ tseed, int tiles_x, int W, int H,
-                                       float nodata) {
-  const int y = blockIdx.y;
-#pragma unroll
-  for (int k = 0; k < kCellsPerThread; k++) {
-    const int x = (blockIdx.x * kCellsPerThread + k) * blockDim.x + threadIdx.x;
-    if (x >= W) break;
-    const int64_t i = (int64_t)y * W + x;
-    const float e = v[i];
-    uint8_t f = 0;
-    if (e == nodata) f = FNODATA;
-    else if (x == 0 || y == 0 || x == W - 1 || y == H - 1 || e == 0.0f) f = FOUTLET | FCLEAN;
-    F[i] = f;
-    Wg[i] = f ? e : (warm ? fmaxf(warm[i], e) : kInf);
-    if (f & FOUTLET) tseed[(y / kTile) * tiles_x + x / kTile] = 1;
-  }
+// A warm start is no lower than the elevation.
+__global__ void fill_warm_start_kernel(const float* __restrict__ v, const float* __restrict__ warm,
+                                       float* __restrict__ Wg, int64_t n) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) Wg[i] = fmaxf(warm[i], v[i]);
 }
 
 // Verification of a warm-started exact fill.  The warm flood keeps clean
@@ -946,220 +388,508 @@ __global__ void fill_init_exact_kernel(const float* __restrict__ v, float* __res
 // fixpoint no cell is above the exact fill either (induction along its
 // optimal path), so a supported cell holds the answer.  Every other cell
 // (started too low, pulled down by one that was, or unreached) restarts
-// from +inf and marks its tile for the repair flood; with every start an
-// upper bound again, the repair flood ends at the exact fill.  Four
-// consecutive cells per thread; the flags are workspace (aligned).  Also
-// resets the work queue's positions.
-__global__ void fill_unsupported_kernel(float* __restrict__ Wg, uint8_t* __restrict__ F,
-                                        uint8_t* __restrict__ tseed, unsigned int* scal,
-                                        int tiles_x, int W, int64_t n) {
+// from +inf, in the grid and in its tile's rim, and marks its tile for the
+// repair flood; with every start an upper bound again, the repair flood ends
+// at the exact fill.  One warp per tile.  Also resets the work queue's
+// positions.
+__global__ void __launch_bounds__(256) fill_unsupported_kernel(LevelArgs a) {
+  const FillWork& w = a.w;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    scal[S_HEAD] = 0u;
-    scal[S_TAIL] = 0u;
-    scal[S_PENDING] = 0u;
+    w.scal[S_HEAD] = 0u;
+    w.scal[S_TAIL] = 0u;
+    w.scal[S_PENDING] = 0u;
   }
-  const int64_t b4 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
-  unsigned int reset = 0;
-  if (b4 < n) {
-    uint8_t fv[4];
-    if (b4 + 4 <= n) {
-      const uchar4 f4 = *reinterpret_cast<const uchar4*>(F + b4);
-      fv[0] = f4.x; fv[1] = f4.y; fv[2] = f4.z; fv[3] = f4.w;
+  const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (t >= w.tiles_x * w.tiles_y) return;
+  // Every tile was visited (a warm start seeds them all).
+  const unsigned int reset = ~(w.mdead[t * kTile + lane] | w.mclean[t * kTile + lane]);
+  const bool any = __any_sync(0xffffffffu, reset != 0);
+  if (lane == 0) w.tseed[t] = any;
+  if (!any) return;
+  float* wp = a.Wg + (int64_t)(t / w.tiles_x) * kTile * w.W + (t % w.tiles_x) * kTile + lane;
+  for (int y = 0; y < kTile; y++)
+    if ((reset >> y) & 1u) wp[(int64_t)y * w.W] = kInf;
+  uint2* rim = w.rim + (size_t)t * kRimCells + lane;
+  const uint2 none = make_uint2(0x7f800000u, 0u);
+  if (reset & 1u) rim[kTop * kTile] = none;
+  if (reset >> 31) rim[kBottom * kTile] = none;
+  const unsigned int l = __shfl_sync(0xffffffffu, reset, 0), r = __shfl_sync(0xffffffffu, reset, 31);
+  if ((l >> lane) & 1u) rim[kLeft * kTile] = none;
+  if ((r >> lane) & 1u) rim[kRight * kTile] = none;
+  const unsigned int n = __reduce_add_sync(0xffffffffu, (unsigned int)__popc(reset));
+  if (lane == 0) {
+    w.tvis[t] = kVisited | kUnsettled;
+    atomicAdd(&w.scal[S_RESET], n);
+  }
+}
+
+// Cells no outlet reaches keep the reference's initial value: only tiles that
+// hold one are touched.  One warp per tile.
+__global__ void __launch_bounds__(256) fill_final_exact_kernel(LevelArgs a) {
+  const FillWork& w = a.w;
+  const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (t >= w.tiles_x * w.tiles_y || !(w.tvis[t] & kUnreached)) return;
+  const unsigned int dead = w.mdead[t * kTile + lane];
+  float* wp = a.Wg + (int64_t)(t / w.tiles_x) * kTile * w.W + (t % w.tiles_x) * kTile + lane;
+  for (int y = 0; y < kTile; y++) {
+    if ((dead >> y) & 1u) continue;  // (cells outside the grid among them)
+    if (wp[(int64_t)y * w.W] == kInf) wp[(int64_t)y * w.W] = 99990000.0f;
+  }
+}
+
+// Whether a cell relays by its own nature: passable and not NODATA.
+__device__ __forceinline__ bool relays(float q, float minE, float nodata) {
+  return q != nodata && passable_quantized(q, minE);
+}
+
+// After the walled flood: the levels of the walls (interior non-passable
+// cells), W = max(q, least relay of the 8 neighbours), and the list of those
+// above their q, which the resolution starts from.  Walls are about 1% of the
+// cells, so the pass reads their masks (0.125 B a cell) and gathers each
+// wall's 8 neighbours.  The levels of listed walls are left marked (see the
+// resolution).  One warp per tile.
+__global__ void __launch_bounds__(256) fill_walls_kernel(LevelArgs a) {
+  const FillWork& w = a.w;
+  const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (t >= w.tiles_x * w.tiles_y) return;
+  unsigned int wall = w.mwall[t * kTile + lane];
+  const int x = (t % w.tiles_x) * kTile + lane, y0 = (t / w.tiles_x) * kTile;
+  const int slab_h = w.slab_h ? w.slab_h : w.H;
+  bool unreached = false;
+  while (__any_sync(0xffffffffu, wall != 0)) {
+    bool lake = false;
+    int64_t i = 0;
+    if (wall) {
+      const int y = y0 + __ffs(wall) - 1;
+      wall &= wall - 1;
+      i = (int64_t)y * w.W + x;
+      const float minE = ordered_to_float(a.minslot[y / slab_h]);
+      const float qv = a.q[i];
+      float m = kInf;
+#pragma unroll
+      for (int k = 0; k < 8; k++) {  // a wall is interior: all 8 are in its slab
+        const int64_t n = i + (int64_t)d8_dy(k) * w.W + d8_dx(k);
+        const float qn = a.q[n], wn = a.Wg[n];
+        if (relays(qn, minE, a.nodata)) m = fminf(m, wn);
+      }
+      const float lv = fmaxf(qv, m);
+      lake = lv > qv && lv < kInf;
+      a.Wg[i] = lake ? -lv : lv;
+      unreached |= lv == kInf;
+      if (lake) {
+        w.flags[i] = kActive;
+        w.aux[i] = __float_as_uint(lv);
+      }
+    }
+    const unsigned int ball = __ballot_sync(0xffffffffu, lake);
+    unsigned int base = 0;
+    if (lane == 0 && ball) base = atomicAdd(&w.scal[S_CAND], (unsigned int)__popc(ball));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (lake) w.cand[base + __popc(ball & ((1u << lane) - 1u))] = (uint32_t)i;
+  }
+  if (__any_sync(0xffffffffu, unreached) && lane == 0) w.tvis[t] |= kUnreached;
+}
+
+// ---- resolution (steps 2 and 3 of the header) --------------------------------
+// Cells are listed once (cand) with the walled flood's level S in aux.  Levels
+// are >= 0 here (quantized elevations), so a float's bits order like the
+// float, and its sign is free: it marks the level of a listed cell, for the
+// length of the resolution.  A fall is one atomicMin of the marked level as a
+// signed integer: marked levels are below every unmarked one and ordered
+// among themselves, and the first to lower a cell gets S back, unmarked.  The
+// other flags are bytes changed by atomics on the word around them.
+struct Resolve {
+  const float* q;
+  float* Wg;
+  FillWork w;
+  float nodata;
+  const unsigned int* minslot;
+  int slab_h;
+
+  __device__ __forceinline__ unsigned int* word(int64_t c) const {
+    return reinterpret_cast<unsigned int*>(w.flags) + (c >> 2);
+  }
+  __device__ __forceinline__ unsigned int set(int64_t c, unsigned int f) const {
+    const int sh = (int)(c & 3) * 8;
+    return (atomicOr(word(c), f << sh) >> sh) & 0xffu;
+  }
+  __device__ __forceinline__ void clear(int64_t c, unsigned int f) const {
+    atomicAnd(word(c), ~(f << ((int)(c & 3) * 8)));
+  }
+  __device__ __forceinline__ unsigned int get(int64_t c) const {
+    return (__ldcg(word(c)) >> ((int)(c & 3) * 8)) & 0xffu;
+  }
+  // Level of a cell that is not NODATA, and whether it is listed.
+  __device__ __forceinline__ float level(int64_t c, bool* listed = nullptr) const {
+    const float v = __ldcg(Wg + c);
+    if (listed) *listed = __float_as_int(v) < 0;
+    return fabsf(v);
+  }
+  __device__ __forceinline__ float walled(int64_t c) const {  // S of a listed cell
+    return __uint_as_float(__ldcg(w.aux + c));
+  }
+  __device__ __forceinline__ bool wall(int64_t c, float qv) const {
+    const int slab = (int)(c / w.W) / slab_h;
+    return !passable_quantized(qv, ordered_to_float(minslot[slab]));
+  }
+};
+
+// Grid barrier of the `nblocks` blocks of the resolution.  Returns whether any
+// thread passed true; *more = the entries listed by then (nothing is listed
+// between the last arrival, which takes the number, and the release); *ok =
+// false on an error (any block's) or a wait limit.
+__device__ bool any_of(const FillWork& w, unsigned int nblocks, bool mine, unsigned int* more,
+                       bool* ok) {
+  __shared__ unsigned int sh_any, sh_more, sh_ok;
+  volatile unsigned int* vs = w.scal;
+  const int block = __syncthreads_or(mine);
+  if (threadIdx.x == 0) {
+    __threadfence();
+    sh_ok = 1u;
+    if (nblocks == 1) {
+      sh_any = block ? 1u : 0u;
+      sh_more = vs[S_MORE];
     } else {
-#pragma unroll
-      for (int k = 0; k < 4; k++) fv[k] = b4 + k < n ? F[b4 + k] : FNODATA;
+      const unsigned int gen = vs[S_BAR_GEN];
+      if (block) atomicOr(&w.scal[S_FLAG], 1u);
+      __threadfence();
+      if (atomicAdd(&w.scal[S_BAR_COUNT], 1u) == nblocks - 1) {
+        vs[S_BAR_COUNT] = 0u;
+        vs[S_RESULT] = vs[S_FLAG];
+        vs[S_FLAG] = 0u;
+        vs[S_MORE_AT] = vs[S_MORE];
+        __threadfence();
+        atomicAdd(&w.scal[S_BAR_GEN], 1u);
+      } else {
+        unsigned int ns = 32;
+        long long polls = 0;
+        while (vs[S_BAR_GEN] == gen) {
+          if (++polls > 20000000LL) {  // several seconds
+            atomicCAS((int*)(w.scal + S_ERR), 0, 1);
+            break;
+          }
+          if ((polls & 63) == 0 && vs[S_ERR]) break;
+          __nanosleep(ns);
+          if (ns < 256) ns <<= 1;
+        }
+      }
+      __threadfence();
+      sh_any = vs[S_RESULT];
+      sh_more = vs[S_MORE_AT];
     }
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const uint8_t f = fv[k];
-      if (f & (FNODATA | FOUTLET | FCLEAN)) continue;
-      const int64_t i = b4 + k;
-      Wg[i] = kInf;
-      F[i] = f & (uint8_t)~FBELOW;
-      const int y = (int)(i / W), x = (int)(i - (int64_t)y * W);
-      tseed[(y / kTile) * tiles_x + x / kTile] = 1;
-      reset++;
-    }
+    if (vs[S_ERR]) sh_ok = 0u;
   }
-  reset = __reduce_add_sync(0xffffffffu, reset);
-  if ((threadIdx.x & 31) == 0 && reset) atomicAdd(&scal[S_RESET], reset);
+  __syncthreads();
+  const bool any = sh_any != 0u;
+  *more = sh_more;
+  *ok = sh_ok != 0u;
+  __syncthreads();
+  return any && *ok;
 }
 
-// Cells no outlet reaches keep the reference's initial value.
-__global__ void fill_final_exact_kernel(float* __restrict__ Wg, int64_t n) {
-#pragma unroll
-  for (int k = 0; k < kCellsPerThread; k++) {
-    const int64_t i = ((int64_t)blockIdx.x * kCellsPerThread + k) * blockDim.x + threadIdx.x;
-    if (i < n && Wg[i] == kInf) Wg[i] = 99990000.0f;
-  }
-}
+constexpr int kResolveThreads = 1024;
+constexpr int kResolveRun = 1024;   // entries of the list a block takes at a time (walls)
+constexpr int kReopenRun = 256;     // the same for the cells of reopened components
+constexpr int kFrontCells = 1024;
 
-// Between the floods.  A clean cell keeps flood A's value and below-q flag,
-// which flood B would give it too (every value flood B relays is a passable
-// level, so a non-passable cell's incoming level never equals its q, and a
-// clean cell's level is reached by a path flood B keeps); nothing of it is
-// written.  Every other cell keeps flood A's result (a lower bound) in aux
-// and FBELOWA, is confirmed when non-passable and reached at a level >= q,
-// restarts from +inf and marks its tile for flood B (tseed).  Four
-// consecutive cells per thread; only the flags of clean cells are read.
-// Also resets the work queue.
-__global__ void fill_classify_kernel(float* __restrict__ Wg, uint8_t* __restrict__ F,
-                                     uint32_t* __restrict__ aux, unsigned int* scal,
-                                     uint8_t* __restrict__ tseed, int tiles_x, int W, int64_t n) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    scal[S_HEAD] = 0u;
-    scal[S_TAIL] = 0u;
-    scal[S_PENDING] = 0u;
-  }
-  const int64_t b4 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
-  if (b4 >= n) return;
-  uint8_t fv[4];
-  if (b4 + 4 <= n) {  // the flags are workspace: 256-byte aligned, b4 % 4 == 0
-    const uchar4 f4 = *reinterpret_cast<const uchar4*>(F + b4);
-    fv[0] = f4.x; fv[1] = f4.y; fv[2] = f4.z; fv[3] = f4.w;
+// A block's front: cells whose level fell (or walls that have come to relay),
+// with that level; one buffer is read while the other fills.  Three counters
+// in turn, so a step needs one block barrier.
+struct Front {
+  uint32_t cell[2][kFrontCells];
+  float level[2][kFrontCells];
+  int n[3];
+  int full;  // an entry did not fit: its cell was marked kActive instead
+};
+
+__device__ __forceinline__ void front_push(const Resolve& r, Front& f, int buf, int cnt, uint32_t c,
+                                           float lv) {
+  const int pos = atomicAdd(&f.n[cnt], 1);
+  if (pos < kFrontCells) {
+    f.cell[buf][pos] = c;
+    f.level[buf][pos] = lv;
   } else {
-#pragma unroll
-    for (int k = 0; k < 4; k++) fv[k] = b4 + k < n ? F[b4 + k] : FNODATA;
-  }
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    uint8_t f = fv[k];
-    if (f & (FNODATA | FOUTLET | FCLEAN)) continue;
-    const int64_t i = b4 + k;
-    const float wa = Wg[i];
-    aux[i] = __float_as_uint(wa);
-    if ((f & FNONPASS) && !(f & FBELOW) && wa < kInf) f |= FCONF;
-    if (f & FBELOW) f |= FBELOWA;
-    F[i] = f & (uint8_t)~FBELOW;
-    Wg[i] = kInf;
-    const int y = (int)(i / W), x = (int)(i - (int64_t)y * W);
-    tseed[(y / kTile) * tiles_x + x / kTile] = 1;
+    __threadfence();  // the level before the mark
+    r.set(c, kActive);
+    f.full = 1;
   }
 }
 
-// Flood B's tile states: a tile without a cell to recompute is done from
-// the start (its cells hold flood B's values already); the others are idle.
-__global__ void fill_tile_states_kernel(int* __restrict__ queued, const uint8_t* __restrict__ tseed,
-                                        int ntiles) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < ntiles) queued[t] = tseed[t] ? kIdle : kDone;
-}
-
-// Between flood B's two launches: the undecided cells -- flood A's lower
-// bound (aux) and flood B's upper bound (Wg) differ in value, or in the
-// blocked status of a non-passable cell -- are flagged FUNSURE, labelled
-// with their own index and appended to the candidate list.  Only tiles that
-// held a cell to recompute (tseed) are read: a clean cell kept flood A's
-// value and flag.  One block per tile, one row segment of 4 cells per
-// thread; the filled grid is the caller's and is read as float4 only when
-// the row segment is 16-byte aligned.
-__global__ void fill_undecided_kernel(const float* __restrict__ Wg, uint8_t* __restrict__ F,
-                                      uint32_t* __restrict__ aux, uint32_t* __restrict__ cand,
-                                      unsigned int* scal, const uint8_t* __restrict__ tseed,
-                                      int tiles_x, int W, int H) {
-  const int t = blockIdx.x;
-  if (!tseed[t]) return;
-  const int y = (t / tiles_x) * kTile + (int)(threadIdx.x >> 3);
-  const int x = (t % tiles_x) * kTile + (int)(threadIdx.x & 7) * 4;
-  if (y >= H || x >= W) return;
-  const int64_t b4 = (int64_t)y * W + x;
-  uint8_t fv[4];
-  float wav[4], wbv[4];
-  // b4 % 4 == 0 aligns the workspace arrays (256-byte aligned bases);
-  // the caller's grid is checked on its own.
-  if (x + 4 <= W && (b4 & 3) == 0 && ((uintptr_t)(Wg + b4) & 15u) == 0) {
-    const uchar4 f4 = *reinterpret_cast<const uchar4*>(F + b4);
-    const uint4 a4 = *reinterpret_cast<const uint4*>(aux + b4);
-    const float4 w4 = *reinterpret_cast<const float4*>(Wg + b4);
-    fv[0] = f4.x; fv[1] = f4.y; fv[2] = f4.z; fv[3] = f4.w;
-    wav[0] = __uint_as_float(a4.x); wav[1] = __uint_as_float(a4.y);
-    wav[2] = __uint_as_float(a4.z); wav[3] = __uint_as_float(a4.w);
-    wbv[0] = w4.x; wbv[1] = w4.y; wbv[2] = w4.z; wbv[3] = w4.w;
-  } else {
+// Relaxes from the active cells among the nl of a list until no level falls.
+// LOWER: the list is cand; walls with S > q relay whatever their level, and a
+// neighbour that falls is listed (from entry nu0 on, *more of them so far);
+// otherwise the list holds the reopened components, confirmed walls above
+// their q relay, and only these cells can fall.
+//
+// The falls travel up to ~70 cells at 4096^2 (~170 at 8192^2) from where they
+// start, so what counts is the time of a step.  Each block follows the fronts
+// of its own entries with no grid barrier in between: 8 lanes per cell, one
+// per neighbour, two dependent L2 accesses (the neighbour's level and
+// elevation, the atomicMin) and one block barrier a step.  Levels fall in any
+// order, and a cell two blocks reach is followed by whichever lowers it.
+// (Grid-wide rounds over the list took 3.3 ms at 8192^2, a flag beside each
+// level -- two accesses more a step -- 0.7 ms.)  Blocks take runs of
+// consecutive entries, which lie in the same tiles.
+template <bool LOWER>
+__device__ unsigned int relax(const Resolve& r, Front& f, const uint32_t* list, unsigned int nl,
+                              unsigned int nblocks, unsigned int* more, bool* ok) {
+  constexpr int kRun = LOWER ? kResolveRun : kReopenRun;
+  const FillWork& w = r.w;
+  const unsigned int nu0 = nl;
+  unsigned int steps = 0;
+  for (bool again = true; again;) {
+    const unsigned int nu = LOWER ? nl + *more : nl;
+    if (threadIdx.x == 0) f.full = 0;
+    for (unsigned int base = blockIdx.x * kRun; base < nu; base += nblocks * kRun) {
+      __syncthreads();
+      if (threadIdx.x < 3) f.n[threadIdx.x] = 0;
+      __syncthreads();
+      // The active entries that can lower a neighbour.
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const bool in = x + k < W;
-      fv[k] = in ? F[b4 + k] : FNODATA;
-      wav[k] = in ? __uint_as_float(aux[b4 + k]) : 0.0f;
-      wbv[k] = in ? Wg[b4 + k] : 0.0f;
+      for (int i = 0; i < (kRun + kResolveThreads - 1) / kResolveThreads; i++) {
+        const unsigned int j = base + i * kResolveThreads + threadIdx.x;
+        if (j >= min(nu, base + kRun)) continue;
+        const uint32_t c = __ldcg(list + j);
+        const unsigned int fl = r.get(c);
+        if (LOWER) {
+          if (j < nu0) w.label[c] = c;
+        } else if (__ldcg(w.label + c) == c) {
+          __stcg(w.aux + c, 0xffffffffu);  // the component's least pending level
+        }
+        if (!(fl & kActive)) continue;
+        r.clear(c, kActive);
+        __threadfence();  // a fall after the read below marks the cell again
+        const float lv = r.level(c), qc = r.q[c];
+        // (LOWER: every active cell is a wall with S > q, or fell, or both.)
+        if (!LOWER && r.wall(c, qc) && !((fl & kConfirmed) && lv > qc)) continue;
+        const int x = (int)(c % (uint32_t)w.W), y = (int)(c / (uint32_t)w.W);
+        bool lowers = false;
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+          const int nx = x + d8_dx(k), ny = y + d8_dy(k);
+          if (nx < 0 || nx >= w.W || ny < 0 || ny >= w.H) continue;
+          const int64_t b = (int64_t)ny * w.W + nx;
+          const float qb = r.q[b];
+          lowers |= fmaxf(qb, lv) < r.level(b) && qb != r.nodata;
+        }
+        if (lowers) front_push(r, f, 0, 0, c, lv);
+      }
+      int buf = 0, cnt = 0;
+      for (;;) {
+        __syncthreads();
+        const int nf = min(f.n[cnt], kFrontCells);
+        const int nxt = cnt == 2 ? 0 : cnt + 1;
+        if (threadIdx.x == 0) f.n[nxt == 2 ? 0 : nxt + 1] = 0;
+        if (nf == 0) break;
+        if (++steps > (1u << 26)) {  // every step lowers a level: far beyond any path
+          if (threadIdx.x == 0) atomicCAS((int*)(w.scal + S_ERR), 0, 4);
+          break;
+        }
+        const int k = threadIdx.x & 7;
+        for (int e = threadIdx.x >> 3; e < nf; e += kResolveThreads / 8) {
+          const uint32_t c = f.cell[buf][e];
+          const float lv = f.level[buf][e];
+          const int nx = (int)(c % (uint32_t)w.W) + d8_dx(k), ny = (int)(c / (uint32_t)w.W) + d8_dy(k);
+          if (nx < 0 || nx >= w.W || ny < 0 || ny >= w.H) continue;
+          const int64_t b = (int64_t)ny * w.W + nx;
+          const float qb = r.q[b], nv = fmaxf(qb, lv);
+          // (Outlets are at their elevation.)
+          if (!(nv < r.level(b)) || qb == r.nodata) continue;
+          const int mine = (int)(__float_as_uint(nv) | 0x80000000u);
+          const int prev = atomicMin(reinterpret_cast<int*>(r.Wg + b), mine);
+          if (LOWER) {
+            const bool first = prev >= 0;
+            const unsigned int pos = warp_append(&w.scal[S_MORE], first);
+            if (first) {
+              __stcg(w.aux + b, (unsigned int)prev);
+              __stcg(w.label + b, (uint32_t)b);
+              __stcg(w.cand + nu0 + pos, (uint32_t)b);
+            }
+          }
+          if (prev <= mine) continue;
+          // A wall that falls was above its q, so LOWER lets it relay.
+          if (LOWER || !r.wall(b, qb) || ((r.get(b) & kConfirmed) && nv > qb))
+            front_push(r, f, buf ^ 1, nxt, (uint32_t)b, nv);
+        }
+        buf ^= 1;
+        cnt = nxt;
+      }
     }
+    __syncthreads();
+    again = any_of(w, nblocks, f.full != 0, more, ok);
   }
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    const uint8_t f = fv[k];
-    // Clean cells agree by construction (their aux and FBELOWA are not kept).
-    const bool unsure = !(f & (FNODATA | FOUTLET | FCLEAN)) &&
-                        (wav[k] != wbv[k] ||
-                         ((f & FNONPASS) && (((f & FBELOWA) != 0) != ((f & FBELOW) != 0))));
-    const int64_t i = b4 + k;
-    if (unsure) {
-      F[i] = f | FUNSURE;
-      aux[i] = (uint32_t)i;
-    }
-    const unsigned int pos = warp_append(&scal[S_CAND], unsure);
-    if (unsure) cand[pos] = (uint32_t)i;
-  }
+  return steps;
 }
 
-// Union of undecided neighbours (W, NW, N, NE: each pair once) into
-// 8-connected components; labels in aux.
-__global__ void fill_unite_kernel(const uint32_t* __restrict__ cand, unsigned int* scal,
-                                  const uint8_t* __restrict__ F, uint32_t* aux, int W) {
-  const unsigned int nu = ((volatile unsigned int*)scal)[S_CAND];
+// Steps 2 and 3, and the cells no outlet reaches.  A cooperative launch; only
+// as many blocks as the list's runs need stay (a barrier among few blocks is
+// cheap, and the list is short on small grids).
+__global__ void __launch_bounds__(kResolveThreads, 1) fill_resolve_kernel(Resolve r) {
+  __shared__ Front front;
+  const FillWork& w = r.w;
+  volatile unsigned int* vs = w.scal;
+  const unsigned int nu0 = vs[S_CAND];  // (final before the launch)
+  const unsigned int nblocks = min(gridDim.x, max(1u, (nu0 + kResolveRun - 1) / kResolveRun));
+  if (blockIdx.x >= nblocks) return;
+  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t nthreads = (int64_t)nblocks * blockDim.x;
+  const unsigned long long t0 = global_ns();
+  int phases = 0;
+  unsigned int more = 0;
   bool ok = true;
-  for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < nu;
-       j += (int64_t)gridDim.x * blockDim.x) {
-    const uint32_t c = cand[j];
-    const int cx = (int)(c % (uint32_t)W), cy = (int)(c / (uint32_t)W);
-    for (int k = 0; k < 4; k++) {
-      const int nx = cx + (k == 0 ? -1 : k - 2), ny = cy + (k == 0 ? 0 : -1);
-      if (nx < 0 || ny < 0 || nx >= W) continue;
-      const uint32_t nb = (uint32_t)ny * (uint32_t)W + (uint32_t)nx;
-      if (F[nb] & FUNSURE) ok &= uf_unite(aux, c, nb);
+  if (nu0) {
+    const unsigned int steps = relax<true>(r, front, w.cand, nu0, nblocks, &more, &ok);
+    if (threadIdx.x == 0) atomicMax(&w.scal[S_STEPS], steps);
+  }
+  const unsigned long long t1 = global_ns();
+  const unsigned int nu = ok ? nu0 + more : 0u;
+  // Members: the cells between the bounds, united with their W, NW, N and NE
+  // neighbours among them (each pair once).  Reopened components: those with
+  // a wall that S left above its q and A took to it.
+  bool reopen = false, united = true;
+  auto member = [&](int64_t c, float* lv, float* s) {
+    bool listed;
+    *lv = r.level(c, &listed);
+    if (!listed || r.q[c] == r.nodata) return false;
+    *s = r.walled(c);
+    return *lv != *s;
+  };
+  for (int64_t j = tid; j < nu; j += nthreads) {
+    const uint32_t c = __ldcg(w.cand + j);
+    float lv, s, lb, sb;
+    if (!member(c, &lv, &s)) continue;
+    r.set(c, kMember);
+    const float qc = r.q[c];
+    reopen |= lv <= qc && s > qc && r.wall(c, qc);
+    const int cx = (int)(c % (uint32_t)w.W), cy = (int)(c / (uint32_t)w.W);
+    for (int d = 0; d < 4; d++) {
+      const int nx = cx + (d == 0 ? -1 : d - 2), ny = cy + (d == 0 ? 0 : -1);
+      if (nx < 0 || ny < 0 || nx >= w.W) continue;
+      const uint32_t b = (uint32_t)ny * (uint32_t)w.W + (uint32_t)nx;
+      if (member(b, &lb, &sb)) united &= uf_unite(w.label, c, b);
     }
   }
-  if (!ok) atomicCAS((int*)(scal + S_ERR), 0, 6);
-}
-
-// Every undecided cell's label becomes its component's root.
-__global__ void fill_flatten_kernel(const uint32_t* __restrict__ cand,
-                                    const unsigned int* scal, uint32_t* aux) {
-  const unsigned int nu = ((const volatile unsigned int*)scal)[S_CAND];
-  for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < nu;
-       j += (int64_t)gridDim.x * blockDim.x) {
-    const uint32_t c = cand[j];
-    aux[c] = uf_root(aux, c);
+  if (!united) atomicCAS((int*)(w.scal + S_ERR), 0, 6);
+  if (nu0 && any_of(w, nblocks, reopen, &more, &ok)) {
+    for (int64_t j = tid; j < nu; j += nthreads) {
+      const uint32_t c = __ldcg(w.cand + j);
+      if (!(r.get(c) & kMember)) continue;
+      const uint32_t root = uf_root(w.label, c);
+      w.label[c] = root;
+      const float qc = r.q[c];
+      if (r.level(c) <= qc && r.walled(c) > qc && r.wall(c, qc)) r.set(root, kReopened);
+    }
+    any_of(w, nblocks, false, &more, &ok);
+    // The cells of reopened components restart at S -- or at what a settled
+    // listed wall beside them offers, if that is less -- with the walls that A
+    // left above their q confirmed, and are listed once more after the others
+    // (where the list fills the array, it is used whole).  From here aux
+    // holds the components' least pending level.
+    const bool apart = 2 * (uint64_t)nu <= (uint64_t)w.W * w.H;
+    for (int64_t j = tid; j < nu && ok; j += nthreads) {
+      const uint32_t c = __ldcg(w.cand + j);
+      if (!(r.get(c) & kMember)) continue;
+      const uint32_t root = __ldcg(w.label + c);
+      // Every label is a root: a cell labelled otherwise would take a
+      // minimum nothing resets.
+      if (__ldcg(w.label + root) != root) atomicCAS((int*)(w.scal + S_ERR), 0, 6);
+      const bool open = r.get(root) & kReopened;
+      if (open) {
+        const float qc = r.q[c], lv = r.level(c), s = r.walled(c);
+        float start = s;
+        const int x = (int)(c % (uint32_t)w.W), y = (int)(c / (uint32_t)w.W);
+#pragma unroll 1
+        for (int k = 0; k < 8; k++) {
+          const int nx = x + d8_dx(k), ny = y + d8_dy(k);
+          if (nx < 0 || nx >= w.W || ny < 0 || ny >= w.H) continue;
+          const int64_t b = (int64_t)ny * w.W + nx;
+          bool listed;
+          const float lb = r.level(b, &listed), qb = r.q[b];
+          if (listed && qb != r.nodata && !(r.get(b) & kMember) && lb > qb && r.wall(b, qb))
+            start = fminf(start, fmaxf(qc, lb));
+        }
+        const bool confirm = lv > qc && s > qc && r.wall(c, qc);
+        if (confirm || start < s) r.set(c, (confirm ? kConfirmed : 0u) | kActive);
+        __stcg(r.Wg + c, -start);
+      }
+      const unsigned int pos = warp_append(&w.scal[S_OPEN], open && apart);
+      if (open && apart) __stcg(w.cand + nu + pos, c);
+    }
+    any_of(w, nblocks, false, &more, &ok);
+    const unsigned int no = apart ? vs[S_OPEN] : nu;
+    const uint32_t* open_list = apart ? w.cand + nu : w.cand;
+    while (ok) {
+      relax<false>(r, front, open_list, no, nblocks, &more, &ok);
+      if (!ok) break;
+      // The unconfirmed walls above their q.
+      auto pending = [&](int64_t j, uint32_t& c, float& lv, float& qc) {
+        c = __ldcg(open_list + j);
+        const unsigned int f = r.get(c);
+        if (!(f & kMember) || (f & kConfirmed)) return false;
+        if (!apart && !(r.get(__ldcg(w.label + c)) & kReopened)) return false;
+        qc = r.q[c];
+        lv = r.level(c);
+        return lv > qc && r.wall(c, qc);
+      };
+      bool some = false;
+      uint32_t c;
+      float lv, qc;
+      for (int64_t j = tid; j < no; j += nthreads) {
+        if (!pending(j, c, lv, qc) || lv == kInf) continue;
+        atomicMin(&w.aux[__ldcg(w.label + c)], __float_as_uint(lv));
+        some = true;
+      }
+      if (!any_of(w, nblocks, some, &more, &ok)) break;
+      // Each phase confirms at least one cell of every component with a
+      // pending one (the cell holding its minimum).
+      if (++phases > (int)min(nu, 0x7fffff00u) + 8) {
+        if (threadIdx.x == 0) atomicCAS((int*)(w.scal + S_ERR), 0, 5);
+        break;  // (in every block)
+      }
+      for (int64_t j = tid; j < no; j += nthreads) {
+        if (!pending(j, c, lv, qc)) continue;
+        const unsigned int m = __ldcg(w.aux + __ldcg(w.label + c));
+        if (m != 0xffffffffu && qc <= __uint_as_float(m)) r.set(c, kConfirmed | kActive);
+      }
+      any_of(w, nblocks, false, &more, &ok);
+    }
+  }
+  // The marks come off, and cells no outlet reached keep q.
+  for (int64_t j = tid; j < nu0 + more; j += nthreads) {
+    const uint32_t c = __ldcg(w.cand + j);
+    const float lv = r.level(c);
+    r.Wg[c] = lv == kInf ? r.q[c] : lv;
+  }
+  // (Only tiles that held one after the flood are read.  One warp per tile.)
+  const int ntiles = w.tiles_x * w.tiles_y, lane = threadIdx.x & 31;
+  for (int64_t t = tid >> 5; t < ntiles; t += nthreads >> 5) {
+    if (!(w.tvis[t] & kUnreached)) continue;
+    const int x = (int)(t % w.tiles_x) * kTile + lane, y0 = (int)(t / w.tiles_x) * kTile;
+    for (int y = y0; y < min(y0 + kTile, w.H) && x < w.W; y++) {
+      const int64_t i = (int64_t)y * w.W + x;
+      if (r.level(i) == kInf) r.Wg[i] = r.q[i];
+    }
+  }
+  if (tid == 0) {
+    vs[S_PASS] = vs[S_PASS] + 1u + (unsigned int)phases;
+    vs[S_PHASES] = (unsigned int)phases;
+    vs[S_US_B] = (unsigned int)((t1 - t0) / 1000);
+    vs[S_US_P] = (unsigned int)((global_ns() - t1) / 1000);
   }
 }
 
-// Cells no outlet reached keep q.  Such a cell was never clean (a clean
-// cell's level is finite and flood B keeps it), so only the tiles flood B
-// worked on (tseed) are read: one block per tile, a row segment of 4 cells
-// per thread.
-__global__ void fill_final_kernel(const float* __restrict__ q, float* __restrict__ Wg,
-                                  const uint8_t* __restrict__ tseed, int tiles_x, int W, int H) {
-  const int t = blockIdx.x;
-  if (!tseed[t]) return;
-  const int y = (t / tiles_x) * kTile + (int)(threadIdx.x >> 3);
-  const int x0 = (t % tiles_x) * kTile + (int)(threadIdx.x & 7) * 4;
-  if (y >= H) return;
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    const int x = x0 + k;
-    if (x >= W) break;
-    const int64_t i = (int64_t)y * W + x;
-    if (Wg[i] == kInf) Wg[i] = q[i];
-  }
-}
-
-__global__ void quantize_min_kernel(float* __restrict__ d, int64_t n, float nodata,
-                                    unsigned int* minslot) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void quantize_min_kernel(float* __restrict__ d, int W, int H, float nodata,
+                                    unsigned int* minslot, uint8_t* __restrict__ tseed,
+                                    int tiles_x) {
+  const unsigned int i = blockIdx.x * blockDim.x + threadIdx.x;
   float m = kInf;
-  if (i < n) {
-    float q = fill_quantize(d[i], nodata);
+  if (i < (unsigned int)W * (unsigned int)H) {
+    const float q = fill_quantize(d[i], nodata);
     d[i] = q;
     m = q;
+    const int y = (int)(i / (unsigned int)W), x = (int)(i - (unsigned int)y * (unsigned int)W);
+    if (q == 0.0f || x == 0 || y == 0 || x == W - 1 || y == H - 1)
+      tseed[(y / kTile) * tiles_x + x / kTile] = 1;
   }
   unsigned int o = float_to_ordered(m);
   o = __reduce_min_sync(0xffffffffu, o);
@@ -1172,153 +902,129 @@ __global__ void quantize_min_kernel(float* __restrict__ d, int64_t n, float noda
   if (threadIdx.x == 0) atomicMin(minslot, bmin);
 }
 
-__global__ void fill_scalars_kernel(unsigned int* s) {
-  for (int i = threadIdx.x; i < S_SIZE; i += blockDim.x)
-    s[i] = (i == S_MIN || (i >= S_M && i < S_M + 3)) ? 0xffffffffu : 0u;
+// Blocks and warps per block of a flood over `ntiles` tiles: one block on
+// every SM (`blocks` of them) as far as there are tiles, with as many warps
+// as the tiles can keep busy.  At 512^2 (256 tiles) a visit takes half as
+// long with 2 warps on each of 128 SMs as with 20 warps on each of 13.
+static void flood_shape(int ntiles, int blocks, int warps, int* grid, int* per_block) {
+  *grid = std::max(1, std::min(blocks, ntiles));
+  *per_block = std::max(1, std::min(warps, (ntiles + *grid - 1) / *grid));
 }
 
-template <int MODE, int WARPS>
-static cageo_status launch_flood_warps(const FloodArgs& a, cudaStream_t s) {
-  const size_t smem = sizeof(WarpSmem<MODE>) * WARPS;
-  auto fn = fill_flood_kernel<MODE, WARPS>;
-  CAGEO_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+template <bool MARKS, int WARPS>
+static cageo_status launch_level_warps(const LevelArgs& a, cudaStream_t s) {
+  const size_t smem = sizeof(LevelSmem) * WARPS;
+  auto fn = level_flood_kernel<MARKS, WARPS>;
   static PerDevice resident;  // one table per instantiation
   int blocks = 0;
   cageo_status st = per_device(resident, &blocks, [&](int dev, int* v) -> cageo_status {
+    CAGEO_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     return resident_blocks((const void*)fn, WARPS * 32, smem, dev, v);
   });
   if (st) return st;
-  FloodArgs args = a;
+  int grid, per;
+  flood_shape(a.w.tiles_x * a.w.tiles_y, blocks, WARPS, &grid, &per);
+  LevelArgs args = a;
   void* params[] = {&args};
-  // No more blocks than the tiles can keep busy (small grids leave the
-  // rest of the GPU idle instead of polling the work queue).
-  const int ntiles = a.w.tiles_x * a.w.tiles_y;
-  const int grid = std::max(1, std::min(blocks, (ntiles + WARPS - 1) / WARPS));
-  CAGEO_CUDA(cudaLaunchCooperativeKernel((const void*)fn, dim3(grid), dim3(WARPS * 32), params,
-                                         smem, s));
+  CAGEO_CUDA(cudaLaunchCooperativeKernel((const void*)fn, dim3(grid), dim3(per * 32), params,
+                                         sizeof(LevelSmem) * per, s));
   return CAGEO_OK;
 }
 
 bool fill_flood_warps_valid(int warps) { return warps == 16 || warps == 20 || warps == 22; }
 
-template <int MODE>
-static cageo_status launch_flood(const FloodArgs& a, cudaStream_t s) {
-  if (MODE == 1) return launch_flood_warps<1, kWarpsB>(a, s);
+template <bool MARKS>
+static cageo_status launch_level(const LevelArgs& a, cudaStream_t s) {
   switch (a.w.flood_warps) {
-    case 16: return launch_flood_warps<MODE == 1 ? 0 : MODE, 16>(a, s);
-    case 20: return launch_flood_warps<MODE == 1 ? 0 : MODE, 20>(a, s);
-    case 22: return launch_flood_warps<MODE == 1 ? 0 : MODE, 22>(a, s);
+    case 16: return launch_level_warps<MARKS, 16>(a, s);
+    case 20: return launch_level_warps<MARKS, 20>(a, s);
+    case 22: return launch_level_warps<MARKS, 22>(a, s);
   }
   set_error("pit filling: %d warps per block is not one of 16, 20, 22", a.w.flood_warps);
   return CAGEO_ERR_ARGUMENT;
 }
 
-cageo_status fill_clear_seeds(const FillWork& w, cudaStream_t s) {
-  CAGEO_CUDA(cudaMemsetAsync(w.tseed, 0, (size_t)w.tiles_x * w.tiles_y, s));
+static cageo_status launch_resolve(const Resolve& r, cudaStream_t s) {
+  static PerDevice resident;
+  int blocks = 0;
+  cageo_status st = per_device(resident, &blocks, [&](int dev, int* v) -> cageo_status {
+    return resident_blocks((const void*)fill_resolve_kernel, kResolveThreads, 0, dev, v);
+  });
+  if (st) return st;
+  Resolve args = r;
+  void* params[] = {&args};
+  // No more blocks than a list of every cell would need.
+  const int64_t n = (int64_t)r.w.W * r.w.H;
+  const int grid = (int)std::min<int64_t>(blocks, (n + kResolveRun - 1) / kResolveRun);
+  CAGEO_CUDA(cudaLaunchCooperativeKernel((const void*)fill_resolve_kernel, dim3(grid),
+                                         dim3(kResolveThreads), params, 0, s));
   return CAGEO_OK;
 }
 
-cageo_status fill_reset_scalars(const FillWork& w, cudaStream_t s) {
-  fill_scalars_kernel<<<1, 32, 0, s>>>(w.scal);
+cageo_status fill_begin(const FillWork& w, cudaStream_t s) {
+  const int ntiles = w.tiles_x * w.tiles_y;
+  // 8 rim words (16 bytes each) per thread, but no more blocks than fill the GPU.
+  const unsigned blocks = (unsigned)std::min<int64_t>(
+      2048, ((int64_t)ntiles * (kRimCells / 2) + kRingSlack + 1023) / 1024);
+  fill_begin_kernel<<<blocks, 256, 0, s>>>(w, ntiles);
   CAGEO_CUDA(cudaGetLastError());
-  CAGEO_CUDA(cudaMemsetAsync(w.queued, 0, sizeof(int) * w.tiles_x * w.tiles_y, s));
   return CAGEO_OK;
 }
+
+static unsigned warp_per_tile_blocks(size_t nt) { return (unsigned)((nt + 7) / 8); }
 
 cageo_status fill_run(const float* q, float* filled, const FillWork& w, float nodata,
                       cudaStream_t s) {
-  const int64_t n = (int64_t)w.W * w.H;
-  const unsigned blocks = (unsigned)((n + 256 * kCellsPerThread - 1) / (256 * kCellsPerThread));
-  const size_t nt = (size_t)w.tiles_x * w.tiles_y;
-  if (!w.front_init) CAGEO_CUDA(cudaMemsetAsync(w.tseed, 0, nt, s));
-  const dim3 rows((unsigned)((w.W + 256 * kCellsPerThread - 1) / (256 * kCellsPerThread)),
-                   (unsigned)w.H);
-  // After a fused front, a few block rows check the slabs' minima and
-  // exit (the set-up is redone only where a minimum is not 0).
-  const dim3 init_rows(rows.x, std::min(rows.y, w.front_init ? 1024u : 65535u));
-  fill_init_kernel<<<init_rows, 256, 0, s>>>(q, filled, w.flags,
-                                             w.slab_min ? w.slab_min : w.scal + S_MIN, w.tseed,
-                                             w.tiles_x, w.W, w.H, w.slab_h ? w.slab_h : w.H, nodata,
-                                             w.front_init ? 1 : 0);
-  CAGEO_CUDA(cudaGetLastError());
-  FloodArgs a{q, filled, w};
-  CAGEO_CUDA(cudaMemsetAsync(w.queued, 0, sizeof(int) * nt, s));  // all idle
-  CAGEO_CUDA(cudaMemsetAsync(w.tconv, 0, nt, s));
-  CAGEO_CUDA(cudaMemsetAsync(w.lists, 0xff, (2 * nt + kRingSlack) * sizeof(int), s));  // empty ring
+  const unsigned tblocks = warp_per_tile_blocks((size_t)w.tiles_x * w.tiles_y);
+  if (!w.seeded) fill_seed_kernel<<<tblocks, 256, 0, s>>>(q, w);
+  const unsigned int* minslot = w.slab_min ? w.slab_min : w.scal + S_MIN;
+  LevelArgs a{q, filled, w, nodata, minslot, 0, 0};
   if (w.marks) CAGEO_CUDA(cudaEventRecord(w.marks[0], s));
-  cageo_status st = launch_flood<2>(a, s);  // flood A with clean marks
+  cageo_status st = launch_level<false>(a, s);
   if (st) return st;
   if (w.marks) CAGEO_CUDA(cudaEventRecord(w.marks[1], s));
-  CAGEO_CUDA(cudaMemsetAsync(w.tseed, 0, nt, s));
-  const unsigned cblocks = (unsigned)((n + 4 * 256 - 1) / (4 * 256));
-  fill_classify_kernel<<<cblocks, 256, 0, s>>>(filled, w.flags, w.aux, w.scal, w.tseed,
-                                               w.tiles_x, w.W, n);
-  fill_tile_states_kernel<<<(unsigned)((nt + 255) / 256), 256, 0, s>>>(w.queued, w.tseed,
-                                                                       (int)nt);
-  CAGEO_CUDA(cudaGetLastError());
-  CAGEO_CUDA(cudaMemsetAsync(w.tconv, 0, nt, s));
-  a.stage = 1;  // flood B's main drain, from the tiles holding a cell to recompute
-  st = launch_flood<1>(a, s);
-  if (st) return st;
-  fill_undecided_kernel<<<(unsigned)nt, 256, 0, s>>>(filled, w.flags, w.aux, w.cand, w.scal,
-                                                     w.tseed, w.tiles_x, w.W, w.H);
-  const unsigned ublocks = (unsigned)std::min<int64_t>((n + 255) / 256, 2048);
-  fill_unite_kernel<<<ublocks, 256, 0, s>>>(w.cand, w.scal, w.flags, w.aux, w.W);
-  fill_flatten_kernel<<<ublocks, 256, 0, s>>>(w.cand, w.scal, w.aux);
+  fill_walls_kernel<<<tblocks, 256, 0, s>>>(a);
   CAGEO_CUDA(cudaGetLastError());
   if (w.marks) CAGEO_CUDA(cudaEventRecord(w.marks[2], s));
-  a.stage = 2;  // the confirmation phases
-  st = launch_flood<1>(a, s);
+  st = launch_resolve(Resolve{q, filled, w, nodata, minslot, w.slab_h ? w.slab_h : w.H}, s);
   if (st) return st;
   if (w.marks) CAGEO_CUDA(cudaEventRecord(w.marks[3], s));
-  fill_final_kernel<<<(unsigned)nt, 256, 0, s>>>(q, filled, w.tseed, w.tiles_x, w.W, w.H);
-  CAGEO_CUDA(cudaGetLastError());
   return CAGEO_OK;
 }
 
 cageo_status fill_run_exact(const float* v, float* filled, const FillWork& w, float nodata,
                             const float* warm, cudaStream_t s) {
   const int64_t n = (int64_t)w.W * w.H;
-  const unsigned blocks = (unsigned)((n + 256 * kCellsPerThread - 1) / (256 * kCellsPerThread));
   const size_t nt = (size_t)w.tiles_x * w.tiles_y;
-  // A warm start may hold values above the answer anywhere: every tile is
-  // visited on the first pass.
-  CAGEO_CUDA(cudaMemsetAsync(w.tseed, warm ? 1 : 0, nt, s));
-  const dim3 rows((unsigned)((w.W + 256 * kCellsPerThread - 1) / (256 * kCellsPerThread)),
-                   (unsigned)w.H);
-  fill_init_exact_kernel<<<rows, 256, 0, s>>>(v, filled, w.flags, warm, w.tseed, w.tiles_x, w.W,
-                                              w.H, nodata);
-  CAGEO_CUDA(cudaGetLastError());
-  CAGEO_CUDA(cudaMemsetAsync(w.queued, 0, sizeof(int) * nt, s));  // all idle
-  CAGEO_CUDA(cudaMemsetAsync(w.tconv, 0, nt, s));
-  CAGEO_CUDA(cudaMemsetAsync(w.lists, 0xff, (2 * nt + kRingSlack) * sizeof(int), s));  // empty ring
-  FloodArgs a{v, filled, w};
+  const unsigned tblocks = warp_per_tile_blocks(nt);
+  LevelArgs a{v, filled, w, nodata, nullptr, warm ? 1 : 0, 0};
   if (!warm) {
-    cageo_status st = launch_flood<0>(a, s);
+    if (!w.seeded) fill_seed_kernel<<<tblocks, 256, 0, s>>>(v, w);
+    cageo_status st = launch_level<false>(a, s);
     if (st) return st;
   } else {
-    // Warm flood with support marks, then the unsupported cells restart
-    // from +inf and the repair flood visits their tiles (the others keep
-    // their states: a tile done in the warm flood holds the answer).
-    cageo_status st = launch_flood<2>(a, s);
+    // A warm start may hold values above the answer anywhere: every tile is
+    // visited.  After the warm flood with support marks, the unsupported
+    // cells restart from +inf and the repair flood visits their tiles.
+    CAGEO_CUDA(cudaMemsetAsync(w.tseed, 1, nt, s));
+    fill_warm_start_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(v, warm, filled, n);
+    cageo_status st = launch_level<true>(a, s);
     if (st) return st;
-    CAGEO_CUDA(cudaMemsetAsync(w.tseed, 0, nt, s));
-    const unsigned ublocks = (unsigned)((n + 4 * 256 - 1) / (4 * 256));
-    fill_unsupported_kernel<<<ublocks, 256, 0, s>>>(filled, w.flags, w.tseed, w.scal,
-                                                    w.tiles_x, w.W, n);
+    fill_unsupported_kernel<<<tblocks, 256, 0, s>>>(a);
     CAGEO_CUDA(cudaGetLastError());
-    CAGEO_CUDA(cudaMemsetAsync(w.tconv, 0, nt, s));
     a.stage = 3;
-    if ((st = launch_flood<0>(a, s))) return st;
+    a.warm = 0;
+    if ((st = launch_level<false>(a, s))) return st;
   }
-  fill_final_exact_kernel<<<blocks, 256, 0, s>>>(filled, n);
+  fill_final_exact_kernel<<<tblocks, 256, 0, s>>>(a);
   CAGEO_CUDA(cudaGetLastError());
   return CAGEO_OK;
 }
 
 cageo_status fill_quantize_min(float* d, const FillWork& w, float nodata, cudaStream_t s) {
   const int64_t n = (int64_t)w.W * w.H;
-  quantize_min_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d, n, nodata, w.scal + S_MIN);
+  quantize_min_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(
+      d, w.W, w.H, nodata, w.scal + S_MIN, w.tseed, w.tiles_x);
   CAGEO_CUDA(cudaGetLastError());
   return CAGEO_OK;
 }
@@ -1356,13 +1062,13 @@ cageo_status fill_check_status(const FillWork& w, int64_t* stats) {
     stats[0] = h[S_PASS];
     stats[1] = h[S_PHASES];
     stats[2] = h[S_PASSES_A];
-    stats[3] = h[S_PASSES_B];
+    stats[3] = h[S_STEPS];
     stats[4] = h[S_US_A];
     stats[5] = h[S_US_B];
     stats[6] = h[S_US_P];
     stats[7] = h[S_TILES_A];
     stats[8] = h[S_ROUNDS_A];
-    stats[9] = h[S_TILES_B];
+    stats[9] = h[S_TILES_B] ? h[S_TILES_B] : h[S_CAND] + h[S_MORE];
     stats[10] = h[S_ROUNDS_B];
     stats[11] = h[S_KCYC_LOAD];
     stats[12] = h[S_KCYC_SWEEP];
@@ -1376,20 +1082,12 @@ cageo_status fill_check_status(const FillWork& w, int64_t* stats) {
                                  "a grid-wide wait hit its limit",
                                  "a warp waited for a tile past its limit",
                                  "a tile's queue state kept changing",
-                                 "the tile visits passed their limit",
+                                 "the tile visits or relaxation rounds passed their limit",
                                  "the confirmation phases passed their limit",
-                                 "the labels of the undecided cells are not settled roots"};
+                                 "the labels of the unsettled cells are not settled roots"};
     const unsigned int e = h[S_ERR];
-    if (e == 5)
-      set_error("pit filling: %s (phases %u, undecided cells %u; pending counted %u, confirmed "
-                "in the last phase %u; a minimum cell %u: level %.9g, q %.9g, minimum read %.9g, "
-                "label %u, its label %u)",
-                what[e], h[S_PHASES], h[S_CAND], h[S_DBG], h[S_DBG + 1], h[S_DBG + 2] - 1,
-                __builtin_bit_cast(float, h[S_DBG + 3]), __builtin_bit_cast(float, h[S_DBG + 4]),
-                ordered_to_float(h[S_DBG + 5]), h[S_DBG + 6], h[S_DBG + 7]);
-    else
-      set_error("pit filling: %s (pending tiles %u, phases %u, undecided cells %u)",
-                e < 7 ? what[e] : "unknown error", h[S_PENDING], h[S_PHASES], h[S_CAND]);
+    set_error("pit filling: %s (pending tiles %u, phases %u, listed cells %u)",
+              e < 7 ? what[e] : "unknown error", h[S_PENDING], h[S_PHASES], h[S_CAND]);
     return CAGEO_ERR_NO_CONVERGENCE;
   }
   return CAGEO_OK;
@@ -1410,7 +1108,7 @@ extern "C" cageo_status cageo_pitfill_exact_warm(const float* d_dem, const float
   cageo_status st = ws.acquire(d_workspace, workspace_bytes, fill_workspace_bytes(W, H), stream);
   if (st) return st;
   FillWork w = fill_carve(ws.ptr, W, H);
-  if ((st = fill_reset_scalars(w, stream))) return st;
+  if ((st = fill_begin(w, stream))) return st;
   if ((st = fill_run_exact(d_dem, d_filled, w, nodata_dem, d_warm, stream))) return st;
   CAGEO_CUDA(cudaStreamSynchronize(stream));
   return fill_check_status(w, h_stats);
@@ -1432,11 +1130,12 @@ extern "C" cageo_status cageo_pitfill(float* d_dem, float* d_filled, int W, int 
   cageo_status st = ws.acquire(d_workspace, workspace_bytes, fill_workspace_bytes(W, H), stream);
   if (st) return st;
   FillWork w = fill_carve(ws.ptr, W, H);
-  if ((st = fill_reset_scalars(w, stream))) return st;
+  if ((st = fill_begin(w, stream))) return st;
   if (mode == CAGEO_FILL_EXACT) {
     if ((st = fill_run_exact(d_dem, d_filled, w, nodata_dem, nullptr, stream))) return st;
   } else {
     if ((st = fill_quantize_min(d_dem, w, nodata_dem, stream))) return st;
+    w.seeded = true;
     if ((st = fill_run(d_dem, d_filled, w, nodata_dem, stream))) return st;
   }
   CAGEO_CUDA(cudaStreamSynchronize(stream));

@@ -7,22 +7,28 @@
 
 namespace cageo {
 
-// Workspace of one fill: per-cell flags, per-tile worklists, counters and
-// the candidate list of the confirmation phases.
+// Workspace of one fill: per-tile states, rims, masks and work queue, and the
+// cell lists of the resolution.
 struct FillWork {
   int W = 0, H = 0;
   int tiles_x = 0, tiles_y = 0;
-  uint8_t* flags = nullptr;      // W*H
+  uint8_t* flags = nullptr;      // W*H: cell flags of the resolution
   int* queued = nullptr;         // ntiles: tile state in the work queue (idle, queued, processing, re-queued, done)
-  int* lists = nullptr;          // 2 * ntiles: tile worklists (double buffer)
-  uint8_t* tseed = nullptr;      // ntiles: tile holds a relaying outlet
-  uint8_t* tconv = nullptr;      // ntiles: tile converged on its last visit
-  uint32_t* cand = nullptr;      // W*H: list of undecided cells of the phases
-  uint32_t* aux = nullptr;       // W*H: flood A's result, then component labels
-  uint32_t* cmin = nullptr;      // W*H: per-component phase minima (at roots)
+  int* lists = nullptr;          // 2 * ntiles + kRingSlack: the work queue's ring
+  uint8_t* tseed = nullptr;      // ntiles: tile holds an outlet (or a cell to repair)
+  uint8_t* tvis = nullptr;       // ntiles: tile state of the flood (levelflood.cuh)
+  uint32_t* cand = nullptr;      // W*H: list of the resolution's cells
+  uint32_t* aux = nullptr;       // W*H: their walled level, then component minima (at roots)
+  uint32_t* label = nullptr;     // W*H: their component labels
+  // The flood (levelflood.cuh), in the space of the labels: per tile the rim
+  // entries (4 sides x 32: level bits, flags), and 32 column masks each (lane
+  // = column, bit = row) of the cells that are clean, that never relay in
+  // the flood, and that are walls (interior and not passable).
+  uint2* rim = nullptr;
+  uint32_t *mclean = nullptr, *mdead = nullptr, *mwall = nullptr;
   unsigned int* scal = nullptr;  // scalar block (see pitfill.cu)
   int max_rounds = 64;           // sweep rounds per tile visit before the tile re-queues itself
-  int flood_warps = 20;          // warps per block (per SM) of flood A: 16, 20 or 22
+  int flood_warps = 20;          // warps per block (per SM) of the flood: 16, 20 or 22
   // Stacked realizations (CPU-compatible fill only): the grid holds
   // H / slab_h realizations of slab_h rows each, one above the other.
   // Every slab's first and last rows are its border (outlets), so no flood
@@ -32,22 +38,24 @@ struct FillWork {
   // minE).  slab_h = 0: one realization, minimum in the scalar block.
   int slab_h = 0;
   const unsigned int* slab_min = nullptr;
-  // The fused front has set up the flags, the start values and the tile
-  // seeds (with minE = 0; fill_clear_seeds must run before it): fill_run
-  // only redoes the set-up of the slabs whose minimum of q is not 0.
-  bool front_init = false;
+  // The fused front (or fill_quantize_min) has set the tile seeds; otherwise
+  // the fill finds them itself.
+  bool seeded = false;
   // Profiling only: when set, fill_run records marks[0] after the set-up,
-  // [1] after flood A, [2] after flood B's main drain and the undecided-cell
-  // kernels, [3] after the confirmation phases.
+  // [1] after the walled flood, [2] after the walls' levels, [3] after the
+  // resolution.
   const cudaEvent_t* marks = nullptr;
 };
 
-// Whether `warps` is a block size flood A is built for.
+// Whether `warps` is a block size the flood is built for.
 bool fill_flood_warps_valid(int warps);
 
 size_t fill_workspace_bytes(int W, int H);
 FillWork fill_carve(void* base, int W, int H);
 
+// First of all: the scalar block, the seeds, the work queue, the tile states
+// and the rims of a fill, in one launch.
+cageo_status fill_begin(const FillWork& w, cudaStream_t s);
 // Fill q (already quantized, min already in scal) into `filled`.  Runs on
 // `s`; does not synchronize.  Errors found on the device are reported by
 // fill_check_status after the stream has drained.
@@ -60,24 +68,22 @@ cageo_status fill_run(const float* q, float* filled, const FillWork& w,
 // flood visits their tiles, so the result is the exact fill for any start.
 cageo_status fill_run_exact(const float* v, float* filled, const FillWork& w, float nodata,
                             const float* warm, cudaStream_t s);
-// Quantize d in place (the reference's step (i)) and reduce its minimum
-// into the scalar block.
+// Quantize d in place (the reference's step (i)), reduce its minimum into the
+// scalar block and set the tile seeds.
 cageo_status fill_quantize_min(float* d, const FillWork& w, float nodata,
                                cudaStream_t s);
-// Clears the tile seeds before a fused front sets them (FillWork::front_init).
-cageo_status fill_clear_seeds(const FillWork& w, cudaStream_t s);
-// Launch-time setup of the scalar block and the ordered minimum of q.
-cageo_status fill_reset_scalars(const FillWork& w, cudaStream_t s);
 unsigned int* fill_min_slot(const FillWork& w);
 // Copies the device status (0 ok) and stats into host memory; the stream
 // must have been synchronized.  stats (kFillStats entries): last pass
-// number, phases, passes of flood A, passes of flood B before the first
-// phase, microseconds of flood A, of flood B to convergence, of the phase
-// loop, tiles and sweep rounds of flood A, tiles and rounds of flood B,
-// kilo-cycles summed over tile visits spent staging, sweeping, storing, and
-// kilo-cycles warps of flood A and of flood B spent waiting for a tile,
-// and the cells a warm-started exact fill restarted from +inf.
+// number, phases, drains of the flood, steps of the lower bound's longest front,
+// microseconds of the flood, of the lower bound (of a warm-started exact fill:
+// of the repair flood), of the phases, tiles and sweep rounds of the flood,
+// tiles and rounds of the repair flood, kilo-cycles summed over tile visits
+// spent staging, sweeping, storing, and kilo-cycles warps of the flood and of
+// the repair flood spent waiting for a tile, and the cells a warm-started
+// exact fill restarted from +inf.
 constexpr int kFillStats = 17;
+constexpr int kFillScalars = 224;  // words of the scalar block
 cageo_status fill_check_status(const FillWork& w, int64_t* stats);
 // Adds the last warm-started exact fill's counters to acc (9 device
 // uint64: fills, fills that restarted cells, cells restarted, warm-flood

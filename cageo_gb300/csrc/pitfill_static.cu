@@ -71,11 +71,12 @@ extern "C" cageo_status cageo_pitfill_static(float* d_dem, float* d_filled, int 
   cageo_status st = static_fill_scratch(&base);
   if (st) return st;
   FillWork w = fill_carve(base, W, H);
-  if ((st = fill_reset_scalars(w, stream))) return st;
+  if ((st = fill_begin(w, stream))) return st;
   if (mode == CAGEO_FILL_EXACT) {
     if ((st = fill_run_exact(d_dem, d_filled, w, nodata_dem, nullptr, stream))) return st;
   } else {
     if ((st = fill_quantize_min(d_dem, w, nodata_dem, stream))) return st;
+    w.seeded = true;
     if ((st = fill_run(d_dem, d_filled, w, nodata_dem, stream))) return st;
   }
   CAGEO_CUDA(cudaStreamSynchronize(stream));

@@ -42,7 +42,7 @@ enum : int { R_NFLAT = 0, R_ERR = 3, R_US_BFS = 8, R_PASSES = 9,
              R_HEAD = 128,     // work-queue tickets handed out (own 128-byte line)
              R_TAIL = 160,     // work-queue entries pushed (own line)
              R_PENDING = 192,  // tiles queued or being searched (own line)
-             R_SIZE = 224 };
+             R_SIZE = kRouteScalars };
 constexpr int kFT = 32;          // flat tile size
 constexpr int kFWarps = 20;      // warps per block of the flat kernel (20 x 9.5 KB smem)
 constexpr int kFRS = 35;         // staged row stride

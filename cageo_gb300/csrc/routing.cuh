@@ -20,6 +20,7 @@ struct RouteWork {
   // their neighbours lie in their own slab.
   int slab_h = 0;
 };
+constexpr int kRouteScalars = 224;  // words of the scalar block
 size_t route_workspace_bytes(int W, int H);
 RouteWork route_carve(void* base, int W, int H);
 // mode: CAGEO_ROUTE_CPU_COMPAT or CAGEO_ROUTE_GPU_ORDER (nodata is used by
