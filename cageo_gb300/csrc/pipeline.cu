@@ -104,7 +104,7 @@ struct cageo_pipeline {
         *filter = nullptr, *tmp = nullptr;
   uint8_t* code = nullptr;
   int8_t* dir = nullptr;
-  int *flatdist = nullptr, *label = nullptr;
+  int* label = nullptr;
   uint32_t* counts = nullptr;
   void *fill_ws = nullptr, *route_ws = nullptr, *trace_ws = nullptr;
   FillWork fw;
@@ -135,10 +135,9 @@ struct cageo_pipeline {
   void* fill_ws_b = nullptr;
   unsigned int* slab_min = nullptr;
   FillWork fwb;
-  // Routing over the stack as well: directions and flat distances of all
-  // slabs, routing workspace for W x batch*H.
+  // Routing over the stack as well: directions of all slabs, routing workspace
+  // for W x batch*H.
   int8_t* dirb = nullptr;
-  int* flatdistb = nullptr;
   void* route_ws_b = nullptr;
   RouteWork rwb;
   cudaGraph_t graph_b = nullptr;
@@ -153,15 +152,13 @@ void free_batch(cageo_pipeline* p) {
   if (p->graph_b) cudaGraphDestroy(p->graph_b);
   p->exec_b = nullptr;
   p->graph_b = nullptr;
-  void* bufs[] = {p->qb, p->filledb, p->fill_ws_b, p->slab_min, p->dirb, p->flatdistb,
-                  p->route_ws_b};
+  void* bufs[] = {p->qb, p->filledb, p->fill_ws_b, p->slab_min, p->dirb, p->route_ws_b};
   for (void* b : bufs)
     if (b) cudaFree(b);
   p->qb = p->filledb = nullptr;
   p->fill_ws_b = nullptr;
   p->slab_min = nullptr;
   p->dirb = nullptr;
-  p->flatdistb = nullptr;
   p->route_ws_b = nullptr;
   p->batch = 1;
 }
@@ -171,7 +168,7 @@ void free_all(cageo_pipeline* p) {
   if (p->exec) cudaGraphExecDestroy(p->exec);
   if (p->graph) cudaGraphDestroy(p->graph);
   void* bufs[] = {p->dem, p->streams, p->noise, p->q, p->filled, p->filter, p->tmp, p->code,
-                  p->dir, p->flatdist, p->label, p->counts, p->fill_ws, p->route_ws,
+                  p->dir, p->label, p->counts, p->fill_ws, p->route_ws,
                   p->trace_ws, p->dscal, p->ws_params, p->warm, p->ws_acc};
   for (void* b : bufs)
     if (b) cudaFree(b);
@@ -197,7 +194,7 @@ cageo_status enqueue_fill(cageo_pipeline* p) {
 }
 
 cageo_status enqueue_route(cageo_pipeline* p) {
-  return route_run(p->filled, p->dir, p->flatdist, p->rw, p->stream,
+  return route_run(p->filled, p->dir, nullptr, p->rw, p->stream,
                    exact_mode(p) ? CAGEO_ROUTE_GPU_ORDER : CAGEO_ROUTE_CPU_COMPAT,
                    p->cfg.nodata_dem);
 }
@@ -271,7 +268,7 @@ cageo_status enqueue_batch(cageo_pipeline* p) {
       return st;
   }
   if ((st = fill_run(p->qb, p->filledb, p->fwb, c.nodata_dem, s))) return st;
-  if ((st = route_run(p->filledb, p->dirb, p->flatdistb, p->rwb, s, CAGEO_ROUTE_CPU_COMPAT,
+  if ((st = route_run(p->filledb, p->dirb, nullptr, p->rwb, s, CAGEO_ROUTE_CPU_COMPAT,
                       c.nodata_dem)))
     return st;
   for (int k = 0; k < K; k++) {
@@ -367,7 +364,7 @@ cageo_status create_common(cageo_pipeline** out, const cageo_pipeline_config* cf
       (st = dalloc(&p->tmp, fb)) ||
       (st = dalloc(&p->filter, sizeof(float) * (2 * kMaxRunRadius + 1) * (2 * kMaxRunRadius + 1))) ||
       (st = dalloc(&p->code, (size_t)p->N)) || (st = dalloc(&p->dir, 2 * (size_t)p->N)) ||
-      (st = dalloc(&p->flatdist, 4 * (size_t)p->N)) || (st = dalloc(&p->label, 4 * (size_t)p->N)) ||
+      (st = dalloc(&p->label, 4 * (size_t)p->N)) ||
       (st = dalloc(&p->counts, 4 * (size_t)p->N)) ||
       (st = dalloc(&p->fill_ws, fill_workspace_bytes(W, H))) ||
       (st = dalloc(&p->route_ws, route_workspace_bytes(W, H))) ||
@@ -839,9 +836,9 @@ extern "C" cageo_status cageo_pipeline_counts_bytes(cageo_pipeline* p, uint8_t* 
   counts_to_float_kernel<<<(unsigned)((p->N + 255) / 256), 256, 0, s>>>(p->counts, p->tmp, p->N);
   CAGEO_CUDA(cudaGetLastError());
   // The byte image is staged in the noise buffer and the min/max pair in the
-  // flat-distance grid; both are rewritten by the next realization.
+  // redo list; both are rewritten by the next realization.
   uint8_t* bytes = (uint8_t*)p->noise;
-  unsigned int* mm = (unsigned int*)p->flatdist;
+  unsigned int* mm = p->dscal + 3;
   cageo_status st = launch_to_bytes(p->tmp, bytes, p->N, mm, s);
   if (st) return st;
   CAGEO_CUDA(cudaMemcpyAsync(h_out, bytes, (size_t)p->N, cudaMemcpyDeviceToHost, s));
@@ -1026,7 +1023,7 @@ extern "C" cageo_status cageo_pipeline_set_batch(cageo_pipeline* p, int batch) {
   if ((st = dalloc(&p->qb, sizeof(float) * nb)) || (st = dalloc(&p->filledb, sizeof(float) * nb)) ||
       (st = dalloc(&p->fill_ws_b, fill_workspace_bytes(p->W, batch * p->H))) ||
       (st = dalloc(&p->slab_min, sizeof(unsigned int) * 64)) ||
-      (st = dalloc(&p->dirb, 2 * nb)) || (st = dalloc(&p->flatdistb, sizeof(int) * nb)) ||
+      (st = dalloc(&p->dirb, 2 * nb)) ||
       (st = dalloc(&p->route_ws_b, route_workspace_bytes(p->W, batch * p->H)))) {
     free_batch(p);
     return st;

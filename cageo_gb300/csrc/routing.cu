@@ -1,23 +1,26 @@
 // routing.cu -- A7 D8 flow routing with the reference CPU path's rules
 // (src/flowrouting/FlowRoutingAlgorithmCPUOpenMP.h:53-249).
 //
-// First pass, one thread per cell: border cells point outward (corners
-// diagonally), cells equal to 0 are streams (flatDist -2, no direction),
-// others take the steepest strictly-descending neighbour in N, NE, E, SE, S,
-// SW, W, NW order with diagonal drops divided by 1.41421356f, the first
-// maximum winning.  Cells with no descending neighbour are flat.
+// First pass: border cells point outward (corners diagonally), cells equal to
+// 0 are streams (flatDist -2, no direction), others take the steepest
+// strictly-descending neighbour in N, NE, E, SE, S, SW, W, NW order with
+// diagonal drops divided by 1.41421356f, the first maximum winning.  Cells
+// with no descending neighbour are flat.
 //
 // Flats: the reference assigns layer k = 1, 2, ... to flat cells that have a
 // neighbour in layer k-1 (layer 0 = cells with a direction, flatDist -1)
 // whose elevation is <= theirs, taking the direction of the LAST such
-// neighbour in N..NW order.  Layer numbers are breadth-first distances, so
-// they are computed here as shortest-path distances by tile relaxation (a
-// persistent cooperative kernel on an asynchronous tile queue: one warp runs
-// a bit-parallel breadth-first search over a 32x32 tile of the tiles that
-// hold flat cells, seeded from its halo, and queues the neighbouring tiles
-// when its border changed), and
-// the directions by one final pass that applies the last-match rule to the
-// finished distances.
+// neighbour in N..NW order.  A flat cell has no lower neighbour, so such a
+// neighbour is at its own elevation, and adjacent flat cells are level with
+// each other: layers 1 need the elevations once (the first pass finds them,
+// with their directions), all later layers only the masks of flat cells.
+// Layer numbers are breadth-first distances; they are computed tile by tile
+// (32x32) from three things only: the tile's mask of flat cells, its mask of
+// layer-1 cells, and the distances on the neighbouring tiles' rims, kept in a
+// compact array (4 sides x 32 per tile).  A visit of the distance flood so
+// moves 0.8 KB, against 9 KB when it staged distances and elevations, and
+// writes back changed rims.  When the rims are final, one pass over the tiles
+// recomputes the distances inside and applies the last-match rule.
 //
 // The GPU-order mode follows the reference's GPU routing instead
 // (src/flowrouting/FlowRoutingAlgorithmGPUCUDAOriginal.cu:200-271 and
@@ -25,7 +28,9 @@
 // layer 1 may drain into any cell with a negative flatDist (streams too)
 // whose non-NODATA elevation is <= the flat cell's; a later layer k drains
 // into a cell of an earlier layer; the FIRST match in the order N, W, E,
-// S, NW, NE, SW, SE wins.  The layer numbers are again BFS distances.
+// S, NW, NE, SW, SE wins.  The layer numbers are again BFS distances (and a
+// stream, at 0, is never level with a flat cell: one above 0 has a direction,
+// one below 0 is lower).
 #include <algorithm>
 #include "common.cuh"
 #include "routing.cuh"
@@ -35,7 +40,6 @@
 namespace cageo {
 
 constexpr int kFlatInf = 0x3fffffff;
-constexpr int kOffGrid = (int)0x80000000;  // staged code of a cell outside the grid
 enum : int { R_NFLAT = 0, R_ERR = 3, R_US_BFS = 8, R_PASSES = 9,
              R_TILES = 10, R_KCYC_LOAD = 11, R_KCYC_BFS = 12, R_KCYC_STORE = 13,
              R_BAR_COUNT = kBarCountSlot, R_BAR_GEN = kBarGenSlot,
@@ -44,12 +48,14 @@ enum : int { R_NFLAT = 0, R_ERR = 3, R_US_BFS = 8, R_PASSES = 9,
              R_PENDING = 192,  // tiles queued or being searched (own line)
              R_SIZE = kRouteScalars };
 constexpr int kFT = 32;          // flat tile size
-constexpr int kFWarps = 20;      // warps per block of the flat kernel (20 x 9.5 KB smem)
-constexpr int kFRS = 35;         // staged row stride
+constexpr int kFWarps = 32;      // most warps per block of the distance flood
+enum : int { kRTop = 0, kRBottom = 1, kRLeft = 2, kRRight = 3 };
+constexpr int kRimCells = 4 * kFT;
 
 size_t route_workspace_bytes(int W, int H) {
   const size_t nt = (size_t)((W + kFT - 1) / kFT) * ((H + kFT - 1) / kFT);
   return align_up(nt, 256) + align_up(nt * 4, 256) + align_up((2 * nt + kRingSlack) * 4, 256) +
+         2 * align_up(nt * kFT * 4, 256) + align_up(nt * kRimCells * 4, 256) +
          align_up(R_SIZE * 4, 256);
 }
 
@@ -59,126 +65,276 @@ RouteWork route_carve(void* base, int W, int H) {
   w.H = H;
   w.tiles_x = (W + kFT - 1) / kFT;
   w.tiles_y = (H + kFT - 1) / kFT;
-  const size_t n = (size_t)W * H, nt = (size_t)w.tiles_x * w.tiles_y;
+  const size_t nt = (size_t)w.tiles_x * w.tiles_y;
   char* p = (char*)base;
-  (void)n;
   w.tflat = (uint8_t*)p;
   p += align_up(nt, 256);
   w.queued = (int*)p;
   p += align_up(nt * 4, 256);
   w.lists = (int*)p;
   p += align_up((2 * nt + kRingSlack) * 4, 256);
+  w.mflat = (uint32_t*)p;
+  p += align_up(nt * kFT * 4, 256);
+  w.mfirst = (uint32_t*)p;
+  p += align_up(nt * kFT * 4, 256);
+  w.rim = (int*)p;
+  p += align_up(nt * kRimCells * 4, 256);
   w.scal = (unsigned int*)p;
   return w;
 }
 
-// Steepest-descent pass.  flatdist: -1 direction, -2 stream, -3 NODATA
-// (GPU order only), kFlatInf flat.  A 32x8 block covers one 32x32 flat
-// tile (4 rows per thread), so the tile's "holds a flat cell" flag and the
-// flat-cell count take one store and one atomic per block.
+// x / 1.41421356237309505f, correctly rounded for magnitudes in (1e-30, 1e30):
+// the product with the rounded reciprocal and one correction by its residue
+// (Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990); equal to the division for every mantissa (checked over
+// all 2^24 floats of [1, 4)).  3 instructions against ~10.
+__device__ __forceinline__ float div_sqrt2(float x) {
+  constexpr float kS = 1.41421356237309505f, kR = 1.0f / kS;
+  const float q = __fmul_rn(x, kR);
+  return __fmaf_rn(__fmaf_rn(-q, kS, x), kR, q);
+}
+
+// The steepest descent from c to its neighbours v in N, NE, E, SE, S, SW, W, NW
+// order, diagonal drops divided by sqrt(2), the first maximum winning: its
+// index, or 8 where no neighbour is lower.  GPU: NODATA neighbours are skipped.
+// All eight slopes at once, their maximum, then the first equal to it: ~45
+// instructions, against ~75 for a running maximum.
+template <bool GPU>
+__device__ __forceinline__ int steepest_of(float c, const float (&v)[8], float nodata) {
+  float s[8];
+#pragma unroll
+  for (int n = 0; n < 8; n++) s[n] = GPU && v[n] == nodata ? 0.0f : __fsub_rn(c, v[n]);
+  const float diag = fmaxf(fmaxf(s[1], s[3]), fmaxf(s[5], s[7]));
+  if (diag > 0.0f && !(diag > 1e-30f && diag < 1e30f)) {
+    // Outside the quick division's range: the largest diagonal drop decides
+    // (a smaller one that rounds to the same quotient is in range with it).
+    float best = 0.0f;
+    int got = 8;
+#pragma unroll
+    for (int n = 0; n < 8; n++) {
+      const float d = n & 1 ? __fdiv_rn(s[n], 1.41421356237309505f) : s[n];
+      if (d > best) {
+        best = d;
+        got = n;
+      }
+    }
+    return got;
+  }
+#pragma unroll
+  for (int n = 1; n < 8; n += 2) s[n] = div_sqrt2(s[n]);
+  const float best = fmaxf(fmaxf(fmaxf(s[0], s[2]), fmaxf(s[4], s[6])),
+                           fmaxf(fmaxf(s[1], s[3]), fmaxf(s[5], s[7])));
+  int got = 8;
+#pragma unroll
+  for (int n = 7; n >= 0; n--)
+    if (s[n] == best) got = n;
+  return best > 0.0f ? got : 8;
+}
+
+// Direction n as (dx, dy); n = 8: none.
+__device__ __forceinline__ char2 d8_dir(int n) {
+  // 2 bits per direction: dx + 1 and dy + 1.
+  const int dx = (int)((0x101a9u >> (2 * n)) & 3u) - 1, dy = (int)((0x11a90u >> (2 * n)) & 3u) - 1;
+  return make_char2((signed char)dx, (signed char)dy);
+}
+
+// Staged elevations of a tile and the two cells around it: rows y0 - 2 ..
+// y0 + 33, columns x0 - 4 .. x0 + 35 (x0 - 2 .. x0 + 33 are used), so that the
+// tile's own columns start on a 16-byte boundary.
+constexpr int kES = 40;
+
+// Whether the cell at staged position (sx, sy) -- column gx, in the grid if
+// `in`, row ys of its slab -- has a direction from the first pass.
+template <bool GPU>
+__device__ __forceinline__ bool has_direction(const float* E, int sx, int sy, bool in, int gx,
+                                              int ys, int W, int slab_h, float nodata) {
+  if (!in) return false;
+  if (gx == 0 || gx == W - 1 || ys == 0 || ys == slab_h - 1) return true;
+  const float* e = E + sy * kES + sx;
+  const float c = *e;
+  if (c == 0.0f || (GPU && c == nodata)) return false;
+  float m = kInf;
+#pragma unroll
+  for (int n = 0; n < 8; n++) {
+    const float v = e[d8_dy(n) * kES + d8_dx(n)];
+    if (!(GPU && v == nodata)) m = fminf(m, v);
+  }
+  return m < c;
+}
+
+// First pass: directions, the masks of flat and of layer-1 cells with the
+// directions of the latter, the rims' first distances, and (fd not null) the
+// flat distances known so far.  A block of 8 warps per 32x32 tile, a warp per
+// 4 rows (lane = column): the three elevations of a row serve three rows of
+// outputs from registers.  A layer-1 cell needs to know which neighbours have
+// a direction, so the ring around the tile is decided too (132 cells).
 template <bool GPU>
 __global__ void __launch_bounds__(256) d8_kernel(const float* __restrict__ dem,
                                                  char2* __restrict__ dir,
                                                  int* __restrict__ fd, RouteWork w, float nodata) {
   const int W = w.W, H = w.H;
   const int slab_h = w.slab_h ? w.slab_h : H;
-  const int x = blockIdx.x * kFT + threadIdx.x;
-  // The tile's elevations and a one-cell halo in shared memory.
-  __shared__ float E[34 * 35];
-  {
-    const int x0 = blockIdx.x * kFT - 1, y0 = blockIdx.y * kFT - 1;
-#pragma unroll
-    for (int k = threadIdx.y * 32 + threadIdx.x; k < 34 * 34; k += 256) {
-      const int hy = k / 34, hx = k - hy * 34;
-      const int gx = x0 + hx, gy = y0 + hy;
-      if (gx >= 0 && gx < W && gy >= 0 && gy < H)
-        cp_async4(&E[hy * 35 + hx], dem + (int64_t)gy * W + gx);  // all in flight at once
-      else
-        E[hy * 35 + hx] = 0.0f;
-    }
-    cp_async_wait();
-  }
-  __syncthreads();
-  int nflat = 0;
-#pragma unroll
-  for (int k = 0; k < kFT / 8; k++) {
-    const int y = blockIdx.y * kFT + threadIdx.y + 8 * k;
-    if (x >= W || y >= H) continue;
-    const int64_t i = (int64_t)y * W + x;
-    int dxi = 0, dyi = 0;
-    const int ys = y % slab_h;  // row within its realization's slab
-    if (x == 0) dxi = -1; else if (x == W - 1) dxi = 1;
-    if (ys == 0) dyi = -1; else if (ys == slab_h - 1) dyi = 1;
-    if (dxi || dyi) {
-      dir[i] = make_char2((signed char)dxi, (signed char)dyi);
-      fd[i] = -1;
-      continue;
-    }
-    const float* ec = &E[(threadIdx.y + 8 * k + 1) * 35 + threadIdx.x + 1];
-    const float c = *ec;
-    if (c == 0.0f) {
-      dir[i] = make_char2(0, 0);
-      fd[i] = -2;
-      continue;
-    }
-    if (GPU && c == nodata) {
-      dir[i] = make_char2(0, 0);
-      fd[i] = -3;
-      continue;
-    }
-    float steepest = 0.0f;
-    int sdx = 0, sdy = 0;
-#pragma unroll
-    for (int n = 0; n < 8; n++) {
-      const int dx = d8_dx(n), dy = d8_dy(n);
-      const float e = ec[dy * 35 + dx];
-      if (GPU && e == nodata) continue;
-      float sl = __fsub_rn(c, e);
-      // A diagonal drop only shrinks when divided by sqrt(2), so the
-      // (slow, correctly rounded) division is needed only when the
-      // undivided drop already beats the steepest so far.
-      if (sl > 0.0f && sl > steepest) {
-        if (n & 1) sl = __fdiv_rn(sl, 1.41421356237309505f);
-        if (sl > steepest) { steepest = sl; sdx = dx; sdy = dy; }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int x0 = blockIdx.x * kFT, y0 = blockIdx.y * kFT;
+  __shared__ __align__(16) float E[36 * kES];
+  __shared__ unsigned int Hd[34];       // cells with a direction, rows -1..32, columns 0..31
+  __shared__ unsigned int Hl, Hr, Hc;   // columns -1 and 32 (bit = row 0..31), corners
+  __shared__ unsigned int F[kFT], S[kFT];
+  if ((W & 3) == 0 && x0 + kFT <= W && ((uintptr_t)dem & 15u) == 0) {
+    // The tile's columns by 16-byte copies, the two beside them on either side
+    // by 4-byte ones: 432 copies instead of 1296.
+    for (int k = threadIdx.x; k < 36 * 8 + 36 * 4; k += 256) {
+      const bool mid = k < 36 * 8;
+      const int j = k - 36 * 8;
+      const int sy = mid ? k >> 3 : j >> 2;
+      const int sx = mid ? 4 + 4 * (k & 7) : (j & 2 ? 36 : 2) + (j & 1);
+      const int gx = x0 - 4 + sx, gy = y0 - 2 + sy;
+      float* e = &E[sy * kES + sx];
+      if (gy >= 0 && gy < H && gx >= 0 && gx < W) {
+        if (mid) cp_async16(e, dem + (int64_t)gy * W + gx);
+        else cp_async4(e, dem + (int64_t)gy * W + gx);
       }
     }
-    if (steepest > 0.0f) {
-      dir[i] = make_char2((signed char)sdx, (signed char)sdy);
-      fd[i] = -1;
-    } else {
-      dir[i] = make_char2(0, 0);
-      fd[i] = kFlatInf;
-      nflat++;
+  } else {
+    for (int k = threadIdx.x; k < 36 * 36; k += 256) {
+      const int sy = k / 36, sx = k - sy * 36 + 2;
+      const int gx = x0 - 4 + sx, gy = y0 - 2 + sy;
+      if (gx >= 0 && gx < W && gy >= 0 && gy < H)
+        cp_async4(&E[sy * kES + sx], dem + (int64_t)gy * W + gx);
     }
   }
-  __shared__ int block_flat;
-  if (threadIdx.x == 0 && threadIdx.y == 0) block_flat = 0;
+  cp_async_wait();
   __syncthreads();
+  const int x = x0 + lane, yw = y0 + 4 * warp;  // this warp's first row
+  const bool xin = x < W, xborder = x == 0 || x == W - 1;
+  const int ys0 = yw % slab_h;  // its row in its slab
+  // Row of the slab `k` rows further (k < 37).
+  auto slab_row = [&](int k) {
+    int ys = ys0 + k;
+    while (ys >= slab_h) ys -= slab_h;
+    return ys;
+  };
+  int code[4];  // 0..7: direction; 8: flat; 9: border; 10: stream, NODATA or outside
+  {
+    const float* e = E + (4 * warp + 1) * kES + lane + 3;  // row above this warp's first
+    float a0 = e[0], a1 = e[1], a2 = e[2];
+    float b0 = e[kES], b1 = e[kES + 1], b2 = e[kES + 2];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const float* r = e + (k + 2) * kES;
+      const float c0 = r[0], c1 = r[1], c2 = r[2];
+      const int ys = slab_row(k);
+      const float v[8] = {a1, a2, b2, c2, c1, c0, b0, a0};
+      int n = steepest_of<GPU>(b1, v, nodata);
+      if (b1 == 0.0f || (GPU && b1 == nodata)) n = 10;
+      if (xborder || ys == 0 || ys == slab_h - 1) n = 9;
+      if (!xin || yw + k >= H) n = 10;
+      code[k] = n;
+      const unsigned int h = __ballot_sync(0xffffffffu, n < 8 || n == 9);
+      const unsigned int f = __ballot_sync(0xffffffffu, n == 8);
+      if (lane == 0) {
+        Hd[4 * warp + k + 1] = h;
+        F[4 * warp + k] = f;
+      }
+      a0 = b0; a1 = b1; a2 = b2;
+      b0 = c0; b1 = c1; b2 = c2;
+    }
+  }
+  // The ring: rows -1 and 32 (warps 0, 1), columns -1 and 32 (2, 3), corners.
+  if (warp < 5) {
+    const bool col = warp == 2 || warp == 3, corner = warp == 4;
+    const int rx = corner ? (lane & 1 ? 32 : -1) : col ? (warp == 2 ? -1 : 32) : lane;
+    const int ry = corner ? (lane & 2 ? 32 : -1) : col ? lane : (warp ? 32 : -1);
+    const int gx = x0 + rx, gy = y0 + ry;
+    const bool in = (!corner || lane < 4) && gx >= 0 && gx < W && gy >= 0 && gy < H;
+    const unsigned int h = __ballot_sync(
+        0xffffffffu, has_direction<GPU>(E, rx + 4, ry + 2, in, gx, in ? gy % slab_h : 0, W,
+                                        slab_h, nodata));
+    if (lane == 0) {
+      if (warp == 2) Hl = h;
+      else if (warp == 3) Hr = h;
+      else if (warp == 4) Hc = h;
+      else Hd[warp ? 33 : 0] = h;
+    }
+  }
+  __syncthreads();
+  // Directions; flat cells look for a level neighbour with a direction.
+  int nflat = 0;
+  // Bits 0..2: the cells at x - 1, x, x + 1 of row r (0..33 for rows -1..32)
+  // that have a direction.
+  auto row3 = [&](int r) {
+    const unsigned int h = Hd[r];
+    const unsigned int l = r == 0 ? Hc : r == 33 ? Hc >> 2 : Hl >> (r - 1);
+    const unsigned int g = r == 0 ? Hc >> 1 : r == 33 ? Hc >> 3 : Hr >> (r - 1);
+    return __funnelshift_r((h << 1) | (l & 1u), (h >> 31) | ((g & 1u) << 1), lane) & 7u;
+  };
+  unsigned int gn = row3(4 * warp), gm = row3(4 * warp + 1);
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const int ty = 4 * warp + k, y = y0 + ty;
+    const unsigned int gs = row3(ty + 2);
+    int n = code[k];
+    bool first = false;
+    if (n == 8) {
+      nflat++;
+      // 8 bits in N..NW order.
+      const unsigned int m = (gn >> 1 & 3u) | (gm & 4u) | (gs & 4u) << 1 | (gs & 2u) << 3 |
+                             (gs & 1u) << 5 | (gm & 1u) << 6 | (gn & 1u) << 7;
+      if (m) {
+        const float* e = E + (ty + 2) * kES + lane + 4;
+        const float c = *e;
+        constexpr int order[8] = {0, 6, 2, 4, 7, 1, 5, 3};  // N W E S NW NE SW SE as D8 indices
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          const int d = GPU ? order[7 - j] : j;  // the last match stays
+          const float v = e[d8_dy(d) * kES + d8_dx(d)];
+          if ((m >> d & 1u) && v <= c && !(GPU && v == nodata)) n = d;
+        }
+        first = n != 8;
+      }
+    }
+    gn = gm;
+    gm = gs;
+    const unsigned int s = __ballot_sync(0xffffffffu, first);
+    if (lane == 0) S[ty] = s;
+    if (!xin || y >= H) continue;
+    const int64_t i = (int64_t)y * W + x;
+    char2 d;
+    if (n == 9) {
+      const int ys = slab_row(k);
+      d = make_char2((signed char)(x == 0 ? -1 : x == W - 1 ? 1 : 0),
+                     (signed char)(ys == 0 ? -1 : ys == slab_h - 1 ? 1 : 0));
+    } else {
+      d = d8_dir(min(n, 8));
+    }
+    dir[i] = d;
+    if (fd) {
+      // Flat cells beyond layer 1 start unresolved (0).
+      fd[i] = code[k] == 8 ? (first ? 1 : 0)
+              : code[k] != 10 ? -1
+              : (GPU && E[(ty + 2) * kES + lane + 4] != 0.0f) ? -3 : -2;
+    }
+  }
   nflat = __reduce_add_sync(0xffffffffu, nflat);
-  if (threadIdx.x == 0 && nflat) atomicAdd(&block_flat, nflat);
   __syncthreads();
-  if (threadIdx.x == 0 && threadIdx.y == 0 && block_flat) {
-    w.tflat[blockIdx.y * w.tiles_x + blockIdx.x] = 1;
-    atomicAdd(&w.scal[R_NFLAT], (unsigned int)block_flat);  // statistics only
+  const int t = blockIdx.y * w.tiles_x + blockIdx.x;
+  if (lane == 0 && nflat) atomicAdd(&w.scal[R_NFLAT], (unsigned int)nflat);  // statistics only
+  if (warp == 4) {
+    const unsigned int f = F[lane], s = S[lane];
+    w.mflat[t * kFT + lane] = f;
+    w.mfirst[t * kFT + lane] = s;
+    const bool more = __any_sync(0xffffffffu, (f & ~s) != 0);
+    if (lane == 0) w.tflat[t] = more;
+  } else if (warp < 4) {
+    // Rim entries: 0 not flat, 1 layer 1, infinite otherwise.
+    const int rx = warp == kRLeft ? 0 : warp == kRRight ? 31 : lane;
+    const int ry = warp == kRTop ? 0 : warp == kRBottom ? 31 : lane;
+    const bool f = F[ry] >> rx & 1u, s = S[ry] >> rx & 1u;
+    w.rim[(size_t)t * kRimCells + warp * kFT + lane] = s ? 1 : f ? kFlatInf : 0;
   }
 }
 
-// ---- flat distances by tile relaxation ----------------------------------
-// Staged value of a cell for its neighbours: 0 for a cell a first-layer flat
-// cell may drain into (CPU: a direction; GPU order: a direction or a stream,
-// with an elevation that is not NODATA), the current distance of a flat
-// cell, "infinite" otherwise.
-__device__ __forceinline__ int flat_relay(int code, float e, bool gpu, float nodata) {
-  if (code >= 0) return code;
-  if (gpu) return ((code == -1 || code == -2) && e != nodata) ? 0 : kFlatInf;
-  return code == -1 ? 0 : kFlatInf;
-}
-
-struct FlatSmem {
-  int R[34 * kFRS];      // staged relay values (tile + halo)
-  float E[34 * kFRS];    // staged elevations
-};
-
+// ---- distances ------------------------------------------------------------
 // The flat BFS's queue (tilequeue.cuh): tile states in w.queued, the ring
 // in w.lists.
 __device__ __forceinline__ TileQueue route_queue(const RouteWork& w) {
@@ -189,11 +345,6 @@ __device__ __forceinline__ TileQueue route_queue(const RouteWork& w) {
                    w.scal + R_TAIL,
                    w.scal + R_PENDING,
                    (int*)(w.scal + R_ERR)};
-}
-
-__device__ __forceinline__ void flat_enqueue(const RouteWork& w, int t) {
-  if (!((volatile uint8_t*)w.tflat)[t]) return;  // no flat cell: nothing to do
-  tq_enqueue(route_queue(w), t);
 }
 
 // Per-warp visit statistics (lane 0), flushed every 64 visits and at the end.
@@ -210,151 +361,91 @@ __device__ __forceinline__ void flush_flat_stats(const RouteWork& w, FlatStats& 
   st = FlatStats{};
 }
 
-__device__ void flat_tile(FlatSmem& s, const float* __restrict__ dem, int* fd, const RouteWork& w,
-                          int t, int lane, bool gpu, float nodata, FlatStats& st) {
-  const int W = w.W, H = w.H;
+// The rim entries around a tile: cells next to its top, bottom, left and right
+// side, corners in lanes 0..3 (TL, TR, BL, BR).  L2: other SMs write them.
+struct FlatHalo {
+  int t, b, l, r, c;
+};
+
+__device__ __forceinline__ FlatHalo flat_halo(const RouteWork& w, int t, int lane) {
   const int tx = t % w.tiles_x, ty = t / w.tiles_x;
-  const int x0 = tx * kFT, y0 = ty * kFT;
-  const long long c0 = clock64();
-  // Stage the raw codes and elevations.  The elevations never change: they
-  // come by asynchronous copies (all in flight at once).  The codes hold
-  // distances other warps write meanwhile: they are read from L2 (an L1
-  // line could hold an older value), in a loop
-  // of their own so that the copies' memory clobber does not keep each load
-  // from being issued before the previous iteration's copy.
-  for (int idx = lane; idx < 34 * 34; idx += 32) {
-    const int hy = idx / 34, hx = idx - hy * 34;
-    const int gx = x0 - 1 + hx, gy = y0 - 1 + hy;
-    float* de = &s.E[hy * kFRS + hx];
-    if (gx >= 0 && gx < W && gy >= 0 && gy < H) cp_async4(de, dem + (int64_t)gy * W + gx);
-    else *de = 0.0f;
-  }
-#pragma unroll 12
-  for (int idx = lane; idx < 34 * 34; idx += 32) {
-    const int hy = idx / 34, hx = idx - hy * 34;
-    const int gx = x0 - 1 + hx, gy = y0 - 1 + hy;
-    int code = kOffGrid;
-    if (gx >= 0 && gx < W && gy >= 0 && gy < H) code = __ldcg(fd + (int64_t)gy * W + gx);
-    s.R[hy * kFRS + hx] = code;
-  }
-  cp_async_wait();
-  __syncwarp();
-  // Lane y: the flat cells of row y, and its exits (cells with a direction
-  // that a first-layer flat cell may drain into: relay 0).  The staged codes
-  // stay raw; the seeds below turn the few they read into relay values.
-  const int y = lane;
-  unsigned int flat = 0, exitm = 0;
-#pragma unroll
-  for (int x = 0; x < kFT; x++) {
-    const int b = (y + 1) * kFRS + (x + 1);
-    const int code = s.R[b];
-    if (code == kFlatInf || code >= 1) flat |= 1u << x;
-    // flat_relay(code) == 0 for a non-flat cell; the elevation matters in
-    // GPU order only.
-    const bool ex = gpu ? ((code == -1 || code == -2) && s.E[b] != nodata) : code == -1;
-    if (ex) exitm |= 1u << x;
-  }
-  __syncwarp();
-  const long long c1 = clock64();
-  // Distances inside the tile by a bit-parallel breadth-first search: lane y
-  // holds row y as a bit mask.  A flat cell is a seed at level 1 + the least
-  // relay among its neighbours that are not flat cells of this tile (halo
-  // cells, or exits inside the tile) and whose elevation is <= its own;
-  // flat cells pass levels on to their flat neighbours (which have the same
-  // elevation, so the elevation test always holds between them).  Levels are
-  // visited in increasing order, so the first level that reaches a cell is
-  // its distance; old values inside the tile came from halo values that can
-  // only have dropped since, so they are never below the new ones.
-  //
-  // Only cells on the tile's rim or next to an exit of the tile (a non-flat
-  // cell with relay 0) can be seeds.  Inside the rim a seed's non-flat
-  // neighbours are all inside the tile, where the least relay is 0 (an exit)
-  // or none, so inner seeds are all at level 1.  Rim seeds are held one per lane: the top and bottom rows by
-  // column (lane = x), the left and right columns by row (lane = y, rows
-  // 1..30); each level's seed masks then come from two ballots.
-  unsigned int fup = __shfl_up_sync(0xffffffffu, flat, 1);
-  unsigned int fdn = __shfl_down_sync(0xffffffffu, flat, 1);
-  if (lane == 0) fup = 0;
-  if (lane == kFT - 1) fdn = 0;
-  // Seed level of cell (cx, cy) (kFlatInf: none); fr = the flat masks of
-  // rows cy-1, cy, cy+1 (bit set = flat cell of this tile).
-  auto seed_of = [&](int cx, int cy, unsigned int fu, unsigned int fm, unsigned int fb) {
-    const int b = (cy + 1) * kFRS + (cx + 1);
-    const float e = s.E[b];
-    int best = kFlatInf;
-#pragma unroll
-    for (int n = 0; n < 8; n++) {
-      const int nx = cx + d8_dx(n), ny = cy + d8_dy(n);
-      const unsigned int row = d8_dy(n) < 0 ? fu : (d8_dy(n) > 0 ? fb : fm);
-      const bool inner = nx >= 0 && nx < kFT && ny >= 0 && ny < kFT && ((row >> nx) & 1u);
-      const int o = b + d8_dy(n) * kFRS + d8_dx(n);
-      const float eo = s.E[o];
-      const int v = flat_relay(s.R[o], eo, gpu, nodata);  // the staged codes are raw
-      if (!inner && v < best && eo <= e) best = v;
-    }
-    return best < kFlatInf ? best + 1 : kFlatInf;
+  const bool up = ty > 0, dn = ty + 1 < w.tiles_y, lf = tx > 0, rt = tx + 1 < w.tiles_x;
+  auto at = [&](bool in, int tile, int side, int k) {
+    return in ? __ldcg(w.rim + (size_t)tile * kRimCells + side * kFT + k) : 0;
   };
-  const unsigned int f0 = __shfl_sync(0xffffffffu, flat, 0);
-  const unsigned int f1 = __shfl_sync(0xffffffffu, flat, 1);
-  const unsigned int f30 = __shfl_sync(0xffffffffu, flat, kFT - 2);
-  const unsigned int f31 = __shfl_sync(0xffffffffu, flat, kFT - 1);
-  // Top row (0, x = lane) and bottom row (31, x = lane).
-  const int tseed = ((f0 >> lane) & 1u) ? seed_of(lane, 0, 0u, f0, f1) : kFlatInf;
-  const int bseed = ((f31 >> lane) & 1u) ? seed_of(lane, kFT - 1, f30, f31, 0u) : kFlatInf;
-  // Left (y, 0) and right (y, 31) columns, rows 1..30 (y = lane).
-  const bool mid = lane >= 1 && lane <= kFT - 2;
-  const int lseed = (mid && (flat & 1u)) ? seed_of(0, y, fup, flat, fdn) : kFlatInf;
-  const int rseed = (mid && (flat >> 31)) ? seed_of(kFT - 1, y, fup, flat, fdn) : kFlatInf;
-  // Inner candidates next to an exit of the tile: level 1 or none (an inner
-  // cell's other non-flat neighbours relay nothing).
-  unsigned int exu = __shfl_up_sync(0xffffffffu, exitm, 1);
-  unsigned int exd = __shfl_down_sync(0xffffffffu, exitm, 1);
-  const unsigned int ex3 = exitm | exu | exd;
-  const unsigned int near_exit = ex3 | (ex3 << 1) | (ex3 >> 1);
-  unsigned int inner1 = 0;
-  if (mid) {
-    for (unsigned int m = flat & near_exit & 0x7ffffffeu; m; m &= m - 1) {
-      const int x = __ffs(m) - 1;
-      if (seed_of(x, y, fup, flat, fdn) == 1) inner1 |= 1u << x;
-    }
-  }
+  FlatHalo h;
+  h.t = at(up, t - w.tiles_x, kRBottom, lane);
+  h.b = at(dn, t + w.tiles_x, kRTop, lane);
+  h.l = at(lf, t - 1, kRRight, lane);
+  h.r = at(rt, t + 1, kRLeft, lane);
+  const bool cdn = lane & 2, crt = lane & 1;
+  h.c = at(lane < 4 && (cdn ? dn : up) && (crt ? rt : lf),
+           t + (cdn ? w.tiles_x : -w.tiles_x) + (crt ? 1 : -1), cdn ? kRTop : kRBottom,
+           crt ? 0 : 31);
+  return h;
+}
+
+// Levels the halo gives this lane's cells of the four sides (top and bottom:
+// lane = column; left and right: lane = row): 1 + the least distance of the
+// flat cells next to it outside the tile.
+struct FlatSeeds {
+  int t, b, l, r;
+};
+
+__device__ __forceinline__ FlatSeeds flat_seeds(const FlatHalo& h, unsigned int flat, int lane) {
+  auto dist = [](int v) { return v == 0 ? kFlatInf : v; };  // not flat: no distance
+  const int c = dist(h.c);
+  const int tl = __shfl_sync(0xffffffffu, c, 0), tr = __shfl_sync(0xffffffffu, c, 1);
+  const int bl = __shfl_sync(0xffffffffu, c, 2), br = __shfl_sync(0xffffffffu, c, 3);
+  auto near = [&](int v, int lo, int hi, bool is_flat) {
+    const int u = __shfl_up_sync(0xffffffffu, v, 1), d = __shfl_down_sync(0xffffffffu, v, 1);
+    const int m = min(v, min(lane == 0 ? lo : u, lane == 31 ? hi : d));
+    return is_flat && m < kFlatInf ? m + 1 : kFlatInf;
+  };
+  const unsigned int f0 = __shfl_sync(0xffffffffu, flat, 0), f31 = __shfl_sync(0xffffffffu, flat, 31);
+  FlatSeeds s;
+  s.t = near(dist(h.t), tl, tr, f0 >> lane & 1u);
+  s.b = near(dist(h.b), bl, br, f31 >> lane & 1u);
+  s.l = near(dist(h.l), tl, bl, flat & 1u);
+  s.r = near(dist(h.r), tr, br, flat >> 31);
+  return s;
+}
+
+// Distances inside a tile by a bit-parallel breadth-first search: lane y holds
+// row y as a bit mask.  Levels are visited in increasing order, one dilation
+// each, so the first level that reaches a cell is its distance; the level of
+// each reached cell is kept as an offset from a base in 6 bit planes and
+// handed to emit(x, level) in one pass per segment of at most 64 consecutive
+// levels (when the front dies out, or after 64), for the cells of `keep`.
+template <class Emit>
+__device__ __forceinline__ void flat_bfs(unsigned int flat, unsigned int first, const FlatSeeds& sd,
+                                         unsigned int keep, int lane, Emit emit) {
   auto next_level = [&](int after) {  // least seed level above `after`
     int m = kFlatInf;
-    if (tseed > after) m = min(m, tseed);
-    if (bseed > after) m = min(m, bseed);
-    if (lseed > after) m = min(m, lseed);
-    if (rseed > after) m = min(m, rseed);
-    if (inner1 && after < 1) m = min(m, 1);
+    if (sd.t > after) m = min(m, sd.t);
+    if (sd.b > after) m = min(m, sd.b);
+    if (sd.l > after) m = min(m, sd.l);
+    if (sd.r > after) m = min(m, sd.r);
+    if (first && after < 1) m = min(m, 1);
     return __reduce_min_sync(0xffffffffu, m);
   };
-  int L = next_level(0);
-  unsigned int visited = 0, front = 0, changed = 0;
-  // The level of each reached cell is kept as an offset from Lb in 6 bit
-  // planes (lane = row, bit = column) and written to the staged tile in one
-  // pass per segment of at most 64 consecutive levels (when the front dies
-  // out, or after 64 levels), so the level loop itself does no shared-memory
-  // traffic.
-  int Lb = L;
-  unsigned int seg = 0, pl0 = 0, pl1 = 0, pl2 = 0, pl3 = 0, pl4 = 0, pl5 = 0;
+  int L = next_level(0), base = L;
+  unsigned int open = flat, front = 0;
+  unsigned int seg = 0, p0 = 0, p1 = 0, p2 = 0, p3 = 0, p4 = 0, p5 = 0;
   auto flush = [&]() {
-    for (unsigned int r = seg; r; r &= r - 1) {
+    for (unsigned int r = seg & keep; r; r &= r - 1) {
       const int x = __ffs(r) - 1;
-      const int off = ((pl0 >> x) & 1) | (((pl1 >> x) & 1) << 1) | (((pl2 >> x) & 1) << 2) |
-                      (((pl3 >> x) & 1) << 3) | (((pl4 >> x) & 1) << 4) |
-                      (((pl5 >> x) & 1) << 5);
-      int* cell = &s.R[(y + 1) * kFRS + (x + 1)];
-      if (Lb + off < *cell) {
-        *cell = Lb + off;
-        changed |= 1u << x;
-      }
+      const int off = ((p0 >> x) & 1) | (((p1 >> x) & 1) << 1) | (((p2 >> x) & 1) << 2) |
+                      (((p3 >> x) & 1) << 3) | (((p4 >> x) & 1) << 4) | (((p5 >> x) & 1) << 5);
+      emit(x, base + off);
     }
-    seg = pl0 = pl1 = pl2 = pl3 = pl4 = pl5 = 0;
+    seg = p0 = p1 = p2 = p3 = p4 = p5 = 0;
   };
   for (int guard = 0; guard < 4 * kFT * kFT && L < kFlatInf; guard++) {
-    const unsigned int tb = __ballot_sync(0xffffffffu, tseed == L);
-    const unsigned int bb = __ballot_sync(0xffffffffu, bseed == L);
-    unsigned int seeds = (L == 1 ? inner1 : 0u) | (lseed == L ? 1u : 0u) |
-                         (rseed == L ? 0x80000000u : 0u);
+    const unsigned int tb = __ballot_sync(0xffffffffu, sd.t == L);
+    const unsigned int bb = __ballot_sync(0xffffffffu, sd.b == L);
+    unsigned int seeds = (L == 1 ? first : 0u) | (sd.l == L ? 1u : 0u) |
+                         (sd.r == L ? 0x80000000u : 0u);
     if (lane == 0) seeds |= tb;
     if (lane == kFT - 1) seeds |= bb;
     unsigned int up = __shfl_up_sync(0xffffffffu, front, 1);
@@ -362,69 +453,94 @@ __device__ void flat_tile(FlatSmem& s, const float* __restrict__ dem, int* fd, c
     if (lane == 0) up = 0;
     if (lane == kFT - 1) dn = 0;
     const unsigned int v = front | up | dn;
-    const unsigned int reach = ((v | (v << 1) | (v >> 1)) | seeds) & flat & ~visited;
-    visited |= reach;
-    front = reach;
-    const int off = L - Lb;  // 0..63
-    seg |= reach;
-    if (off & 1) pl0 |= reach;
-    if (off & 2) pl1 |= reach;
-    if (off & 4) pl2 |= reach;
-    if (off & 8) pl3 |= reach;
-    if (off & 16) pl4 |= reach;
-    if (off & 32) pl5 |= reach;
+    front = ((v | (v << 1) | (v >> 1)) | seeds) & open;
+    open &= ~front;
+    const int off = L - base;  // 0..63
+    seg |= front;
+    if (off & 1) p0 |= front;
+    if (off & 2) p1 |= front;
+    if (off & 4) p2 |= front;
+    if (off & 8) p3 |= front;
+    if (off & 16) p4 |= front;
+    if (off & 32) p5 |= front;
     // Next level, or jump to the next seed level when the front died out.
     if (__any_sync(0xffffffffu, front != 0)) {
-      if (++L - Lb == 64) {
+      if (++L - base == 64) {
         flush();
-        Lb = L;
+        base = L;
       }
     } else {
+      if (!__any_sync(0xffffffffu, open != 0)) break;
       flush();
       L = next_level(L);
-      Lb = L;
+      base = L;
     }
   }
   flush();
   __syncwarp();
-  const long long c2 = clock64();
-  const bool capped = false;
-  // Write back the changed distances (lane = column now); note the sides.
-  for (int yy = 0; yy < kFT; yy++) {
-    const unsigned int row = __shfl_sync(0xffffffffu, changed, yy);
-    if ((row >> lane) & 1u)
-      fd[(int64_t)(y0 + yy) * W + (x0 + lane)] = s.R[(yy + 1) * kFRS + (lane + 1)];
-  }
-  // The write-back is visible before any neighbour is queued or the tile's
-  // state changes.  A visit that changed nothing wrote nothing.
-  if (__any_sync(0xffffffffu, changed != 0)) __threadfence();
-  __syncwarp();
-  const unsigned int top = __shfl_sync(0xffffffffu, changed, 0);
-  const unsigned int bot = __shfl_sync(0xffffffffu, changed, kFT - 1);
-  const unsigned int lcol = __ballot_sync(0xffffffffu, changed & 1u);
-  const unsigned int rcol = __ballot_sync(0xffffffffu, changed >> 31);
-  unsigned int sides = (lcol ? 1u : 0u) | (rcol ? 2u : 0u) | (top ? 4u : 0u) | (bot ? 8u : 0u) |
-                       ((top & 1u) ? 16u : 0u) | ((top >> 31) ? 32u : 0u) |
-                       ((bot & 1u) ? 64u : 0u) | ((bot >> 31) ? 128u : 0u);
-  if (lane < 9) {
-    int dx = 0, dy = 0;
-    bool want = false;
-    switch (lane) {
-      case 0: want = capped; break;
-      case 1: dx = -1; want = sides & 1; break;
-      case 2: dx = 1; want = sides & 2; break;
-      case 3: dy = -1; want = sides & 4; break;
-      case 4: dy = 1; want = sides & 8; break;
-      case 5: dx = -1; dy = -1; want = sides & 16; break;
-      case 6: dx = 1; dy = -1; want = sides & 32; break;
-      case 7: dx = -1; dy = 1; want = sides & 64; break;
-      case 8: dx = 1; dy = 1; want = sides & 128; break;
+}
+
+// One visit: the distances on the tile's rim for its halo.  A neighbour is
+// queued only when a rim cell that fell is more than one step below a flat
+// cell next to it (distances only fall, so what holds for the staged ones
+// holds for the present ones).
+__device__ void flat_tile(int* rim_new, const RouteWork& w, int t, int lane, FlatStats& st) {
+  const long long c0 = clock64();
+  int* own = w.rim + (size_t)t * kRimCells + lane;
+  const unsigned int flat = w.mflat[t * kFT + lane], first = w.mfirst[t * kFT + lane];
+  const FlatHalo h = flat_halo(w, t, lane);
+  const int oT = __ldcg(own + kRTop * kFT), oB = __ldcg(own + kRBottom * kFT);
+  const int oL = __ldcg(own + kRLeft * kFT), oR = __ldcg(own + kRRight * kFT);
+  const bool visited = ((volatile uint8_t*)w.tflat)[t] == 2;
+  const FlatSeeds sd = flat_seeds(h, flat, lane);
+  const long long c1 = clock64();
+  long long c2 = c1;
+  unsigned int want = 0;  // neighbours to queue: 1 L, 2 R, 4 T, 8 B, 16 TL, 32 TR, 64 BL, 128 BR
+  const bool lower = sd.t < oT || sd.b < oB || sd.l < oL || sd.r < oR;
+  if (!visited || __any_sync(0xffffffffu, lower)) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) rim_new[k * kFT + lane] = kFlatInf;
+    __syncwarp();
+    const bool edge = lane == 0 || lane == 31;
+    flat_bfs(flat, first, sd, edge ? ~0u : 0x80000001u, lane, [&](int x, int level) {
+      if (lane == 0) rim_new[kRTop * kFT + x] = level;
+      if (lane == 31) rim_new[kRBottom * kFT + x] = level;
+      if (x == 0) rim_new[kRLeft * kFT + lane] = level;
+      if (x == 31) rim_new[kRRight * kFT + lane] = level;
+    });
+    c2 = clock64();
+    if (!visited && lane == 0) w.tflat[t] = 2;
+    auto side = [&](int which, int o, int hv, unsigned int bit, int clo, int chi,
+                    unsigned int lobit, unsigned int hibit) {
+      const int v = rim_new[which * kFT + lane];
+      const bool fell = v < o;
+      if (!__any_sync(0xffffffffu, fell)) return;
+      if (fell) own[which * kFT] = v;
+      const int u = __shfl_up_sync(0xffffffffu, hv, 1), d = __shfl_down_sync(0xffffffffu, hv, 1);
+      if (__any_sync(0xffffffffu, fell && v + 1 < max(hv, max(u, d)))) want |= bit;
+      const int lo = __shfl_sync(0xffffffffu, h.c, clo), hi = __shfl_sync(0xffffffffu, h.c, chi);
+      const unsigned int at = __ballot_sync(0xffffffffu, fell && v + 1 < (lane == 0 ? lo : hi));
+      if (at & 1u) want |= lobit;
+      if (at >> 31) want |= hibit;
+    };
+    side(kRTop, oT, h.t, 4u, 0, 1, 16u, 32u);
+    side(kRBottom, oB, h.b, 8u, 2, 3, 64u, 128u);
+    side(kRLeft, oL, h.l, 1u, 0, 2, 16u, 64u);
+    side(kRRight, oR, h.r, 2u, 1, 3, 32u, 128u);
+    // The rims are visible before any neighbour is queued or the tile's state
+    // changes.
+    __threadfence();
+    __syncwarp();
+    if (lane >= 1 && lane < 9 && (want >> (lane - 1) & 1u)) {
+      // (A side is wanted only where a neighbour lies: outside the grid the
+      // staged entries are 0.)
+      const int dx = lane == 1 || lane == 5 || lane == 7 ? -1 : lane == 2 || lane == 6 || lane == 8 ? 1 : 0;
+      const int dy = lane == 3 || lane == 5 || lane == 6 ? -1 : lane == 4 || lane == 7 || lane == 8 ? 1 : 0;
+      const int n = t + dy * w.tiles_x + dx;
+      if (((volatile uint8_t*)w.tflat)[n]) tq_enqueue(route_queue(w), n);
     }
-    const int nx = tx + dx, ny = ty + dy;
-    if (want && nx >= 0 && ny >= 0 && nx < w.tiles_x && ny < w.tiles_y)
-      flat_enqueue(w, ny * w.tiles_x + nx);
+    __syncwarp();
   }
-  __syncwarp();
   if (lane == 0) {
     const long long c3 = clock64();
     st.tiles++;
@@ -434,33 +550,27 @@ __device__ void flat_tile(FlatSmem& s, const float* __restrict__ dem, int* fd, c
   }
 }
 
-// The flat BFS: every tile holding a flat cell is queued, one 2x2 parity
-// class of tiles after another (grid barrier between), so tiles searched at
-// the same time are rarely neighbours and each class starts from the
-// finished borders of the classes before it; then the warps drain the
-// asynchronous queue (tilequeue.cuh), a tile whose border distances changed
-// queueing its neighbours.  No pass barriers: a free warp takes the next
-// queued tile at once.  A CPU simulation of the queue needed no more tile
-// visits than pass-synchronous worklists (2.70 against 2.71 per tile at
-// 2048^2); on the GPU it took 149 k visits against 186 k at 8192^2.  Waits
-// are bounded; a limit sets the error flag.
-__global__ void __launch_bounds__(kFWarps * 32, 1)
-flat_relax_kernel(const float* __restrict__ dem, int* fd, RouteWork w, int gpu, float nodata) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  FlatSmem& s = reinterpret_cast<FlatSmem*>(smraw)[warp];
+// The distance flood: every tile with flat cells beyond layer 1 is queued, one
+// 2x2 parity class of tiles after another (grid barrier between), so tiles
+// searched at the same time are rarely neighbours and each class starts from
+// the finished rims of the classes before it; then the warps drain the
+// asynchronous queue (tilequeue.cuh).  No pass barriers: a free warp takes the
+// next queued tile at once.  Waits are bounded; a limit sets the error flag.
+__global__ void __launch_bounds__(kFWarps * 32, 1) flat_relax_kernel(RouteWork w) {
+  __shared__ int rims[kFWarps][kRimCells];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   const int ntiles = w.tiles_x * w.tiles_y;
   GridSync gs{w.scal + R_BAR_COUNT, w.scal + R_BAR_GEN, (int*)(w.scal + R_ERR)};
   volatile unsigned int* vs = w.scal;
   const TileQueue q = route_queue(w);
   unsigned long long t0;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-  const int gwarp = blockIdx.x * kFWarps + warp, nwarps = gridDim.x * kFWarps;
+  const int gthread = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
   bool go = true;
   for (int c = 0; c < 4 && go; c++) {
-    for (int i = gwarp; i < ntiles; i += nwarps) {
+    for (int i = gthread; i < ntiles; i += nthreads) {
       const int tx = i % w.tiles_x, ty = i / w.tiles_x;
-      if (lane == 0 && ((tx & 1) | ((ty & 1) << 1)) == c && w.tflat[i]) tq_enqueue(q, i);
+      if (((tx & 1) | ((ty & 1) << 1)) == c && w.tflat[i]) tq_enqueue(q, i);
     }
     go = grid_barrier(gs, gridDim.x);
   }
@@ -474,7 +584,7 @@ flat_relax_kernel(const float* __restrict__ dem, int* fd, RouteWork w, int gpu, 
       if (lane == 0) t = tq_try_dequeue(q, &ticket);
       t = __shfl_sync(0xffffffffu, t, 0);
       if (t >= 0) {
-        flat_tile(s, dem, fd, w, t, lane, gpu != 0, nodata, st);
+        flat_tile(rims[warp], w, t, lane, st);
         if (lane == 0) {
           tq_finish(q, t, false);
           if (st.tiles >= 64) flush_flat_stats(w, st);
@@ -486,12 +596,12 @@ flat_relax_kernel(const float* __restrict__ dem, int* fd, RouteWork w, int gpu, 
       }
       if (vs[R_ERR]) break;
       if (vs[R_PENDING] == 0u) break;
-      if (++idle > (1LL << 24) || vs[R_TILES] > visit_cap) {
+      if (++idle > (1LL << 25) || vs[R_TILES] > visit_cap) {
         if (lane == 0) atomicCAS((int*)(w.scal + R_ERR), 0, 2);
         break;
       }
       __nanosleep(ns);
-      if (ns < 1024) ns <<= 1;
+      if (ns < 512) ns <<= 1;
     }
   }
   if (lane == 0) flush_flat_stats(w, st);
@@ -503,120 +613,90 @@ flat_relax_kernel(const float* __restrict__ dem, int* fd, RouteWork w, int gpu, 
   }
 }
 
-// Directions of flat cells, and flatDist 0 for the flats left unresolved,
-// over the tiles that hold flat cells only (a 32x8 block per 32x32 tile, 4
-// rows per thread).  CPU rules: the LAST neighbour in N..NW order in the
-// previous layer (flatDist -1 for layer 1) whose elevation is <= the
-// cell's.  GPU order: the FIRST neighbour in N, W, E, S, NW, NE, SW, SE
-// order that is (layer 1) a non-NODATA cell with a negative flatDist and an
-// elevation <= the cell's, or (layer d > 1) a cell of layers 1..d-1.  A
-// neighbour reset from "unresolved" to 0 meanwhile matches neither rule
-// before or after, so the reset can share the pass.
+// Directions (and, fd not null, flatDist) of the flat cells beyond layer 1,
+// one warp per tile that holds any: the distances inside from the final rims,
+// then, lane = column, a row at a time: CPU rules: the LAST neighbour in N..NW
+// order in the previous layer; GPU order: the FIRST neighbour in N, W, E, S,
+// NW, NE, SW, SE order in an earlier layer (which is the previous one).
+constexpr int kDS = 35;  // row stride of the staged distances (34 used)
+constexpr int kDirWarps = 8;
 template <bool GPU>
-__global__ void __launch_bounds__(256) flat_dir_kernel(const float* __restrict__ dem,
-                                                       char2* __restrict__ dir,
-                                                       int* __restrict__ fd, RouteWork w,
-                                                       float nodata) {
-  if (!w.tflat[blockIdx.y * w.tiles_x + blockIdx.x]) return;
-  const int W = w.W, H = w.H;
-  const int x = blockIdx.x * kFT + threadIdx.x;
+__global__ void __launch_bounds__(kDirWarps * 32) flat_dir_kernel(char2* __restrict__ dir,
+                                                                  int* __restrict__ fd, RouteWork w) {
+  __shared__ int Ds[kDirWarps][34 * kDS];
+  const int lane = threadIdx.x & 31, t = blockIdx.x * kDirWarps + (threadIdx.x >> 5);
+  if (t >= w.tiles_x * w.tiles_y || !w.tflat[t]) return;
+  int* D = Ds[threadIdx.x >> 5];
+  const unsigned int flat = w.mflat[t * kFT + lane], first = w.mfirst[t * kFT + lane];
+  const FlatHalo h = flat_halo(w, t, lane);
+  const FlatSeeds sd = flat_seeds(h, flat, lane);
+#pragma unroll 8
+  for (int y = 0; y < kFT; y++) D[(y + 1) * kDS + lane + 1] = 0;  // 0: no distance
+  D[lane + 1] = h.t;
+  D[33 * kDS + lane + 1] = h.b;
+  D[(lane + 1) * kDS] = h.l;
+  D[(lane + 1) * kDS + 33] = h.r;
+  if (lane < 4) D[(lane & 2 ? 33 : 0) * kDS + (lane & 1 ? 33 : 0)] = h.c;
+  __syncwarp();
+  flat_bfs(flat, first, sd, ~0u, lane, [&](int x, int level) { D[(lane + 1) * kDS + x + 1] = level; });
+  const unsigned int later = flat & ~first;
+  const int x = (t % w.tiles_x) * kFT + lane, y0 = (t / w.tiles_x) * kFT;
   constexpr int order[8] = {0, 6, 2, 4, 7, 1, 5, 3};  // N W E S NW NE SW SE as D8 indices
-  // Codes and elevations of the tile and a one-cell halo (outside: kOffGrid).
-  __shared__ int F[34 * 35];
-  __shared__ float E[34 * 35];
-  {
-    const int x0 = blockIdx.x * kFT - 1, y0 = blockIdx.y * kFT - 1;
+  for (unsigned int rows = __ballot_sync(0xffffffffu, later != 0); rows; rows &= rows - 1) {
+    const int y = __ffs(rows) - 1;
+    const unsigned int row = __shfl_sync(0xffffffffu, later, y);
+    if (!((row >> lane) & 1u)) continue;
+    const int* c = &D[(y + 1) * kDS + lane + 1];
+    const int d = *c;
+    if (d == 0) continue;  // unresolved
+    int got = 8;
 #pragma unroll
-    for (int k = threadIdx.y * 32 + threadIdx.x; k < 34 * 34; k += 256) {
-      const int hy = k / 34, hx = k - hy * 34;
-      const int gx = x0 + hx, gy = y0 + hy;
-      if (gx >= 0 && gx < W && gy >= 0 && gy < H) {
-        const int64_t i = (int64_t)gy * W + gx;
-        cp_async4(&F[hy * 35 + hx], fd + i);  // all in flight at once
-        cp_async4(&E[hy * 35 + hx], dem + i);
-      } else {
-        F[hy * 35 + hx] = kOffGrid;
-        E[hy * 35 + hx] = 0.0f;
-      }
+    for (int j = 0; j < 8; j++) {
+      const int n = GPU ? order[7 - j] : j;  // the last match stays
+      if (c[d8_dy(n) * kDS + d8_dx(n)] == d - 1) got = n;
     }
-    cp_async_wait();
-  }
-  __syncthreads();
-#pragma unroll 1
-  for (int k = 0; k < kFT / 8; k++) {
-    const int y = blockIdx.y * kFT + threadIdx.y + 8 * k;
-    if (x >= W || y >= H) continue;
-    const int64_t c = (int64_t)y * W + x;
-    const int b = (threadIdx.y + 8 * k + 1) * 35 + threadIdx.x + 1;
-    const int d = F[b];
-    if (d == kFlatInf) {
-      fd[c] = 0;
-      continue;
-    }
-    if (d < 1) continue;  // not a flat cell with a layer
-    const float e = E[b];
-    int nf[8];
-    float ne[8];
-#pragma unroll
-    for (int n = 0; n < 8; n++) {
-      nf[n] = F[b + d8_dy(n) * 35 + d8_dx(n)];
-      ne[n] = E[b + d8_dy(n) * 35 + d8_dx(n)];
-    }
-    int got = -1;
-    if (GPU) {
-#pragma unroll
-      for (int q = 7; q >= 0; q--) {
-        const int n = order[q];
-        const bool ok = d == 1 ? (nf[n] < 0 && nf[n] != kOffGrid && ne[n] != nodata && ne[n] <= e)
-                               : (nf[n] >= 1 && nf[n] <= d - 1);
-        if (ok) got = n;
-      }
-    } else {
-      const int want = d == 1 ? -1 : d - 1;
-#pragma unroll
-      for (int n = 0; n < 8; n++)
-        if (nf[n] == want && ne[n] <= e) got = n;
-    }
-    if (got >= 0) dir[c] = make_char2((signed char)d8_dx(got), (signed char)d8_dy(got));
+    const int64_t i = (int64_t)(y0 + y) * w.W + x;
+    dir[i] = d8_dir(got);
+    if (fd) fd[i] = d;
   }
 }
 
-__global__ void route_scalars_kernel(unsigned int* s) {
-  for (int i = threadIdx.x; i < R_SIZE; i += blockDim.x) s[i] = 0u;
+// Start of a routing: the scalar block, no tile queued, an empty ring.
+__global__ void route_begin_kernel(RouteWork w, int ntiles) {
+  const int tid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
+  for (int i = tid; i < R_SIZE; i += nthreads) w.scal[i] = 0u;
+  for (int64_t i = tid; i < 2 * (int64_t)ntiles + kRingSlack; i += nthreads) {
+    w.lists[i] = kEmptySlot;
+    if (i < ntiles) w.queued[i] = kIdle;
+  }
 }
 
 cageo_status route_run(const float* filled, int8_t* dir, int* fd, const RouteWork& w,
                        cudaStream_t s, int mode, float nodata) {
   const bool gpu = mode == CAGEO_ROUTE_GPU_ORDER;
-  const size_t nt = (size_t)w.tiles_x * w.tiles_y;
-  route_scalars_kernel<<<1, 128, 0, s>>>(w.scal);
-  CAGEO_CUDA(cudaMemsetAsync(w.tflat, 0, nt, s));
-  CAGEO_CUDA(cudaMemsetAsync(w.queued, 0, nt * 4, s));  // all idle
-  CAGEO_CUDA(cudaMemsetAsync(w.lists, 0xff, (2 * nt + kRingSlack) * 4, s));  // empty ring
-  dim3 b(32, 8), g(w.tiles_x, w.tiles_y);
-  if (gpu) d8_kernel<true><<<g, b, 0, s>>>(filled, (char2*)dir, fd, w, nodata);
-  else d8_kernel<false><<<g, b, 0, s>>>(filled, (char2*)dir, fd, w, nodata);
+  const int nt = w.tiles_x * w.tiles_y;
+  route_begin_kernel<<<(unsigned)std::min((2 * (int64_t)nt + kRingSlack + 255) / 256, (int64_t)1024),
+                       256, 0, s>>>(w, nt);
+  const dim3 g(w.tiles_x, w.tiles_y);
+  if (gpu) d8_kernel<true><<<g, 256, 0, s>>>(filled, (char2*)dir, fd, w, nodata);
+  else d8_kernel<false><<<g, 256, 0, s>>>(filled, (char2*)dir, fd, w, nodata);
   CAGEO_CUDA(cudaGetLastError());
   static PerDevice resident;
-  const size_t smem = sizeof(FlatSmem) * kFWarps;
   int coop = 0;
   cageo_status st = per_device(resident, &coop, [&](int dev, int* v) -> cageo_status {
-    CAGEO_CUDA(cudaFuncSetAttribute(flat_relax_kernel,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    return resident_blocks((const void*)flat_relax_kernel, kFWarps * 32, smem, dev, v);
+    return resident_blocks((const void*)flat_relax_kernel, kFWarps * 32, 0, dev, v);
   });
   if (st) return st;
-  const float* f = filled;
-  int* fdp = fd;
   RouteWork wc = w;
-  int gflag = gpu ? 1 : 0;
-  float nd = nodata;
-  void* params[] = {(void*)&f, (void*)&fdp, (void*)&wc, (void*)&gflag, (void*)&nd};
-  const int fgrid = std::max(1, std::min(coop, (int)((nt + kFWarps - 1) / kFWarps)));
+  void* params[] = {(void*)&wc};
+  // A small grid's tiles are spread over all SMs, with fewer warps each.
+  const int fgrid = std::max(1, std::min(coop, nt));
+  const int warps = std::max(1, std::min(kFWarps, (nt + fgrid - 1) / fgrid));
   CAGEO_CUDA(cudaLaunchCooperativeKernel((const void*)flat_relax_kernel, dim3(fgrid),
-                                         dim3(kFWarps * 32), params, smem, s));
-  if (gpu) flat_dir_kernel<true><<<g, b, 0, s>>>(filled, (char2*)dir, fd, w, nodata);
-  else flat_dir_kernel<false><<<g, b, 0, s>>>(filled, (char2*)dir, fd, w, nodata);
+                                         dim3(warps * 32), params, 0, s));
+  const unsigned dblocks = (unsigned)((nt + kDirWarps - 1) / kDirWarps);
+  if (gpu) flat_dir_kernel<true><<<dblocks, kDirWarps * 32, 0, s>>>((char2*)dir, fd, w);
+  else flat_dir_kernel<false><<<dblocks, kDirWarps * 32, 0, s>>>((char2*)dir, fd, w);
   CAGEO_CUDA(cudaGetLastError());
   return CAGEO_OK;
 }
@@ -646,7 +726,7 @@ using namespace cageo;
 
 extern "C" size_t cageo_route_workspace_size(int W, int H) {
   if (!valid_dims(W, H)) return 0;
-  return route_workspace_bytes(W, H) + align_up((size_t)W * H * 4, 256);
+  return route_workspace_bytes(W, H);
 }
 
 extern "C" cageo_status cageo_route_d8_mode(const float* d_filled, int8_t* d_dir,
@@ -660,9 +740,7 @@ extern "C" cageo_status cageo_route_d8_mode(const float* d_filled, int8_t* d_dir
                                cageo_route_workspace_size(W, H), stream);
   if (st) return st;
   RouteWork w = route_carve(ws.ptr, W, H);
-  int* fd = d_flatdist ? d_flatdist
-                       : (int*)((char*)ws.ptr + route_workspace_bytes(W, H));
-  if ((st = route_run(d_filled, d_dir, fd, w, stream, mode, nodata_dem))) return st;
+  if ((st = route_run(d_filled, d_dir, d_flatdist, w, stream, mode, nodata_dem))) return st;
   CAGEO_CUDA(cudaStreamSynchronize(stream));
   return route_check_status(w, nullptr);
 }

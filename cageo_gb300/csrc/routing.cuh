@@ -10,9 +10,12 @@ namespace cageo {
 struct RouteWork {
   int W = 0, H = 0;
   int tiles_x = 0, tiles_y = 0;
-  uint8_t* tflat = nullptr;      // per 32x32 tile: holds a flat cell
-  int* queued = nullptr;         // per tile: last pass it was queued for
-  int* lists = nullptr;          // 2 * ntiles: tile worklists
+  uint8_t* tflat = nullptr;      // per 32x32 tile: holds a flat cell beyond layer 1 (2: visited)
+  int* queued = nullptr;         // per tile: state in the work queue
+  int* lists = nullptr;          // 2 * ntiles + kRingSlack: the work queue's ring
+  uint32_t* mflat = nullptr;     // per tile, 32 row masks (bit = column): flat cells
+  uint32_t* mfirst = nullptr;    // the same: flat cells of layer 1
+  int* rim = nullptr;            // per tile, 4 sides x 32: distance, 0 where not flat
   unsigned int* scal = nullptr;  // counters, barrier, error
   // Stacked realizations: H / slab_h grids of slab_h rows each, one above
   // the other; each slab's first and last rows are its border (0: one grid).
@@ -24,7 +27,7 @@ constexpr int kRouteScalars = 224;  // words of the scalar block
 size_t route_workspace_bytes(int W, int H);
 RouteWork route_carve(void* base, int W, int H);
 // mode: CAGEO_ROUTE_CPU_COMPAT or CAGEO_ROUTE_GPU_ORDER (nodata is used by
-// the latter only).
+// the latter only).  flatdist may be null.
 cageo_status route_run(const float* filled, int8_t* dir, int* flatdist,
                        const RouteWork& w, cudaStream_t s, int mode, float nodata);
 // stats (7 entries, may be null): flat relaxation passes, flat cells,
