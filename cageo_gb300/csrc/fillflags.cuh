@@ -17,8 +17,9 @@ namespace cageo {
 // Other values take the general test.
 __device__ __forceinline__ bool passable_quantized(float q, float minE) {
   if (minE == 0.0f && q >= 0.0f && q < 4096.0f) {
+    // rint(p) by adding and taking away 2^23 (0 <= p < 2^22).
     const float p = __fmul_rn(1000.0f, q);
-    return p >= rintf(p);
+    return p >= __fsub_rn(__fadd_rn(p, 8388608.0f), 8388608.0f);
   }
   return fill_passable(q, minE);
 }

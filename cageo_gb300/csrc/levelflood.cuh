@@ -3,16 +3,20 @@
 // registers.
 //
 // What bounds a flood is the instructions and the dependent chains of its
-// tile visits, not memory (a visit moves ~9 KB).  So a warp holds its 32x32
-// tile's levels in registers, one column per lane (R[y]), and a sweep step is
-// two shuffles, a three-way minimum, and max/min with the cell's elevation
-// (one conflict-free shared load): ~7 instructions a row against ~25 when the
-// levels lay in shared memory with a flag byte per cell.  Sweeping along rows
-// needs the transpose, which goes through shared memory (stride 33, 64
-// accesses) between the two directions.  No flags are read inside the sweeps:
-// a cell that never relays (outside the grid, NODATA, not passable) is staged
-// as level +inf with elevation +inf, an outlet as level = elevation, and both
-// are fixed points of the update.
+// tile visits, not memory (a visit moves ~9 KB).  A warp stages its 32x32 tile
+// as (level, elevation) pairs in shared memory (row stride 33, so rows and
+// columns are both read without bank conflicts) and sweeps it a line at a
+// time, the line before in registers: per cell one 8-byte load, two shuffles,
+// a three-way minimum, max/min with the elevation, and a store if the level
+// fell -- ~9 instructions against ~25 with a flag byte per cell and scalar
+// neighbour loads.  No flags are read inside the sweeps: a cell that never
+// relays (outside the grid, NODATA, not passable) is staged as level +inf with
+// elevation +inf, an outlet as level = elevation, and both are fixed points of
+// the update.  Lines go in groups of 4 in a loop of small body.  (With the
+// levels in 32 registers, every line unrolled and a transpose between the two
+// directions, a visit took as many instructions, but warps waited for
+// instruction fetches more than for anything else: 1.33 ms at 8192^2 against
+// 1.07.)
 //
 // Tiles see each other through their rims only: 4 sides x 32 cells per tile
 // in a compact array, each entry the cell's relayed level with its flags in
@@ -30,6 +34,7 @@
 #include "common.cuh"
 #include "fillflags.cuh"
 #include "pitfill.cuh"
+#include "tilequeue.cuh"
 
 namespace cageo {
 
@@ -46,11 +51,9 @@ constexpr int kRimCells = 4 * kTile;   // rim entries per tile
 // Tile states of the flood (FillWork::tvis).
 constexpr uint8_t kVisited = 1, kUnsettled = 2, kUnreached = 4;
 
-// Per warp: the elevations (+inf where a cell never relays) and the
-// transposition buffer.
+// Per warp: (level, elevation) of the tile's cells.
 struct LevelSmem {
-  float Q[kTile * kLS];
-  float T[kTile * kLS];
+  float2 C[kTile * kLS];
 };
 
 struct LevelArgs {
@@ -73,63 +76,66 @@ struct VisitStats {
 __device__ __forceinline__ float min3(float a, float b, float c) { return fminf(fminf(a, b), c); }
 __device__ __forceinline__ float max3(float a, float b, float c) { return fmaxf(fmaxf(a, b), c); }
 
-// Forward and backward sweep of the lines held in R (registers are lines,
-// lanes the positions along them), interleaved so their dependency chains
-// overlap: step f updates line f from line f - 1 and line 31 - f from line
-// 32 - f.  Bit k of pf (pb) = line k has to be evaluated against line k - 1
-// (k + 1); lines go in groups of 4, and a group with nothing pending is
-// skipped.  A change sets the bits of the lines that read it; a bit set for a
-// line that its sweep has passed stays for the next phase, so empty masks
-// mean a fixed point.  Returns the lanes that changed.
-template <int QS>
-__device__ __forceinline__ unsigned int sweep_lines(float (&R)[kTile], const float* q,
-                                                    unsigned int& pf, unsigned int& pb) {
+// Forward and backward sweep over the tile's lines (ROWS: rows, down and up,
+// lane = column; otherwise columns, right and left, lane = row), interleaved
+// so their dependency chains overlap: step f updates line f from line f - 1
+// and line 31 - f from line 32 - f.  Bit k of pf (pb) = line k has to be
+// evaluated against line k - 1 (k + 1); lines go in groups of 4, loaded ahead,
+// and a group with nothing pending is skipped.  A change sets the bits of the
+// lines that read it; a bit set for a line that its sweep has passed stays for
+// the next phase, so empty masks mean a fixed point.  Returns the lanes that
+// changed.
+template <bool ROWS>
+__device__ __forceinline__ unsigned int sweep_lines(float2* C, int lane, unsigned int& pf,
+                                                    unsigned int& pb) {
+  constexpr int S = ROWS ? kLS : 1;
+  float2* c = C + (ROWS ? lane : lane * kLS);
   unsigned int lanes = 0;
-#pragma unroll
-  for (int g = 0; g < 8; g++) {
+#pragma unroll 1
+  for (int f0 = 0; f0 < kTile; f0 += 4) {
     constexpr unsigned int kGroup = 0xfu;
-    const int f0 = 4 * g, b0 = 28 - 4 * g;
-    if (((pf >> f0) | (pb >> b0)) & kGroup) {
-      bool cf = false, cb = false;
+    const int b0 = 28 - f0;
+    if (!(((pf >> f0) | (pb >> b0)) & kGroup)) continue;
+    float2 vf[4], vb[4];
 #pragma unroll
-      for (int k = 0; k < 4; k++) {
-        const int f = f0 + k, b = 31 - f;
-        float nf = 0.0f, nb = 0.0f;
-        if (f > 0) {
-          const float c = R[f - 1];
-          const float m = min3(c, __shfl_up_sync(0xffffffffu, c, 1),
-                               __shfl_down_sync(0xffffffffu, c, 1));
-          nf = fminf(R[f], fmaxf(q[f * QS], m));
-        }
-        if (b < 31) {
-          const float c = R[b + 1];
-          const float m = min3(c, __shfl_up_sync(0xffffffffu, c, 1),
-                               __shfl_down_sync(0xffffffffu, c, 1));
-          nb = fminf(R[b], fmaxf(q[b * QS], m));
-        }
-        if (f > 0) {
-          cf |= nf < R[f];
-          R[f] = nf;
-        }
-        if (b < 31) {
-          cb |= nb < R[b];
-          R[b] = nb;
-        }
-      }
-      const unsigned int bf = __ballot_sync(0xffffffffu, cf), bb = __ballot_sync(0xffffffffu, cb);
-      pf &= ~(kGroup << f0);
-      pb &= ~(kGroup << b0);
-      if (bf) {
-        if (f0 + 4 < kTile) pf |= 1u << ((f0 + 4) & 31);
-        pb |= (kGroup << f0) >> 1;
-      }
-      if (bb) {
-        if (b0 > 0) pb |= 1u << ((b0 - 1) & 31);
-        pf |= (kGroup << b0) << 1;
-      }
-      lanes |= bf | bb;
+    for (int k = 0; k < 4; k++) {
+      vf[k] = c[(f0 + k) * S];
+      vb[k] = c[(b0 + 3 - k) * S];
     }
+    // (Lines 0 and 31 have none before them.)
+    float pvf = f0 > 0 ? c[(f0 - 1) * S].x : kInf, pvb = f0 > 0 ? c[(b0 + 4) * S].x : kInf;
+    bool cf = false, cb = false;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const float mf = min3(pvf, __shfl_up_sync(0xffffffffu, pvf, 1),
+                            __shfl_down_sync(0xffffffffu, pvf, 1));
+      const float mb = min3(pvb, __shfl_up_sync(0xffffffffu, pvb, 1),
+                            __shfl_down_sync(0xffffffffu, pvb, 1));
+      pvf = fminf(vf[k].x, fmaxf(vf[k].y, mf));
+      pvb = fminf(vb[k].x, fmaxf(vb[k].y, mb));
+      if (pvf < vf[k].x) {
+        c[(f0 + k) * S].x = pvf;
+        cf = true;
+      }
+      if (pvb < vb[k].x) {
+        c[(b0 + 3 - k) * S].x = pvb;
+        cb = true;
+      }
+    }
+    const unsigned int bf = __ballot_sync(0xffffffffu, cf), bb = __ballot_sync(0xffffffffu, cb);
+    pf &= ~(kGroup << f0);
+    pb &= ~(kGroup << b0);
+    if (bf) {
+      pf |= (1u << f0) << 4;
+      pb |= (kGroup << f0) >> 1;
+    }
+    if (bb) {
+      pb |= (1u << b0) >> 1;
+      pf |= (kGroup << b0) << 1;
+    }
+    lanes |= bf | bb;
   }
+  __syncwarp();
   return lanes;
 }
 
@@ -185,28 +191,26 @@ __device__ __forceinline__ CellMasks cell_masks(const FillWork& w, const unsigne
 // over with one shuffle per mask), on the rows around an open cell only; then
 // the marks spread by bit operations until no lane changes, at most 1024
 // rounds, each marking a cell.
-__device__ __forceinline__ unsigned int spread_clean(const float (&R)[kTile], unsigned int cl,
+__device__ __forceinline__ unsigned int spread_clean(const float2* C, unsigned int cl,
                                                      unsigned int open, int lane) {
   const unsigned int need = __reduce_or_sync(0xffffffffu, open & ~cl);
   if (!need) return cl;
   unsigned int qN = 0, qS = 0, qE = 0, qNE = 0, qSE = 0;  // this lane's cell takes from ...
   unsigned int eW = 0, eNW = 0, eSW = 0;                  // the right-hand lane's cell takes from ...
-#pragma unroll
   for (int y = 0; y < kTile; y++) {
-    if (need & ((1u << y) | (y + 1 < kTile ? 2u << y : 0u))) {
-      const float a = R[y], ar = __shfl_down_sync(0xffffffffu, a, 1);
-      if (ar <= a) qE |= 1u << y;
-      if (a <= ar) eW |= 1u << y;
-      if (y + 1 < kTile) {
-        const float b = R[(y + 1) & 31], br = __shfl_down_sync(0xffffffffu, b, 1);
-        const unsigned int below = 1u << ((y + 1) & 31);
-        if (b <= a) qS |= 1u << y;
-        if (a <= b) qN |= below;
-        if (br <= a) qSE |= 1u << y;
-        if (a <= br) eNW |= below;
-        if (b <= ar) eSW |= 1u << y;
-        if (ar <= b) qNE |= below;
-      }
+    const unsigned int bit = 1u << y, below = bit << 1;
+    if (!(need & (bit | below))) continue;
+    const float a = C[y * kLS + lane].x, ar = __shfl_down_sync(0xffffffffu, a, 1);
+    if (ar <= a) qE |= bit;
+    if (a <= ar) eW |= bit;
+    if (y + 1 < kTile) {
+      const float b = C[(y + 1) * kLS + lane].x, br = __shfl_down_sync(0xffffffffu, b, 1);
+      if (b <= a) qS |= bit;
+      if (a <= b) qN |= below;
+      if (br <= a) qSE |= bit;
+      if (a <= br) eNW |= below;
+      if (b <= ar) eSW |= bit;
+      if (ar <= b) qNE |= below;
     }
   }
   const unsigned int qW = __shfl_up_sync(0xffffffffu, eW, 1);
@@ -272,79 +276,70 @@ __device__ __forceinline__ float near_max(float v, int lane) {
 __device__ __forceinline__ float takes_level(const Rim& r) { return r.f & kRimFinal ? -kInf : r.v; }
 __device__ __forceinline__ float takes_mark(const Rim& r) { return r.f & kRimClean ? -kInf : r.v; }
 
-// One visit of tile t by a warp.  Returns false when the sweeps hit the
-// round limit (the tile then queues itself).  `enqueue(tile)` queues a tile.
-template <bool MARKS, class Enqueue>
-__device__ __forceinline__ void level_visit(LevelSmem& s, const LevelArgs& a, int t, int lane,
-                                            VisitStats& st, Enqueue enqueue) {
+// One visit of tile t by a warp.  (When the sweeps hit the round limit the tile
+// queues itself.)
+template <bool MARKS>
+__device__ __forceinline__ void level_visit(LevelSmem& s, const LevelArgs& a, const TileQueue& queue,
+                                            int t, int lane, VisitStats& st) {
   const FillWork& w = a.w;
   const int W = w.W, H = w.H;
   const int tx = t % w.tiles_x, ty = t / w.tiles_x;
   const int x0 = tx * kTile, y0 = ty * kTile, gx = x0 + lane;
   const long long c0 = clock64();
-  const uint8_t ts = __ldcg(w.tvis + t);
-  const bool first = ts == 0;
   const bool full = x0 + kTile <= W && y0 + kTile <= H;
   const int64_t base = (int64_t)y0 * W + gx;
-  // Elevations: asynchronous copies, in flight with everything below.
+  float2* col = s.C + lane;              // this lane's column, row stride kLS
+  float2* row = s.C + lane * kLS;        // this lane's row
+  // Levels of the visit before and elevations: asynchronous copies, all in
+  // flight with the rims and masks (a first visit copies levels it does not
+  // use rather than wait for the tile's state).  The levels were last written
+  // by whichever SM visited the tile before; taking it from the queue ended in
+  // a fence, which orders these loads after that visit's stores.
   if (full) {
     const float* qp = a.q + base;
-#pragma unroll
-    for (int y = 0; y < kTile; y++) cp_async4(&s.Q[y * kLS + lane], qp + (int64_t)y * W);
+    const float* wp = a.Wg + base;
+#pragma unroll 8
+    for (int y = 0; y < kTile; y++) {
+      cp_async4(&col[y * kLS].x, wp + (int64_t)y * W);
+      cp_async4(&col[y * kLS].y, qp + (int64_t)y * W);
+    }
   } else {
     for (int y = 0; y < kTile; y++) {
-      if (gx < W && y0 + y < H) cp_async4(&s.Q[y * kLS + lane], a.q + base + (int64_t)y * W);
-      else s.Q[y * kLS + lane] = kInf;
+      if (gx < W && y0 + y < H) {
+        cp_async4(&col[y * kLS].x, a.Wg + base + (int64_t)y * W);
+        cp_async4(&col[y * kLS].y, a.q + base + (int64_t)y * W);
+      } else {
+        col[y * kLS] = make_float2(kInf, kInf);
+      }
     }
   }
   Rim hT, hB, hL, hR, hC;
   load_halo(w, t, tx, ty, lane, hT, hB, hL, hR, hC);
-  // Own levels, masks and left and right rim of the visit before.
-  float R[kTile];
-  unsigned int dead = 0, cl = 0;
-  Rim oL{kInf, 0u}, oR{kInf, 0u};
-  if (!first || a.warm) {
-    const float* wp = a.Wg + base;
-    if (full) {
-#pragma unroll
-      for (int y = 0; y < kTile; y++) R[y] = __ldcg(wp + (int64_t)y * W);
-    } else {
-#pragma unroll
-      for (int y = 0; y < kTile; y++)
-        R[y] = gx < W && y0 + y < H ? __ldcg(wp + (int64_t)y * W) : kInf;
-    }
-  }
-  if (!first) {
-    dead = __ldcg(w.mdead + t * kTile + lane);
-    if (MARKS) cl = __ldcg(w.mclean + t * kTile + lane);
-    oL = load_rim(w, true, t, kLeft, lane);
-    oR = load_rim(w, true, t, kRight, lane);
-  }
+  // Masks and left and right rim of the visit before.
+  const uint8_t ts = __ldcg(w.tvis + t);
+  const bool first = ts == 0;
+  unsigned int dead = __ldcg(w.mdead + t * kTile + lane);
+  unsigned int cl = MARKS ? __ldcg(w.mclean + t * kTile + lane) : 0u;
+  Rim oL = load_rim(w, true, t, kLeft, lane), oR = load_rim(w, true, t, kRight, lane);
+  if (first) cl = 0;
   cp_async_wait();
   __syncwarp();
   if (first) {
     const CellMasks m = cell_masks(w, a.minslot, a.nodata, gx, y0,
-                                   [&](int y) { return s.Q[y * kLS + lane]; });
+                                   [&](int y) { return col[y * kLS].y; });
     dead = m.dead;
     cl = m.outlet;
     w.mdead[t * kTile + lane] = dead;
     w.mwall[t * kTile + lane] = m.wall;
-#pragma unroll
+#pragma unroll 4
     for (int y = 0; y < kTile; y++) {
-      const float start = a.warm ? R[y] : kInf;
-      R[y] = (m.outlet >> y) & 1u ? s.Q[y * kLS + lane] : start;
+      if ((m.outlet >> y) & 1u) col[y * kLS].x = col[y * kLS].y;
+      else if (!a.warm) col[y * kLS].x = kInf;
     }
   }
-  if (__any_sync(0xffffffffu, dead != 0)) {
-#pragma unroll
-    for (int y = 0; y < kTile; y++)
-      if ((dead >> y) & 1u) {
-        R[y] = kInf;
-        s.Q[y * kLS + lane] = kInf;
-      }
-    __syncwarp();
-  }
-  const float oT = first ? kInf : R[0], oB = first ? kInf : R[31];
+  for (unsigned int m = dead; m; m &= m - 1) col[(__ffs(m) - 1) * kLS] = make_float2(kInf, kInf);
+  __syncwarp();
+  const float oT = first ? kInf : col[0].x, oB = first ? kInf : col[31 * kLS].x;
   const unsigned int cl0 = first ? 0u : cl;
   // The least relay each rim cell has outside the tile.
   const float tl = __shfl_sync(0xffffffffu, hC.v, 0), tr = __shfl_sync(0xffffffffu, hC.v, 1);
@@ -357,104 +352,53 @@ __device__ __forceinline__ void level_visit(LevelSmem& s, const LevelArgs& a, in
   // inside: only what its halo changes has to spread.
   const bool settled = (ts & (kVisited | kUnsettled)) == kVisited;
   unsigned int pd = settled ? 0u : ~0u, pu = pd, pr = pd, pl = pd;
-  bool sides = !settled;    // the left and right halo have yet to be applied
-  bool moved = first;       // a level changed on this visit
+  bool moved = first;  // a level changed on this visit
+  auto offer = [&](float2* c, float m) {  // the lanes whose rim cell falls
+    const float2 v = *c;
+    const float n = fminf(v.x, fmaxf(v.y, m));
+    if (n < v.x) c->x = n;
+    return __ballot_sync(0xffffffffu, n < v.x);
+  };
   {
-    const float n0 = fminf(R[0], fmaxf(s.Q[lane], mT));
-    const float n1 = fminf(R[31], fmaxf(s.Q[31 * kLS + lane], mB));
-    const unsigned int b0 = __ballot_sync(0xffffffffu, n0 < R[0]);
-    const unsigned int b1 = __ballot_sync(0xffffffffu, n1 < R[31]);
-    R[0] = n0;
-    R[31] = n1;
-    if (b0) pd |= 2u;
-    if (b1) pu |= 1u << 30;
-    const unsigned int b = b0 | b1;
-    pr |= b << 1;
-    pl |= b >> 1;
-    moved |= b != 0;
-    if (settled)
-      sides = __any_sync(0xffffffffu, fminf(oL.v, fmaxf(s.Q[lane * kLS], mL)) < oL.v ||
-                                          fminf(oR.v, fmaxf(s.Q[lane * kLS + 31], mR)) < oR.v);
+    const unsigned int bT = offer(col, mT), bB = offer(col + 31 * kLS, mB);
+    __syncwarp();
+    const unsigned int bL = offer(row, mL), bR = offer(row + 31, mR);
+    __syncwarp();
+    const unsigned int h = bT | bB, v = bL | bR;
+    pd |= (bT ? 2u : 0u) | v << 1;
+    pu |= (bB ? 1u << 30 : 0u) | v >> 1;
+    pr |= (bL ? 2u : 0u) | h << 1;
+    pl |= (bR ? 1u << 30 : 0u) | h >> 1;
+    moved |= (h | v) != 0;
   }
-  bool fresh = false;  // T holds the current levels
   int rounds = 0;
-  for (; rounds < w.max_rounds && (pd | pu | pr | pl | (unsigned int)sides); rounds++) {
+  for (; rounds < w.max_rounds && (pd | pu | pr | pl); rounds++) {
     if (pd | pu) {
-      const unsigned int cols = sweep_lines<kLS>(R, &s.Q[lane], pd, pu);
-      if (cols) {
-        pr |= cols << 1;
-        pl |= cols >> 1;
-        moved = true;
-        fresh = false;
-      }
+      const unsigned int cols = sweep_lines<true>(s.C, lane, pd, pu);
+      pr |= cols << 1;
+      pl |= cols >> 1;
+      moved |= cols != 0;
     }
-    if (pr | pl | (unsigned int)sides) {
-#pragma unroll
-      for (int y = 0; y < kTile; y++) s.T[y * kLS + lane] = R[y];
-      __syncwarp();
-#pragma unroll
-      for (int x = 0; x < kTile; x++) R[x] = s.T[lane * kLS + x];
-      __syncwarp();
-      unsigned int rows = 0;
-      if (sides) {
-        const float n0 = fminf(R[0], fmaxf(s.Q[lane * kLS], mL));
-        const float n1 = fminf(R[31], fmaxf(s.Q[lane * kLS + 31], mR));
-        const unsigned int b0 = __ballot_sync(0xffffffffu, n0 < R[0]);
-        const unsigned int b1 = __ballot_sync(0xffffffffu, n1 < R[31]);
-        R[0] = n0;
-        R[31] = n1;
-        if (b0) pr |= 2u;
-        if (b1) pl |= 1u << 30;
-        rows = b0 | b1;
-        sides = false;
-      }
-      rows |= sweep_lines<1>(R, &s.Q[lane * kLS], pr, pl);
-      if (rows) {
-        pd |= rows << 1;
-        pu |= rows >> 1;
-        moved = true;
-      }
-#pragma unroll
-      for (int x = 0; x < kTile; x++) s.T[lane * kLS + x] = R[x];
-      __syncwarp();
-#pragma unroll
-      for (int y = 0; y < kTile; y++) R[y] = s.T[y * kLS + lane];
-      fresh = true;
+    if (pr | pl) {
+      const unsigned int rows = sweep_lines<false>(s.C, lane, pr, pl);
+      pd |= rows << 1;
+      pu |= rows >> 1;
+      moved |= rows != 0;
     }
   }
   const bool capped = (pd | pu | pr | pl) != 0;
-  if (moved && !fresh) {
-    __syncwarp();
-#pragma unroll
-    for (int y = 0; y < kTile; y++) s.T[y * kLS + lane] = R[y];
-    __syncwarp();
-  }
-  // This lane's row of the left and right columns.
-  const float nL = moved ? s.T[lane * kLS] : oL.v, nR = moved ? s.T[lane * kLS + 31] : oR.v;
-  // Cells no outlet has reached (and cells that never relay) are at +inf.
-  unsigned int inf = 0;
-  const bool work = moved || !settled;
-  if (MARKS || work) {
-    float mx = R[0];
-#pragma unroll
-    for (int y = 1; y < kTile; y++) mx = fmaxf(mx, R[y]);
-    if (__any_sync(0xffffffffu, mx == kInf)) {
-#pragma unroll
-      for (int y = 0; y < kTile; y++)
-        if (R[y] == kInf) inf |= 1u << y;
-    }
-  }
+  // New rim: this lane's column of the top and bottom rows, its row of the
+  // left and right columns.
+  const float2 nT = col[0], nB = col[31 * kLS], nL = row[0], nR = row[31];
   if constexpr (MARKS) {
     // A level that fell withdraws its mark (its clean path may not reach the
     // new level); the pass below derives it again.
-    if (moved && !first && __any_sync(0xffffffffu, cl != 0)) {
-      const float* wp = a.Wg + base;
-#pragma unroll
-      for (int y = 0; y < kTile; y++) {
-        const float old = full || (gx < W && y0 + y < H) ? __ldcg(wp + (int64_t)y * W) : kInf;
-        if (R[y] < old) cl &= ~(1u << y);
-      }
-      // Dead cells hold their elevation there; outlets never change.
+    unsigned int inf = 0;
+    for (int y = 0; y < kTile; y++) {
+      const float v = col[y * kLS].x;
+      if (v == kInf) inf |= 1u << y;
+      else if (moved && ((cl0 >> y) & 1u) && v < __ldcg(a.Wg + base + (int64_t)y * W)) cl &= ~(1u << y);
+      // (Dead cells are at +inf here; outlets never change.)
     }
     const unsigned int open = ~(cl | inf);
     if (__any_sync(0xffffffffu, open != 0)) {
@@ -465,24 +409,31 @@ __device__ __forceinline__ void level_visit(LevelSmem& s, const LevelArgs& a, in
       const float sB = near_min(hB.f & kRimRelay ? hB.v : kInf, cbl, cbr, lane);
       const float sL = near_min(hL.f & kRimRelay ? hL.v : kInf, ctl, cbl, lane);
       const float sR = near_min(hR.f & kRimRelay ? hR.v : kInf, ctr, cbr, lane);
-      const unsigned int bl_ = __ballot_sync(0xffffffffu, sL <= nL);
-      const unsigned int br_ = __ballot_sync(0xffffffffu, sR <= nR);
-      unsigned int offered = (sT <= R[0] ? 1u : 0u) | (sB <= R[31] ? 1u << 31 : 0u);
+      const unsigned int bl_ = __ballot_sync(0xffffffffu, sL <= nL.x);
+      const unsigned int br_ = __ballot_sync(0xffffffffu, sR <= nR.x);
+      unsigned int offered = (sT <= nT.x ? 1u : 0u) | (sB <= nB.x ? 1u << 31 : 0u);
       if (lane == 0) offered |= bl_;
       if (lane == 31) offered |= br_;
       cl |= offered & open;
-      cl = spread_clean(R, cl, open, lane);
+      cl = spread_clean(s.C, cl, open, lane);
     }
   }
   const long long c2 = clock64();
   // Write back.  Dead cells keep their elevation in the filled grid (written
   // by the first visit).
+  bool unreached = (ts & kUnreached) != 0;
   if (moved) {
     float* wp = a.Wg + base;
-#pragma unroll
+    bool inf = false;
+#pragma unroll 8
     for (int y = 0; y < kTile; y++) {
-      if (!((dead >> y) & 1u)) wp[(int64_t)y * W] = R[y];
+      const float v = col[y * kLS].x;
+      if (!((dead >> y) & 1u)) {
+        wp[(int64_t)y * W] = v;
+        inf |= v == kInf;
+      }
     }
+    unreached = __any_sync(0xffffffffu, inf);
     if (first) {
       for (unsigned int m = dead; m; m &= m - 1) {
         const int y = __ffs(m) - 1;
@@ -503,10 +454,10 @@ __device__ __forceinline__ void level_visit(LevelSmem& s, const LevelArgs& a, in
     return (MARKS ? (relay ? kRimRelay : 0u) | (clean ? kRimClean : 0u) : 0u) |
            (v == q ? kRimFinal : 0u);
   };
-  const unsigned int fT = flags(cl & 1u, cd & 1u, R[0], s.Q[lane]);
-  const unsigned int fB = flags(cl >> 31, cd >> 31, R[31], s.Q[31 * kLS + lane]);
-  const unsigned int fL = flags((clL >> lane) & 1u, (cdL >> lane) & 1u, nL, s.Q[lane * kLS]);
-  const unsigned int fR = flags((clR >> lane) & 1u, (cdR >> lane) & 1u, nR, s.Q[lane * kLS + 31]);
+  const unsigned int fT = flags(cl & 1u, cd & 1u, nT.x, nT.y);
+  const unsigned int fB = flags(cl >> 31, cd >> 31, nB.x, nB.y);
+  const unsigned int fL = flags((clL >> lane) & 1u, (cdL >> lane) & 1u, nL.x, nL.y);
+  const unsigned int fR = flags((clR >> lane) & 1u, (cdR >> lane) & 1u, nR.x, nR.y);
   uint2* rim = w.rim + (size_t)t * kRimCells + lane;
   // Publishes a side's new entries; returns whether any changed.
   auto publish = [&](int which, float v, unsigned int f, float ov, unsigned int of) {
@@ -533,10 +484,10 @@ __device__ __forceinline__ void level_visit(LevelSmem& s, const LevelArgs& a, in
     if (at >> 31) to |= hibit;
     return to;
   };
-  const unsigned int ofT = first ? 0u : flags(cl0 & 1u, cd0 & 1u, oT, s.Q[lane]);
-  const unsigned int ofB = first ? 0u : flags(cl0 >> 31, cd0 >> 31, oB, s.Q[31 * kLS + lane]);
-  const bool pT = publish(kTop, R[0], fT, oT, ofT), pB = publish(kBottom, R[31], fB, oB, ofB);
-  const bool pL = publish(kLeft, nL, fL, oL.v, oL.f), pR = publish(kRight, nR, fR, oR.v, oR.f);
+  const unsigned int ofT = first ? 0u : flags(cl0 & 1u, cd0 & 1u, oT, nT.y);
+  const unsigned int ofB = first ? 0u : flags(cl0 >> 31, cd0 >> 31, oB, nB.y);
+  const bool pT = publish(kTop, nT.x, fT, oT, ofT), pB = publish(kBottom, nB.x, fB, oB, ofB);
+  const bool pL = publish(kLeft, nL.x, fL, oL.v, oL.f), pR = publish(kRight, nR.x, fR, oR.v, oR.f);
   Rim kT = hT, kB = hB, kL = hL, kR = hR, kC = hC;
   if constexpr (MARKS) {
     // A mark here and a withdrawn one there may cross: with marks the
@@ -553,32 +504,29 @@ __device__ __forceinline__ void level_visit(LevelSmem& s, const LevelArgs& a, in
                                         newer(kR, hR) || newer(kC, hC)) &&
             __any_sync(0xffffffffu, (~cd) != 0);
   }
-  if (pT) want |= wants(R[0], fT, oT, ofT, kT, kC, 4u, 0, 1, 16u, 32u);
-  if (pB) want |= wants(R[31], fB, oB, ofB, kB, kC, 8u, 2, 3, 64u, 128u);
-  if (pL) want |= wants(nL, fL, oL.v, oL.f, kL, kC, 1u, 0, 2, 16u, 64u);
-  if (pR) want |= wants(nR, fR, oR.v, oR.f, kR, kC, 2u, 1, 3, 32u, 128u);
+  if (pT) want |= wants(nT.x, fT, oT, ofT, kT, kC, 4u, 0, 1, 16u, 32u);
+  if (pB) want |= wants(nB.x, fB, oB, ofB, kB, kC, 8u, 2, 3, 64u, 128u);
+  if (pL) want |= wants(nL.x, fL, oL.v, oL.f, kL, kC, 1u, 0, 2, 16u, 64u);
+  if (pR) want |= wants(nR.x, fR, oR.v, oR.f, kR, kC, 2u, 1, 3, 32u, 128u);
   }
   if (lane == 0) {
     st.tiles++;
     st.rounds += (unsigned int)rounds;
   }
-  if (work) {
-    const bool unreached = __any_sync(0xffffffffu, (inf & ~dead) != 0);
-    if (lane == 0)
-      w.tvis[t] = kVisited | (capped ? kUnsettled : 0) | (unreached ? kUnreached : 0);
-  }
+  if ((moved || !settled) && lane == 0)
+    w.tvis[t] = kVisited | (capped ? kUnsettled : 0) | (unreached ? kUnreached : 0);
   // Everything written is visible before a neighbour is queued or the tile's
   // state changes.
   __threadfence();
   __syncwarp();
-  if (lane < 9) {
+  want = (want << 1) | (capped || again ? 1u : 0u);
+  if (want) {
     const int dx = lane == 1 || lane == 5 || lane == 7 ? -1 : lane == 2 || lane == 6 || lane == 8 ? 1 : 0;
     const int dy = lane == 3 || lane == 5 || lane == 6 ? -1 : lane == 4 || lane == 7 || lane == 8 ? 1 : 0;
-    const bool q = lane == 0 ? capped || again : (want >> (lane - 1)) & 1u;
     const int nx = tx + dx, ny = ty + dy;
-    if (q && nx >= 0 && ny >= 0 && nx < w.tiles_x && ny < w.tiles_y) enqueue(ny * w.tiles_x + nx);
+    tq_enqueue(queue, lane < 9 && ((want >> lane) & 1u) && nx >= 0 && ny >= 0 && nx < w.tiles_x &&
+                          ny < w.tiles_y, ny * w.tiles_x + nx);
   }
-  __syncwarp();
   if (lane == 0) {
     const long long c3 = clock64();
     st.kload += (unsigned int)((c1 - c0) >> 10);

@@ -85,7 +85,7 @@ enum : int {
   S_KCYC_IDLE_B = 104, // the same for a repair flood
   S_HEAD = 128,      // work-queue tickets handed out (own 128-byte line)
   S_TAIL = 160,      // work-queue entries pushed (own line)
-  S_PENDING = 192,   // tiles queued or being processed (own line)
+  S_DONE = 192,      // tiles finished (own line)
   S_BAR_COUNT = kBarCountSlot,
   S_BAR_GEN = kBarGenSlot,
   S_SIZE = kFillScalars
@@ -162,11 +162,9 @@ __device__ __forceinline__ TileQueue fill_queue(const FillWork& w) {
                    2u * (unsigned int)(w.tiles_x * w.tiles_y) + kRingSlack,
                    w.scal + S_HEAD,
                    w.scal + S_TAIL,
-                   w.scal + S_PENDING,
+                   w.scal + S_DONE,
                    (int*)(w.scal + S_ERR)};
 }
-
-__device__ __forceinline__ void enqueue(const FillWork& w, int t) { tq_enqueue(fill_queue(w), t); }
 
 __device__ __forceinline__ void flush_stats(const FillWork& w, VisitStats& st, bool b_slots) {
   if (!st.tiles && !st.kidle) return;
@@ -217,32 +215,31 @@ __device__ __forceinline__ bool uf_unite(uint32_t* lab, uint32_t a, uint32_t b) 
   return false;
 }
 
-// One warp: process queued tiles (visit(t, stats), which returns whether the
-// tile can never change again) until no tile is queued or being processed
-// anywhere.  During a drain only a warp processing a tile can queue one, and
-// that tile keeps `pending` above 0, so pending == 0 means no push can come: a
-// ticket still waiting then is abandoned (head and tail are reset after the
-// drain).  b_slots: the statistics go to flood B's counters.  False on an
-// error or a wait limit.
+// One warp: process queued tiles (visit(t, stats)) until no tile is queued or
+// being processed anywhere; a ticket still waiting then is abandoned (head,
+// tail and done are reset after the drain).  b_slots: the statistics go to the
+// repair flood's counters.  False on an error or a wait limit.
 template <class Visit>
 __device__ bool drain(const FillWork& w, int lane, int ntiles, bool b_slots, Visit visit) {
   volatile unsigned int* vs = w.scal;
   const unsigned int visit_cap = 1000u * (unsigned int)min(ntiles, 4000000);
+  const TileQueue q = fill_queue(w);
   long long ticket = -1;
-  unsigned int ns = 32;
+  unsigned int ns = 32, finished = 0;
   VisitStats st;
   bool ok = true;
   long long idle_from = -1;  // clock when this warp last found no tile (-1: busy)
   for (long long idle = 0;;) {
     int t = -1;
-    if (lane == 0) t = tq_try_dequeue(fill_queue(w), &ticket);
+    if (lane == 0) t = tq_try_dequeue(q, &ticket);
     t = __shfl_sync(0xffffffffu, t, 0);
     if (t >= 0) {
       if (lane == 0 && idle_from >= 0) st.kidle += (unsigned int)((clock64() - idle_from) >> 10);
       idle_from = -1;
-      const bool done = visit(t, st);
+      visit(t, st);
       if (lane == 0) {
-        tq_finish(fill_queue(w), t, done);
+        tq_finish(q, t);
+        finished++;
         if (st.tiles >= 64) flush_stats(w, st, b_slots);
       }
       __syncwarp();
@@ -250,17 +247,20 @@ __device__ bool drain(const FillWork& w, int lane, int ntiles, bool b_slots, Vis
       ns = 32;
       continue;
     }
-    if (vs[S_ERR]) {
-      ok = false;
+    int end = 0;  // 1 drained, 2 error, 3 limit
+    if (lane == 0) {
+      if (tq_drained(q, &finished)) end = 1;
+      else if (vs[S_ERR]) end = 2;
+      else if (idle > (1LL << 25)) end = 3;
+      else if (vs[b_slots ? S_TILES_B : S_TILES_A] > visit_cap) end = 4;
+    }
+    end = __shfl_sync(0xffffffffu, end, 0);
+    if (end) {
+      ok = end == 1;
+      if (lane == 0 && end > 2) atomicCAS((int*)(w.scal + S_ERR), 0, end == 3 ? 2 : 4);
       break;
     }
-    if (vs[S_PENDING] == 0u) break;
-    const bool idle_limit = ++idle > (1LL << 25);
-    if (idle_limit || vs[b_slots ? S_TILES_B : S_TILES_A] > visit_cap) {
-      if (lane == 0) atomicCAS((int*)(w.scal + S_ERR), 0, idle_limit ? 2 : 4);
-      ok = false;
-      break;
-    }
+    idle++;
     if (idle_from < 0) idle_from = clock64();
     __nanosleep(ns);
     if (ns < 512) ns <<= 1;
@@ -284,11 +284,11 @@ __device__ bool drain(const FillWork& w, int lane, int ntiles, bool b_slots, Vis
 __device__ __forceinline__ bool seed_queue(const FillWork& w, const GridSync& gs, int gwarp,
                                            int nwarps, int lane, int ntiles) {
   bool go = true;
-  const int gthread = gwarp * 32 + lane, nthreads = nwarps * 32;
+  const TileQueue q = fill_queue(w);
   for (int c = 0; c < 4 && go; c++) {
-    for (int i = gthread; i < ntiles; i += nthreads) {
-      const int tx = i % w.tiles_x, ty = i / w.tiles_x;
-      if (((tx & 1) | ((ty & 1) << 1)) == c && w.tseed[i]) enqueue(w, i);
+    for (int base = gwarp * 32; base < ntiles; base += nwarps * 32) {
+      const int i = base + lane, tx = i % w.tiles_x, ty = i / w.tiles_x;
+      tq_enqueue(q, i < ntiles && ((tx & 1) | ((ty & 1) << 1)) == c && w.tseed[i], i);
     }
     go = grid_barrier(gs, gridDim.x);
   }
@@ -312,8 +312,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) level_flood_kernel(LevelArgs a)
   const bool repair = a.stage == 3;
   if (go)
     go = drain(w, lane, ntiles, repair, [&](int t, VisitStats& st) {
-      level_visit<MARKS>(s, a, t, lane, st, [&](int n) { enqueue(w, n); });
-      return false;
+      level_visit<MARKS>(s, a, fill_queue(w), t, lane, st);
     });
   grid_barrier(gs, gridDim.x);
   // Tiles no outlet reaches were never queued: their masks and start levels
@@ -397,7 +396,7 @@ __global__ void __launch_bounds__(256) fill_unsupported_kernel(LevelArgs a) {
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     w.scal[S_HEAD] = 0u;
     w.scal[S_TAIL] = 0u;
-    w.scal[S_PENDING] = 0u;
+    w.scal[S_DONE] = 0u;
   }
   const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (t >= w.tiles_x * w.tiles_y) return;
@@ -1086,8 +1085,8 @@ cageo_status fill_check_status(const FillWork& w, int64_t* stats) {
                                  "the confirmation phases passed their limit",
                                  "the labels of the unsettled cells are not settled roots"};
     const unsigned int e = h[S_ERR];
-    set_error("pit filling: %s (pending tiles %u, phases %u, listed cells %u)",
-              e < 7 ? what[e] : "unknown error", h[S_PENDING], h[S_PHASES], h[S_CAND]);
+    set_error("pit filling: %s (tiles finished %u, phases %u, listed cells %u)",
+              e < 7 ? what[e] : "unknown error", h[S_DONE], h[S_PHASES], h[S_CAND]);
     return CAGEO_ERR_NO_CONVERGENCE;
   }
   return CAGEO_OK;

@@ -45,7 +45,7 @@ enum : int { R_NFLAT = 0, R_ERR = 3, R_US_BFS = 8, R_PASSES = 9,
              R_BAR_COUNT = kBarCountSlot, R_BAR_GEN = kBarGenSlot,
              R_HEAD = 128,     // work-queue tickets handed out (own 128-byte line)
              R_TAIL = 160,     // work-queue entries pushed (own line)
-             R_PENDING = 192,  // tiles queued or being searched (own line)
+             R_DONE = 192,     // tiles finished (own line)
              R_SIZE = kRouteScalars };
 constexpr int kFT = 32;          // flat tile size
 constexpr int kFWarps = 32;      // most warps per block of the distance flood
@@ -343,7 +343,7 @@ __device__ __forceinline__ TileQueue route_queue(const RouteWork& w) {
                    2u * (unsigned int)(w.tiles_x * w.tiles_y) + kRingSlack,
                    w.scal + R_HEAD,
                    w.scal + R_TAIL,
-                   w.scal + R_PENDING,
+                   w.scal + R_DONE,
                    (int*)(w.scal + R_ERR)};
 }
 
@@ -531,15 +531,15 @@ __device__ void flat_tile(int* rim_new, const RouteWork& w, int t, int lane, Fla
     // changes.
     __threadfence();
     __syncwarp();
-    if (lane >= 1 && lane < 9 && (want >> (lane - 1) & 1u)) {
+    if (want) {
       // (A side is wanted only where a neighbour lies: outside the grid the
       // staged entries are 0.)
       const int dx = lane == 1 || lane == 5 || lane == 7 ? -1 : lane == 2 || lane == 6 || lane == 8 ? 1 : 0;
       const int dy = lane == 3 || lane == 5 || lane == 6 ? -1 : lane == 4 || lane == 7 || lane == 8 ? 1 : 0;
       const int n = t + dy * w.tiles_x + dx;
-      if (((volatile uint8_t*)w.tflat)[n]) tq_enqueue(route_queue(w), n);
+      const bool go = lane >= 1 && lane < 9 && (want >> (lane - 1) & 1u);
+      tq_enqueue(route_queue(w), go && ((volatile uint8_t*)w.tflat)[n], n);
     }
-    __syncwarp();
   }
   if (lane == 0) {
     const long long c3 = clock64();
@@ -565,12 +565,12 @@ __global__ void __launch_bounds__(kFWarps * 32, 1) flat_relax_kernel(RouteWork w
   const TileQueue q = route_queue(w);
   unsigned long long t0;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-  const int gthread = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
+  const int gwarp = blockIdx.x * warps + warp, nwarps = gridDim.x * warps;
   bool go = true;
   for (int c = 0; c < 4 && go; c++) {
-    for (int i = gthread; i < ntiles; i += nthreads) {
-      const int tx = i % w.tiles_x, ty = i / w.tiles_x;
-      if (((tx & 1) | ((ty & 1) << 1)) == c && w.tflat[i]) tq_enqueue(q, i);
+    for (int base = gwarp * 32; base < ntiles; base += nwarps * 32) {
+      const int i = base + lane, tx = i % w.tiles_x, ty = i / w.tiles_x;
+      tq_enqueue(q, i < ntiles && ((tx & 1) | ((ty & 1) << 1)) == c && w.tflat[i], i);
     }
     go = grid_barrier(gs, gridDim.x);
   }
@@ -578,15 +578,16 @@ __global__ void __launch_bounds__(kFWarps * 32, 1) flat_relax_kernel(RouteWork w
   if (go) {
     const unsigned int visit_cap = 1000u * (unsigned int)min(ntiles, 4000000);
     long long ticket = -1;
-    unsigned int ns = 32;
-    for (long long idle = 0;;) {
+    unsigned int ns = 32, finished = 0;
+    for (long long idle = 0;; idle++) {
       int t = -1;
       if (lane == 0) t = tq_try_dequeue(q, &ticket);
       t = __shfl_sync(0xffffffffu, t, 0);
       if (t >= 0) {
         flat_tile(rims[warp], w, t, lane, st);
         if (lane == 0) {
-          tq_finish(q, t, false);
+          tq_finish(q, t);
+          finished++;
           if (st.tiles >= 64) flush_flat_stats(w, st);
         }
         __syncwarp();
@@ -594,10 +595,14 @@ __global__ void __launch_bounds__(kFWarps * 32, 1) flat_relax_kernel(RouteWork w
         ns = 32;
         continue;
       }
-      if (vs[R_ERR]) break;
-      if (vs[R_PENDING] == 0u) break;
-      if (++idle > (1LL << 25) || vs[R_TILES] > visit_cap) {
-        if (lane == 0) atomicCAS((int*)(w.scal + R_ERR), 0, 2);
+      int end = 0;
+      if (lane == 0) {
+        if (tq_drained(q, &finished) || vs[R_ERR]) end = 1;
+        else if (idle > (1LL << 25) || vs[R_TILES] > visit_cap) end = 2;
+      }
+      end = __shfl_sync(0xffffffffu, end, 0);
+      if (end) {
+        if (lane == 0 && end == 2) atomicCAS((int*)(w.scal + R_ERR), 0, 2);
         break;
       }
       __nanosleep(ns);

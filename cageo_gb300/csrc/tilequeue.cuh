@@ -7,18 +7,25 @@
 // must not happen is two warps processing one tile at once (a slower warp's
 // write-back could undo a faster one's lower values).  Each tile therefore
 // has a state: idle, queued, processing, processing and queued again
-// meanwhile (re-queued when its processing ends), or done (never queued
-// again).  `pending` counts tiles that are queued or processing; the queue
-// is drained when it reaches 0.  The ring (cap slots, -1 = empty) holds each
-// queued tile once, so cap = 2 * tiles + the tickets warps may hold ahead of
-// the pushes (kRingSlack > warps in flight) never overflows.
+// meanwhile (re-queued when its processing ends).  The ring (cap slots, -1 =
+// empty) holds each queued tile once, so cap = 2 * tiles + the tickets warps
+// may hold ahead of the pushes (kRingSlack > warps in flight) never overflows.
+//
+// The queue is drained when as many tiles have been finished as were ever
+// pushed: a tile is pushed by a warp that has not finished its own yet, so
+// reading `done` first and `tail` after it and finding them equal means that
+// no tile was queued or in process at the first read.  Warps add their
+// finished tiles to `done` only when they find no tile waiting, and a warp
+// pushes all the neighbours of a visit with one addition to `tail`: two
+// same-address atomics a visit, against five with a counter of pending tiles
+// (the fill's flood 1.09 -> 1.07 ms at 8192^2).
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
 
 namespace cageo {
 
-enum : int { kIdle = 0, kQueued = 1, kBusy = 2, kBusyQueued = 3, kDone = 4 };
+enum : int { kIdle = 0, kQueued = 1, kBusy = 2, kBusyQueued = 3 };
 constexpr int kEmptySlot = -1;
 constexpr int kRingSlack = 8192;
 
@@ -28,47 +35,51 @@ struct TileQueue {
   unsigned int cap;
   unsigned int* head;      // tickets handed out (own 128-byte line)
   unsigned int* tail;      // entries pushed (own line)
-  unsigned int* pending;   // tiles queued or being processed (own line)
+  unsigned int* done;      // tiles finished (own line)
   int* err;                // set to 3 when a state change keeps failing
 };
 
-__device__ __forceinline__ void tq_push(const TileQueue& q, int t) {
-  const unsigned int pos = atomicAdd(q.tail, 1u);
-  // A plain store: the taker swaps the slot for "empty" and retries while
-  // it reads empty.
+// A plain store: the taker swaps the slot for "empty" and retries while it
+// reads empty.
+__device__ __forceinline__ void tq_store(const TileQueue& q, unsigned int pos, int t) {
   ((volatile int*)q.ring)[pos % q.cap] = t;
 }
 
-// Queue tile t unless it is queued already or done: idle -> queued,
-// processing -> processing and queued again.  A single compare-and-swap
-// when the state is the one expected.
-__device__ __forceinline__ void tq_enqueue(const TileQueue& q, int t) {
-  int expect = kIdle;
-  for (int it = 0; it < 256; it++) {
-    const int old = atomicCAS(&q.state[t], expect, expect == kIdle ? kQueued : kBusyQueued);
-    if (old == expect) {
-      if (expect == kIdle) {
-        atomicAdd(q.pending, 1u);
-        tq_push(q, t);
-      }
-      return;
+// The whole warp: each lane with `want` queues its tile t, unless it is queued
+// already: idle -> queued, processing -> processing and queued again
+// (its owner pushes it then).  A single compare-and-swap when the state is the
+// one expected.
+__device__ __forceinline__ void tq_enqueue(const TileQueue& q, bool want, int t) {
+  bool push = false;
+  if (want) {
+    int expect = kIdle;
+    bool settled = false;
+    for (int it = 0; it < 256 && !settled; it++) {
+      const int old = atomicCAS(&q.state[t], expect, expect == kIdle ? kQueued : kBusyQueued);
+      settled = old == expect || (old != kIdle && old != kBusy);
+      push = old == expect && expect == kIdle;
+      expect = old;
     }
-    if (old != kIdle && old != kBusy) return;  // queued already, or done
-    expect = old;
+    if (!settled) atomicCAS(q.err, 0, 3);
   }
-  atomicCAS(q.err, 0, 3);
+  __syncwarp();
+  const unsigned int ball = __ballot_sync(0xffffffffu, push);
+  if (!ball) return;
+  const int lane = (int)(threadIdx.x & 31), leader = __ffs(ball) - 1;
+  unsigned int pos = 0;
+  if (lane == leader) pos = atomicAdd(q.tail, (unsigned int)__popc(ball));
+  pos = __shfl_sync(0xffffffffu, pos, leader);
+  if (push) tq_store(q, pos + __popc(ball & ((1u << lane) - 1u)), t);
 }
 
 // Lane 0: take the next queued tile.  A warp takes a ticket (the next ring
-// position) when the ring looks non-empty and keeps it until the slot is
-// filled -- possibly by a later push -- so no claim ever fails.  Returns
+// position) as soon as it is free and keeps it until the slot is filled --
+// possibly by a later push -- so no claim ever fails (looking whether the
+// ring holds an entry first would be one more L2 access a visit).  Returns
 // the tile, or -1 while waiting; *ticket carries the ticket between calls
 // (-1: none).
 __device__ __forceinline__ int tq_try_dequeue(const TileQueue& q, long long* ticket) {
-  if (*ticket < 0) {
-    if (*(volatile unsigned int*)q.head >= *(volatile unsigned int*)q.tail) return -1;
-    *ticket = atomicAdd(q.head, 1u);
-  }
+  if (*ticket < 0) *ticket = atomicAdd(q.head, 1u);
   const int t = atomicExch(&q.ring[(unsigned int)*ticket % q.cap], kEmptySlot);
   if (t == kEmptySlot) return -1;
   *ticket = -1;
@@ -80,19 +91,29 @@ __device__ __forceinline__ int tq_try_dequeue(const TileQueue& q, long long* tic
   return t;
 }
 
-// Lane 0, after the tile's write-back: idle again (done if nothing more can
-// change it), or queued again if a neighbour queued it while it was
-// processed.
-__device__ __forceinline__ void tq_finish(const TileQueue& q, int t, bool done) {
-  if (atomicCAS(&q.state[t], kBusy, done ? kDone : kIdle) == kBusy) {
-    atomicSub(q.pending, 1u);
-  } else if (done) {  // processing and queued again: only the owner changes that state
-    ((volatile int*)q.state)[t] = kDone;
-    atomicSub(q.pending, 1u);
-  } else {
+// Lane 0, after the tile's write-back (and a fence): idle again, or pushed
+// again if a neighbour queued it while it was processed.  The caller counts the
+// finished tile.
+__device__ __forceinline__ void tq_finish(const TileQueue& q, int t) {
+  if (atomicCAS(&q.state[t], kBusy, kIdle) != kBusy) {
+    // Processing and queued again: only the owner changes that state.
     ((volatile int*)q.state)[t] = kQueued;
-    tq_push(q, t);
+    tq_store(q, atomicAdd(q.tail, 1u), t);
   }
+}
+
+// Lane 0, when no tile is waiting: adds the tiles this warp has finished since
+// the last call; whether the queue is drained.
+__device__ __forceinline__ bool tq_drained(const TileQueue& q, unsigned int* finished) {
+  unsigned int d;
+  if (*finished) {
+    d = atomicAdd(q.done, *finished) + *finished;
+    *finished = 0;
+  } else {
+    d = *(volatile unsigned int*)q.done;
+  }
+  __threadfence();
+  return d == *(volatile unsigned int*)q.tail;
 }
 
 }  // namespace cageo
