@@ -41,11 +41,10 @@ struct FrontParams {
   float factor[kMaxBurnClasses + 1];  // factor[0] unused
 };
 
-// Writes one output of the fused front (cell i at column x, row y) from the
-// convolved value and the cell's DEM value and static code; returns q for
-// the min reduction.
-__device__ inline float front_epilogue(const FrontParams& p, int64_t i, int x, int y, float conv,
-                                       float dem, uint8_t c) {
+// One output of the fused front (column x, row y of this grid) from the
+// convolved value and the cell's DEM value and static code: the quantized
+// burned elevation.  Flags what the precomputed factors cannot cover.
+__device__ __forceinline__ float front_value(const FrontParams& p, float conv, float dem, uint8_t c) {
   float v = realistic_value(dem, conv, p.nodata_dem);
   if (c & kCodeBurnStream) {
     // The reference tests a stream neighbour's elevation against NODATA;
@@ -53,13 +52,17 @@ __device__ inline float front_epilogue(const FrontParams& p, int64_t i, int x, i
     if (v == p.nodata_dem) atomicExch(p.anomaly, 1);
     v = 0.0f;
   }
-  int k = c & 0x1f;
+  const int k = c & 0x1f;
   if (k) v = __fmul_rn(v, p.factor[k]);
-  float q = p.quantize ? fill_quantize(v, p.nodata_dem) : v;
-  p.q[i] = q;
-  if (q == 0.0f || x == 0 || y == 0 || x == p.W - 1 || y == p.H - 1)
-    p.tseed[((p.row0 + y) >> 5) * p.tiles_x + (x >> 5)] = 1;
-  return q;
+  return p.quantize ? fill_quantize(v, p.nodata_dem) : v;
+}
+
+// Whether the cell is an outlet of the pit fill, and the mark of its tile.
+__device__ __forceinline__ bool front_outlet(const FrontParams& p, int x, int y, float q) {
+  return q == 0.0f || x == 0 || y == 0 || x == p.W - 1 || y == p.H - 1;
+}
+__device__ __forceinline__ void front_seed(const FrontParams& p, int x, int y) {
+  p.tseed[((p.row0 + y) >> 5) * p.tiles_x + (x >> 5)] = 1;
 }
 
 }  // namespace cageo

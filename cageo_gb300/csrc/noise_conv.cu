@@ -6,6 +6,14 @@
 // add), so they equal ConvolutionAlgorithm_CPU_OpenMP bit for bit.  The
 // same kernels, instantiated with the FrontEpilogue, fuse the realistic-DEM,
 // burning and quantization steps of a realization into their store.
+//
+// What bounds them is the single-precision pipe: 2 taps products and 2 sums an
+// output, each rounded on its own.  Both are issued packed, two outputs of
+// neighbouring lines at a time (64-bit register pairs that the sliding windows
+// never take apart), so products, sums and loads each cost half an
+// instruction; results go through shared memory once more to be written in
+// 16-byte pieces along the rows.
+#include <algorithm>
 #include <type_traits>
 #include "common.cuh"
 #include "front.cuh"
@@ -80,28 +88,46 @@ __device__ __forceinline__ int wrap_idx(int v, int n) {
   return v;
 }
 
-// Epilogues: pre(i) loads what the output at i needs besides the
-// convolved value (issued before the convolution so the loads overlap it);
-// operator() writes the output.
+// Epilogues: what happens to the convolved values of a tile.  cell() takes one,
+// quad() four along a row at once (`aligned` says that it may: the grids then
+// start on 16-byte boundaries and W is a multiple of 4).  They return the least
+// of the values written.
 struct StoreEpilogue {
   float* out;
-  struct Pre {};
-  __device__ inline Pre pre(int64_t) const { return {}; }
-  __device__ inline float operator()(int64_t i, int, int, float v, Pre) const {
+  bool aligned;
+  __device__ __forceinline__ float cell(int64_t i, int, int, float v) const {
     out[i] = v;
     return v;
+  }
+  __device__ __forceinline__ float quad(int64_t i, int, int, float4 v) const {
+    *reinterpret_cast<float4*>(out + i) = v;
+    return 0.0f;
   }
 };
 
 struct FrontEpilogue {
   FrontParams p;
-  struct Pre {
-    float dem;
-    uint8_t code;
-  };
-  __device__ inline Pre pre(int64_t i) const { return {p.dem[i], p.code[i]}; }
-  __device__ inline float operator()(int64_t i, int x, int y, float v, Pre pr) const {
-    return front_epilogue(p, i, x, y, v, pr.dem, pr.code);
+  bool aligned;
+  __device__ __forceinline__ float cell(int64_t i, int x, int y, float v) const {
+    const float q = front_value(p, v, p.dem[i], p.code[i]);
+    p.q[i] = q;
+    if (front_outlet(p, x, y, q)) front_seed(p, x, y);
+    return q;
+  }
+  __device__ __forceinline__ float quad(int64_t i, int x, int y, float4 v) const {
+    const float4 d = *reinterpret_cast<const float4*>(p.dem + i);
+    const unsigned int c = *reinterpret_cast<const unsigned int*>(p.code + i);
+    float4 q;
+    q.x = front_value(p, v.x, d.x, (uint8_t)c);
+    q.y = front_value(p, v.y, d.y, (uint8_t)(c >> 8));
+    q.z = front_value(p, v.z, d.z, (uint8_t)(c >> 16));
+    q.w = front_value(p, v.w, d.w, (uint8_t)(c >> 24));
+    *reinterpret_cast<float4*>(p.q + i) = q;
+    // (The four cells lie in one fill tile: x is a multiple of 4.)
+    if (front_outlet(p, x, y, q.x) || front_outlet(p, x + 1, y, q.y) ||
+        front_outlet(p, x + 2, y, q.z) || front_outlet(p, x + 3, y, q.w))
+      front_seed(p, x, y);
+    return fminf(fminf(q.x, q.y), fminf(q.z, q.w));
   }
 };
 
@@ -125,153 +151,132 @@ __device__ inline void block_min_out(float local_min, const FrontEpilogue& e) {
   }
 }
 
-// a0 += w0 * t and a1 += w1 * t, each product and each sum rounded to
-// nearest on its own (as __fmul_rn / __fadd_rn, no contraction): the two
-// products as one packed single-precision multiply, the sums as scalar
-// __fadd_rn.  (A packed multiply feeding a packed add is contracted into a
-// fused multiply-add by the assembler, .rn notwithstanding: one rounding
-// fewer, different last bits.  A packed multiply feeding scalar adds, or
-// scalar multiplies feeding a packed add, keep both roundings; both were
-// checked against __fmul_rn + __fadd_rn over 4 M random operand pairs.)
-__device__ __forceinline__ void muladd2_rn(float& a0, float& a1, float w0, float w1, float t) {
-  float p0, p1;
-  asm("{\n\t.reg .b64 wa, tt;\n\t"
-      "mov.b64 wa, {%2, %3};\n\t"
-      "mov.b64 tt, {%4, %4};\n\t"
-      "mul.rn.f32x2 wa, wa, tt;\n\t"
-      "mov.b64 {%0, %1}, wa;\n\t}"
-      : "=f"(p0), "=f"(p1)
-      : "f"(w0), "f"(w1), "f"(t));
-  a0 = __fadd_rn(a0, p0);
-  a1 = __fadd_rn(a1, p1);
-}
-
-// 8 outputs along a line from a sliding window of 8 registers: out[j] =
-// sum_t v[j + t] * taps[t], t ascending, each sum starting at 0.  LC > 0:
-// the tap count is a compile-time constant and the loop is fully unrolled
-// (the window shifts become register renames); LC = 0: runtime count L.
-template <int LC>
-__device__ __forceinline__ void conv_line8(const float* __restrict__ v, int stride,
-                                           const float* __restrict__ taps, int L,
-                                           float acc[8]) {
-  float win[8];
-#pragma unroll
-  for (int j = 0; j < 8; j++) {
-    win[j] = v[j * stride];
-    acc[j] = 0.0f;
-  }
-  if (LC > 0) {
-#pragma unroll
-    for (int t = 0; t < LC; t++) {
-      const float tap = taps[t];
-#pragma unroll
-      for (int j = 0; j < 8; j += 2) muladd2_rn(acc[j], acc[j + 1], win[j], win[j + 1], tap);
-#pragma unroll
-      for (int j = 0; j < 7; j++) win[j] = win[j + 1];
-      if (t + 1 < LC) win[7] = v[(t + 8) * stride];
+// The tile's convolved values (rows of s_out, stride OS, a multiple of 4) into
+// the epilogue, consecutive threads along the rows.
+template <int TW, int TH, class Epi>
+__device__ __forceinline__ void tile_out(const float* s_out, int OS, int x0, int y0, int W, int H,
+                                         const Epi& epi) {
+  float local_min = kInf;
+  if (epi.aligned && x0 + TW <= W) {
+    constexpr int QW = TW / 4;
+#pragma unroll 2
+    for (int k = threadIdx.x; k < QW * TH; k += blockDim.x) {
+      const int y = k / QW, x = 4 * (k - y * QW);
+      if (y0 + y >= H) break;
+      const float4 v = *reinterpret_cast<const float4*>(s_out + y * OS + x);
+      local_min = fminf(local_min, epi.quad((int64_t)(y0 + y) * W + x0 + x, x0 + x, y0 + y, v));
     }
   } else {
-#pragma unroll 8
-    for (int t = 0; t < L; t++) {
-      const float tap = taps[t];
-#pragma unroll
-      for (int j = 0; j < 8; j += 2) muladd2_rn(acc[j], acc[j + 1], win[j], win[j + 1], tap);
-#pragma unroll
-      for (int j = 0; j < 7; j++) win[j] = win[j + 1];
-      win[7] = (t + 1 < L) ? v[(t + 8) * stride] : 0.0f;
+    for (int k = threadIdx.x; k < TW * TH; k += blockDim.x) {
+      const int y = k / TW, x = k - y * TW;
+      if (y0 + y >= H) break;
+      if (x0 + x < W)
+        local_min = fminf(local_min, epi.cell((int64_t)(y0 + y) * W + x0 + x, x0 + x, y0 + y,
+                                              s_out[y * OS + x]));
     }
   }
+  block_min_out(local_min, epi);
 }
 
-// p0 = w0 * t and p1 = w1 * t, each rounded to nearest, as one packed
-// single-precision multiply.
-__device__ __forceinline__ void mul2_rn(float& p0, float& p1, float w0, float w1, float t) {
-  asm("{\n\t.reg .b64 wa, tt;\n\t"
-      "mov.b64 wa, {%2, %3};\n\t"
-      "mov.b64 tt, {%4, %4};\n\t"
-      "mul.rn.f32x2 wa, wa, tt;\n\t"
-      "mov.b64 {%0, %1}, wa;\n\t}"
-      : "=f"(p0), "=f"(p1)
-      : "f"(w0), "f"(w1), "f"(t));
+// Packed pairs of floats.  acc + w * t with the product and the sum each
+// rounded to nearest (as __fmul_rn and __fadd_rn, no contraction): a packed
+// multiply, and the packed sum as fma(product, 1, acc) with a 1 the compiler
+// cannot see -- the assembler contracts a packed multiply feeding a packed add
+// into one rounding, .rn notwithstanding; the product with 1 is exact, so this
+// fused operation rounds the sum alone.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f32x2 muladd2_rn(f32x2 acc, f32x2 w, f32x2 t, f32x2 one) {
+  f32x2 p;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(p) : "l"(w), "l"(t));
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(p) : "l"(p), "l"(one), "l"(acc));
+  return p;
 }
 
-// conv_line8 for two lines at once (v0, v1; same stride and taps): the
-// window values of the two lines at one position are multiplied as one
-// packed pair, and the two windows shift together, so the pairs stay put
-// in registers.  ADJ: the lines are adjacent columns (v1 = v0 + 1, v0
-// 8-byte aligned), loaded as one float2.  Each sum runs over t ascending,
-// as in conv_line8.
-template <int LC, bool ADJ>
-__device__ __forceinline__ void conv_line8x2(const float* __restrict__ v0,
-                                             const float* __restrict__ v1, int stride,
-                                             const float* __restrict__ taps, int L,
-                                             float a0[8], float a1[8]) {
-  float w0[8], w1[8];
-  auto load = [&](int k, float& x0, float& x1) {
-    if (ADJ) {
-      const float2 p = *reinterpret_cast<const float2*>(v0 + k * stride);
-      x0 = p.x;
-      x1 = p.y;
-    } else {
-      x0 = v0[k * stride];
-      x1 = v1[k * stride];
-    }
-  };
+// 8 outputs along a line for two neighbouring lines at once: acc[j] = sum_t
+// v(j + t) * tap(t), t ascending, each sum starting at 0.  The window of 8
+// pairs is a ring of registers: tap t + u of a group of 8 finds output j's
+// value at (j + u) % 8 and replaces entry u.  LC > 0: the tap count is a
+// compile-time constant; LC = 0: runtime count L.
+template <int LC, class V, class Tap>
+__device__ __forceinline__ void conv_line8(int L, f32x2 one, V v, Tap tap, f32x2 (&acc)[8]) {
+  f32x2 win[8];
 #pragma unroll
   for (int j = 0; j < 8; j++) {
-    load(j, w0[j], w1[j]);
-    a0[j] = 0.0f;
-    a1[j] = 0.0f;
+    win[j] = v(j);
+    acc[j] = 0;
   }
-  auto tap_step = [&](float tap) {
+  const int n = LC > 0 ? LC : L;
+#pragma unroll(LC > 0 ? (LC + 7) / 8 : 1)
+  for (int t = 0; t < n; t += 8) {
 #pragma unroll
-    for (int j = 0; j < 8; j++) {
-      float p0, p1;
-      mul2_rn(p0, p1, w0[j], w1[j], tap);
-      a0[j] = __fadd_rn(a0[j], p0);
-      a1[j] = __fadd_rn(a1[j], p1);
-    }
+    for (int u = 0; u < 8; u++) {
+      if (t + u < n) {
+        const f32x2 w = tap(t + u);
 #pragma unroll
-    for (int j = 0; j < 7; j++) {
-      w0[j] = w0[j + 1];
-      w1[j] = w1[j + 1];
-    }
-  };
-  if (LC > 0) {
-#pragma unroll
-    for (int t = 0; t < LC; t++) {
-      tap_step(taps[t]);
-      if (t + 1 < LC) load(t + 8, w0[7], w1[7]);
-    }
-  } else {
-#pragma unroll 4
-    for (int t = 0; t < L; t++) {
-      tap_step(taps[t]);
-      if (t + 1 < L) load(t + 8, w0[7], w1[7]);
+        for (int j = 0; j < 8; j++) acc[j] = muladd2_rn(acc[j], win[(j + u) & 7], w, one);
+        if (t + u + 1 < n) win[u] = v(t + u + 8);
+      }
     }
   }
 }
 
+// Staged columns left and right of the tile: the radius, rounded up so that
+// rows start on a 16-byte boundary.
+__host__ __device__ inline int sep_pad(int r) { return (r + 3) & ~3; }
+
+// Blocks per SM the registers are held to: 5 (at 8192^2, radius 15, 64 x 32
+// tiles: 0.58 ms; 4: 0.61), but 4 for radius 23, whose longer unrolled lines
+// would spill (16384^2: 3.14 ms; 5: 3.27).  128 or 192 threads, or 6 blocks,
+// are slower for both.  The lines are unrolled for these two radii (the
+// runtime loop takes 0.61 and 3.5 ms).
 template <class Epi, int LC, int TW, int TH>
-__global__ void __launch_bounds__(kSepThreads)
+__global__ void __launch_bounds__(kSepThreads, LC == 47 ? 4 : 5)
 conv_sep_kernel(const float* __restrict__ in, int W, int H,
-                const float* __restrict__ taps, int r, Epi epi) {
+                const float* __restrict__ taps, int r, float one, Epi epi) {
   static_assert(TW % 8 == 0 && TH % 8 == 0, "items are 8 outputs wide / 8 rows tall");
-  extern __shared__ float sm[];
-  const int L = 2 * r + 1;
-  const int IW = TW + 2 * r, IH = TH + 2 * r;
-  float* s_taps = sm;
-  float* s_in = sm + ((L + 3) & ~3);
-  float* s_tmp = s_in + IW * IH;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const int L = 2 * r + 1, rp = sep_pad(r);
+  const int IW = TW + 2 * rp, IH = TH + 2 * r, TS = IW + 1;
+  f32x2* s_taps = reinterpret_cast<f32x2*>(smraw);                          // (tap, tap)
+  float* s_in = reinterpret_cast<float*>(s_taps + ((L + 1) & ~1));  // IH x IW, then the outputs
+  const int in_floats = IH * IW > TH * (TW + 4) ? IH * IW : TH * (TW + 4);
+  f32x2* s_tmp = reinterpret_cast<f32x2*>(s_in + in_floats);        // TH/2 x TS: rows 2j, 2j + 1
   const int x0 = blockIdx.x * TW, y0 = blockIdx.y * TH;
-  for (int t = threadIdx.x; t < L; t += blockDim.x) s_taps[t] = taps[t];
-  {
-    // Row and column of this thread's element, stepped by blockDim.x.
+  const f32x2 one2 = pack2(one, one);
+  for (int t = threadIdx.x; t < L; t += kSepThreads) {
+    const float v = taps[t];
+    s_taps[t] = pack2(v, v);
+  }
+  if (x0 >= rp && x0 + TW + rp <= W && (W & 3) == 0 && ((uintptr_t)in & 15u) == 0) {
+    // No column wraps: 16-byte copies.
+    const int CW = IW / 4;
+    int iy = threadIdx.x / CW, ic = threadIdx.x - iy * CW;
+    const int dy = kSepThreads / CW, dc = kSepThreads - dy * CW;
+#pragma unroll 2
+    for (int k = threadIdx.x; k < IH * CW; k += kSepThreads) {
+      const int gy = wrap_idx(y0 - r + iy, H);
+      cp_async16(s_in + 4 * k, in + (int64_t)gy * W + x0 - rp + 4 * ic);
+      iy += dy;
+      ic += dc;
+      if (ic >= CW) {
+        ic -= CW;
+        iy++;
+      }
+    }
+  } else {
     int iy = threadIdx.x / IW, ix = threadIdx.x - iy * IW;
-    const int dy = blockDim.x / IW, dx = blockDim.x - dy * IW;
+    const int dy = kSepThreads / IW, dx = kSepThreads - dy * IW;
 #pragma unroll 4
-    for (int idx = threadIdx.x; idx < IW * IH; idx += blockDim.x) {
-      const int gy = wrap_idx(y0 - r + iy, H), gx = wrap_idx(x0 - r + ix, W);
+    for (int idx = threadIdx.x; idx < IW * IH; idx += kSepThreads) {
+      const int gy = wrap_idx(y0 - r + iy, H), gx = wrap_idx(x0 - rp + ix, W);
       cp_async4(&s_in[idx], &in[(int64_t)gy * W + gx]);  // all of them in flight at once
       iy += dy;
       ix += dx;
@@ -280,70 +285,96 @@ conv_sep_kernel(const float* __restrict__ in, int W, int H,
         iy++;
       }
     }
-    cp_async_wait();
   }
+  cp_async_wait();
   __syncthreads();
-  // Column pass: tmp[y][ix] = sum_t in[y+t][ix] * taps[t]; an item is 8
-  // rows of two adjacent columns (IW is even).
-  const int IW2 = IW / 2;
-  for (int item = threadIdx.x; item < IW2 * (TH / 8); item += blockDim.x) {
-    const int g = item / IW2, ix = 2 * (item - g * IW2);
-    float a0[8], a1[8];
-    conv_line8x2<LC, true>(s_in + (8 * g) * IW + ix, nullptr, IW, s_taps, L, a0, a1);
+  // Column pass: tmp[y][ix] = sum_t in[y+t][ix] * taps[t]; an item is 8 rows
+  // of two adjacent columns.  The results are kept as pairs of rows, which is
+  // what the row pass multiplies; its row stride is odd, so 16 row pairs are
+  // read without bank conflicts.
+  const int p0 = (rp - r) >> 1, np = ((rp + TW + r + 1) >> 1) - p0;
+  for (int item = threadIdx.x; item < np * (TH / 8); item += kSepThreads) {
+    const int g = item / np, ix = 2 * (p0 + item - g * np);
+    const float* base = s_in + (8 * g) * IW + ix;
+    f32x2 acc[8];
+    conv_line8<LC>(L, one2,
+                   [&](int k) { return *reinterpret_cast<const f32x2*>(base + k * IW); },
+                   [&](int t) { return s_taps[t]; }, acc);
 #pragma unroll
-    for (int j = 0; j < 8; j++)
-      *reinterpret_cast<float2*>(&s_tmp[(8 * g + j) * IW + ix]) = make_float2(a0[j], a1[j]);
-  }
-  __syncthreads();
-  // Row pass (8 consecutive outputs per item) and store.
-  float local_min = kInf;
-  for (int item = threadIdx.x; item < TH * (TW / 8); item += blockDim.x) {
-    const int y = item / (TW / 8), g = item - y * (TW / 8);
-    const int gy = y0 + y;
-    typename Epi::Pre pre[8];
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-      const int gx = x0 + 8 * g + j;
-      if (gy < H && gx < W) pre[j] = epi.pre((int64_t)gy * W + gx);
-    }
-    float acc[8];
-    conv_line8<LC>(s_tmp + y * IW + 8 * g, 1, s_taps, L, acc);
-    if (gy >= H) continue;
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-      const int gx = x0 + 8 * g + j;
-      if (gx < W) local_min = fminf(local_min, epi((int64_t)gy * W + gx, gx, gy, acc[j], pre[j]));
+    for (int j = 0; j < 4; j++) {
+      float a0, a1, b0, b1;
+      unpack2(acc[2 * j], a0, a1);
+      unpack2(acc[2 * j + 1], b0, b1);
+      f32x2* o = s_tmp + (4 * g + j) * TS + ix;
+      o[0] = pack2(a0, b0);
+      o[1] = pack2(a1, b1);
     }
   }
-  block_min_out(local_min, epi);
+  __syncthreads();
+  // Row pass: an item is 8 consecutive outputs of two rows.
+  constexpr int OS = TW + 4;
+  float* s_out = s_in;
+  for (int item = threadIdx.x; item < (TH / 2) * (TW / 8); item += kSepThreads) {
+    const int g = item / (TH / 2), j = item - g * (TH / 2);
+    const f32x2* base = s_tmp + j * TS + 8 * g + (rp - r);
+    f32x2 acc[8];
+    conv_line8<LC>(L, one2, [&](int k) { return base[k]; }, [&](int t) { return s_taps[t]; }, acc);
+    float* o = s_out + 2 * j * OS + 8 * g;
+#pragma unroll
+    for (int k = 0; k < 8; k++) unpack2(acc[k], o[k], o[OS + k]);
+  }
+  __syncthreads();
+  tile_out<TW, TH>(s_out, OS, x0, y0, W, H, epi);
 }
 
 // ---- A3 full 2D (exponential) -----------------------------------------------
-// A block computes a 64 x 32 tile; a thread 8 consecutive outputs of one row
-// from a sliding window of 8 registers, so each tap costs one shared-memory
-// load of input (and a broadcast load of the tap) per 8 outputs.  Each
-// output's sum runs over the filter rows, and inside a row over its taps,
-// in ascending order, as the reference's 2D loop does.
-constexpr int kTwoDTW = 64, kTwoDTH = 32, kTwoDThreads = 256;
+// A block computes a 64 x TH tile; a thread 8 consecutive outputs of rows j and
+// j + TH/2 as packed pairs from a sliding window.  PAIRED: the input is staged
+// as those pairs and the taps twice, so a tap costs one load of input and one
+// broadcast load of the tap per 16 outputs; larger filters, whose pairs would
+// not fit shared memory, load the two rows and pack the tap.  Lane = row, and
+// the row stride is odd: no bank conflicts.
+// Each output's sum runs over the filter rows, and inside a row over its taps,
+// in ascending order, as the reference's 2D loop does.  TH = 64 where the grid
+// then still has 8 tiles per SM to balance; 32 otherwise.
+constexpr int kTwoDTW = 64;
+constexpr int kTwoDBlocks = 8 * 152;
+constexpr int kTwoDPairedRadius = 31;
 
-template <class Epi>
-__global__ void __launch_bounds__(kTwoDThreads)
+template <class Epi, int TH, bool PAIRED>
+__global__ void __launch_bounds__(4 * TH)
 conv_2d_kernel(const float* __restrict__ in, int W, int H,
-               const float* __restrict__ filt, int r, Epi epi) {
-  extern __shared__ float sm[];
+               const float* __restrict__ filt, int r, float one, Epi epi) {
+  constexpr int NT = 4 * TH, NP = TH / 2;
+  extern __shared__ __align__(16) unsigned char smraw[];
   const int L = 2 * r + 1;
-  const int IW = kTwoDTW + 2 * r, IH = kTwoDTH + 2 * r;
-  float* s_f = sm;
-  float* s_in = sm + ((L * L + 3) & ~3);
-  const int x0 = blockIdx.x * kTwoDTW, y0 = blockIdx.y * kTwoDTH;
-  for (int t = threadIdx.x; t < L * L; t += blockDim.x) s_f[t] = filt[t];
+  const int IW = kTwoDTW + 2 * r, IH = TH + 2 * r, S = IW | 1;
+  float* s_f = reinterpret_cast<float*>(smraw);
+  f32x2* s_f2 = reinterpret_cast<f32x2*>(smraw);
+  unsigned char* rows = smraw + sizeof(float) * (((PAIRED ? 2 : 1) * L * L + 3) & ~3);
+  f32x2* s_in2 = reinterpret_cast<f32x2*>(rows);  // PAIRED: rows y, y + NP
+  float* s_in = reinterpret_cast<float*>(rows);
+  const f32x2 one2 = pack2(one, one);
+  const int x0 = blockIdx.x * kTwoDTW, y0 = blockIdx.y * TH;
+  for (int t = threadIdx.x; t < L * L; t += NT) {
+    const float v = filt[t];
+    if (PAIRED) s_f2[t] = pack2(v, v);
+    else s_f[t] = v;
+  }
   {
     int iy = threadIdx.x / IW, ix = threadIdx.x - iy * IW;
-    const int dy = blockDim.x / IW, dx = blockDim.x - dy * IW;
+    const int dy = NT / IW, dx = NT - dy * IW;
 #pragma unroll 4
-    for (int idx = threadIdx.x; idx < IW * IH; idx += blockDim.x) {
+    for (int idx = threadIdx.x; idx < IW * IH; idx += NT) {
       const int gy = wrap_idx(y0 - r + iy, H), gx = wrap_idx(x0 - r + ix, W);
-      cp_async4(&s_in[idx], &in[(int64_t)gy * W + gx]);  // all of them in flight at once
+      const float* src = &in[(int64_t)gy * W + gx];
+      if (PAIRED) {  // all of them in flight at once
+        float* d = reinterpret_cast<float*>(s_in2 + iy * S + ix);
+        if (iy < NP + 2 * r) cp_async4(d, src);
+        if (iy >= NP) cp_async4(d - 2 * NP * S + 1, src);
+      } else {
+        cp_async4(&s_in[iy * S + ix], src);
+      }
       iy += dy;
       ix += dx;
       if (ix >= IW) {
@@ -354,53 +385,63 @@ conv_2d_kernel(const float* __restrict__ in, int W, int H,
     cp_async_wait();
   }
   __syncthreads();
-  const int ox = 8 * (threadIdx.x & 7), ty = threadIdx.x >> 3;
-  const int gy = y0 + ty;
-  typename Epi::Pre pre[8];
+  const int j = threadIdx.x % NP, g = threadIdx.x / NP;
+  f32x2 acc[8];
 #pragma unroll
-  for (int j = 0; j < 8; j++) {
-    const int gx = x0 + ox + j;
-    if (gy < H && gx < W) pre[j] = epi.pre((int64_t)gy * W + gx);
-  }
-  float acc[8];
-#pragma unroll
-  for (int j = 0; j < 8; j++) acc[j] = 0.0f;
+  for (int k = 0; k < 8; k++) acc[k] = 0;
   for (int fy = 0; fy < L; fy++) {
-    const float* row = s_in + (ty + fy) * IW + ox;
-    const float* frow = s_f + fy * L;
-    float win[8];
+    const int f = fy * L, o = (j + fy) * S + 8 * g;
+    auto tap = [&](int t) { return PAIRED ? s_f2[f + t] : pack2(s_f[f + t], s_f[f + t]); };
+    auto value = [&](int k) { return PAIRED ? s_in2[o + k] : pack2(s_in[o + k], s_in[o + NP * S + k]); };
+    f32x2 win[8];
 #pragma unroll
-    for (int j = 0; j < 8; j++) win[j] = row[j];
-#pragma unroll 8
-    for (int fx = 0; fx < L; fx++) {
-      const float f = frow[fx];
+    for (int k = 0; k < 8; k++) win[k] = value(k);
+    int t = 0;
+#pragma unroll 1
+    for (; t + 8 < L; t += 8) {
 #pragma unroll
-      for (int j = 0; j < 8; j += 2) muladd2_rn(acc[j], acc[j + 1], win[j], win[j + 1], f);
+      for (int u = 0; u < 8; u++) {
+        const f32x2 w = tap(t + u);
 #pragma unroll
-      for (int j = 0; j < 7; j++) win[j] = win[j + 1];
-      win[7] = (fx + 1 < L) ? row[fx + 8] : 0.0f;
+        for (int k = 0; k < 8; k++) acc[k] = muladd2_rn(acc[k], win[(k + u) & 7], w, one2);
+        win[u] = value(t + u + 8);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+      if (t + u >= L) break;
+      const f32x2 w = tap(t + u);
+#pragma unroll
+      for (int k = 0; k < 8; k++) acc[k] = muladd2_rn(acc[k], win[(k + u) & 7], w, one2);
+      if (t + u + 1 < L) win[u] = value(t + u + 8);
     }
   }
-  float local_min = kInf;
-  if (gy < H) {
+  __syncthreads();
+  constexpr int OS = kTwoDTW + 4;
+  float* s_out = s_in;
 #pragma unroll
-    for (int j = 0; j < 8; j++) {
-      const int gx = x0 + ox + j;
-      if (gx < W) local_min = fminf(local_min, epi((int64_t)gy * W + gx, gx, gy, acc[j], pre[j]));
-    }
-  }
-  block_min_out(local_min, epi);
+  for (int k = 0; k < 8; k++)
+    unpack2(acc[k], s_out[j * OS + 8 * g + k], s_out[(j + NP) * OS + 8 * g + k]);
+  __syncthreads();
+  tile_out<kTwoDTW, TH>(s_out, OS, x0, y0, W, H, epi);
+}
+
+size_t conv_2d_smem_bytes(int r, int th) {
+  const int L = 2 * r + 1, S = (kTwoDTW + 2 * r) | 1;
+  const bool paired = r <= kTwoDPairedRadius;
+  return sizeof(float) * ((((paired ? 2 : 1) * L * L + 3) & ~3) +
+                          std::max((size_t)(paired ? th + 4 * r : th + 2 * r) * S,
+                                   (size_t)th * (kTwoDTW + 4)));
 }
 
 size_t conv_smem_bytes(int model, int r, int tile) {
-  int L = 2 * r + 1;
-  if (model == CAGEO_FILTER_GAUSSIAN) {
-    const SepTile t = kSepTiles[tile];
-    int IW = t.tw + 2 * r, IH = t.th + 2 * r;
-    return sizeof(float) * (((L + 3) & ~3) + (size_t)IW * IH + (size_t)IW * t.th);
-  }
-  int IW = kTwoDTW + 2 * r, IH = kTwoDTH + 2 * r;
-  return sizeof(float) * (((L * L + 3) & ~3) + (size_t)IW * IH);
+  if (model != CAGEO_FILTER_GAUSSIAN) return conv_2d_smem_bytes(r, 32);
+  const int L = 2 * r + 1;
+  const SepTile t = kSepTiles[tile];
+  const int IW = t.tw + 2 * sep_pad(r), IH = t.th + 2 * r;
+  return sizeof(float) * (2 * ((L + 1) & ~1) +
+                          std::max((size_t)IW * IH, (size_t)t.th * (t.tw + 4)) +
+                          (size_t)t.th * (IW + 1));
 }
 
 // Whether a tile shape of the fused front applies: Gaussian filters (the
@@ -418,7 +459,7 @@ bool conv_tile_applies(int model, int r, int tile) {
 // The separable kernel for a tile shape and radius: fully unrolled for the
 // 60 m and 90 m ranges at 10 m cells (radius 15 and 23).
 template <class Epi>
-using SepKernel = void (*)(const float*, int, int, const float*, int, Epi);
+using SepKernel = void (*)(const float*, int, int, const float*, int, float, Epi);
 
 template <class Epi, int TW, int TH>
 SepKernel<Epi> sep_kernel_for(int r) {
@@ -460,8 +501,8 @@ cageo_status launch_conv(const float* in, int W, int H, int model,
     CAGEO_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, *limit));
     return CAGEO_OK;
   };
-  const size_t smem = conv_smem_bytes(model, r, tile);
   if (model == CAGEO_FILTER_GAUSSIAN) {
+    const size_t smem = conv_smem_bytes(model, r, tile);
     const SepKernel<Epi> fn = sep_kernel<Epi>(r, tile);
     int limit = 0;
     cageo_status st = raise_limit((const void*)fn, &limit);
@@ -472,17 +513,28 @@ cageo_status launch_conv(const float* in, int W, int H, int model,
     }
     const SepTile t = kSepTiles[tile];
     dim3 grid((W + t.tw - 1) / t.tw, (H + t.th - 1) / t.th);
-    fn<<<grid, kSepThreads, smem, s>>>(in, W, H, filt, r, epi);
+    fn<<<grid, kSepThreads, smem, s>>>(in, W, H, filt, r, 1.0f, epi);
   } else {
-    int limit = 0;
-    cageo_status st = raise_limit((const void*)conv_2d_kernel<Epi>, &limit);
-    if (st) return st;
-    if (smem > (size_t)limit) {
-      set_error("filter radius %d needs %zu bytes of shared memory (%d available)", r, smem, limit);
-      return CAGEO_ERR_ARGUMENT;
+    using Kernel = SepKernel<Epi>;
+    const bool paired = r <= kTwoDPairedRadius;
+    const int gx = (W + kTwoDTW - 1) / kTwoDTW;
+    int th = gx * ((H + 63) / 64) >= kTwoDBlocks ? 64 : 32, limit = 0;
+    for (;; th = 32) {
+      const Kernel fn = th == 64 ? (paired ? (Kernel)conv_2d_kernel<Epi, 64, true>
+                                        : (Kernel)conv_2d_kernel<Epi, 64, false>)
+                                 : (paired ? (Kernel)conv_2d_kernel<Epi, 32, true>
+                                        : (Kernel)conv_2d_kernel<Epi, 32, false>);
+      cageo_status st = raise_limit((const void*)fn, &limit);
+      if (st) return st;
+      const size_t bytes = conv_2d_smem_bytes(r, th);
+      if (bytes > (size_t)limit && th == 64) continue;
+      if (bytes > (size_t)limit) {
+        set_error("filter radius %d needs %zu bytes of shared memory (%d available)", r, bytes, limit);
+        return CAGEO_ERR_ARGUMENT;
+      }
+      fn<<<dim3(gx, (H + th - 1) / th), 4 * th, bytes, s>>>(in, W, H, filt, r, 1.0f, epi);
+      break;
     }
-    dim3 grid((W + kTwoDTW - 1) / kTwoDTW, (H + kTwoDTH - 1) / kTwoDTH);
-    conv_2d_kernel<Epi><<<grid, kTwoDThreads, smem, s>>>(in, W, H, filt, r, epi);
   }
   CAGEO_CUDA(cudaGetLastError());
   return CAGEO_OK;
@@ -503,7 +555,8 @@ cageo_status launch_noise(float* d, int64_t n, uint64_t seed, uint32_t realizati
 cageo_status launch_front(const float* noise, int W, int H, int model,
                           const float* filt, int r, const FrontParams& fp,
                           cudaStream_t s, int tile) {
-  FrontEpilogue e{fp};
+  const uintptr_t ptrs = (uintptr_t)fp.dem | (uintptr_t)fp.q;
+  FrontEpilogue e{fp, (W & 3) == 0 && (ptrs & 15u) == 0 && ((uintptr_t)fp.code & 3u) == 0};
   return launch_conv(noise, W, H, model, filt, r, e, s, tile);
 }
 
@@ -555,6 +608,6 @@ extern "C" cageo_status cageo_convolve(const float* d_in, float* d_out, int W,
                   "filter model");
   CAGEO_CHECK_ARG(radius >= 0 && radius < W && radius < H,
                   "filter radius must be below the grid width and height");
-  StoreEpilogue e{d_out};
+  StoreEpilogue e{d_out, (W & 3) == 0 && ((uintptr_t)d_out & 15u) == 0};
   return launch_conv(d_in, W, H, model, d_filter, radius, e, stream);
 }
