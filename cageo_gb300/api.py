@@ -401,8 +401,8 @@ class Pipeline:
         _check(lib().cageo_pipeline_run(self._p, first, count))
 
     def set_batch(self, batch):
-        """Realizations per batched step (1: one at a time); see
-        cageo_pipeline_set_batch."""
+        """Realizations per stacked step (1: one at a time; by default small grids
+        are stacked by themselves); see cageo_pipeline_set_batch."""
         _check(lib().cageo_pipeline_set_batch(self._p, int(batch)))
 
     def run_filter(self, first, count, filter_model, practical_range, error_mean, error_stddev):

@@ -27,9 +27,9 @@ constexpr int kConvTiles = 4;
 struct FrontParams {
   const float* dem;        // W*H
   const uint8_t* code;     // W*H static codes
-  float* q;                // W*H output: quantized burned realistic DEM
-  unsigned int* min_ord;   // ordered-uint min of q (pit-fill minE)
-  int* anomaly;            // set when the precomputed burn factor may not apply
+  float* q;                // W*H output: quantized burned realistic DEM (of a stack's first grid)
+  unsigned int* min_ord;   // ordered-uint min of q (pit-fill minE), one per grid of a stack
+  int* anomaly;            // set when the precomputed burn factor may not apply (per grid of a stack)
   float nodata_dem;
   int quantize;            // 1: the CPU fill's 1 mm quantization; 0: raw (exact fill)
   // The pit fill's seeds: a tile holding an outlet (a border cell or a cell

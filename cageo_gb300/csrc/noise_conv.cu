@@ -31,6 +31,9 @@ __global__ void noise_kernel(float* __restrict__ out, int64_t n, uint32_t k0,
   int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t base = g * 4;
   if (base >= n) return;
+  // blockIdx.y: the field of a stack, one realization further each.
+  out += blockIdx.y * n;
+  realization += blockIdx.y;
   if (dreal) realization += *dreal;  // an offset from the device counter
   U4 ctr = {(uint32_t)g, realization, kNoiseTag, (uint32_t)(g >> 32)};
   U4 r = philox4x32_10(ctr, k0, k1);
@@ -95,6 +98,7 @@ __device__ __forceinline__ int wrap_idx(int v, int n) {
 struct StoreEpilogue {
   float* out;
   bool aligned;
+  __device__ __forceinline__ void slab(int, int64_t) {}
   __device__ __forceinline__ float cell(int64_t i, int, int, float v) const {
     out[i] = v;
     return v;
@@ -108,6 +112,12 @@ struct StoreEpilogue {
 struct FrontEpilogue {
   FrontParams p;
   bool aligned;
+  __device__ __forceinline__ void slab(int k, int64_t n) {
+    p.q += k * n;
+    p.min_ord += k;
+    p.anomaly += k;
+    p.row0 += k * p.H;
+  }
   __device__ __forceinline__ float cell(int64_t i, int x, int y, float v) const {
     const float q = front_value(p, v, p.dem[i], p.code[i]);
     p.q[i] = q;
@@ -250,6 +260,8 @@ conv_sep_kernel(const float* __restrict__ in, int W, int H,
   const int in_floats = IH * IW > TH * (TW + 4) ? IH * IW : TH * (TW + 4);
   f32x2* s_tmp = reinterpret_cast<f32x2*>(s_in + in_floats);        // TH/2 x TS: rows 2j, 2j + 1
   const int x0 = blockIdx.x * TW, y0 = blockIdx.y * TH;
+  in += blockIdx.z * (int64_t)W * H;  // a field of a stack
+  epi.slab(blockIdx.z, (int64_t)W * H);
   const f32x2 one2 = pack2(one, one);
   for (int t = threadIdx.x; t < L; t += kSepThreads) {
     const float v = taps[t];
@@ -356,6 +368,8 @@ conv_2d_kernel(const float* __restrict__ in, int W, int H,
   float* s_in = reinterpret_cast<float*>(rows);
   const f32x2 one2 = pack2(one, one);
   const int x0 = blockIdx.x * kTwoDTW, y0 = blockIdx.y * TH;
+  in += blockIdx.z * (int64_t)W * H;  // a field of a stack
+  epi.slab(blockIdx.z, (int64_t)W * H);
   for (int t = threadIdx.x; t < L * L; t += NT) {
     const float v = filt[t];
     if (PAIRED) s_f2[t] = pack2(v, v);
@@ -483,7 +497,7 @@ SepKernel<Epi> sep_kernel(int r, int tile) {
 template <class Epi>
 cageo_status launch_conv(const float* in, int W, int H, int model,
                          const float* filt, int r, const Epi& epi,
-                         cudaStream_t s, int tile = 0) {
+                         cudaStream_t s, int tile = 0, int slabs = 1) {
   if (!std::is_same<Epi, FrontEpilogue>::value || tile < 0 || tile >= kConvTiles) tile = 0;
   // The kernels' dynamic shared-memory limit is raised to the most the
   // device allows (its opt-in maximum less the kernel's static shared
@@ -512,13 +526,13 @@ cageo_status launch_conv(const float* in, int W, int H, int model,
       return CAGEO_ERR_ARGUMENT;
     }
     const SepTile t = kSepTiles[tile];
-    dim3 grid((W + t.tw - 1) / t.tw, (H + t.th - 1) / t.th);
+    dim3 grid((W + t.tw - 1) / t.tw, (H + t.th - 1) / t.th, slabs);
     fn<<<grid, kSepThreads, smem, s>>>(in, W, H, filt, r, 1.0f, epi);
   } else {
     using Kernel = SepKernel<Epi>;
     const bool paired = r <= kTwoDPairedRadius;
     const int gx = (W + kTwoDTW - 1) / kTwoDTW;
-    int th = gx * ((H + 63) / 64) >= kTwoDBlocks ? 64 : 32, limit = 0;
+    int th = (int64_t)slabs * gx * ((H + 63) / 64) >= kTwoDBlocks ? 64 : 32, limit = 0;
     for (;; th = 32) {
       const Kernel fn = th == 64 ? (paired ? (Kernel)conv_2d_kernel<Epi, 64, true>
                                         : (Kernel)conv_2d_kernel<Epi, 64, false>)
@@ -532,7 +546,7 @@ cageo_status launch_conv(const float* in, int W, int H, int model,
         set_error("filter radius %d needs %zu bytes of shared memory (%d available)", r, bytes, limit);
         return CAGEO_ERR_ARGUMENT;
       }
-      fn<<<dim3(gx, (H + th - 1) / th), 4 * th, bytes, s>>>(in, W, H, filt, r, 1.0f, epi);
+      fn<<<dim3(gx, (H + th - 1) / th, slabs), 4 * th, bytes, s>>>(in, W, H, filt, r, 1.0f, epi);
       break;
     }
   }
@@ -541,11 +555,11 @@ cageo_status launch_conv(const float* in, int W, int H, int model,
 }
 
 cageo_status launch_noise(float* d, int64_t n, uint64_t seed, uint32_t realization,
-                          const uint32_t* dreal, float mean, float sd, cudaStream_t s) {
+                          const uint32_t* dreal, float mean, float sd, cudaStream_t s, int slabs) {
   int64_t groups = (n + 3) / 4;
   int threads = 256;
   int64_t blocks = (groups + threads - 1) / threads;
-  noise_kernel<<<(unsigned)blocks, threads, 0, s>>>(d, n, (uint32_t)seed,
+  noise_kernel<<<dim3((unsigned)blocks, slabs), threads, 0, s>>>(d, n, (uint32_t)seed,
                                                     (uint32_t)(seed >> 32), realization,
                                                     dreal, mean, sd);
   CAGEO_CUDA(cudaGetLastError());
@@ -554,10 +568,10 @@ cageo_status launch_noise(float* d, int64_t n, uint64_t seed, uint32_t realizati
 
 cageo_status launch_front(const float* noise, int W, int H, int model,
                           const float* filt, int r, const FrontParams& fp,
-                          cudaStream_t s, int tile) {
+                          cudaStream_t s, int tile, int slabs) {
   const uintptr_t ptrs = (uintptr_t)fp.dem | (uintptr_t)fp.q;
   FrontEpilogue e{fp, (W & 3) == 0 && (ptrs & 15u) == 0 && ((uintptr_t)fp.code & 3u) == 0};
-  return launch_conv(noise, W, H, model, filt, r, e, s, tile);
+  return launch_conv(noise, W, H, model, filt, r, e, s, tile, slabs);
 }
 
 }  // namespace cageo
@@ -569,8 +583,8 @@ extern "C" cageo_status cageo_noise_philox(float* d_field, int W, int H,
                                            float mean, float stddev,
                                            cudaStream_t stream) {
   CAGEO_CHECK_ARG(d_field && valid_dims(W, H), "field pointer and size");
-  return launch_noise(d_field, (int64_t)W * H, seed, realization, nullptr, mean, stddev,
-                      stream);
+  return launch_noise(d_field, (int64_t)W * H, seed, realization, nullptr, mean, stddev, stream,
+                      1);
 }
 
 // Raw Philox4x32-10 blocks: block i is philox4x32_10((c0 + i, c1, c2, c3),

@@ -17,6 +17,7 @@
 // such a realization is not counted by the fast path and is recomputed with
 // the stage kernels, which follow the reference step by step.  With a
 // NODATA of 0 every realization takes the stage path.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -32,9 +33,9 @@
 
 namespace cageo {
 cageo_status launch_noise(float* d, int64_t n, uint64_t seed, uint32_t realization,
-                          const uint32_t* dreal, float mean, float sd, cudaStream_t s);
+                          const uint32_t* dreal, float mean, float sd, cudaStream_t s, int slabs);
 cageo_status launch_front(const float* noise, int W, int H, int model, const float* filt,
-                          int r, const FrontParams& fp, cudaStream_t s, int tile);
+                          int r, const FrontParams& fp, cudaStream_t s, int tile, int slabs);
 bool conv_tile_applies(int model, int r, int tile);
 cageo_status launch_burn_code(const float* streams, uint8_t* code, int W, int H,
                               float nodata_stream, int bevel, float* factor_out,
@@ -49,19 +50,25 @@ cageo_status launch_to_bytes(const float* in, uint8_t* out, int64_t n, unsigned 
 cageo_status ws_infer(const float* params, const float* v, float* warm, float* depth, int W,
                       int H, float nodata, float threshold, cudaStream_t s);
 
-// End of a step of `count` realizations: record the realizations of a
-// flagged step (none of them was counted), clear the flag and advance the
-// device realization counter.
+// Layout of the device scalars (cageo_pipeline::dscal).
+constexpr int kMaxStack = 64;               // realizations of a step
+constexpr int kFlags = 4;                   // their anomaly flags
+constexpr int kRedo = kFlags + kMaxStack;   // realizations to redo
+constexpr unsigned int kMaxRedo = 4096;
+
+// End of a step of `count` realizations: list the flagged ones (they were not
+// counted), clear their flags and advance the device realization counter.
 __global__ void realization_end_kernel(uint32_t* real, int* anomaly, uint32_t* redo,
                                        unsigned int* nredo, unsigned int count) {
-  if (threadIdx.x == 0) {
-    if (*anomaly) {
-      const unsigned int k = atomicAdd(nredo, count);
-      for (unsigned int j = 0; j < count && k + j < 4096; j++) redo[k + j] = *real + j;
-      *anomaly = 0;
+  for (unsigned int j = threadIdx.x; j < count; j += blockDim.x) {
+    if (anomaly[j]) {
+      const unsigned int k = atomicAdd(nredo, 1u);
+      if (k < kMaxRedo) redo[k] = *real + j;
+      anomaly[j] = 0;
     }
-    *real += count;
   }
+  __syncthreads();
+  if (threadIdx.x == 0) *real += count;
 }
 
 // Order-independent 64-bit digest of a float grid: the wrapping sum over
@@ -110,7 +117,9 @@ struct cageo_pipeline {
   FillWork fw;
   RouteWork rw;
   TraceWork tw;
-  // device scalars: [0] realization counter, [1] anomaly, [2] nredo, [3..] redo list
+  // device scalars: [0] realization counter, [1] -, [2] nredo, [3] the run's
+  // last realization (the one whose labels are kept), [4..] the anomaly flags
+  // of a step's slabs, then the redo list
   uint32_t* dscal = nullptr;
   FrontParams fp{};
   cudaGraph_t graph = nullptr;
@@ -126,45 +135,55 @@ struct cageo_pipeline {
   float ws_threshold = 0.0f;
   // Digest of the DEM and stream grids (grid_digest_kernel), for checkpoints.
   unsigned long long input_digest = 0;
-  // Batched steps (cageo_pipeline_set_batch): `batch` realizations share one
-  // fill over a stack of their q grids (qb, filledb: batch * N floats, fill
-  // workspace fwb for W x batch*H), each slab's minimum of q in slab_min.
+  // Stacked steps: `stack` realizations (the capacity; `step` of the last
+  // step) one above the other through every stage -- q grids, filled grids,
+  // directions, workspaces for W x K*H, each slab's minimum of q, and for
+  // small grids their noise.  batch > 1: what cageo_pipeline_set_batch asked
+  // for; 1: steps are sized by the grid (stack_of).
   int batch = 1;
+  bool plain = false;  // batch 1 was asked for: one realization at a time
+  int stack = 0, step = 0;
   int conv_tile = 0;  // the fused front's convolution tile shape (kConvTiles)
-  float *qb = nullptr, *filledb = nullptr;
-  void* fill_ws_b = nullptr;
+  float *qb = nullptr, *filledb = nullptr, *noiseb = nullptr;
+  void *fill_ws_b = nullptr, *route_ws_b = nullptr, *trace_ws_b = nullptr;
   unsigned int* slab_min = nullptr;
   FillWork fwb;
-  // Routing over the stack as well: directions of all slabs, routing workspace
-  // for W x batch*H.
   int8_t* dirb = nullptr;
-  void* route_ws_b = nullptr;
   RouteWork rwb;
+  TraceWork twb;
+  int graph_k = 0;  // realizations of the captured step
+  int last_k = 0;   // realizations of the last run's steps
   cudaGraph_t graph_b = nullptr;
   cudaGraphExec_t exec_b = nullptr;
-  bool last_batched = false;  // the last realization ran in a batched step
+  bool last_batched = false;  // the last realization ran in a stacked step (its top slab)
 };
 
 namespace {
 
-void free_batch(cageo_pipeline* p) {
+void drop_step_graph(cageo_pipeline* p) {
   if (p->exec_b) cudaGraphExecDestroy(p->exec_b);
   if (p->graph_b) cudaGraphDestroy(p->graph_b);
   p->exec_b = nullptr;
   p->graph_b = nullptr;
-  void* bufs[] = {p->qb, p->filledb, p->fill_ws_b, p->slab_min, p->dirb, p->route_ws_b};
+  p->graph_k = 0;
+}
+
+void free_stack(cageo_pipeline* p) {
+  drop_step_graph(p);
+  void* bufs[] = {p->qb, p->filledb, p->noiseb, p->fill_ws_b, p->slab_min, p->dirb,
+                  p->route_ws_b, p->trace_ws_b};
   for (void* b : bufs)
     if (b) cudaFree(b);
-  p->qb = p->filledb = nullptr;
-  p->fill_ws_b = nullptr;
+  p->qb = p->filledb = p->noiseb = nullptr;
+  p->fill_ws_b = p->route_ws_b = p->trace_ws_b = nullptr;
   p->slab_min = nullptr;
   p->dirb = nullptr;
-  p->route_ws_b = nullptr;
-  p->batch = 1;
+  p->stack = p->step = 0;
+  p->last_batched = false;
 }
 
 void free_all(cageo_pipeline* p) {
-  free_batch(p);
+  free_stack(p);
   if (p->exec) cudaGraphExecDestroy(p->exec);
   if (p->graph) cudaGraphDestroy(p->graph);
   void* bufs[] = {p->dem, p->streams, p->noise, p->q, p->filled, p->filter, p->tmp, p->code,
@@ -203,19 +222,15 @@ int trace_mode(const cageo_pipeline* p) {
   return exact_mode(p) ? CAGEO_TRACE_DEAD_END_ERROR : CAGEO_TRACE_CPU_COMPAT;
 }
 
-// Tracing with labels (the learned path reads them before the border).
-cageo_status enqueue_trace(cageo_pipeline* p) {
-  return trace_run(p->dir, p->streams, p->label, p->tw, p->stream, trace_mode(p), true);
-}
-
 // Tracing whose labels are decoded by the border pass (one pass fewer);
-// gate: skip the accumulation when set (null: always accumulate).
-cageo_status enqueue_trace_border(cageo_pipeline* p, const int* gate) {
-  cageo_status st = trace_run(p->dir, p->streams, p->label, p->tw, p->stream, trace_mode(p),
-                              false);
+// gate: skip the accumulation when set (null: always accumulate); every:
+// write the labels whichever realization it is.
+cageo_status enqueue_trace_border(cageo_pipeline* p, const int* gate, bool every) {
+  cageo_status st = trace_run(p->dir, p->streams, p->code, p->label, p->tw, p->stream,
+                              trace_mode(p), false);
   if (st) return st;
-  return border_u32_from_state(p->tw, p->label, p->counts, gate,
-                               trace_mode(p), p->stream);
+  return border_u32_from_state(p->tw, p->label, p->counts, gate, trace_mode(p), p->dscal,
+                               every ? nullptr : p->dscal + 3, p->stream);
 }
 
 // Launch sequence of one realization on the fast path.  The realization
@@ -225,61 +240,65 @@ cageo_status enqueue_fast(cageo_pipeline* p) {
   const cageo_pipeline_config& c = p->cfg;
   cageo_status st;
   if ((st = fill_begin(p->fw, s))) return st;
-  if ((st = launch_noise(p->noise, p->N, c.seed, 0, p->dscal, c.error_mean, c.error_stddev, s)))
+  if ((st = launch_noise(p->noise, p->N, c.seed, 0, p->dscal, c.error_mean, c.error_stddev, s, 1)))
     return st;
   if ((st = launch_front(p->noise, p->W, p->H, c.filter_model, p->filter, p->radius, p->fp, s,
-                         p->conv_tile)))
+                         p->conv_tile, 1)))
     return st;
   if ((st = enqueue_fill(p))) return st;
   if ((st = enqueue_route(p))) return st;
-  if ((st = enqueue_trace_border(p, (const int*)p->dscal + 1))) return st;
-  realization_end_kernel<<<1, 32, 0, s>>>(p->dscal, (int*)p->dscal + 1, p->dscal + 3,
+  if ((st = enqueue_trace_border(p, (const int*)p->dscal + kFlags, false))) return st;
+  realization_end_kernel<<<1, 32, 0, s>>>(p->dscal, (int*)p->dscal + kFlags, p->dscal + kRedo,
                                           p->dscal + 2, 1u);
   CAGEO_CUDA(cudaGetLastError());
   return CAGEO_OK;
 }
 
-// Launch sequence of one batched step: `p->batch` realizations from the
-// device counter on.  Noise and the fused front run per realization, each
-// into its slab of the stacked q grid (with its own minimum); one fill
-// covers the whole stack (slabs cannot exchange values: see FillWork), and
-// so does the routing (flat cells are interior: their neighbours lie in
-// their own slab); tracing and the border counts run per slab.  The results
-// equal `batch` single realizations bit for bit.
-cageo_status enqueue_batch(cageo_pipeline* p) {
+// Launch sequence of one stacked step: p->step realizations from the device
+// counter on, one above the other (slabs cannot exchange values: every slab's
+// border cells are outlets of the fill and drain outward).  Every stage runs
+// once over the stack; for grids above kStackNoise cells noise and front run
+// slab by slab, which spares a noise grid per slab and loses nothing.  The
+// results equal single realizations bit for bit.
+constexpr int64_t kStackNoise = (int64_t)1 << 22;
+
+cageo_status enqueue_step(cageo_pipeline* p) {
   cudaStream_t s = p->stream;
   const cageo_pipeline_config& c = p->cfg;
-  const int K = p->batch;
+  const int K = p->step;
   cageo_status st;
   if ((st = fill_begin(p->fwb, s))) return st;
   CAGEO_CUDA(cudaMemsetAsync(p->slab_min, 0xff, sizeof(unsigned int) * K, s));
-  for (int k = 0; k < K; k++) {
-    if ((st = launch_noise(p->noise, p->N, c.seed, (uint32_t)k, p->dscal, c.error_mean,
-                           c.error_stddev, s)))
+  FrontParams fp = p->fp;
+  fp.tseed = p->fwb.tseed;
+  fp.tiles_x = p->fwb.tiles_x;
+  const int each = p->noiseb ? K : 1;  // slabs per launch of noise and front
+  for (int k = 0; k < K; k += each) {
+    float* noise = p->noiseb ? p->noiseb : p->noise;
+    if ((st = launch_noise(noise, p->N, c.seed, (uint32_t)k, p->dscal, c.error_mean,
+                           c.error_stddev, s, each)))
       return st;
-    FrontParams fp = p->fp;
     fp.q = p->qb + (size_t)k * p->N;
     fp.min_ord = p->slab_min + k;
-    fp.tseed = p->fwb.tseed;
-    fp.tiles_x = p->fwb.tiles_x;
+    fp.anomaly = p->fp.anomaly + k;
     fp.row0 = k * p->H;
-    if ((st = launch_front(p->noise, p->W, p->H, c.filter_model, p->filter, p->radius, fp, s,
-                           p->conv_tile)))
+    if ((st = launch_front(noise, p->W, p->H, c.filter_model, p->filter, p->radius, fp, s,
+                           p->conv_tile, each)))
       return st;
   }
-  if ((st = fill_run(p->qb, p->filledb, p->fwb, c.nodata_dem, s))) return st;
-  if ((st = route_run(p->filledb, p->dirb, nullptr, p->rwb, s, CAGEO_ROUTE_CPU_COMPAT,
+  if (exact_mode(p)) st = fill_run_exact(p->qb, p->filledb, p->fwb, c.nodata_dem, nullptr, s);
+  else st = fill_run(p->qb, p->filledb, p->fwb, c.nodata_dem, s);
+  if (st) return st;
+  if ((st = route_run(p->filledb, p->dirb, nullptr, p->rwb, s,
+                      exact_mode(p) ? CAGEO_ROUTE_GPU_ORDER : CAGEO_ROUTE_CPU_COMPAT,
                       c.nodata_dem)))
     return st;
-  for (int k = 0; k < K; k++) {
-    const int8_t* dir = p->dirb + 2 * (size_t)k * p->N;
-    if ((st = trace_run(dir, p->streams, p->label, p->tw, s, CAGEO_TRACE_CPU_COMPAT, false)))
-      return st;
-    if ((st = border_u32_from_state(p->tw, p->label, p->counts, (const int*)p->dscal + 1,
-                                    CAGEO_TRACE_CPU_COMPAT, s)))
-      return st;
-  }
-  realization_end_kernel<<<1, 32, 0, s>>>(p->dscal, (int*)p->dscal + 1, p->dscal + 3,
+  if ((st = trace_run(p->dirb, p->streams, p->code, p->label, p->twb, s, trace_mode(p), false)))
+    return st;
+  if ((st = border_u32_from_state(p->twb, p->label, p->counts, (const int*)p->dscal + kFlags,
+                                  trace_mode(p), p->dscal, p->dscal + 3, s)))
+    return st;
+  realization_end_kernel<<<1, 32, 0, s>>>(p->dscal, (int*)p->dscal + kFlags, p->dscal + kRedo,
                                           p->dscal + 2, (unsigned int)K);
   CAGEO_CUDA(cudaGetLastError());
   return CAGEO_OK;
@@ -291,7 +310,7 @@ cageo_status run_stage_path(cageo_pipeline* p, uint32_t r) {
   const cageo_pipeline_config& c = p->cfg;
   cageo_status st;
   if ((st = fill_begin(p->fw, s))) return st;
-  if ((st = launch_noise(p->noise, p->N, c.seed, r, nullptr, c.error_mean, c.error_stddev, s)))
+  if ((st = launch_noise(p->noise, p->N, c.seed, r, nullptr, c.error_mean, c.error_stddev, s, 1)))
     return st;
   if ((st = cageo_convolve(p->noise, p->tmp, p->W, p->H, c.filter_model, p->filter, p->radius, s)))
     return st;
@@ -306,7 +325,7 @@ cageo_status run_stage_path(cageo_pipeline* p, uint32_t r) {
   p->fw.seeded = true;
   if (st) return st;
   if ((st = enqueue_route(p))) return st;
-  if ((st = enqueue_trace_border(p, nullptr))) return st;
+  if ((st = enqueue_trace_border(p, nullptr, true))) return st;
   return CAGEO_OK;
 }
 
@@ -369,7 +388,7 @@ cageo_status create_common(cageo_pipeline** out, const cageo_pipeline_config* cf
       (st = dalloc(&p->fill_ws, fill_workspace_bytes(W, H))) ||
       (st = dalloc(&p->route_ws, route_workspace_bytes(W, H))) ||
       (st = dalloc(&p->trace_ws, trace_workspace_bytes(W, H))) ||
-      (st = dalloc(&p->dscal, sizeof(uint32_t) * (3 + 4096))))
+      (st = dalloc(&p->dscal, sizeof(uint32_t) * (kRedo + kMaxRedo))))
     return fail(st);
   p->fw = fill_carve(p->fill_ws, W, H);
   p->rw = route_carve(p->route_ws, W, H);
@@ -384,15 +403,15 @@ cageo_status create_common(cageo_pipeline** out, const cageo_pipeline_config* cf
   PCUDA(cudaMemcpyAsync(p->dem, dem, fb, kind, s));
   PCUDA(cudaMemcpyAsync(p->streams, streams, fb, kind, s));
   PCUDA(cudaMemsetAsync(p->counts, 0, 4 * (size_t)p->N, s));
-  PCUDA(cudaMemsetAsync(p->dscal, 0, sizeof(uint32_t) * 3, s));
+  PCUDA(cudaMemsetAsync(p->dscal, 0, sizeof(uint32_t) * kRedo, s));
   // Status words of workspaces that a run may read without having used them
   // (batched steps have workspaces of their own).
   PCUDA(cudaMemsetAsync(p->fw.scal, 0, kFillScalars * sizeof(unsigned int), s));
   PCUDA(cudaMemsetAsync(p->rw.scal, 0, kRouteScalars * sizeof(unsigned int), s));
   PCUDA(cudaMemsetAsync(p->tw.scal, 0, kScalarSlots * sizeof(unsigned int), s));
   {
-    // dscal[4..5] holds the digest until the first realization.
-    unsigned long long* dig = (unsigned long long*)(p->dscal + 4);
+    // The redo list's place holds the digest until the first realization.
+    unsigned long long* dig = (unsigned long long*)(p->dscal + kRedo);
     PCUDA(cudaMemsetAsync(dig, 0, 8, s));
     grid_digest_kernel<<<1024, 256, 0, s>>>(p->dem, p->N, 0x44454dull, dig);
     grid_digest_kernel<<<1024, 256, 0, s>>>(p->streams, p->N, 0x535452ull << 20, dig);
@@ -406,7 +425,7 @@ cageo_status create_common(cageo_pipeline** out, const cageo_pipeline_config* cf
   p->fp.code = p->code;
   p->fp.q = p->q;
   p->fp.min_ord = fill_min_slot(p->fw);
-  p->fp.anomaly = (int*)p->dscal + 1;
+  p->fp.anomaly = (int*)p->dscal + kFlags;
   p->fp.nodata_dem = cfg->nodata_dem;
   p->fp.quantize = cfg->fill_mode == CAGEO_FILL_EXACT ? 0 : 1;
   // The front's epilogue sets the fill's seeds.
@@ -441,49 +460,133 @@ extern "C" cageo_status cageo_pipeline_create_device(cageo_pipeline** out,
   });
 }
 
+// Room for stacks of K realizations.
+static cageo_status ensure_stack(cageo_pipeline* p, int K) {
+  if (p->stack >= K) return CAGEO_OK;
+  CAGEO_CUDA(cudaStreamSynchronize(p->stream));
+  free_stack(p);
+  const size_t nb = (size_t)K * p->N;
+  cageo_status st;
+  if ((st = dalloc(&p->qb, sizeof(float) * nb)) || (st = dalloc(&p->filledb, sizeof(float) * nb)) ||
+      (p->N <= kStackNoise && (st = dalloc(&p->noiseb, sizeof(float) * nb))) ||
+      (st = dalloc(&p->fill_ws_b, fill_workspace_bytes(p->W, K * p->H))) ||
+      (st = dalloc(&p->slab_min, sizeof(unsigned int) * K)) || (st = dalloc(&p->dirb, 2 * nb)) ||
+      (st = dalloc(&p->route_ws_b, route_workspace_bytes(p->W, K * p->H))) ||
+      (st = dalloc(&p->trace_ws_b, trace_workspace_bytes(p->W, K * p->H)))) {
+    free_stack(p);
+    cudaGetLastError();
+    return st;
+  }
+  p->stack = K;
+  return CAGEO_OK;
+}
+
+// The workspaces of a step of K realizations (K <= p->stack), with the single
+// fill's tuning.
+static void set_step(cageo_pipeline* p, int K) {
+  p->step = K;
+  p->rwb = route_carve(p->route_ws_b, p->W, K * p->H);
+  p->rwb.slab_h = p->H;
+  p->twb = trace_carve(p->trace_ws_b, p->W, K * p->H);
+  p->twb.slab_h = p->H;
+  p->fwb = fill_carve(p->fill_ws_b, p->W, K * p->H);
+  p->fwb.slab_h = p->H;
+  p->fwb.slab_min = p->slab_min;
+  p->fwb.seeded = true;
+  p->fwb.max_rounds = p->fw.max_rounds;
+  p->fwb.flood_warps = p->fw.flood_warps;
+}
+
+// Realizations stacked per step where none was asked for.  A realization of a
+// small grid is a chain of ~15 launches that leave most of the GPU idle (330
+// us at 512^2, 20 of them stacked: 860 us), so as many are stacked as
+// make up kStackCells cells (about 35 bytes a cell: 1.2 GB); above that a
+// single grid fills the GPU (four at 4096^2 in two steps: 5.1 ms, singly 6.5).
+constexpr int64_t kStackCells = (int64_t)1 << 25;
+
+static int stack_of(const cageo_pipeline* p, int count) {
+  // (Launches over tiles have their rows in grid.y: 65535 at most.)
+  const int64_t fit = std::min<int64_t>({kMaxStack, kStackCells / p->N, 65535 * 32 / p->H});
+  if (p->plain || fit < 2 || count < 2) return 1;
+  const int steps = (int)((count + fit - 1) / fit);
+  return (count + steps - 1) / steps;  // even steps
+}
+
+// `steps` stacked steps of K realizations, replaying a captured graph where
+// one is wanted: it is captured on first use, and again for another K once
+// that has been used by two runs in a row.
+static cageo_status run_steps(cageo_pipeline* p, int K, int steps) {
+  cudaStream_t s = p->stream;
+  cageo_status st;
+  if (p->step != K) set_step(p, K);
+  int b = 0;
+  if (p->cfg.use_graphs && p->graph_k != K && (p->graph_k == 0 || p->last_k == K)) {
+    drop_step_graph(p);
+    // Warm-up outside capture, then capture one step.
+    if ((st = enqueue_step(p))) return st;
+    b = 1;
+    CAGEO_CUDA(cudaStreamSynchronize(s));
+    cudaGraph_t g = nullptr;
+    if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+      cageo_status cst = enqueue_step(p);
+      cudaError_t e = cudaStreamEndCapture(s, &g);
+      if (cst != CAGEO_OK || e != cudaSuccess ||
+          cudaGraphInstantiate(&p->exec_b, g, 0) != cudaSuccess) {
+        p->exec_b = nullptr;
+      }
+      cudaGetLastError();
+    }
+    // Kept even when the capture failed: graph_k marks it as tried (steps then
+    // run as direct launches).
+    p->graph_b = g;
+    p->graph_k = K;
+  }
+  p->last_k = K;
+  for (; b < steps; b++) {
+    if (p->exec_b && p->graph_k == K) CAGEO_CUDA(cudaGraphLaunch(p->exec_b, s));
+    else if ((st = enqueue_step(p))) return st;
+  }
+  return CAGEO_OK;
+}
+
 static cageo_status pipeline_run(cageo_pipeline* p, uint32_t first, int count) {
   CAGEO_CHECK_ARG(p && count >= 0, "pipeline and count");
   cudaStream_t s = p->stream;
   cageo_status st;
-  CAGEO_CUDA(cudaMemcpyAsync(p->dscal, &first, sizeof(uint32_t), cudaMemcpyHostToDevice, s));
-  CAGEO_CUDA(cudaMemsetAsync(p->dscal + 1, 0, 2 * sizeof(uint32_t), s));
+  const uint32_t scalars[kRedo] = {first, 0, 0, first + (uint32_t)count - 1u};
+  CAGEO_CUDA(cudaMemcpyAsync(p->dscal, scalars, sizeof(scalars), cudaMemcpyHostToDevice, s));
   const bool stage_only = p->cfg.nodata_dem == 0.0f;
-  // Learned warm starts run on the fast path too (never batched).
+  // Learned warm starts run on the fast path too (never stacked).
   const bool learned = p->ws_params != nullptr && !stage_only;
   int done = 0;
-  // Whole batched steps first (cageo_pipeline_set_batch), then single
-  // realizations for the rest.  Both advance the same device counter.
-  const int K = p->batch;
-  const bool batched = !stage_only && !learned && K > 1 && count >= K;
-  const int in_batches = batched ? count / K * K : 0;
-  if (batched) {
-    const int nb = count / K;
-    int b = 0;
-    if (p->cfg.use_graphs && !p->exec_b && !p->graph_b) {
-      // Warm-up outside capture, then capture one batched step.
-      if ((st = enqueue_batch(p))) return st;
-      b = 1;
-      CAGEO_CUDA(cudaStreamSynchronize(s));
-      cudaGraph_t g = nullptr;
-      if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-        cageo_status cst = enqueue_batch(p);
-        cudaError_t e = cudaStreamEndCapture(s, &g);
-        if (cst != CAGEO_OK || e != cudaSuccess ||
-            cudaGraphInstantiate(&p->exec_b, g, 0) != cudaSuccess) {
-          p->exec_b = nullptr;
-        }
-        cudaGetLastError();
-      }
-      // Kept even when the capture failed: it marks the capture as tried
-      // (batched steps then run as direct launches).
-      p->graph_b = g;
-    }
-    for (; b < nb; b++) {
-      if (p->exec_b) CAGEO_CUDA(cudaGraphLaunch(p->exec_b, s));
-      else if ((st = enqueue_batch(p))) return st;
-    }
-    done = nb * K;
+  int64_t fs[kFillStats] = {}, rs[7] = {}, jumps = 0;
+  // Stacked steps first: whole ones of the batch asked for, the rest singly;
+  // or, sized by the grid, all realizations (the last step may be smaller).
+  // All advance the same device counter.
+  const bool asked = p->batch > 1;
+  int K = stage_only || learned ? 1 : asked ? p->batch : stack_of(p, count);
+  if (K > 1 && !asked && ensure_stack(p, K)) {
+    p->plain = true;  // no memory for a stack: singly from now on
+    K = 1;
   }
+  const bool stacked = K > 1 && count >= K;
+  auto step_status = [&]() -> cageo_status {
+    CAGEO_CUDA(cudaStreamSynchronize(s));
+    cageo_status e;
+    if ((e = fill_check_status(p->fwb, fs)) || (e = route_check_status(p->rwb, rs))) return e;
+    return trace_check_status(p->twb, &jumps);
+  };
+  if (stacked) {
+    const int steps = count / K, tail = asked ? 0 : count - steps * K;
+    if ((st = run_steps(p, K, steps))) return st;
+    if (tail && (st = step_status())) return st;
+    if (tail) {
+      set_step(p, tail);
+      if ((st = enqueue_step(p))) return st;
+    }
+    done = steps * K + tail;
+  }
+  if (count > 0) p->last_batched = stacked && done == count;
   if (!stage_only && count > done && p->cfg.use_graphs && !p->graph_ok && !p->exec) {
     // Warm-up outside capture (kernel attributes, occupancy caches), then
     // capture one realization.
@@ -517,27 +620,30 @@ static cageo_status pipeline_run(cageo_pipeline* p, uint32_t first, int count) {
     }
   }
   CAGEO_CUDA(cudaStreamSynchronize(s));
-  int64_t fs[kFillStats] = {}, rs[7] = {}, jumps = 0;
-  p->last_batched = batched && in_batches == count;
-  if (batched && (st = fill_check_status(p->fwb, p->last_batched ? fs : nullptr))) return st;
-  if (batched && (st = route_check_status(p->rwb, p->last_batched ? rs : nullptr))) return st;
-  if ((st = fill_check_status(p->fw, p->last_batched ? nullptr : fs))) return st;
-  if ((st = route_check_status(p->rw, p->last_batched ? nullptr : rs))) return st;
-  if ((st = trace_check_status(p->tw, &jumps))) return st;
+  if (p->last_batched) {
+    if ((st = step_status())) return st;
+  } else {
+    if ((st = fill_check_status(p->fw, fs))) return st;
+    if ((st = route_check_status(p->rw, rs))) return st;
+    if ((st = trace_check_status(p->tw, &jumps))) return st;
+  }
   uint32_t nredo = 0;
   CAGEO_CUDA(cudaMemcpy(&nredo, p->dscal + 2, sizeof(uint32_t), cudaMemcpyDeviceToHost));
   if (nredo) {
-    if (nredo > 4096) {
+    if (nredo > kMaxRedo) {
       set_error("more than 4096 realizations need the exact burning path in one run");
       return CAGEO_ERR_NO_CONVERGENCE;
     }
     std::vector<uint32_t> redo(nredo);
-    CAGEO_CUDA(cudaMemcpy(redo.data(), p->dscal + 3, sizeof(uint32_t) * nredo,
+    CAGEO_CUDA(cudaMemcpy(redo.data(), p->dscal + kRedo, sizeof(uint32_t) * nredo,
                           cudaMemcpyDeviceToHost));
+    std::sort(redo.begin(), redo.end(),
+              [=](uint32_t a, uint32_t b) { return a - first < b - first; });
     for (uint32_t r : redo)
       if ((st = run_stage_path(p, r))) return st;
     CAGEO_CUDA(cudaStreamSynchronize(s));
     if ((st = fill_check_status(p->fw, fs))) return st;
+    p->last_batched = false;  // the last realization computed is the last redone
   }
   p->stats[0] = fs[0];
   p->stats[1] = fs[1];
@@ -569,6 +675,7 @@ extern "C" cageo_status cageo_pipeline_profile(cageo_pipeline* p, uint32_t reali
   CAGEO_CHECK_ARG(p->cfg.nodata_dem != 0.0f, "profiling needs the fused path (NODATA != 0)");
   cudaStream_t s = p->stream;
   const cageo_pipeline_config& c = p->cfg;
+  p->last_batched = false;
   cudaEvent_t ev[7], fm[4];
   for (auto& e : ev) CAGEO_CUDA(cudaEventCreate(&e));
   for (auto& e : fm) CAGEO_CUDA(cudaEventCreate(&e));
@@ -580,11 +687,11 @@ extern "C" cageo_status cageo_pipeline_profile(cageo_pipeline* p, uint32_t reali
     }
     if ((st = fill_begin(p->fw, s))) break;
     cudaEventRecord(ev[0], s);
-    if ((st = launch_noise(p->noise, p->N, c.seed, 0, p->dscal, c.error_mean, c.error_stddev, s)))
+    if ((st = launch_noise(p->noise, p->N, c.seed, 0, p->dscal, c.error_mean, c.error_stddev, s, 1)))
       break;
     cudaEventRecord(ev[1], s);
     if ((st = launch_front(p->noise, p->W, p->H, c.filter_model, p->filter, p->radius, p->fp, s,
-                           p->conv_tile)))
+                           p->conv_tile, 1)))
       break;
     cudaEventRecord(ev[2], s);
     if (!exact_mode(p)) p->fw.marks = fm;
@@ -594,12 +701,13 @@ extern "C" cageo_status cageo_pipeline_profile(cageo_pipeline* p, uint32_t reali
     cudaEventRecord(ev[3], s);
     if ((st = enqueue_route(p))) break;
     cudaEventRecord(ev[4], s);
-    if ((st = trace_run(p->dir, p->streams, p->label, p->tw, s, trace_mode(p), false))) break;
-    cudaEventRecord(ev[5], s);  // the border stage decodes the labels
-    if ((st = border_u32_from_state(p->tw, p->label, p->counts,
-                                    (const int*)p->dscal + 1, trace_mode(p), s)))
+    if ((st = trace_run(p->dir, p->streams, p->code, p->label, p->tw, s, trace_mode(p), false)))
       break;
-    realization_end_kernel<<<1, 32, 0, s>>>(p->dscal, (int*)p->dscal + 1, p->dscal + 3,
+    cudaEventRecord(ev[5], s);  // the border stage decodes the labels
+    if ((st = border_u32_from_state(p->tw, p->label, p->counts, (const int*)p->dscal + kFlags,
+                                    trace_mode(p), p->dscal, nullptr, s)))
+      break;
+    realization_end_kernel<<<1, 32, 0, s>>>(p->dscal, (int*)p->dscal + kFlags, p->dscal + kRedo,
                                             p->dscal + 2, 1u);
     cudaEventRecord(ev[6], s);
     if (cudaStreamSynchronize(s) != cudaSuccess) {
@@ -658,13 +766,10 @@ static cageo_status pipeline_run_filter(cageo_pipeline* p, uint32_t first, int c
   // The captured graphs hold the old filter's launch shapes: drop them.
   if (p->exec) cudaGraphExecDestroy(p->exec);
   if (p->graph) cudaGraphDestroy(p->graph);
-  if (p->exec_b) cudaGraphExecDestroy(p->exec_b);
-  if (p->graph_b) cudaGraphDestroy(p->graph_b);
   p->exec = nullptr;
   p->graph = nullptr;
-  p->exec_b = nullptr;
-  p->graph_b = nullptr;
   p->graph_ok = false;
+  drop_step_graph(p);
   p->cfg.use_graphs = 0;
   return pipeline_run(p, first, count);
 }
@@ -838,7 +943,7 @@ extern "C" cageo_status cageo_pipeline_counts_bytes(cageo_pipeline* p, uint8_t* 
   // The byte image is staged in the noise buffer and the min/max pair in the
   // redo list; both are rewritten by the next realization.
   uint8_t* bytes = (uint8_t*)p->noise;
-  unsigned int* mm = p->dscal + 3;
+  unsigned int* mm = p->dscal + kRedo;
   cageo_status st = launch_to_bytes(p->tmp, bytes, p->N, mm, s);
   if (st) return st;
   CAGEO_CUDA(cudaMemcpyAsync(h_out, bytes, (size_t)p->N, cudaMemcpyDeviceToHost, s));
@@ -850,11 +955,11 @@ extern "C" cageo_status cageo_pipeline_last_stages(cageo_pipeline* p, float* h_f
                                                    int8_t* h_dir, int* h_label) {
   CAGEO_CHECK_ARG(p, "null pipeline");
   cudaStream_t s = p->stream;
-  // After a batched step the last realization's filled grid is its top slab.
-  const float* filled = p->last_batched ? p->filledb + (size_t)(p->batch - 1) * p->N : p->filled;
+  // After a stacked step the last realization's filled grid is its top slab.
+  const float* filled = p->last_batched ? p->filledb + (size_t)(p->step - 1) * p->N : p->filled;
   if (h_filled)
     CAGEO_CUDA(cudaMemcpyAsync(h_filled, filled, 4 * p->N, cudaMemcpyDeviceToHost, s));
-  const int8_t* dir = p->last_batched ? p->dirb + 2 * (size_t)(p->batch - 1) * p->N : p->dir;
+  const int8_t* dir = p->last_batched ? p->dirb + 2 * (size_t)(p->step - 1) * p->N : p->dir;
   if (h_dir) CAGEO_CUDA(cudaMemcpyAsync(h_dir, dir, 2 * p->N, cudaMemcpyDeviceToHost, s));
   if (h_label) CAGEO_CUDA(cudaMemcpyAsync(h_label, p->label, 4 * p->N, cudaMemcpyDeviceToHost, s));
   CAGEO_CUDA(cudaStreamSynchronize(s));
@@ -892,19 +997,15 @@ extern "C" int cageo_autotune_candidates(cageo_tuning* h_out, int n) {
 static void drop_graph(cageo_pipeline* p) {
   if (p->exec) cudaGraphExecDestroy(p->exec);
   if (p->graph) cudaGraphDestroy(p->graph);
-  if (p->exec_b) cudaGraphExecDestroy(p->exec_b);
-  if (p->graph_b) cudaGraphDestroy(p->graph_b);
   p->exec = nullptr;
   p->graph = nullptr;
-  p->exec_b = nullptr;
-  p->graph_b = nullptr;
   p->graph_ok = false;
+  drop_step_graph(p);
 }
 
-// The batched fill runs with the single fill's tuning.
-static void sync_batch_tuning(cageo_pipeline* p) {
-  p->fwb.max_rounds = p->fw.max_rounds;
-  p->fwb.flood_warps = p->fw.flood_warps;
+// Stacked steps run with the single fill's tuning.
+static void sync_step_tuning(cageo_pipeline* p) {
+  if (p->step) set_step(p, p->step);
 }
 
 extern "C" cageo_status cageo_pipeline_set_tuning(cageo_pipeline* p, const cageo_tuning* t) {
@@ -919,7 +1020,7 @@ extern "C" cageo_status cageo_pipeline_set_tuning(cageo_pipeline* p, const cageo
   p->fw.max_rounds = t->fill_rounds;
   p->fw.flood_warps = t->fill_warps;
   p->conv_tile = t->conv_tile;
-  sync_batch_tuning(p);
+  sync_step_tuning(p);
   drop_graph(p);  // captured with the old launch shapes
   return CAGEO_OK;
 }
@@ -946,6 +1047,7 @@ extern "C" cageo_status cageo_pipeline_autotune(cageo_pipeline* p, uint32_t firs
   CAGEO_CUDA(cudaEventCreate(&e0));
   CAGEO_CUDA(cudaEventCreate(&e1));
   cageo_status st = CAGEO_OK;
+  p->last_batched = false;
   float best_ms = 0.0f;
   cageo_tuning best{p->fw.max_rounds, p->fw.flood_warps, p->conv_tile};
   cageo_tuning cand[kTuneCandidates];
@@ -968,8 +1070,10 @@ extern "C" cageo_status cageo_pipeline_autotune(cageo_pipeline* p, uint32_t firs
       p->fw.flood_warps = best.fill_warps;
     }
     p->conv_tile = cand[c].conv_tile;
-    uint32_t r0 = first + (uint32_t)(c * (trials + 1));
-    if (cudaMemcpyAsync(p->dscal, &r0, sizeof(r0), cudaMemcpyHostToDevice, s) != cudaSuccess) {
+    const uint32_t r0 = first + (uint32_t)(c * (trials + 1));
+    const uint32_t scalars[4] = {r0, 0, 0, r0 + (uint32_t)trials};
+    if (cudaMemcpyAsync(p->dscal, scalars, sizeof(scalars), cudaMemcpyHostToDevice, s) !=
+        cudaSuccess) {
       st = cuda_fail(cudaGetLastError(), "cudaMemcpyAsync");
       break;
     }
@@ -997,44 +1101,31 @@ extern "C" cageo_status cageo_pipeline_autotune(cageo_pipeline* p, uint32_t firs
   p->fw.max_rounds = best.fill_rounds;
   p->fw.flood_warps = best.fill_warps;
   p->conv_tile = best.conv_tile;
-  sync_batch_tuning(p);
+  sync_step_tuning(p);
   drop_graph(p);
   if (h_best) *h_best = best;
   CAGEO_CUDA(cudaMemsetAsync(p->counts, 0, 4 * (size_t)p->N, s));
-  CAGEO_CUDA(cudaMemsetAsync(p->dscal + 1, 0, 2 * sizeof(uint32_t), s));
+  CAGEO_CUDA(cudaMemsetAsync(p->dscal + 1, 0, (kRedo - 1) * sizeof(uint32_t), s));
   CAGEO_CUDA(cudaStreamSynchronize(s));
   return CAGEO_OK;
 }
 
 extern "C" cageo_status cageo_pipeline_set_batch(cageo_pipeline* p, int batch) {
   CAGEO_CHECK_ARG(p, "null pipeline");
-  CAGEO_CHECK_ARG(batch >= 1 && batch <= 64, "batch must be 1..64 realizations");
+  CAGEO_CHECK_ARG(batch >= 1 && batch <= kMaxStack, "batch must be 1..64 realizations");
   if (batch > 1) {
     CAGEO_CHECK_ARG(p->cfg.fill_mode == CAGEO_FILL_CPU_COMPAT,
                     "batched steps need the CPU-compatible fill mode");
     CAGEO_CHECK_ARG((int64_t)batch * p->N < kMaxCells, "batch * grid cells must stay below 2^31");
   }
   CAGEO_CUDA(cudaStreamSynchronize(p->stream));
-  free_batch(p);
-  p->last_batched = false;
+  free_stack(p);
+  p->batch = 1;
+  p->plain = batch == 1;
   if (batch == 1) return CAGEO_OK;
-  const size_t nb = (size_t)batch * p->N;
-  cageo_status st;
-  if ((st = dalloc(&p->qb, sizeof(float) * nb)) || (st = dalloc(&p->filledb, sizeof(float) * nb)) ||
-      (st = dalloc(&p->fill_ws_b, fill_workspace_bytes(p->W, batch * p->H))) ||
-      (st = dalloc(&p->slab_min, sizeof(unsigned int) * 64)) ||
-      (st = dalloc(&p->dirb, 2 * nb)) ||
-      (st = dalloc(&p->route_ws_b, route_workspace_bytes(p->W, batch * p->H)))) {
-    free_batch(p);
-    return st;
-  }
-  p->rwb = route_carve(p->route_ws_b, p->W, batch * p->H);
-  p->rwb.slab_h = p->H;
-  p->fwb = fill_carve(p->fill_ws_b, p->W, batch * p->H);
-  p->fwb.slab_h = p->H;
-  p->fwb.slab_min = p->slab_min;
-  p->fwb.seeded = true;
-  sync_batch_tuning(p);
+  const cageo_status st = ensure_stack(p, batch);
+  if (st) return st;
+  set_step(p, batch);
   p->batch = batch;
   return CAGEO_OK;
 }
@@ -1075,8 +1166,9 @@ extern "C" cageo_status cageo_pipeline_warmstart_stats(cageo_pipeline* p, int64_
 
 extern "C" cageo_status cageo_pipeline_graph_kernels(cageo_pipeline* p, int64_t* h_count) {
   CAGEO_CHECK_ARG(p && h_count, "null argument");
-  // The batched step's graph when batching is on and it was captured.
-  cudaGraph_t g = (p->batch > 1 && p->exec_b) ? p->graph_b : (p->graph_ok ? p->graph : nullptr);
+  // The stacked step's graph where steps are stacked and it was captured.
+  cudaGraph_t g = (p->exec_b && (p->batch > 1 || !p->graph_ok)) ? p->graph_b
+                  : (p->graph_ok ? p->graph : nullptr);
   CAGEO_CHECK_ARG(g, "no step has been captured in a CUDA graph");
   size_t n = 0;
   CAGEO_CUDA(cudaGraphGetNodes(g, nullptr, &n));

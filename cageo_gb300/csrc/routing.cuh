@@ -40,29 +40,31 @@ struct TraceWork {
   int* state = nullptr;          // W*H: label, or the tile-border cell the path leaves by
   int* bstate = nullptr;         // 124 per 32x32 tile: the same for the tiles' border cells
   unsigned int* scal = nullptr;
+  // Stacked realizations: H / slab_h grids of slab_h rows each, one above the
+  // other, over one stream raster of slab_h rows; paths end at their slab's
+  // edge (0: one grid).
+  int slab_h = 0;
 };
 size_t trace_workspace_bytes(int W, int H);
 TraceWork trace_carve(void* base, int W, int H);
 // is_stream(c) = streams[c] >= 0; the label of a stream terminal is
-// (int)(-streams[c]).
+// (int)(-streams[c]).  code (may be null): the burn codes (front.cuh), whose
+// stream bit is read instead of the streams.
 // mode CAGEO_TRACE_DEAD_END_ERROR: cells whose path ends without an
 // outlet are ERROR instead of taking cell 0's label.
 // write_labels = false leaves the labels to border_u32_from_state.
-cageo_status trace_run(const int8_t* dir, const float* streams, int* label,
+cageo_status trace_run(const int8_t* dir, const float* streams, const uint8_t* code, int* label,
                        const TraceWork& w, cudaStream_t s, int mode, bool write_labels);
 cageo_status trace_check_status(const TraceWork& w, int64_t* jumps);
 
-// count[i] += border(label) for float (stage API) or uint32 (pipeline) counts.
+// count[i] += border(label) (stage API).
 cageo_status border_float(const int* label, float* count, int W, int H,
                           cudaStream_t s);
-cageo_status border_u32(const int* label, uint32_t* count, int W, int H,
-                        cudaStream_t s);
-// From the trace states of a trace_run without labels: writes the labels
-// (mode as for tracing) and adds the border mask unless *gate is set.
+// From the trace states of a trace_run without labels: adds the border masks
+// of all slabs unless *gate is set, and writes the labels (mode as for
+// tracing) of slab k where *real + k == *last (last null: of every slab).
 cageo_status border_u32_from_state(const TraceWork& w, int* label, uint32_t* count,
-                                   const int* gate, int mode, cudaStream_t s);
-// The same, skipped entirely when *gate (device) is non-zero.
-cageo_status border_u32_gated(const int* label, uint32_t* count, int W, int H,
-                              const int* gate, cudaStream_t s);
+                                   const int* gate, int mode, const uint32_t* real,
+                                   const uint32_t* last, cudaStream_t s);
 
 }  // namespace cageo

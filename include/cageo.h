@@ -321,22 +321,20 @@ cageo_status cageo_pipeline_run(cageo_pipeline* p, uint32_t first_realization,
 cageo_status cageo_pipeline_run_filter(cageo_pipeline* p, uint32_t first_realization,
                                        int count, int model, float practical_range,
                                        float error_mean, float error_stddev);
-/* Batched steps (no counterpart in the reference, whose Monte Carlo loop
- * runs one realization after another, src/main.cpp:180-283): with batch > 1
- * cageo_pipeline_run processes realizations `batch` at a time.  Their noise
- * and fused front run one after another into the slabs of a stacked grid,
- * one pit fill covers the whole stack (the slabs' borders are outlets, so no
- * value crosses between them), so does the routing (flat cells are interior
- * to their slab), and tracing and the border counts run per realization; a
- * batched step is captured in a CUDA graph of its own.
- * The counts and every stage output equal single realizations bit for bit;
- * batching only shares the persistent launches of the fill and the flat
- * BFS (their grid barriers and idle tails) among the realizations of a step.  A run
- * of `count` realizations takes count / batch batched steps and the rest
- * singly.  1 <= batch <= 64, batch * cells < 2^31, CPU-compatible fill
- * mode only.  Allocates the stacked grids and the fill and routing
- * workspaces for them (about 27 bytes per cell per realization); batch = 1
- * frees them. */
+/* Stacked steps (no counterpart in the reference, whose Monte Carlo loop
+ * runs one realization after another, src/main.cpp:180-283): realizations are
+ * processed several at a time, one above the other, each stage running once
+ * over the stack (the slabs' borders are outlets of the fill and drain
+ * outward, so nothing crosses between them).  The counts and every stage
+ * output equal single realizations bit for bit.  A step is captured in a CUDA
+ * graph of its own.
+ * Without a call of this, cageo_pipeline_run stacks the realizations of small
+ * grids by itself (up to 64, as many as make up 2^25 cells; both fill modes;
+ * not with a learned warm start) and runs singly where the memory for a stack
+ * (about 35 bytes per cell per realization, allocated by the first such run)
+ * cannot be had.  batch = 1: one realization at a time, no stacks; frees them.
+ * batch > 1: steps of that many whatever the grid, the rest of `count` singly;
+ * batch <= 64, batch * cells < 2^31, CPU-compatible fill mode only. */
 cageo_status cageo_pipeline_set_batch(cageo_pipeline* p, int batch);
 /* Border counts so far as float (the reference's CatchmentBorderType). */
 cageo_status cageo_pipeline_counts(cageo_pipeline* p, float* h_out);
@@ -364,8 +362,8 @@ cageo_status cageo_pipeline_load(cageo_pipeline* p, const char* path,
                                  uint32_t* next_realization);
 cudaStream_t cageo_pipeline_stream(cageo_pipeline* p);
 /* Kernel launches in the CUDA graph that one step replays (the graph's
- * kernel nodes; memset nodes are not counted): the batched step's graph when
- * batching is on and captured, else the single realization's.
+ * kernel nodes; memset nodes are not counted): the stacked step's graph where
+ * steps are stacked, else the single realization's.
  * CAGEO_ERR_ARGUMENT until a run has captured one.  No counterpart in the
  * reference. */
 cageo_status cageo_pipeline_graph_kernels(cageo_pipeline* p, int64_t* h_count);
