@@ -19,32 +19,16 @@
 //   W1[32][4][9], b1[32], W2[32][32][9], b2[32], W3[1][32][9], b3[1]
 // with taps t = (dy+1)*3 + (dx+1), a cell's output reading input (y+dy, x+dx).
 //
-// Training kernels (plain fp32 CUDA cores, planar [batch][channel][H][W]
-// activations): forward convolution, input gradients as the forward
-// convolution with flipped, transposed weights, weight gradients as per
-// (output, input) channel reductions, mean-squared-error loss, Adam.
-// Inference: one fused kernel per 32x16 tile of cells that computes the
-// features and the three layers in shared memory with bf16 mma.sync tensor
-// instructions (fp32 accumulation) and writes the warm surface.
+// Training: learned_train.cu.  Inference: one fused kernel per 32x16 tile of
+// cells that computes the features and the three layers in shared memory with
+// bf16 mma.sync tensor instructions (fp32 accumulation) and writes the warm
+// surface.
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
-#include <cuda_bf16.h>
-#include "common.cuh"
+#include "learned.cuh"
 
 namespace cageo {
-
-constexpr int kWsCin = 4, kWsCh = 32;
-constexpr int kOffW1 = 0, kOffB1 = 1152, kOffW2 = 1184, kOffB2 = 10400, kOffW3 = 10432,
-              kOffB3 = 10720, kWsParams = 10721;
-static_assert(kOffB1 == kWsCh * kWsCin * 9 && kOffW2 == kOffB1 + kWsCh &&
-                  kOffB2 == kOffW2 + kWsCh * kWsCh * 9 && kOffW3 == kOffB2 + kWsCh &&
-                  kOffB3 == kOffW3 + kWsCh * 9 && kWsParams == kOffB3 + 1,
-              "parameter layout");
-
-__host__ __device__ inline float bf16_round(float x) {
-  return __bfloat162float(__float2bfloat16_rn(x));
-}
 
 // ---- features ----------------------------------------------------------------
 // Per cell, from the burned realistic elevations v over the valid (in-grid,
@@ -95,141 +79,6 @@ __global__ void ws_features_kernel(const float* __restrict__ v, float* __restric
   ws_features(g[c], nodata, at, f);
   for (int k = 0; k < 4; k++) feat[((int64_t)b * 4 + k) * n + c] = f[k];
 }
-
-// ---- training: convolution forward (also used for input gradients) ----------
-// out[b][co](y,x) = bias[co] + sum_ci sum_t w[co][ci][t] * in[b][ci](y+dy, x+dx),
-// zero outside; optional ReLU.  Weights (bf16-rounded) staged in shared
-// memory; one thread per output cell, all output channels in registers.
-template <int COUT>
-__global__ void __launch_bounds__(128) ws_conv_fwd_kernel(const float* __restrict__ in,
-                                                          int cin, const float* __restrict__ w,
-                                                          const float* __restrict__ bias,
-                                                          float* __restrict__ out, int W, int H,
-                                                          int B, int relu) {
-  extern __shared__ float sw[];  // [COUT][cin][9]
-  for (int k = threadIdx.x; k < COUT * cin * 9; k += blockDim.x) sw[k] = bf16_round(w[k]);
-  __syncthreads();
-  const int64_t n = (int64_t)W * H;
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n * B) return;
-  const int b = (int)(i / n);
-  const int64_t c = i - (int64_t)b * n;
-  const int x = (int)(c % W), y = (int)(c / W);
-  float acc[COUT];
-#pragma unroll
-  for (int co = 0; co < COUT; co++) acc[co] = bias ? bf16_round(bias[co]) : 0.0f;
-  for (int ci = 0; ci < cin; ci++) {
-    const float* plane = in + ((int64_t)b * cin + ci) * n;
-#pragma unroll
-    for (int t = 0; t < 9; t++) {
-      const int xx = x + t % 3 - 1, yy = y + t / 3 - 1;
-      if (xx < 0 || yy < 0 || xx >= W || yy >= H) continue;
-      const float a = plane[(int64_t)yy * W + xx];
-#pragma unroll
-      for (int co = 0; co < COUT; co++) acc[co] = fmaf(sw[(co * cin + ci) * 9 + t], a, acc[co]);
-    }
-  }
-  float* o = out + (int64_t)b * COUT * n + c;
-#pragma unroll
-  for (int co = 0; co < COUT; co++) o[(int64_t)co * n] = relu ? fmaxf(acc[co], 0.0f) : acc[co];
-}
-
-// wt[ci][co][t] = w[co][ci][8 - t]: the weights of the input-gradient pass.
-__global__ void ws_flip_kernel(const float* __restrict__ w, float* __restrict__ wt, int cout,
-                               int cin) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= cout * cin * 9) return;
-  const int t = k % 9, ci = (k / 9) % cin, co = k / (9 * cin);
-  wt[(ci * cout + co) * 9 + (8 - t)] = w[k];
-}
-
-// g *= (a > 0): the ReLU's gradient mask.
-__global__ void ws_relu_mask_kernel(float* __restrict__ g, const float* __restrict__ a,
-                                    int64_t n) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n && !(a[i] > 0.0f)) g[i] = 0.0f;
-}
-
-// Weight gradients of one (output, input) channel pair per block:
-// gw[co][ci][t] += sum_b sum_cell dz[b][co](y,x) * a[b][ci](y+dy, x+dx);
-// the blocks with ci == 0 also add gb[co] += sum dz[b][co].
-__global__ void __launch_bounds__(256) ws_wgrad_kernel(const float* __restrict__ dz, int cout,
-                                                       const float* __restrict__ a, int cin,
-                                                       float* __restrict__ gw,
-                                                       float* __restrict__ gb, int W, int H,
-                                                       int B) {
-  const int co = blockIdx.x / cin, ci = blockIdx.x % cin;
-  const int64_t n = (int64_t)W * H;
-  float s[10] = {};
-  for (int b = 0; b < B; b++) {
-    const float* d = dz + ((int64_t)b * cout + co) * n;
-    const float* p = a + ((int64_t)b * cin + ci) * n;
-    for (int64_t c = threadIdx.x; c < n; c += blockDim.x) {
-      const float g = d[c];
-      if (g == 0.0f) continue;
-      const int x = (int)(c % W), y = (int)(c / W);
-#pragma unroll
-      for (int t = 0; t < 9; t++) {
-        const int xx = x + t % 3 - 1, yy = y + t / 3 - 1;
-        if (xx < 0 || yy < 0 || xx >= W || yy >= H) continue;
-        s[t] = fmaf(g, p[(int64_t)yy * W + xx], s[t]);
-      }
-      s[9] += g;
-    }
-  }
-  __shared__ float red[8][10];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int t = 0; t < 10; t++) {
-    float v = s[t];
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) red[wid][t] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x < 10) {
-    float v = 0.0f;
-    for (int k = 0; k < (int)(blockDim.x >> 5); k++) v += red[k][threadIdx.x];
-    if (threadIdx.x < 9) gw[(co * cin + ci) * 9 + threadIdx.x] += v;
-    else if (ci == 0 && gb) gb[co] += v;
-  }
-}
-
-// Mean squared error over the cells at least `margin` cells inside each
-// grid: dy = 2 (y - t) / count there, 0 elsewhere; loss (sum) accumulated.
-__global__ void ws_mse_kernel(const float* __restrict__ y, const float* __restrict__ t,
-                              float* __restrict__ dy, float* __restrict__ loss, int W, int H,
-                              int B, int margin, float inv_count) {
-  const int64_t n = (int64_t)W * H;
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  float l = 0.0f;
-  if (i < n * B) {
-    const int64_t c = i % n;
-    const int x = (int)(c % W), yy = (int)(c / W);
-    const bool in = x >= margin && yy >= margin && x < W - margin && yy < H - margin;
-    const float d = y[i] - t[i];
-    dy[i] = in ? 2.0f * d * inv_count : 0.0f;
-    l = in ? d * d * inv_count : 0.0f;
-  }
-  for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-  if ((threadIdx.x & 31) == 0 && l != 0.0f) atomicAdd(loss, l);
-}
-
-__global__ void ws_adam_kernel(float* __restrict__ p, const float* __restrict__ g,
-                               float* __restrict__ m, float* __restrict__ v, int n, float lr,
-                               float b1, float b2, float eps, float c1, float c2) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float gi = g[i];
-  const float mi = b1 * m[i] + (1.0f - b1) * gi;
-  const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-  m[i] = mi;
-  v[i] = vi;
-  p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-}
-
-}  // namespace cageo
-
-namespace cageo {
 
 // ---- inference: fused features + 3 layers on bf16 tensor instructions --------
 // A block owns a 32x16 tile of outputs; the layers need one more cell of
@@ -574,79 +423,6 @@ extern "C" cageo_status cageo_ws_features(const float* d_v, float* d_feat, int W
   CAGEO_CHECK_ARG(d_v && d_feat && valid_dims(W, H) && B >= 1, "pointers, size and batch");
   const int64_t n = (int64_t)W * H * B;
   ws_features_kernel<<<nblk(n, 256), 256, 0, stream>>>(d_v, d_feat, W, H, B, nodata_dem);
-  CAGEO_CUDA(cudaGetLastError());
-  return CAGEO_OK;
-}
-
-extern "C" cageo_status cageo_ws_forward(const float* d_params, const float* d_feat, int W,
-                                         int H, int B, float* d_a1, float* d_a2, float* d_out,
-                                         cudaStream_t stream) {
-  CAGEO_CHECK_ARG(d_params && d_feat && d_a1 && d_a2 && d_out && valid_dims(W, H) && B >= 1,
-                  "pointers, size and batch");
-  const int64_t n = (int64_t)W * H * B;
-  const unsigned g = nblk(n, 128);
-  ws_conv_fwd_kernel<32><<<g, 128, 32 * 4 * 9 * 4, stream>>>(
-      d_feat, 4, d_params + kOffW1, d_params + kOffB1, d_a1, W, H, B, 1);
-  ws_conv_fwd_kernel<32><<<g, 128, 32 * 32 * 9 * 4, stream>>>(
-      d_a1, 32, d_params + kOffW2, d_params + kOffB2, d_a2, W, H, B, 1);
-  ws_conv_fwd_kernel<1><<<g, 128, 32 * 9 * 4, stream>>>(d_a2, 32, d_params + kOffW3,
-                                                         d_params + kOffB3, d_out, W, H, B, 0);
-  CAGEO_CUDA(cudaGetLastError());
-  return CAGEO_OK;
-}
-
-extern "C" cageo_status cageo_ws_backward(const float* d_params, const float* d_feat,
-                                          const float* d_a1, const float* d_a2,
-                                          const float* d_dout, int W, int H, int B,
-                                          float* d_grad, float* d_tmp1, float* d_tmp2,
-                                          float* d_wflip, cudaStream_t stream) {
-  CAGEO_CHECK_ARG(d_params && d_feat && d_a1 && d_a2 && d_dout && d_grad && d_tmp1 && d_tmp2 &&
-                      d_wflip && valid_dims(W, H) && B >= 1,
-                  "pointers, size and batch");
-  const int64_t n = (int64_t)W * H * B, n32 = 32 * n;
-  const unsigned g = nblk(n, 128);
-  // Layer 3: weight gradients, then the gradient of its input (ReLU-masked).
-  ws_wgrad_kernel<<<32, 256, 0, stream>>>(d_dout, 1, d_a2, 32, d_grad + kOffW3,
-                                          d_grad + kOffB3, W, H, B);
-  ws_flip_kernel<<<nblk(288, 256), 256, 0, stream>>>(d_params + kOffW3, d_wflip, 1, 32);
-  ws_conv_fwd_kernel<32><<<g, 128, 32 * 1 * 9 * 4, stream>>>(d_dout, 1, d_wflip, nullptr, d_tmp1,
-                                                             W, H, B, 0);
-  ws_relu_mask_kernel<<<nblk(n32, 256), 256, 0, stream>>>(d_tmp1, d_a2, n32);
-  // Layer 2.
-  ws_wgrad_kernel<<<32 * 32, 256, 0, stream>>>(d_tmp1, 32, d_a1, 32, d_grad + kOffW2,
-                                               d_grad + kOffB2, W, H, B);
-  ws_flip_kernel<<<nblk(9216, 256), 256, 0, stream>>>(d_params + kOffW2, d_wflip, 32, 32);
-  ws_conv_fwd_kernel<32><<<g, 128, 32 * 32 * 9 * 4, stream>>>(d_tmp1, 32, d_wflip, nullptr,
-                                                              d_tmp2, W, H, B, 0);
-  ws_relu_mask_kernel<<<nblk(n32, 256), 256, 0, stream>>>(d_tmp2, d_a1, n32);
-  // Layer 1 (its input, the features, needs no gradient).
-  ws_wgrad_kernel<<<32 * 4, 256, 0, stream>>>(d_tmp2, 32, d_feat, 4, d_grad + kOffW1,
-                                              d_grad + kOffB1, W, H, B);
-  CAGEO_CUDA(cudaGetLastError());
-  return CAGEO_OK;
-}
-
-extern "C" cageo_status cageo_ws_mse(const float* d_y, const float* d_target, float* d_dy,
-                                     float* d_loss, int W, int H, int B, int margin,
-                                     cudaStream_t stream) {
-  CAGEO_CHECK_ARG(d_y && d_target && d_dy && d_loss && valid_dims(W, H) && B >= 1,
-                  "pointers, size and batch");
-  CAGEO_CHECK_ARG(margin >= 0 && 2 * margin < W && 2 * margin < H, "margin");
-  const int64_t n = (int64_t)W * H * B;
-  const float cnt = (float)(W - 2 * margin) * (float)(H - 2 * margin) * (float)B;
-  ws_mse_kernel<<<nblk(n, 256), 256, 0, stream>>>(d_y, d_target, d_dy, d_loss, W, H, B, margin,
-                                                  1.0f / cnt);
-  CAGEO_CUDA(cudaGetLastError());
-  return CAGEO_OK;
-}
-
-extern "C" cageo_status cageo_ws_adam(float* d_params, const float* d_grad, float* d_m,
-                                      float* d_v, int n, float lr, float beta1, float beta2,
-                                      float eps, int step, cudaStream_t stream) {
-  CAGEO_CHECK_ARG(d_params && d_grad && d_m && d_v && n > 0 && step >= 1, "arguments");
-  const float c1 = 1.0f - powf(beta1, (float)step), c2 = 1.0f - powf(beta2, (float)step);
-  ws_adam_kernel<<<nblk(n, 256), 256, 0, stream>>>(d_params, d_grad, d_m, d_v, n, lr, beta1,
-                                                   beta2, eps, c1, c2);
   CAGEO_CUDA(cudaGetLastError());
   return CAGEO_OK;
 }

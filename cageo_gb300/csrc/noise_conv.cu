@@ -16,6 +16,7 @@
 #include <algorithm>
 #include <type_traits>
 #include "common.cuh"
+#include "f32x2.cuh"
 #include "front.cuh"
 #include "stage_math.cuh"
 
@@ -194,15 +195,6 @@ __device__ __forceinline__ void tile_out(const float* s_out, int OS, int x0, int
 // cannot see -- the assembler contracts a packed multiply feeding a packed add
 // into one rounding, .rn notwithstanding; the product with 1 is exact, so this
 // fused operation rounds the sum alone.
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pack2(float a, float b) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
 __device__ __forceinline__ f32x2 muladd2_rn(f32x2 acc, f32x2 w, f32x2 t, f32x2 one) {
   f32x2 p;
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(p) : "l"(w), "l"(t));

@@ -6,7 +6,7 @@ a 1024 x 1024 fBm tile (Hurst 0.8, relief scaled from 300 m over 8192 cells
 to the tile's extent, pits, streams at accumulation 2000) plus one Philox
 noise realization (Gaussian filter, 60 m range, 1.5 m sd) gives the burned
 realistic grid v; the exact fill F of v gives the depth F - v.  The network
-(csrc/learned.cu) learns min(depth, cap) from the features of v: mean
+(csrc/learned_train.cu) learns min(depth, cap) from the features of v: mean
 squared error over random 128 x 128 crops with a 3-cell margin, Adam.  One
 pair per step, each (tile, realization) used once.
 
