@@ -27,7 +27,7 @@ constexpr int kConvTiles = 4;
 struct FrontParams {
   const float* dem;        // W*H
   const uint8_t* code;     // W*H static codes
-  float* q;                // W*H output: quantized burned realistic DEM (of a stack's first grid)
+  float* q;                // W*H output: quantized burned realistic DEM (grid blockIdx.z of a stack after it)
   unsigned int* min_ord;   // ordered-uint min of q (pit-fill minE), one per grid of a stack
   int* anomaly;            // set when the precomputed burn factor may not apply (per grid of a stack)
   float nodata_dem;
@@ -49,7 +49,7 @@ __device__ __forceinline__ float front_value(const FrontParams& p, float conv, f
   if (c & kCodeBurnStream) {
     // The reference tests a stream neighbour's elevation against NODATA;
     // the precomputed factors assume that test passes.
-    if (v == p.nodata_dem) atomicExch(p.anomaly, 1);
+    if (v == p.nodata_dem) atomicExch(p.anomaly + blockIdx.z, 1);
     v = 0.0f;
   }
   const int k = c & 0x1f;
@@ -62,7 +62,7 @@ __device__ __forceinline__ bool front_outlet(const FrontParams& p, int x, int y,
   return q == 0.0f || x == 0 || y == 0 || x == p.W - 1 || y == p.H - 1;
 }
 __device__ __forceinline__ void front_seed(const FrontParams& p, int x, int y) {
-  p.tseed[((p.row0 + y) >> 5) * p.tiles_x + (x >> 5)] = 1;
+  p.tseed[((p.row0 + (int)blockIdx.z * p.H + y) >> 5) * p.tiles_x + (x >> 5)] = 1;
 }
 
 }  // namespace cageo

@@ -99,7 +99,6 @@ __device__ __forceinline__ int wrap_idx(int v, int n) {
 struct StoreEpilogue {
   float* out;
   bool aligned;
-  __device__ __forceinline__ void slab(int, int64_t) {}
   __device__ __forceinline__ float cell(int64_t i, int, int, float v) const {
     out[i] = v;
     return v;
@@ -113,15 +112,13 @@ struct StoreEpilogue {
 struct FrontEpilogue {
   FrontParams p;
   bool aligned;
-  __device__ __forceinline__ void slab(int k, int64_t n) {
-    p.q += k * n;
-    p.min_ord += k;
-    p.anomaly += k;
-    p.row0 += k * p.H;
-  }
+  // The output grid: blockIdx.z is the grid of a stack.  (The parameters stay
+  // as they are: a changed copy would live in local memory, 0.72 instead of
+  // 0.58 ms at 8192^2.)
+  __device__ __forceinline__ float* out() const { return p.q + blockIdx.z * ((int64_t)p.W * p.H); }
   __device__ __forceinline__ float cell(int64_t i, int x, int y, float v) const {
     const float q = front_value(p, v, p.dem[i], p.code[i]);
-    p.q[i] = q;
+    out()[i] = q;
     if (front_outlet(p, x, y, q)) front_seed(p, x, y);
     return q;
   }
@@ -133,7 +130,7 @@ struct FrontEpilogue {
     q.y = front_value(p, v.y, d.y, (uint8_t)(c >> 8));
     q.z = front_value(p, v.z, d.z, (uint8_t)(c >> 16));
     q.w = front_value(p, v.w, d.w, (uint8_t)(c >> 24));
-    *reinterpret_cast<float4*>(p.q + i) = q;
+    *reinterpret_cast<float4*>(out() + i) = q;
     // (The four cells lie in one fill tile: x is a multiple of 4.)
     if (front_outlet(p, x, y, q.x) || front_outlet(p, x + 1, y, q.y) ||
         front_outlet(p, x + 2, y, q.z) || front_outlet(p, x + 3, y, q.w))
@@ -158,7 +155,7 @@ __device__ inline void block_min_out(float local_min, const FrontEpilogue& e) {
     float m = lane < nw ? red[lane] : kInf;
     for (int o = 16; o > 0; o >>= 1)
       m = fminf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if (lane == 0 && m < kInf) atomicMin(e.p.min_ord, float_to_ordered(m));
+    if (lane == 0 && m < kInf) atomicMin(e.p.min_ord + blockIdx.z, float_to_ordered(m));
   }
 }
 
@@ -253,7 +250,6 @@ conv_sep_kernel(const float* __restrict__ in, int W, int H,
   f32x2* s_tmp = reinterpret_cast<f32x2*>(s_in + in_floats);        // TH/2 x TS: rows 2j, 2j + 1
   const int x0 = blockIdx.x * TW, y0 = blockIdx.y * TH;
   in += blockIdx.z * (int64_t)W * H;  // a field of a stack
-  epi.slab(blockIdx.z, (int64_t)W * H);
   const f32x2 one2 = pack2(one, one);
   for (int t = threadIdx.x; t < L; t += kSepThreads) {
     const float v = taps[t];
@@ -361,7 +357,6 @@ conv_2d_kernel(const float* __restrict__ in, int W, int H,
   const f32x2 one2 = pack2(one, one);
   const int x0 = blockIdx.x * kTwoDTW, y0 = blockIdx.y * TH;
   in += blockIdx.z * (int64_t)W * H;  // a field of a stack
-  epi.slab(blockIdx.z, (int64_t)W * H);
   for (int t = threadIdx.x; t < L * L; t += NT) {
     const float v = filt[t];
     if (PAIRED) s_f2[t] = pack2(v, v);
