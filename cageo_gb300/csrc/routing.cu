@@ -32,6 +32,7 @@
 // stream, at 0, is never level with a flat cell: one above 0 has a direction,
 // one below 0 is lower).
 #include <algorithm>
+#include <type_traits>
 #include "common.cuh"
 #include "routing.cuh"
 #include "stage_math.cuh"
@@ -131,11 +132,11 @@ __device__ __forceinline__ int steepest_of(float c, const float (&v)[8], float n
   return best > 0.0f ? got : 8;
 }
 
-// Direction n as (dx, dy); n = 8: none.
-__device__ __forceinline__ char2 d8_dir(int n) {
-  // 2 bits per direction: dx + 1 and dy + 1.
-  const int dx = (int)((0x101a9u >> (2 * n)) & 3u) - 1, dy = (int)((0x11a90u >> (2 * n)) & 3u) - 1;
-  return make_char2((signed char)dx, (signed char)dy);
+// Direction n as (dx, dy) bytes; n = 8: none.
+__device__ __forceinline__ unsigned int d8_dir(int n) {
+  const unsigned int dx = __byte_perm(0x01010100u, 0xffffff00u, n);
+  const unsigned int dy = __byte_perm(0x0100ffffu, 0xff000101u, n);
+  return n < 8 ? __byte_perm(dx, dy, 0x0040u) & 0xffffu : 0u;
 }
 
 // Staged elevations of a tile and the two cells around it: rows y0 - 2 ..
@@ -214,8 +215,14 @@ __global__ void __launch_bounds__(256) d8_kernel(const float* __restrict__ dem,
     while (ys >= slab_h) ys -= slab_h;
     return ys;
   };
-  int code[4];  // 0..7: direction; 8: flat; 9: border; 10: stream, NODATA or outside
-  {
+  // A tile of interior cells only needs no test of the border or the grid.
+  const int top = y0 % slab_h;
+  const bool plain = x0 > 0 && x0 + kFT < W && top > 0 && top + kFT < slab_h && y0 + kFT <= H;
+  // 0..7: direction; 8: flat (| the level neighbours << 4, a bit per direction);
+  // 9: border; 10: stream, NODATA or outside
+  int code[4];
+  auto directions = [&](auto interior) {
+    constexpr bool kPlain = decltype(interior)::value;
     const float* e = E + (4 * warp + 1) * kES + lane + 3;  // row above this warp's first
     float a0 = e[0], a1 = e[1], a2 = e[2];
     float b0 = e[kES], b1 = e[kES + 1], b2 = e[kES + 2];
@@ -223,15 +230,24 @@ __global__ void __launch_bounds__(256) d8_kernel(const float* __restrict__ dem,
     for (int k = 0; k < 4; k++) {
       const float* r = e + (k + 2) * kES;
       const float c0 = r[0], c1 = r[1], c2 = r[2];
-      const int ys = slab_row(k);
       const float v[8] = {a1, a2, b2, c2, c1, c0, b0, a0};
       int n = steepest_of<GPU>(b1, v, nodata);
       if (b1 == 0.0f || (GPU && b1 == nodata)) n = 10;
-      if (xborder || ys == 0 || ys == slab_h - 1) n = 9;
-      if (!xin || yw + k >= H) n = 10;
-      code[k] = n;
-      const unsigned int h = __ballot_sync(0xffffffffu, n < 8 || n == 9);
+      if constexpr (!kPlain) {
+        const int ys = slab_row(k);
+        if (xborder || ys == 0 || ys == slab_h - 1) n = 9;
+        if (!xin || yw + k >= H) n = 10;
+      }
       const unsigned int f = __ballot_sync(0xffffffffu, n == 8);
+      const unsigned int h = __ballot_sync(0xffffffffu, kPlain ? n < 8 : n < 8 || n == 9);
+      code[k] = n;
+      if (f) {  // (no neighbour is lower: <= is level)
+        int level = 0;
+#pragma unroll
+        for (int d = 0; d < 8; d++)
+          if (v[d] <= b1 && !(GPU && v[d] == nodata)) level |= 16 << d;
+        if (n == 8) code[k] |= level;
+      }
       if (lane == 0) {
         Hd[4 * warp + k + 1] = h;
         F[4 * warp + k] = f;
@@ -239,7 +255,9 @@ __global__ void __launch_bounds__(256) d8_kernel(const float* __restrict__ dem,
       a0 = b0; a1 = b1; a2 = b2;
       b0 = c0; b1 = c1; b2 = c2;
     }
-  }
+  };
+  if (plain) directions(std::true_type());
+  else directions(std::false_type());
   // The ring: rows -1 and 32 (warps 0, 1), columns -1 and 32 (2, 3), corners.
   if (warp < 5) {
     const bool col = warp == 2 || warp == 3, corner = warp == 4;
@@ -273,24 +291,22 @@ __global__ void __launch_bounds__(256) d8_kernel(const float* __restrict__ dem,
   for (int k = 0; k < 4; k++) {
     const int ty = 4 * warp + k, y = y0 + ty;
     const unsigned int gs = row3(ty + 2);
-    int n = code[k];
+    int n = code[k] & 15;
     bool first = false;
     if (n == 8) {
       nflat++;
-      // 8 bits in N..NW order.
-      const unsigned int m = (gn >> 1 & 3u) | (gm & 4u) | (gs & 4u) << 1 | (gs & 2u) << 3 |
-                             (gs & 1u) << 5 | (gm & 1u) << 6 | (gn & 1u) << 7;
-      if (m) {
-        const float* e = E + (ty + 2) * kES + lane + 4;
-        const float c = *e;
+      // 8 bits in N..NW order: level neighbours with a direction.
+      const unsigned int m = ((gn >> 1 & 3u) | (gm & 4u) | (gs & 4u) << 1 | (gs & 2u) << 3 |
+                              (gs & 1u) << 5 | (gm & 1u) << 6 | (gn & 1u) << 7) &
+                             (unsigned int)code[k] >> 4;
+      first = m != 0;
+      if (GPU) {
         constexpr int order[8] = {0, 6, 2, 4, 7, 1, 5, 3};  // N W E S NW NE SW SE as D8 indices
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-          const int d = GPU ? order[7 - j] : j;  // the last match stays
-          const float v = e[d8_dy(d) * kES + d8_dx(d)];
-          if ((m >> d & 1u) && v <= c && !(GPU && v == nodata)) n = d;
-        }
-        first = n != 8;
+        for (int j = 7; j >= 0; j--)
+          if (m >> order[j] & 1u) n = order[j];
+      } else if (first) {
+        n = 31 - __clz(m);  // the last in D8 order
       }
     }
     gn = gm;
@@ -299,18 +315,16 @@ __global__ void __launch_bounds__(256) d8_kernel(const float* __restrict__ dem,
     if (lane == 0) S[ty] = s;
     if (!xin || y >= H) continue;
     const int64_t i = (int64_t)y * W + x;
-    char2 d;
+    unsigned int d = d8_dir(n);
     if (n == 9) {
       const int ys = slab_row(k);
-      d = make_char2((signed char)(x == 0 ? -1 : x == W - 1 ? 1 : 0),
-                     (signed char)(ys == 0 ? -1 : ys == slab_h - 1 ? 1 : 0));
-    } else {
-      d = d8_dir(min(n, 8));
+      const int dx = x == 0 ? -1 : x == W - 1 ? 1 : 0, dy = ys == 0 ? -1 : ys == slab_h - 1 ? 1 : 0;
+      d = (dx & 0xff) | (dy & 0xff) << 8;
     }
-    dir[i] = d;
+    reinterpret_cast<unsigned short*>(dir)[i] = (unsigned short)d;
     if (fd) {
       // Flat cells beyond layer 1 start unresolved (0).
-      fd[i] = code[k] == 8 ? (first ? 1 : 0)
+      fd[i] = (code[k] & 15) == 8 ? (first ? 1 : 0)
               : code[k] != 10 ? -1
               : (GPU && E[(ty + 2) * kES + lane + 4] != 0.0f) ? -3 : -2;
     }
@@ -661,7 +675,7 @@ __global__ void __launch_bounds__(kDirWarps * 32) flat_dir_kernel(char2* __restr
       if (c[d8_dy(n) * kDS + d8_dx(n)] == d - 1) got = n;
     }
     const int64_t i = (int64_t)(y0 + y) * w.W + x;
-    dir[i] = d8_dir(got);
+    reinterpret_cast<unsigned short*>(dir)[i] = (unsigned short)d8_dir(got);
     if (fd) fd[i] = d;
   }
 }
