@@ -58,8 +58,7 @@ namespace cageo {
 enum : int {
   S_MIN = 0,       // ordered min of q (minE)
   S_ERR = 3,       // 0 ok; 1 barrier wait; 2 idle wait; 3 queue state; 4 visits; 5 phases; 6 union
-  S_FLAG = 7,      // resolution: something happened in this round
-  S_RESULT = 8,    // ... and its value at the last barrier
+  S_RESULT = 8,    // resolution: whether a thread passed true to the last barrier
   S_MORE_AT = 9,   // S_MORE at the last barrier
   S_CAND = 10,     // walls on the list of the resolution
   S_MORE = 22,     // cells listed by the resolution itself
@@ -180,17 +179,6 @@ __device__ __forceinline__ void flush_stats(const FillWork& w, VisitStats& st, b
 // Lock-free union-find over the cells of the resolution (w.label): links
 // always point to a smaller cell index, so no cycle can form; roots are
 // hooked with CAS, paths halved with plain stores.  Bounded loops.
-__device__ __forceinline__ uint32_t uf_find(uint32_t* lab, uint32_t x) {
-  for (int it = 0; it < (1 << 20); it++) {
-    uint32_t p = ((volatile uint32_t*)lab)[x];
-    if (p == x) return x;
-    uint32_t g = ((volatile uint32_t*)lab)[p];
-    if (g != p) lab[x] = g;
-    x = p;
-  }
-  return x;
-}
-
 // The root without path halving: the flattening pass writes each cell's
 // root while other threads walk the same paths, and a halving store that
 // landed after such a write would replace the root by an ancestor below
@@ -205,12 +193,23 @@ __device__ __forceinline__ uint32_t uf_root(const uint32_t* lab, uint32_t x) {
   return x;
 }
 
+// Both paths are climbed at once, so a step's two reads overlap.
 __device__ __forceinline__ bool uf_unite(uint32_t* lab, uint32_t a, uint32_t b) {
-  for (int it = 0; it < (1 << 16); it++) {
-    uint32_t ra = uf_find(lab, a), rb = uf_find(lab, b);
-    if (ra == rb) return true;
-    if (ra > rb) { uint32_t t = ra; ra = rb; rb = t; }
-    if (atomicCAS(&lab[rb], rb, ra) == rb) return true;
+  volatile uint32_t* l = lab;
+  for (int it = 0; it < (1 << 20); it++) {
+    if (a == b) return true;
+    const uint32_t pa = l[a], pb = l[b];
+    if (pa == a && pb == b) {
+      const uint32_t lo = min(a, b), hi = max(a, b);
+      if (atomicCAS(&lab[hi], hi, lo) == hi) return true;
+      continue;
+    }
+    // Two steps up where there are two; the cell passed points there, too.
+    const uint32_t ga = l[pa], gb = l[pb];
+    if (ga != pa) lab[a] = ga;
+    if (gb != pb) lab[b] = gb;
+    a = ga;
+    b = gb;
   }
   return false;
 }
@@ -550,12 +549,11 @@ __device__ bool any_of(const FillWork& w, unsigned int nblocks, bool mine, unsig
       sh_more = vs[S_MORE];
     } else {
       const unsigned int gen = vs[S_BAR_GEN];
-      if (block) atomicOr(&w.scal[S_FLAG], 1u);
-      __threadfence();
-      if (atomicAdd(&w.scal[S_BAR_COUNT], 1u) == nblocks - 1) {
+      // The count of the arrivals, and 65536 times that of those with a true.
+      const unsigned int arrived = atomicAdd(&w.scal[S_BAR_COUNT], block ? 65537u : 1u);
+      if ((arrived & 0xffffu) == nblocks - 1) {
         vs[S_BAR_COUNT] = 0u;
-        vs[S_RESULT] = vs[S_FLAG];
-        vs[S_FLAG] = 0u;
+        vs[S_RESULT] = block || arrived >> 16 ? 1u : 0u;
         vs[S_MORE_AT] = vs[S_MORE];
         __threadfence();
         atomicAdd(&w.scal[S_BAR_GEN], 1u);
@@ -587,9 +585,11 @@ __device__ bool any_of(const FillWork& w, unsigned int nblocks, bool mine, unsig
 }
 
 constexpr int kResolveThreads = 1024;
-constexpr int kResolveRun = 1024;   // entries of the list a block takes at a time (walls)
-constexpr int kReopenRun = 256;     // the same for the cells of reopened components
-constexpr int kFrontCells = 1024;
+// Entries of the list a block takes at a time at most (walls; cells of reopened
+// components), and entries per block of the launch: with 1024 a block (one
+// on a grid of 512x512) the passes over the list took several turns each.
+constexpr unsigned int kResolveRun = 1024, kReopenRun = 256, kResolveShare = 256;
+constexpr int kFrontCells = 1024, kFreshCells = 2048;
 
 // A block's front: cells whose level fell (or walls that have come to relay),
 // with that level; one buffer is read while the other fills.  Three counters
@@ -599,7 +599,25 @@ struct Front {
   float level[2][kFrontCells];
   int n[3];
   int full;  // an entry did not fit: its cell was marked kActive instead
+  // Cells to list.  They are listed many at a time: an addition to the list's
+  // length in every step made it three dependent L2 accesses instead of two.
+  uint32_t fresh[kFreshCells];
+  int nfresh;
+  unsigned int at;
 };
+
+// The whole block: lists the fresh cells from entry `end` + S_MORE on.
+__device__ void list_fresh(const Resolve& r, Front& f, unsigned int end) {
+  __syncthreads();
+  const int n = min(f.nfresh, kFreshCells);
+  if (n == 0) return;
+  if (threadIdx.x == 0) f.at = atomicAdd(&r.w.scal[S_MORE], (unsigned int)n);
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += blockDim.x) __stcg(r.w.cand + end + f.at + i, f.fresh[i]);
+  __syncthreads();
+  if (threadIdx.x == 0) f.nfresh = 0;
+  __syncthreads();
+}
 
 __device__ __forceinline__ void front_push(const Resolve& r, Front& f, int buf, int cnt, uint32_t c,
                                            float lv) {
@@ -624,7 +642,8 @@ __device__ __forceinline__ void front_push(const Resolve& r, Front& f, int buf, 
 // start, so what counts is the time of a step.  Each block follows the fronts
 // of its own entries with no grid barrier in between: 8 lanes per cell, one
 // per neighbour, two dependent L2 accesses (the neighbour's level and
-// elevation, the atomicMin) and one block barrier a step.  Levels fall in any
+// elevation, the atomicMin) and one block barrier a step (1.2 us; 1.6 with the
+// list's length raised in every step).  Levels fall in any
 // order, and a cell two blocks reach is followed by whichever lowers it.
 // (Grid-wide rounds over the list took 3.3 ms at 8192^2, a flag beside each
 // level -- two accesses more a step -- 0.7 ms.)  Blocks take runs of
@@ -632,22 +651,21 @@ __device__ __forceinline__ void front_push(const Resolve& r, Front& f, int buf, 
 template <bool LOWER>
 __device__ unsigned int relax(const Resolve& r, Front& f, const uint32_t* list, unsigned int nl,
                               unsigned int nblocks, unsigned int* more, bool* ok) {
-  constexpr int kRun = LOWER ? kResolveRun : kReopenRun;
   const FillWork& w = r.w;
   const unsigned int nu0 = nl;
   unsigned int steps = 0;
   for (bool again = true; again;) {
     const unsigned int nu = LOWER ? nl + *more : nl;
-    if (threadIdx.x == 0) f.full = 0;
-    for (unsigned int base = blockIdx.x * kRun; base < nu; base += nblocks * kRun) {
+    const unsigned int run = min(LOWER ? kResolveRun : kReopenRun, (nu + nblocks - 1) / nblocks);
+    if (threadIdx.x == 0) f.full = f.nfresh = 0;
+    for (unsigned int base = blockIdx.x * run; base < nu; base += nblocks * run) {
       __syncthreads();
       if (threadIdx.x < 3) f.n[threadIdx.x] = 0;
       __syncthreads();
       // The active entries that can lower a neighbour.
-#pragma unroll
-      for (int i = 0; i < (kRun + kResolveThreads - 1) / kResolveThreads; i++) {
-        const unsigned int j = base + i * kResolveThreads + threadIdx.x;
-        if (j >= min(nu, base + kRun)) continue;
+      static_assert(kResolveRun <= kResolveThreads && kReopenRun <= kResolveThreads, "one a thread");
+      const unsigned int j = base + threadIdx.x;
+      for (bool once = j < min(nu, base + run); once; once = false) {
         const uint32_t c = __ldcg(list + j);
         const unsigned int fl = r.get(c);
         if (LOWER) {
@@ -675,7 +693,9 @@ __device__ unsigned int relax(const Resolve& r, Front& f, const uint32_t* list, 
       }
       int buf = 0, cnt = 0;
       for (;;) {
-        __syncthreads();
+        // (A half full buffer is emptied; what does not fit a step is listed at once.)
+        if (__syncthreads_or(LOWER && threadIdx.x == 0 && f.nfresh > kFreshCells / 2))
+          list_fresh(r, f, nu0);
         const int nf = min(f.n[cnt], kFrontCells);
         const int nxt = cnt == 2 ? 0 : cnt + 1;
         if (threadIdx.x == 0) f.n[nxt == 2 ? 0 : nxt + 1] = 0;
@@ -692,28 +712,31 @@ __device__ unsigned int relax(const Resolve& r, Front& f, const uint32_t* list, 
           if (nx < 0 || nx >= w.W || ny < 0 || ny >= w.H) continue;
           const int64_t b = (int64_t)ny * w.W + nx;
           const float qb = r.q[b], nv = fmaxf(qb, lv);
+          const unsigned int fl = LOWER ? 0u : r.get(b);  // (kConfirmed does not change meanwhile)
           // (Outlets are at their elevation.)
           if (!(nv < r.level(b)) || qb == r.nodata) continue;
           const int mine = (int)(__float_as_uint(nv) | 0x80000000u);
           const int prev = atomicMin(reinterpret_cast<int*>(r.Wg + b), mine);
           if (LOWER) {
             const bool first = prev >= 0;
-            const unsigned int pos = warp_append(&w.scal[S_MORE], first);
+            const unsigned int at = warp_append((unsigned int*)&f.nfresh, first);
             if (first) {
               __stcg(w.aux + b, (unsigned int)prev);
               __stcg(w.label + b, (uint32_t)b);
-              __stcg(w.cand + nu0 + pos, (uint32_t)b);
+              if (at < kFreshCells) f.fresh[at] = (uint32_t)b;
+              else __stcg(w.cand + nu0 + atomicAdd(&w.scal[S_MORE], 1u), (uint32_t)b);
             }
           }
           if (prev <= mine) continue;
           // A wall that falls was above its q, so LOWER lets it relay.
-          if (LOWER || !r.wall(b, qb) || ((r.get(b) & kConfirmed) && nv > qb))
+          if (LOWER || !r.wall(b, qb) || ((fl & kConfirmed) && nv > qb))
             front_push(r, f, buf ^ 1, nxt, (uint32_t)b, nv);
         }
         buf ^= 1;
         cnt = nxt;
       }
     }
+    if (LOWER) list_fresh(r, f, nu0);
     __syncthreads();
     again = any_of(w, nblocks, f.full != 0, more, ok);
   }
@@ -728,7 +751,7 @@ __global__ void __launch_bounds__(kResolveThreads, 1) fill_resolve_kernel(Resolv
   const FillWork& w = r.w;
   volatile unsigned int* vs = w.scal;
   const unsigned int nu0 = vs[S_CAND];  // (final before the launch)
-  const unsigned int nblocks = min(gridDim.x, max(1u, (nu0 + kResolveRun - 1) / kResolveRun));
+  const unsigned int nblocks = min(gridDim.x, max(1u, (nu0 + kResolveShare - 1) / kResolveShare));
   if (blockIdx.x >= nblocks) return;
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t nthreads = (int64_t)nblocks * blockDim.x;
@@ -746,27 +769,26 @@ __global__ void __launch_bounds__(kResolveThreads, 1) fill_resolve_kernel(Resolv
   // neighbours among them (each pair once).  Reopened components: those with
   // a wall that S left above its q and A took to it.
   bool reopen = false, united = true;
-  auto member = [&](int64_t c, float* lv, float* s) {
-    bool listed;
-    *lv = r.level(c, &listed);
-    if (!listed || r.q[c] == r.nodata) return false;
-    *s = r.walled(c);
-    return *lv != *s;
-  };
-  for (int64_t j = tid; j < nu; j += nthreads) {
-    const uint32_t c = __ldcg(w.cand + j);
-    float lv, s, lb, sb;
-    if (!member(c, &lv, &s)) continue;
-    r.set(c, kMember);
-    const float qc = r.q[c];
-    reopen |= lv <= qc && s > qc && r.wall(c, qc);
+  // Four threads a cell, one per neighbour.  (Their levels first: most
+  // neighbours are not listed.)
+  for (int64_t j = tid; j < 4 * (int64_t)nu; j += nthreads) {
+    const int d = (int)(j & 3);
+    const uint32_t c = __ldcg(w.cand + (j >> 2));
     const int cx = (int)(c % (uint32_t)w.W), cy = (int)(c / (uint32_t)w.W);
-    for (int d = 0; d < 4; d++) {
-      const int nx = cx + (d == 0 ? -1 : d - 2), ny = cy + (d == 0 ? 0 : -1);
-      if (nx < 0 || ny < 0 || nx >= w.W) continue;
-      const uint32_t b = (uint32_t)ny * (uint32_t)w.W + (uint32_t)nx;
-      if (member(b, &lb, &sb)) united &= uf_unite(w.label, c, b);
+    const int nx = cx + (d == 0 ? -1 : d - 2), ny = cy + (d == 0 ? 0 : -1);
+    const bool in = nx >= 0 && ny >= 0 && nx < w.W;
+    const uint32_t b = in ? (uint32_t)ny * (uint32_t)w.W + (uint32_t)nx : c;
+    bool lb;
+    const float wc = r.level(c), wb = r.level(b, &lb);
+    const float qc = r.q[c], sc = r.walled(c);
+    if (wc == sc || qc == r.nodata) continue;  // not a member
+    if (d == 0) {
+      r.set(c, kMember);
+      reopen |= wc <= qc && sc > qc && r.wall(c, qc);
     }
+    if (!in || !lb) continue;
+    const float qb = r.q[b], sb = r.walled(b);
+    if (wb != sb && qb != r.nodata) united &= uf_unite(w.label, c, b);
   }
   if (!united) atomicCAS((int*)(w.scal + S_ERR), 0, 6);
   if (nu0 && any_of(w, nblocks, reopen, &more, &ok)) {
@@ -797,15 +819,23 @@ __global__ void __launch_bounds__(kResolveThreads, 1) fill_resolve_kernel(Resolv
         const float qc = r.q[c], lv = r.level(c), s = r.walled(c);
         float start = s;
         const int x = (int)(c % (uint32_t)w.W), y = (int)(c / (uint32_t)w.W);
-#pragma unroll 1
+        unsigned int near = 0;  // the listed neighbours
+        float lb[8];
+#pragma unroll
         for (int k = 0; k < 8; k++) {
           const int nx = x + d8_dx(k), ny = y + d8_dy(k);
           if (nx < 0 || nx >= w.W || ny < 0 || ny >= w.H) continue;
-          const int64_t b = (int64_t)ny * w.W + nx;
           bool listed;
-          const float lb = r.level(b, &listed), qb = r.q[b];
-          if (listed && qb != r.nodata && !(r.get(b) & kMember) && lb > qb && r.wall(b, qb))
-            start = fminf(start, fmaxf(qc, lb));
+          lb[k] = r.level((int64_t)ny * w.W + nx, &listed);
+          if (listed) near |= 1u << k;
+        }
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+          if (!(near >> k & 1u)) continue;
+          const int64_t b = (int64_t)(y + d8_dy(k)) * w.W + x + d8_dx(k);
+          const float qb = r.q[b];
+          if (lb[k] > qb && qb != r.nodata && !(r.get(b) & kMember) && r.wall(b, qb))
+            start = fminf(start, fmaxf(qc, lb[k]));
         }
         const bool confirm = lv > qc && s > qc && r.wall(c, qc);
         if (confirm || start < s) r.set(c, (confirm ? kConfirmed : 0u) | kActive);
@@ -824,10 +854,10 @@ __global__ void __launch_bounds__(kResolveThreads, 1) fill_resolve_kernel(Resolv
       auto pending = [&](int64_t j, uint32_t& c, float& lv, float& qc) {
         c = __ldcg(open_list + j);
         const unsigned int f = r.get(c);
-        if (!(f & kMember) || (f & kConfirmed)) return false;
-        if (!apart && !(r.get(__ldcg(w.label + c)) & kReopened)) return false;
         qc = r.q[c];
         lv = r.level(c);
+        if (!(f & kMember) || (f & kConfirmed)) return false;
+        if (!apart && !(r.get(__ldcg(w.label + c)) & kReopened)) return false;
         return lv > qc && r.wall(c, qc);
       };
       bool some = false;
@@ -954,7 +984,7 @@ static cageo_status launch_resolve(const Resolve& r, cudaStream_t s) {
   void* params[] = {&args};
   // No more blocks than a list of every cell would need.
   const int64_t n = (int64_t)r.w.W * r.w.H;
-  const int grid = (int)std::min<int64_t>(blocks, (n + kResolveRun - 1) / kResolveRun);
+  const int grid = (int)std::min<int64_t>(blocks, (n + kResolveShare - 1) / kResolveShare);
   CAGEO_CUDA(cudaLaunchCooperativeKernel((const void*)fill_resolve_kernel, dim3(grid),
                                          dim3(kResolveThreads), params, 0, s));
   return CAGEO_OK;

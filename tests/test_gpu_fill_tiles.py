@@ -95,3 +95,24 @@ def test_batched_only_pipeline_reports_its_own_status(cuda):
     one = api.Pipeline(dem, streams, error_stddev=1.5, seed=4)
     one.run(0, 4)
     assert np.array_equal(p.counts(), one.counts())
+
+
+@pytest.mark.parametrize("n", [60, 600])
+def test_basin_behind_one_wall_cell(cuda, oracle, n):
+    """A flat basin that drains through a single non-passable cell of a flooded
+    tunnel: the resolution lowers n x n cells from one entry, in steps that
+    outgrow its buffers."""
+    import torch
+    from cageo_gb300 import api
+    k = np.arange(2001, 4000)
+    q = (k / 1000).astype(np.float32)
+    wall = q[np.trunc(np.float32(1000) * q) < k][0]
+    dem = np.full((n + 40, n + 30), 100.0, np.float32)
+    dem[0] = dem[-1] = dem[:, 0] = dem[:, -1] = 1.0
+    dem[0, 0] = 0.0
+    dem[20, 1], dem[20, 2:10], dem[20, 10] = 20.0, 2.0, wall
+    dem[15:15 + n, 11:11 + n] = 10.0
+    _, f_ref = oracle.pitfill(dem)
+    assert f_ref[300 if n == 600 else 40, 40] == 20.0
+    f = api.pitfill(torch.from_numpy(dem).to(cuda))
+    assert np.array_equal(bits(f.cpu().numpy()), bits(f_ref))
