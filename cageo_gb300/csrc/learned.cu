@@ -26,6 +26,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <type_traits>
 #include "learned.cuh"
 
 namespace cageo {
@@ -85,25 +86,42 @@ __global__ void ws_features_kernel(const float* __restrict__ v, float* __restric
 // context each: layer-2 outputs over 34x18, layer-1 outputs over 36x20,
 // features over 38x22, elevations over 44x28 (the 7x7 feature window).
 // Everything outside the grid is zero for the convolutions (their padding).
+//
+// Two blocks of 8 warps share an SM, so that one computes features or waits
+// where the other keeps the tensor cores busy, and a layer's 32 to 45 m-tiles
+// divide well among the warps: 908 -> @T us for 3001x2003 cells (one block of
+// 16 warps: layer 2's 39 m-tiles took 3 turns of which the last had 7 warps,
+// and nothing ran beside the features).  What makes two blocks fit is one
+// 64-byte row per activation (swizzled, not padded), the features in the layer
+// 2 buffer until that layer runs, and layer 3's weights without the output
+// columns that do not exist.  The elevations of the next tile arrive during
+// the layers.  The order of every sum is the layers' k order.
 constexpr int kTX = 32, kTY = 16;
 constexpr int kVX = kTX + 12, kVY = kTY + 12;    // elevations
 constexpr int kFX = kTX + 6, kFY = kTY + 6;      // features
 constexpr int kA1X = kTX + 4, kA1Y = kTY + 4;    // layer-1 outputs
 constexpr int kA2X = kTX + 2, kA2Y = kTY + 2;    // layer-2 outputs
-constexpr int kAS = 40;                          // activation row stride (bf16), 80 B
 constexpr int kW1S = 56, kW2S = 296;             // weight row strides (bf16)
-constexpr int kInferWarps = 16;
+constexpr int kInferWarps = 8;
 
-struct InferSmem {
-  float v[kVY * kVX];
-  __nv_bfloat16 f[kFY * kFX * 4];
-  __nv_bfloat16 a1[kA1Y * kA1X * kAS];
-  __nv_bfloat16 a2[kA2Y * kA2X * kAS];
-  __nv_bfloat16 w1[kWsCh * kW1S];     // [n][k], k = tap*4 + ci (36 used, 48 in the k-steps)
+struct __align__(128) InferSmem {
+  __nv_bfloat16 a1[kA1Y * kA1X * kWsCh];  // rows swizzled, see act()
+  union {
+    __nv_bfloat16 a2[kA2Y * kA2X * kWsCh];
+    __nv_bfloat16 f[kFY * kFX * 4];
+  };
   __nv_bfloat16 w2[kWsCh * kW2S];     // [n][k], k = tap*32 + ci
-  __nv_bfloat16 w3[8 * kW2S];         // [n][k], only n = 0 non-zero
+  __nv_bfloat16 w1[kWsCh * kW1S];     // [n][k], k = tap*4 + ci (36 used, 48 in the k-steps)
+  __nv_bfloat16 w3[kWsCh * 9];        // [k], k = tap*32 + ci
+  float v[kVY * kVX];
   float b1[kWsCh], b2[kWsCh], b3;
 };
+static_assert(2 * (sizeof(InferSmem) + 1024) <= 227 * 1024, "two blocks per SM");
+
+// Index of channel chunk c (8 channels, 16 bytes) of activation r.  The chunks
+// of a row of 64 bytes are permuted by the row's index, so that the same chunk
+// of 8 consecutive rows lies in 8 different 16-byte columns of the banks.
+__device__ __forceinline__ int act(int r, int c) { return r * kWsCh + ((c ^ ((r >> 1) & 3)) << 3); }
 
 __device__ __forceinline__ uint32_t ld32(const __nv_bfloat16* p) {
   return *reinterpret_cast<const uint32_t*>(p);
@@ -118,7 +136,7 @@ __device__ __forceinline__ void mma_bf16(float c[4], uint32_t a0, uint32_t a1, u
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// ldmatrix: four (two) 8x8 b16 matrices from shared memory; lane i gives
+// ldmatrix: four 8x8 b16 matrices from shared memory; lane i gives
 // the address of row i % 8 of matrix i / 8 (16 contiguous bytes, 16-byte
 // aligned), and receives the elements (row i / 4, columns 2 (i % 4) and
 // 2 (i % 4) + 1) of each matrix in order: the mma.sync fragment layout.
@@ -131,20 +149,12 @@ __device__ __forceinline__ void ldsm_x4(uint32_t& r0, uint32_t& r1, uint32_t& r2
                : "memory");
 }
 
-__device__ __forceinline__ void ldsm_x2(uint32_t& r0, uint32_t& r1, const void* p) {
-  const unsigned a = (unsigned)__cvta_generic_to_shared(p);
-  asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];\n"
-               : "=r"(r0), "=r"(r1)
-               : "r"(a)
-               : "memory");
-}
-
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
-__global__ void __launch_bounds__(kInferWarps * 32, 1)
+__global__ void __launch_bounds__(kInferWarps * 32, 2)
 ws_infer_kernel(const float* __restrict__ params, const float* __restrict__ vg,
                 float* __restrict__ warm, float* __restrict__ depth, int W, int H, float nodata,
                 float threshold) {
@@ -165,37 +175,27 @@ ws_infer_kernel(const float* __restrict__ params, const float* __restrict__ vg,
     if (kk < 288) w = params[kOffW2 + (n * kWsCh + kk % 32) * 9 + kk / 32];
     s.w2[k] = __float2bfloat16_rn(w);
   }
-  for (int k = tid; k < 8 * kW2S; k += blockDim.x) {
-    const int n = k / kW2S, kk = k % kW2S;
-    float w = 0.0f;
-    if (n == 0 && kk < 288) w = params[kOffW3 + (kk % 32) * 9 + kk / 32];
-    s.w3[k] = __float2bfloat16_rn(w);
-  }
+  for (int k = tid; k < kWsCh * 9; k += blockDim.x)
+    s.w3[k] = __float2bfloat16_rn(params[kOffW3 + (k % 32) * 9 + k / 32]);
   if (tid < kWsCh) {
     s.b1[tid] = bf16_round(params[kOffB1 + tid]);
     s.b2[tid] = bf16_round(params[kOffB2 + tid]);
   }
   if (tid == 0) s.b3 = bf16_round(params[kOffB3]);
-  __syncthreads();  // weights staged
-  // Layer 3's B fragments for its 18 k-steps (only output column 0 is used).
-  uint32_t b3[36];
-  {
-    const int bn = lane & 7, bkoff = ((lane >> 3) & 1) << 3;
-#pragma unroll
-    for (int ks = 0; ks < 18; ks++)
-      ldsm_x2(b3[2 * ks], b3[2 * ks + 1], &s.w3[bn * kW2S + ks * 16 + bkoff]);
-  }
-  const int tiles_x = (W + kTX - 1) / kTX, tiles_y = (H + kTY - 1) / kTY;
-  for (int tile = blockIdx.x; tile < tiles_x * tiles_y; tile += gridDim.x) {
-    const int x0 = (tile % tiles_x) * kTX, y0 = (tile / tiles_x) * kTY;
-    __syncthreads();  // weights staged / previous tile done
-    for (int k = tid; k < kVY * kVX; k += blockDim.x) {
+  const int tiles_x = (W + kTX - 1) / kTX, tiles = tiles_x * ((H + kTY - 1) / kTY);
+  auto fetch = [&](int tile) {
+    const int x0 = tile % tiles_x * kTX, y0 = tile / tiles_x * kTY;
+    for (int k = tid; k < kVY * kVX && tile < tiles; k += blockDim.x) {
       const int gy = y0 - 6 + k / kVX, gx = x0 - 6 + k % kVX;
       if (gx < 0 || gy < 0 || gx >= W || gy >= H) s.v[k] = NAN;
       else cp_async4(&s.v[k], vg + (int64_t)gy * W + gx);  // all in flight at once
     }
+  };
+  fetch(blockIdx.x);
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const int x0 = (tile % tiles_x) * kTX, y0 = (tile / tiles_x) * kTY;
     cp_async_wait();
-    __syncthreads();
+    __syncthreads();  // elevations (and weights) staged, previous tile done
     // Features (ws_features), separably: first per elevation row and
     // feature column the 7-wide minimum, maximum, sum and count of the
     // valid cells and the 3-wide minimum, then the 7-high (3-high) column
@@ -257,6 +257,7 @@ ws_infer_kernel(const float* __restrict__ params, const float* __restrict__ vg,
       }
     }
     __syncthreads();
+    fetch(tile + gridDim.x);
     // Layer 1: M = 36x20 cells (45 m-tiles), K = 9 taps x 4 features (3 k-steps), N = 32.
     for (int mt = warp; mt < kA1X * kA1Y / 16; mt += kInferWarps) {
       float acc[4][4] = {};
@@ -292,7 +293,7 @@ ws_infer_kernel(const float* __restrict__ params, const float* __restrict__ vg,
           const int n = j * 8 + 2 * tq;
           const float lo = in ? fmaxf(acc[j][2 * h] + s.b1[n], 0.0f) : 0.0f;
           const float hi = in ? fmaxf(acc[j][2 * h + 1] + s.b1[n + 1], 0.0f) : 0.0f;
-          *reinterpret_cast<uint32_t*>(&s.a1[r * kAS + n]) = pack_bf16(lo, hi);
+          *reinterpret_cast<uint32_t*>(&s.a1[act(r, j) + 2 * tq]) = pack_bf16(lo, hi);
         }
       }
     }
@@ -301,87 +302,122 @@ ws_infer_kernel(const float* __restrict__ params, const float* __restrict__ vg,
     // K = 9 taps x 32 channels (18 k-steps), N = 32.  A and B fragments come
     // from ldmatrix: the A rows are cells (the 16 channels of a k-step are
     // 32 contiguous bytes of a cell), the B rows output channels.  A warp
-    // takes two m-tiles at a time so each k-step's B fragments serve both.
+    // takes its 5 m-tiles as 3 and 2, so a k-step's B fragments serve several.
     constexpr int kM2 = kA2X * kA2Y, kMT2 = (kM2 + 15) / 16;
-    {
-      const int arow = lane & 15, akoff = (lane >> 4) << 3;
+    static_assert(kMT2 <= 5 * kInferWarps, "3 + 2 m-tiles per warp");
+    const int arow = lane & 15, achunk = lane >> 4;
+    auto layer2 = [&](auto count, int mt0) {
+      constexpr int kN = decltype(count)::value;
       const int bn = (lane & 7) + ((lane >> 4) << 3), bkoff = ((lane >> 3) & 1) << 3;
-      for (int mt = warp; mt < kMT2; mt += 2 * kInferWarps) {
-        const int mtb = mt + kInferWarps;
-        const bool two = mtb < kMT2;
-        const int ra = min(mt * 16 + arow, kM2 - 1), rb = min(mtb * 16 + arow, kM2 - 1);
-        const int pa = (ra / kA2X) * kA1X + ra % kA2X, pb = (rb / kA2X) * kA1X + rb % kA2X;
-        float acc[2][4][4] = {};
-#pragma unroll 2
-        for (int ks = 0; ks < 18; ks++) {
-          const int tap = ks >> 1, cb = (ks & 1) * 16;
-          const int off = (tap / 3) * kA1X + tap % 3;
-          uint32_t b[8];
-          ldsm_x4(b[0], b[1], b[2], b[3], &s.w2[bn * kW2S + ks * 16 + bkoff]);
-          ldsm_x4(b[4], b[5], b[6], b[7], &s.w2[(bn + 16) * kW2S + ks * 16 + bkoff]);
-          uint32_t a[4];
-          ldsm_x4(a[0], a[1], a[2], a[3], &s.a1[(pa + off) * kAS + cb + akoff]);
+      const __nv_bfloat16* wb = &s.w2[bn * kW2S + bkoff];
+      int pos[kN];
+      float acc[kN][4][4] = {};
 #pragma unroll
-          for (int j = 0; j < 4; j++) mma_bf16(acc[0][j], a[0], a[1], a[2], a[3], b[2 * j], b[2 * j + 1]);
-          if (two) {
-            ldsm_x4(a[0], a[1], a[2], a[3], &s.a1[(pb + off) * kAS + cb + akoff]);
+      for (int m = 0; m < kN; m++) {
+        const int r = min((mt0 + m * kInferWarps) * 16 + arow, kM2 - 1);
+        pos[m] = (r / kA2X) * kA1X + r % kA2X;
+      }
+#pragma unroll 1
+      for (int dy = 0; dy < 3; dy++) {
 #pragma unroll
-            for (int j = 0; j < 4; j++)
-              mma_bf16(acc[1][j], a[0], a[1], a[2], a[3], b[2 * j], b[2 * j + 1]);
-          }
-        }
+        for (int dx = 0; dx < 3; dx++) {
+          int at[kN];
 #pragma unroll
-        for (int m = 0; m < 2; m++) {
-          if (m == 1 && !two) break;
-          const int r0 = (m ? mtb : mt) * 16 + g, r1 = r0 + 8;
+          for (int m = 0; m < kN; m++) at[m] = act(pos[m] + dx, achunk);
 #pragma unroll
           for (int h = 0; h < 2; h++) {
-            const int r = h ? r1 : r0;
-            if (r >= kM2) continue;
-            const int gy = y0 - 1 + r / kA2X, gx = x0 - 1 + r % kA2X;
-            const bool in = gx >= 0 && gy >= 0 && gx < W && gy < H;
+            uint32_t b[8];
+            ldsm_x4(b[0], b[1], b[2], b[3], wb + (dx * 2 + h) * 16);
+            ldsm_x4(b[4], b[5], b[6], b[7], wb + 16 * kW2S + (dx * 2 + h) * 16);
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-              const int n = j * 8 + 2 * tq;
-              const float lo = in ? fmaxf(acc[m][j][2 * h] + s.b2[n], 0.0f) : 0.0f;
-              const float hi = in ? fmaxf(acc[m][j][2 * h + 1] + s.b2[n + 1], 0.0f) : 0.0f;
-              *reinterpret_cast<uint32_t*>(&s.a2[r * kAS + n]) = pack_bf16(lo, hi);
+            for (int m = 0; m < kN; m++) {
+              uint32_t a[4];
+              ldsm_x4(a[0], a[1], a[2], a[3], &s.a1[at[m] ^ (h << 4)]);  // chunk + 2
+#pragma unroll
+              for (int j = 0; j < 4; j++)
+                mma_bf16(acc[m][j], a[0], a[1], a[2], a[3], b[2 * j], b[2 * j + 1]);
             }
           }
         }
-      }
-    }
-    __syncthreads();
-    // Layer 3: M = 32x16 outputs (32 m-tiles), K = 288, N = 8 (only column 0
-    // used).  The B fragments of all 18 k-steps are the same for every
-    // m-tile and stay in registers (b3, loaded once per block).
-    for (int mt = warp; mt < kTX * kTY / 16; mt += kInferWarps) {
-      // Two accumulators (even and odd k-steps) halve the dependent chain.
-      float acc[4] = {}, acc2[4] = {};
-      const int r0 = mt * 16 + g, r1 = r0 + 8;
-      const int ar = mt * 16 + (lane & 15), akoff = (lane >> 4) << 3;
-      const int pa = (ar / kTX) * kA2X + ar % kTX;
 #pragma unroll
-      for (int ks = 0; ks < 18; ks++) {
-        const int tap = ks >> 1, cb = (ks & 1) * 16;
-        const int off = (tap / 3) * kA2X + tap % 3;
-        uint32_t a[4];
-        ldsm_x4(a[0], a[1], a[2], a[3], &s.a2[(pa + off) * kAS + cb + akoff]);
-        mma_bf16((ks & 1) ? acc2 : acc, a[0], a[1], a[2], a[3], b3[2 * ks], b3[2 * ks + 1]);
+        for (int m = 0; m < kN; m++) pos[m] += kA1X;
+        wb += 6 * 16;
       }
 #pragma unroll
-      for (int q = 0; q < 4; q++) acc[q] += acc2[q];
-      if (tq == 0) {
+      for (int m = 0; m < kN; m++) {
+        const int r0 = (mt0 + m * kInferWarps) * 16 + g;
 #pragma unroll
         for (int h = 0; h < 2; h++) {
-          const int r = h ? r1 : r0;
-          const int gy = y0 + r / kTX, gx = x0 + r % kTX;
-          if (gx >= W || gy >= H) continue;
-          const int64_t i = (int64_t)gy * W + gx;
-          const float d = acc[2 * h] + s.b3;
-          if (depth) depth[i] = d;
-          if (warm) warm[i] = d < threshold ? vg[i] : kInf;
+          const int r = r0 + 8 * h;
+          if (r >= kM2) continue;
+          const int gy = y0 - 1 + r / kA2X, gx = x0 - 1 + r % kA2X;
+          const bool in = gx >= 0 && gy >= 0 && gx < W && gy < H;
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            const int n = j * 8 + 2 * tq;
+            const float lo = in ? fmaxf(acc[m][j][2 * h] + s.b2[n], 0.0f) : 0.0f;
+            const float hi = in ? fmaxf(acc[m][j][2 * h + 1] + s.b2[n + 1], 0.0f) : 0.0f;
+            *reinterpret_cast<uint32_t*>(&s.a2[act(r, j) + 2 * tq]) = pack_bf16(lo, hi);
+          }
         }
+      }
+    };
+    layer2(std::integral_constant<int, 3>(), warp);
+    if (warp + 4 * kInferWarps < kMT2)
+      layer2(std::integral_constant<int, 2>(), warp + 3 * kInferWarps);
+    else
+      layer2(std::integral_constant<int, 1>(), warp + 3 * kInferWarps);
+    __syncthreads();
+    // Layer 3: M = 32x16 outputs (32 m-tiles, two at a time), K = 288, N = 8
+    // of which only column 0 exists: lanes 0..3 hold its B fragments.
+    static_assert(kTX * kTY == 4 * 16 * kInferWarps, "4 m-tiles per warp");
+#pragma unroll 1
+    for (int mt = warp; mt < kTX * kTY / 16; mt += 2 * kInferWarps) {
+      // Two accumulators (even and odd k-steps) halve the dependent chain.
+      float acc[2][2][4] = {};
+      int pos[2];
+#pragma unroll
+      for (int m = 0; m < 2; m++) {
+        const int r = (mt + m * kInferWarps) * 16 + arow;
+        pos[m] = (r / kTX) * kA2X + r % kTX;
+      }
+      const __nv_bfloat16* wb = &s.w3[2 * tq];
+#pragma unroll 1
+      for (int dy = 0; dy < 3; dy++) {
+#pragma unroll
+        for (int dx = 0; dx < 3; dx++) {
+          int at[2];
+#pragma unroll
+          for (int m = 0; m < 2; m++) at[m] = act(pos[m] + dx, achunk);
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            uint32_t b0 = ld32(wb + (dx * 2 + h) * 16), b1 = ld32(wb + (dx * 2 + h) * 16 + 8);
+            if (g != 0) b0 = b1 = 0u;
+#pragma unroll
+            for (int m = 0; m < 2; m++) {
+              uint32_t a[4];
+              ldsm_x4(a[0], a[1], a[2], a[3], &s.a2[at[m] ^ (h << 4)]);
+              mma_bf16(acc[m][h], a[0], a[1], a[2], a[3], b0, b1);
+            }
+          }
+        }
+        pos[0] += kA2X;
+        pos[1] += kA2X;
+        wb += 6 * 16;
+      }
+      if (tq == 0) {
+#pragma unroll
+        for (int m = 0; m < 2; m++)
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            const int r = (mt + m * kInferWarps) * 16 + g + 8 * h;
+            const int gy = y0 + r / kTX, gx = x0 + r % kTX;
+            if (gx >= W || gy >= H) continue;
+            const int64_t i = (int64_t)gy * W + gx;
+            const float d = (acc[m][0][2 * h] + acc[m][1][2 * h]) + s.b3;
+            if (depth) depth[i] = d;
+            if (warm) warm[i] = d < threshold ? vg[i] : kInf;
+          }
       }
     }
   }
@@ -397,7 +433,7 @@ cageo_status ws_infer(const float* params, const float* v, float* warm, float* d
                                     (int)smem));
     int sms = 0;
     CAGEO_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    *v = sms > 1 ? sms : 1;
+    *v = 2 * (sms > 1 ? sms : 1);
     return CAGEO_OK;
   });
   if (st) return st;
