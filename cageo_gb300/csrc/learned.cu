@@ -89,13 +89,15 @@ __global__ void ws_features_kernel(const float* __restrict__ v, float* __restric
 //
 // Two blocks of 8 warps share an SM, so that one computes features or waits
 // where the other keeps the tensor cores busy, and a layer's 32 to 45 m-tiles
-// divide well among the warps: 908 -> @T us for 3001x2003 cells (one block of
+// divide well among the warps: 908 -> 587 us for 3001x2003 cells (one block of
 // 16 warps: layer 2's 39 m-tiles took 3 turns of which the last had 7 warps,
 // and nothing ran beside the features).  What makes two blocks fit is one
-// 64-byte row per activation (swizzled, not padded), the features in the layer
-// 2 buffer until that layer runs, and layer 3's weights without the output
-// columns that do not exist.  The elevations of the next tile arrive during
-// the layers.  The order of every sum is the layers' k order.
+// 64-byte row per activation (swizzled, not padded) and that layer 2's
+// activations stay in registers: layer 3 multiplies them there by the weights
+// of its nine taps (4 mma a 16 cells instead of 18 with one useful column of
+// eight, and no activations written and read back), and the taps' products of
+// neighbouring cells are added from shared memory.  The elevations of the next
+// tile arrive during the layers.
 constexpr int kTX = 32, kTY = 16;
 constexpr int kVX = kTX + 12, kVY = kTY + 12;    // elevations
 constexpr int kFX = kTX + 6, kFY = kTY + 6;      // features
@@ -107,12 +109,12 @@ constexpr int kInferWarps = 8;
 struct __align__(128) InferSmem {
   __nv_bfloat16 a1[kA1Y * kA1X * kWsCh];  // rows swizzled, see act()
   union {
-    __nv_bfloat16 a2[kA2Y * kA2X * kWsCh];
+    float p3[kA2Y * kA2X * 9];         // layer 3's products by tap
     __nv_bfloat16 f[kFY * kFX * 4];
   };
   __nv_bfloat16 w2[kWsCh * kW2S];     // [n][k], k = tap*32 + ci
   __nv_bfloat16 w1[kWsCh * kW1S];     // [n][k], k = tap*4 + ci (36 used, 48 in the k-steps)
-  __nv_bfloat16 w3[kWsCh * 9];        // [k], k = tap*32 + ci
+  __nv_bfloat16 w3[9 * kWsCh];        // [tap][ci]
   float v[kVY * kVX];
   float b1[kWsCh], b2[kWsCh], b3;
 };
@@ -259,6 +261,15 @@ ws_infer_kernel(const float* __restrict__ params, const float* __restrict__ vg,
     __syncthreads();
     fetch(tile + gridDim.x);
     // Layer 1: M = 36x20 cells (45 m-tiles), K = 9 taps x 4 features (3 k-steps), N = 32.
+    uint32_t w1[3][4][2];
+#pragma unroll
+    for (int ks = 0; ks < 3; ks++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const __nv_bfloat16* wb = &s.w1[(j * 8 + g) * kW1S + ks * 16 + 2 * tq];
+        w1[ks][j][0] = ld32(wb);
+        w1[ks][j][1] = ld32(wb + 8);
+      }
     for (int mt = warp; mt < kA1X * kA1Y / 16; mt += kInferWarps) {
       float acc[4][4] = {};
       const int r0 = mt * 16 + g, r1 = r0 + 8;
@@ -278,10 +289,8 @@ ws_infer_kernel(const float* __restrict__ params, const float* __restrict__ vg,
           }
         }
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-          const __nv_bfloat16* wb = &s.w1[(j * 8 + g) * kW1S + ks * 16 + 2 * tq];
-          mma_bf16(acc[j], a[0], a[1], a[2], a[3], ld32(wb), ld32(wb + 8));
-        }
+        for (int j = 0; j < 4; j++)
+          mma_bf16(acc[j], a[0], a[1], a[2], a[3], w1[ks][j][0], w1[ks][j][1]);
       }
 #pragma unroll
       for (int h = 0; h < 2; h++) {
@@ -343,13 +352,25 @@ ws_infer_kernel(const float* __restrict__ params, const float* __restrict__ vg,
         for (int m = 0; m < kN; m++) pos[m] += kA1X;
         wb += 6 * 16;
       }
+      // Layer 3 on the activations as they lie in the registers (the
+      // accumulators' layout is the A fragments'): per cell its product with
+      // the 32 weights of each tap, summed over the cells' neighbours below.
+      uint32_t w3[2][2][2];
+#pragma unroll
+      for (int ks = 0; ks < 2; ks++)
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+#pragma unroll
+          for (int h = 0; h < 2; h++)
+            w3[ks][j][h] = j == 0 ? ld32(&s.w3[g * kWsCh + ks * 16 + 2 * tq + 8 * h])
+                           : g == 0 ? ld32(&s.w3[8 * kWsCh + ks * 16 + 2 * tq + 8 * h]) : 0u;
 #pragma unroll
       for (int m = 0; m < kN; m++) {
         const int r0 = (mt0 + m * kInferWarps) * 16 + g;
+        uint32_t a[4][2];  // [channels / 8][row half]
 #pragma unroll
         for (int h = 0; h < 2; h++) {
           const int r = r0 + 8 * h;
-          if (r >= kM2) continue;
           const int gy = y0 - 1 + r / kA2X, gx = x0 - 1 + r % kA2X;
           const bool in = gx >= 0 && gy >= 0 && gx < W && gy < H;
 #pragma unroll
@@ -357,8 +378,24 @@ ws_infer_kernel(const float* __restrict__ params, const float* __restrict__ vg,
             const int n = j * 8 + 2 * tq;
             const float lo = in ? fmaxf(acc[m][j][2 * h] + s.b2[n], 0.0f) : 0.0f;
             const float hi = in ? fmaxf(acc[m][j][2 * h + 1] + s.b2[n + 1], 0.0f) : 0.0f;
-            *reinterpret_cast<uint32_t*>(&s.a2[act(r, j) + 2 * tq]) = pack_bf16(lo, hi);
+            a[j][h] = pack_bf16(lo, hi);
           }
+        }
+        float p[2][4] = {};
+#pragma unroll
+        for (int ks = 0; ks < 2; ks++)
+#pragma unroll
+          for (int j = 0; j < 2; j++)
+            mma_bf16(p[j], a[2 * ks][0], a[2 * ks][1], a[2 * ks + 1][0], a[2 * ks + 1][1],
+                     w3[ks][j][0], w3[ks][j][1]);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const int r = r0 + 8 * h;
+          if (r >= kM2) continue;
+          float* d = &s.p3[r * 9];
+          d[2 * tq] = p[0][2 * h];
+          d[2 * tq + 1] = p[0][2 * h + 1];
+          if (tq == 0) d[8] = p[1][2 * h];
         }
       }
     };
@@ -368,57 +405,17 @@ ws_infer_kernel(const float* __restrict__ params, const float* __restrict__ vg,
     else
       layer2(std::integral_constant<int, 1>(), warp + 3 * kInferWarps);
     __syncthreads();
-    // Layer 3: M = 32x16 outputs (32 m-tiles, two at a time), K = 288, N = 8
-    // of which only column 0 exists: lanes 0..3 hold its B fragments.
-    static_assert(kTX * kTY == 4 * 16 * kInferWarps, "4 m-tiles per warp");
-#pragma unroll 1
-    for (int mt = warp; mt < kTX * kTY / 16; mt += 2 * kInferWarps) {
-      // Two accumulators (even and odd k-steps) halve the dependent chain.
-      float acc[2][2][4] = {};
-      int pos[2];
+    for (int k = tid; k < kTX * kTY; k += blockDim.x) {
+      const int gy = y0 + k / kTX, gx = x0 + k % kTX;
+      if (gx >= W || gy >= H) continue;
+      const float* p = &s.p3[(k / kTX * kA2X + k % kTX) * 9];
+      float d = 0.0f;
 #pragma unroll
-      for (int m = 0; m < 2; m++) {
-        const int r = (mt + m * kInferWarps) * 16 + arow;
-        pos[m] = (r / kTX) * kA2X + r % kTX;
-      }
-      const __nv_bfloat16* wb = &s.w3[2 * tq];
-#pragma unroll 1
-      for (int dy = 0; dy < 3; dy++) {
-#pragma unroll
-        for (int dx = 0; dx < 3; dx++) {
-          int at[2];
-#pragma unroll
-          for (int m = 0; m < 2; m++) at[m] = act(pos[m] + dx, achunk);
-#pragma unroll
-          for (int h = 0; h < 2; h++) {
-            uint32_t b0 = ld32(wb + (dx * 2 + h) * 16), b1 = ld32(wb + (dx * 2 + h) * 16 + 8);
-            if (g != 0) b0 = b1 = 0u;
-#pragma unroll
-            for (int m = 0; m < 2; m++) {
-              uint32_t a[4];
-              ldsm_x4(a[0], a[1], a[2], a[3], &s.a2[at[m] ^ (h << 4)]);
-              mma_bf16(acc[m][h], a[0], a[1], a[2], a[3], b0, b1);
-            }
-          }
-        }
-        pos[0] += kA2X;
-        pos[1] += kA2X;
-        wb += 6 * 16;
-      }
-      if (tq == 0) {
-#pragma unroll
-        for (int m = 0; m < 2; m++)
-#pragma unroll
-          for (int h = 0; h < 2; h++) {
-            const int r = (mt + m * kInferWarps) * 16 + g + 8 * h;
-            const int gy = y0 + r / kTX, gx = x0 + r % kTX;
-            if (gx >= W || gy >= H) continue;
-            const int64_t i = (int64_t)gy * W + gx;
-            const float d = (acc[m][0][2 * h] + acc[m][1][2 * h]) + s.b3;
-            if (depth) depth[i] = d;
-            if (warm) warm[i] = d < threshold ? vg[i] : kInf;
-          }
-      }
+      for (int t = 0; t < 9; t++) d += p[((t / 3) * kA2X + t % 3) * 9 + t];
+      d += s.b3;
+      const int64_t i = (int64_t)gy * W + gx;
+      if (depth) depth[i] = d;
+      if (warm) warm[i] = d < threshold ? vg[i] : kInf;
     }
   }
 }
