@@ -33,8 +33,12 @@ inline bool valid_dims(int W, int H) {
   return W > 0 && H > 0 && (int64_t)W * H < kMaxCells;
 }
 
-// Stream-ordered scratch: the caller's workspace when given, else
-// cudaMallocAsync / cudaFreeAsync on the stream.
+// Gives back what the stage calls' scratch pool keeps (for an allocation that
+// failed).
+void scratch_trim();
+
+// Stream-ordered scratch: the caller's workspace when given, else from the
+// library's pool, in stream order.
 struct Scratch {
   void* ptr = nullptr;
   bool owned = false;

@@ -352,6 +352,9 @@ constexpr int kMaxRunRadius = 64;
 
 template <typename T>
 cageo_status dalloc(T** ptr, size_t bytes) {
+  if (cudaMalloc((void**)ptr, bytes ? bytes : 16) == cudaSuccess) return CAGEO_OK;
+  cudaGetLastError();
+  scratch_trim();
   CAGEO_CUDA(cudaMalloc((void**)ptr, bytes ? bytes : 16));
   return CAGEO_OK;
 }
