@@ -427,13 +427,13 @@ __device__ __forceinline__ FlatSeeds flat_seeds(const FlatHalo& h, unsigned int 
 
 // Distances inside a tile by a bit-parallel breadth-first search: lane y holds
 // row y as a bit mask.  Levels are visited in increasing order, one dilation
-// each, so the first level that reaches a cell is its distance; the level of
-// each reached cell is kept as an offset from a base in 6 bit planes and
-// handed to emit(x, level) in one pass per segment of at most 64 consecutive
-// levels (when the front dies out, or after 64), for the cells of `keep`.
-template <class Emit>
-__device__ __forceinline__ void flat_bfs(unsigned int flat, unsigned int first, const FlatSeeds& sd,
-                                         unsigned int keep, int lane, Emit emit) {
+// each, so the first level that reaches a cell is its distance: step(front, L)
+// gets the cells of each level.  Four levels between two looks whether the
+// front has died out (the search then jumps to the next level that has seeds);
+// every(L) is called there, before levels L .. L + 3.
+template <class Every, class Step>
+__device__ __forceinline__ void flat_levels(unsigned int flat, unsigned int first,
+                                            const FlatSeeds& sd, int lane, Every every, Step step) {
   auto next_level = [&](int after) {  // least seed level above `after`
     int m = kFlatInf;
     if (sd.t > after) m = min(m, sd.t);
@@ -443,11 +443,44 @@ __device__ __forceinline__ void flat_bfs(unsigned int flat, unsigned int first, 
     if (first && after < 1) m = min(m, 1);
     return __reduce_min_sync(0xffffffffu, m);
   };
-  int L = next_level(0), base = L;
+  int L = next_level(0);
   unsigned int open = flat, front = 0;
+  for (int guard = 0; guard < 4 * kFT * kFT && L < kFlatInf; guard++) {
+    every(L);
+#pragma unroll
+    for (int k = 0; k < 4; k++, L++) {
+      const unsigned int tb = __ballot_sync(0xffffffffu, sd.t == L);
+      const unsigned int bb = __ballot_sync(0xffffffffu, sd.b == L);
+      unsigned int seeds = (L == 1 ? first : 0u) | (sd.l == L ? 1u : 0u) |
+                           (sd.r == L ? 0x80000000u : 0u);
+      if (lane == 0) seeds |= tb;
+      if (lane == kFT - 1) seeds |= bb;
+      unsigned int up = __shfl_up_sync(0xffffffffu, front, 1);
+      unsigned int dn = __shfl_down_sync(0xffffffffu, front, 1);
+      if (lane == 0) up = 0;
+      if (lane == kFT - 1) dn = 0;
+      const unsigned int v = front | up | dn;
+      front = ((v | (v << 1) | (v >> 1)) | seeds) & open;
+      open &= ~front;
+      step(front, L);
+    }
+    if (!__any_sync(0xffffffffu, front != 0)) {
+      if (!__any_sync(0xffffffffu, open != 0)) break;
+      L = next_level(L - 1);
+    }
+  }
+}
+
+// Every reached cell's distance to emit(x, level) (this lane's row).  The
+// levels are kept as offsets from a base in 6 bit planes and handed over once
+// per segment of at most 64 consecutive levels.
+template <class Emit>
+__device__ __forceinline__ void flat_bfs(unsigned int flat, unsigned int first, const FlatSeeds& sd,
+                                         int lane, Emit emit) {
+  int base = 0, after = 0;  // the segment's levels: base .. after - 1
   unsigned int seg = 0, p0 = 0, p1 = 0, p2 = 0, p3 = 0, p4 = 0, p5 = 0;
   auto flush = [&]() {
-    for (unsigned int r = seg & keep; r; r &= r - 1) {
+    for (unsigned int r = seg; r; r &= r - 1) {
       const int x = __ffs(r) - 1;
       const int off = ((p0 >> x) & 1) | (((p1 >> x) & 1) << 1) | (((p2 >> x) & 1) << 2) |
                       (((p3 >> x) & 1) << 3) | (((p4 >> x) & 1) << 4) | (((p5 >> x) & 1) << 5);
@@ -455,41 +488,24 @@ __device__ __forceinline__ void flat_bfs(unsigned int flat, unsigned int first, 
     }
     seg = p0 = p1 = p2 = p3 = p4 = p5 = 0;
   };
-  for (int guard = 0; guard < 4 * kFT * kFT && L < kFlatInf; guard++) {
-    const unsigned int tb = __ballot_sync(0xffffffffu, sd.t == L);
-    const unsigned int bb = __ballot_sync(0xffffffffu, sd.b == L);
-    unsigned int seeds = (L == 1 ? first : 0u) | (sd.l == L ? 1u : 0u) |
-                         (sd.r == L ? 0x80000000u : 0u);
-    if (lane == 0) seeds |= tb;
-    if (lane == kFT - 1) seeds |= bb;
-    unsigned int up = __shfl_up_sync(0xffffffffu, front, 1);
-    unsigned int dn = __shfl_down_sync(0xffffffffu, front, 1);
-    if (lane == 0) up = 0;
-    if (lane == kFT - 1) dn = 0;
-    const unsigned int v = front | up | dn;
-    front = ((v | (v << 1) | (v >> 1)) | seeds) & open;
-    open &= ~front;
-    const int off = L - base;  // 0..63
-    seg |= front;
-    if (off & 1) p0 |= front;
-    if (off & 2) p1 |= front;
-    if (off & 4) p2 |= front;
-    if (off & 8) p3 |= front;
-    if (off & 16) p4 |= front;
-    if (off & 32) p5 |= front;
-    // Next level, or jump to the next seed level when the front died out.
-    if (__any_sync(0xffffffffu, front != 0)) {
-      if (++L - base == 64) {
-        flush();
-        base = L;
-      }
-    } else {
-      if (!__any_sync(0xffffffffu, open != 0)) break;
-      flush();
-      L = next_level(L);
-      base = L;
-    }
-  }
+  flat_levels(flat, first, sd, lane,
+              [&](int L) {
+                if (L != after || L - base == 64) {
+                  flush();
+                  base = L;
+                }
+                after = L + 4;
+              },
+              [&](unsigned int front, int L) {
+                const int off = L - base;  // 0..63
+                seg |= front;
+                if (off & 1) p0 |= front;
+                if (off & 2) p1 |= front;
+                if (off & 4) p2 |= front;
+                if (off & 8) p3 |= front;
+                if (off & 16) p4 |= front;
+                if (off & 32) p5 |= front;
+              });
   flush();
   __syncwarp();
 }
@@ -498,7 +514,7 @@ __device__ __forceinline__ void flat_bfs(unsigned int flat, unsigned int first, 
 // queued only when a rim cell that fell is more than one step below a flat
 // cell next to it (distances only fall, so what holds for the staged ones
 // holds for the present ones).
-__device__ void flat_tile(int* rim_new, const RouteWork& w, int t, int lane, FlatStats& st) {
+__device__ void flat_tile(const RouteWork& w, int t, int lane, FlatStats& st) {
   const long long c0 = clock64();
   int* own = w.rim + (size_t)t * kRimCells + lane;
   const unsigned int flat = w.mflat[t * kFT + lane], first = w.mfirst[t * kFT + lane];
@@ -512,21 +528,21 @@ __device__ void flat_tile(int* rim_new, const RouteWork& w, int t, int lane, Fla
   unsigned int want = 0;  // neighbours to queue: 1 L, 2 R, 4 T, 8 B, 16 TL, 32 TR, 64 BL, 128 BR
   const bool lower = sd.t < oT || sd.b < oB || sd.l < oL || sd.r < oR;
   if (!visited || __any_sync(0xffffffffu, lower)) {
-#pragma unroll
-    for (int k = 0; k < 4; k++) rim_new[k * kFT + lane] = kFlatInf;
-    __syncwarp();
-    const bool edge = lane == 0 || lane == 31;
-    flat_bfs(flat, first, sd, edge ? ~0u : 0x80000001u, lane, [&](int x, int level) {
-      if (lane == 0) rim_new[kRTop * kFT + x] = level;
-      if (lane == 31) rim_new[kRBottom * kFT + x] = level;
-      if (x == 0) rim_new[kRLeft * kFT + lane] = level;
-      if (x == 31) rim_new[kRRight * kFT + lane] = level;
+    // Only the rim's distances are wanted: each lane notes the level that
+    // reaches its cell of each side.
+    int nT = kFlatInf, nB = kFlatInf, nL = kFlatInf, nR = kFlatInf;
+    flat_levels(flat, first, sd, lane, [](int) {}, [&](unsigned int front, int L) {
+      const unsigned int top = __shfl_sync(0xffffffffu, front, 0);
+      const unsigned int bottom = __shfl_sync(0xffffffffu, front, 31);
+      if (top >> lane & 1u) nT = L;
+      if (bottom >> lane & 1u) nB = L;
+      if (front & 1u) nL = L;
+      if (front >> 31) nR = L;
     });
     c2 = clock64();
     if (!visited && lane == 0) w.tflat[t] = 2;
-    auto side = [&](int which, int o, int hv, unsigned int bit, int clo, int chi,
+    auto side = [&](int which, int v, int o, int hv, unsigned int bit, int clo, int chi,
                     unsigned int lobit, unsigned int hibit) {
-      const int v = rim_new[which * kFT + lane];
       const bool fell = v < o;
       if (!__any_sync(0xffffffffu, fell)) return;
       if (fell) own[which * kFT] = v;
@@ -537,10 +553,10 @@ __device__ void flat_tile(int* rim_new, const RouteWork& w, int t, int lane, Fla
       if (at & 1u) want |= lobit;
       if (at >> 31) want |= hibit;
     };
-    side(kRTop, oT, h.t, 4u, 0, 1, 16u, 32u);
-    side(kRBottom, oB, h.b, 8u, 2, 3, 64u, 128u);
-    side(kRLeft, oL, h.l, 1u, 0, 2, 16u, 64u);
-    side(kRRight, oR, h.r, 2u, 1, 3, 32u, 128u);
+    side(kRTop, nT, oT, h.t, 4u, 0, 1, 16u, 32u);
+    side(kRBottom, nB, oB, h.b, 8u, 2, 3, 64u, 128u);
+    side(kRLeft, nL, oL, h.l, 1u, 0, 2, 16u, 64u);
+    side(kRRight, nR, oR, h.r, 2u, 1, 3, 32u, 128u);
     // The rims are visible before any neighbour is queued or the tile's state
     // changes.
     __threadfence();
@@ -571,7 +587,6 @@ __device__ void flat_tile(int* rim_new, const RouteWork& w, int t, int lane, Fla
 // asynchronous queue (tilequeue.cuh).  No pass barriers: a free warp takes the
 // next queued tile at once.  Waits are bounded; a limit sets the error flag.
 __global__ void __launch_bounds__(kFWarps * 32, 1) flat_relax_kernel(RouteWork w) {
-  __shared__ int rims[kFWarps][kRimCells];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   const int ntiles = w.tiles_x * w.tiles_y;
   GridSync gs{w.scal + R_BAR_COUNT, w.scal + R_BAR_GEN, (int*)(w.scal + R_ERR)};
@@ -598,7 +613,7 @@ __global__ void __launch_bounds__(kFWarps * 32, 1) flat_relax_kernel(RouteWork w
       if (lane == 0) t = tq_try_dequeue(q, &ticket);
       t = __shfl_sync(0xffffffffu, t, 0);
       if (t >= 0) {
-        flat_tile(rims[warp], w, t, lane, st);
+        flat_tile(w, t, lane, st);
         if (lane == 0) {
           tq_finish(q, t);
           finished++;
@@ -657,7 +672,7 @@ __global__ void __launch_bounds__(kDirWarps * 32) flat_dir_kernel(char2* __restr
   D[(lane + 1) * kDS + 33] = h.r;
   if (lane < 4) D[(lane & 2 ? 33 : 0) * kDS + (lane & 1 ? 33 : 0)] = h.c;
   __syncwarp();
-  flat_bfs(flat, first, sd, ~0u, lane, [&](int x, int level) { D[(lane + 1) * kDS + x + 1] = level; });
+  flat_bfs(flat, first, sd, lane, [&](int x, int level) { D[(lane + 1) * kDS + x + 1] = level; });
   const unsigned int later = flat & ~first;
   const int x = (t % w.tiles_x) * kFT + lane, y0 = (t / w.tiles_x) * kFT;
   constexpr int order[8] = {0, 6, 2, 4, 7, 1, 5, 3};  // N W E S NW NE SW SE as D8 indices
