@@ -276,9 +276,10 @@ cageo_status enqueue_fast(cageo_pipeline* p) {
 // counter on, one above the other (slabs cannot exchange values: every slab's
 // border cells are outlets of the fill and drain outward).  Every stage runs
 // once over the stack; for grids above kStackNoise cells noise and front run
-// slab by slab, which spares a noise grid per slab and loses nothing.  The
-// results equal single realizations bit for bit.
-constexpr int64_t kStackNoise = (int64_t)1 << 22;
+// slab by slab, which spares a noise grid per slab and loses nothing there (four
+// at 4096^2: 4.00 ms slab by slab, 3.93 stacked).  The results equal single
+// realizations bit for bit.
+constexpr int64_t kStackNoise = (int64_t)1 << 24;
 
 cageo_status enqueue_step(cageo_pipeline* p) {
   cudaStream_t s = p->stream;
@@ -521,9 +522,10 @@ static void set_step(cageo_pipeline* p, int K) {
 // Realizations stacked per step where none was asked for.  A realization of a
 // small grid is a chain of ~15 launches that leave most of the GPU idle (330
 // us at 512^2, 20 of them stacked: 860 us), so as many are stacked as
-// make up kStackCells cells (about 35 bytes a cell: 1.2 GB); above that a
-// single grid fills the GPU (four at 4096^2 in two steps: 5.1 ms, singly 6.5).
-constexpr int64_t kStackCells = (int64_t)1 << 25;
+// make up kStackCells cells (about 35 bytes a cell: 2.4 GB).  Four at 4096^2:
+// 3.9 ms in one step, 4.5 in two (6.5 singly, measured with slower stages);
+// twice as many cells a step gain nothing there.
+constexpr int64_t kStackCells = (int64_t)1 << 26;
 
 static int stack_of(const cageo_pipeline* p, int count) {
   // (Launches over tiles have their rows in grid.y: 65535 at most.)

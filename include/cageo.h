@@ -329,7 +329,7 @@ cageo_status cageo_pipeline_run_filter(cageo_pipeline* p, uint32_t first_realiza
  * output equal single realizations bit for bit.  A step is captured in a CUDA
  * graph of its own.
  * Without a call of this, cageo_pipeline_run stacks the realizations of small
- * grids by itself (up to 64, as many as make up 2^25 cells; both fill modes;
+ * grids by itself (up to 64, as many as make up 2^26 cells; both fill modes;
  * not with a learned warm start) and runs singly where the memory for a stack
  * (about 35 bytes per cell per realization, allocated by the first such run)
  * cannot be had.  batch = 1: one realization at a time, no stacks; frees them.

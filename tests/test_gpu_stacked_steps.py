@@ -29,9 +29,9 @@ def _same(one, many):
     (33, 50, (3, 66), dict(use_graphs=False)),
     (257, 131, (7, 2, 7, 7), dict(filter_model=0)),
     (130, 97, (6, 4), dict(fill_mode=1)),
-    (1100, 700, (50,), dict(error_stddev=0.5)),       # two steps of 25
-    (1501, 1333, (17,), dict(fill_mode=1)),           # fit 16: 9 and 8
-    (2100, 2300, (7, 7), {}),                         # noise slab by slab, 4 and 3
+    (1100, 700, (67,), dict(error_stddev=0.5)),       # two steps: 34 and 33
+    (1501, 1333, (35,), dict(fill_mode=1)),           # fit 33: 18 and 17
+    (4200, 4100, (4, 4), {}),                         # noise slab by slab, fit 3: 2 and 2
 ])
 def test_stacked_equals_single(cuda, W, H, counts, kw):
     dem, streams = make_case(W, H, seed=W + H, plateaus=0.1, nodata_cells=W * H // 500)
