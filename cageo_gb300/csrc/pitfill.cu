@@ -584,11 +584,14 @@ __device__ bool any_of(const FillWork& w, unsigned int nblocks, bool mine, unsig
   return any && *ok;
 }
 
-constexpr int kResolveThreads = 1024;
+// Two blocks on an SM: a step's few cells leave most of a block waiting (batch
+// 8 at 8192^2: 27.1 ms; one block of 1024 28.1; four of 256 27.5, and slower on
+// long lists of few fronts).
+constexpr int kResolveThreads = 512;
 // Entries of the list a block takes at a time at most (walls; cells of reopened
 // components), and entries per block of the launch: with 1024 a block (one
 // on a grid of 512x512) the passes over the list took several turns each.
-constexpr unsigned int kResolveRun = 1024, kReopenRun = 256, kResolveShare = 256;
+constexpr unsigned int kResolveRun = 512, kReopenRun = 256, kResolveShare = 128;
 constexpr int kFrontCells = 1024, kFreshCells = 2048;
 
 // A block's front: cells whose level fell (or walls that have come to relay),
@@ -746,7 +749,7 @@ __device__ unsigned int relax(const Resolve& r, Front& f, const uint32_t* list, 
 // Steps 2 and 3, and the cells no outlet reaches.  A cooperative launch; only
 // as many blocks as the list's runs need stay (a barrier among few blocks is
 // cheap, and the list is short on small grids).
-__global__ void __launch_bounds__(kResolveThreads, 1) fill_resolve_kernel(Resolve r) {
+__global__ void __launch_bounds__(kResolveThreads, 2) fill_resolve_kernel(Resolve r) {
   __shared__ Front front;
   const FillWork& w = r.w;
   volatile unsigned int* vs = w.scal;
