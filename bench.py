@@ -47,14 +47,14 @@ FALLBACK_HBM = 6800.0
 # Algorithmic bytes per cell of each stage (unfused compulsory I/O).
 STAGE_BYTES = {"noise": 4, "front": 40, "fill": 8, "route": 5, "trace": 6, "border": 12}
 PIPE_BYTES = 75
-# The dominant kernel is the pit fill's lower-bound flood (fill_flood_kernel
-# with clean marks, 35% of a realization).  Its algorithmic bytes are those
+# The dominant kernel is the pit fill's walled flood (level_flood_kernel,
+# 28% of a realization).  Its algorithmic bytes are those
 # of one fill pass: read q (4 B) and write the filled value (4 B) per cell.
 # Its DRAM bytes per launch come from an ncu capture of the 4096^2 workload
 # (dram__bytes_read.sum + dram__bytes_write.sum of that launch divided by
 # its 16.8 M cells), applied per cell to the benchmark grid.
 FLOOD_A_BYTES_PER_CELL = 8
-FLOOD_A_TRAFFIC_PER_CELL = 614.9e6 / (4096 * 4096)
+FLOOD_A_TRAFFIC_PER_CELL = 488.5e6 / (4096 * 4096)
 
 
 _T0 = time.time()
@@ -480,7 +480,7 @@ def main():
         "fill_stats": stats,
         "fill_parts_ms": fill_parts_ms,
         "roofline": {"bound": "hbm",
-                     "kernel": "fill_flood_kernel (pit fill, lower-bound flood with clean marks)",
+                     "kernel": "level_flood_kernel (pit fill, walled flood)",
                      "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                      "traffic": FLOOD_A_TRAFFIC_PER_CELL * N,
                      "traffic_note": "DRAM bytes of one launch: ncu at 4096^2, scaled by cells",

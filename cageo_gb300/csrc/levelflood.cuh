@@ -1,6 +1,6 @@
 // levelflood.cuh -- one tile visit of the pit fill's flood (the walled flood of
 // the CPU-compatible fill, and the whole of the exact fill): levels relaxed in
-// registers.
+// shared memory.
 //
 // What bounds a flood is the instructions and the dependent chains of its
 // tile visits, not memory (a visit moves ~9 KB).  A warp stages its 32x32 tile

@@ -5,11 +5,11 @@
 // burning + quantization (front) -> pit fill -> routing -> tracing ->
 // border counts.  In exact mode the front does not quantize and the fill,
 // routing and tracing follow the reference's GPU path instead of its CPU
-// path.  The launch sequence of one realization reads the
-// realization number from device memory, so it is captured once in a CUDA
-// graph and replayed; the data-dependent loops (fill passes, flat BFS
-// layers, pointer jumps) run inside persistent kernels and need no host
-// round trip.  Counts accumulate in uint32.
+// path.  The launch sequence of a step -- one realization, or several stacked
+// one above the other -- reads the realization number from device memory, so it
+// is captured once in a CUDA graph and replayed; the data-dependent loops (fill
+// passes, flat BFS layers, pointer jumps) run inside persistent kernels and
+// need no host round trip.  Counts accumulate in uint32.
 //
 // The fused front uses a burn code precomputed from the stream raster.  It
 // flags a realization where that code may differ from the reference's
@@ -523,7 +523,7 @@ static void set_step(cageo_pipeline* p, int K) {
 // Realizations stacked per step where none was asked for.  A realization of a
 // small grid is a chain of ~15 launches that leave most of the GPU idle (330
 // us at 512^2, 20 of them stacked: 860 us), so as many are stacked as
-// make up kStackCells cells (about 35 bytes a cell: 2.4 GB).  Four at 4096^2:
+// make up kStackCells cells (about 32 bytes a cell: 2.1 GB).  Four at 4096^2:
 // 3.9 ms in one step, 4.5 in two (6.5 singly, measured with slower stages);
 // twice as many cells a step gain nothing there.
 constexpr int64_t kStackCells = (int64_t)1 << 26;
@@ -739,8 +739,8 @@ extern "C" cageo_status cageo_pipeline_profile(cageo_pipeline* p, uint32_t reali
       break;
     }
     for (int i = 0; i < 6 && i < n; i++) cudaEventElapsedTime(&h_ms[i], ev[i], ev[i + 1]);
-    // The fill's parts (CPU-compatible mode): set-up, flood A, flood B with
-    // the undecided-cell kernels, confirmation phases, final pass.
+    // The fill's parts (CPU-compatible mode): set-up, walled flood, the walls'
+    // levels, resolution, and a last part that is empty now.
     const cudaEvent_t fill_marks[6] = {ev[2], fm[0], fm[1], fm[2], fm[3], ev[3]};
     for (int i = 0; i < 5 && 6 + i < n; i++) {
       if (exact_mode(p)) h_ms[6 + i] = 0.0f;

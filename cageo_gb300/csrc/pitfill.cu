@@ -1,7 +1,7 @@
 // pitfill.cu -- A6 pit filling with the semantics of the reference's CPU
 // path (src/pitfilling/PitFillingAlgorithmCPUOpenMP.h:68-242), and the exact
 // float fill of its GPU path (src/pitfilling/PitFillingAlgorithmGPUCUDA.cu:
-// 201-381) as a second mode: flood A alone on the unquantized grid, every
+// 201-381) as a second mode: the flood alone on the unquantized grid, every
 // outlet relaying, unreached cells ending at the GPU path's 99990000.
 //
 // The CPU fill is a bucket priority-flood over 1 mm levels in which a
@@ -295,8 +295,9 @@ __device__ __forceinline__ bool seed_queue(const FillWork& w, const GridSync& gs
 }
 
 // The walled flood, the exact fill (no walls), the warm-started exact fill
-// (MARKS: with clean marks) and its repair flood.  Blocks of at most WARPS warps, one per SM; a
-// small grid's tiles are spread over all SMs with fewer warps each.
+// (MARKS: with clean marks) and its repair flood.  Blocks of at most WARPS
+// warps, one per SM; a small grid's tiles are spread over all SMs with fewer
+// warps each.
 template <bool MARKS, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 1) level_flood_kernel(LevelArgs a) {
   extern __shared__ __align__(16) unsigned char smraw[];

@@ -1,7 +1,7 @@
 // pitfill_static.cu -- pit filling that allocates nothing.
 //
-// cageo_pitfill needs about 5 bytes of device scratch per cell, which it
-// takes from the caller's workspace or allocates with cudaMallocAsync.
+// cageo_pitfill needs about 13 bytes of device scratch per cell, which it
+// takes from the caller's workspace or allocates in stream order.
 // Some callers can do neither: a host application that has reserved the
 // GPU's memory for its own allocator and forbids plug-ins from calling
 // cudaMalloc, or a loop that must not pay an allocation's latency or

@@ -331,7 +331,7 @@ cageo_status cageo_pipeline_run_filter(cageo_pipeline* p, uint32_t first_realiza
  * Without a call of this, cageo_pipeline_run stacks the realizations of small
  * grids by itself (up to 64, as many as make up 2^26 cells; both fill modes;
  * not with a learned warm start) and runs singly where the memory for a stack
- * (about 35 bytes per cell per realization, allocated by the first such run)
+ * (28 to 32 bytes per cell per realization, allocated by the first such run)
  * cannot be had.  batch = 1: one realization at a time, no stacks; frees them.
  * batch > 1: steps of that many whatever the grid, the rest of `count` singly;
  * batch <= 64, batch * cells < 2^31, CPU-compatible fill mode only. */
@@ -371,28 +371,29 @@ cageo_status cageo_pipeline_graph_kernels(cageo_pipeline* p, int64_t* h_count);
  * it is accumulated like any other.  h_ms[0..5]: noise, front
  * (convolution + realistic DEM + burning + quantization), pit fill,
  * routing, tracing, border (milliseconds); with n >= 11, h_ms[6..10]: the
- * pit fill's parts -- set-up, lower-bound flood, walled flood with the
- * undecided-cell kernels, confirmation phases, final pass (0 in exact
- * mode). */
+ * pit fill's parts -- set-up, walled flood, the walls' levels, resolution
+ * (lower bound, components, confirmation phases), and a fifth part that is
+ * empty (0 in exact mode). */
 cageo_status cageo_pipeline_profile(cageo_pipeline* p, uint32_t realization,
                                     float* h_ms, int n);
 /* Counters of the last run: [0] fill work-queue drains, [1] confirmation
  * phases, [2] flat-BFS passes, [3] trace jumps, [4] burn re-runs, [5] drains
- * of the lower-bound flood, [6] drains of the walled flood before the first
- * phase, [7..9] microseconds of the lower-bound flood, of the walled flood
- * to convergence and of the phase loop, [10..13] tiles and sweep rounds of
- * the two floods, [14] flat cells, [15] microseconds of the flat BFS,
- * [16..18] kilo-cycles summed over the fill's tile visits spent staging,
- * sweeping and storing, [19] tile visits of the flat BFS, [20..22]
- * kilo-cycles summed over them spent staging, searching and storing,
- * [23..24] kilo-cycles the warps of the fill's lower-bound flood and of its
- * walled flood spent waiting for a tile, end of the queue included (last
- * realization). */
+ * of the flood, [6] most steps of a front in the resolution (drains of the
+ * repair flood with a warm start), [7..9] microseconds of the flood, of the
+ * resolution's lower bound (of the repair flood) and of the rest of the
+ * resolution, [10..11] tile visits and sweep rounds of the flood, [12..13]
+ * cells listed by the resolution and 0 (visits and rounds of the repair
+ * flood), [14] flat cells, [15] microseconds of the flat BFS, [16..18]
+ * kilo-cycles summed over the fill's tile visits spent staging, sweeping and
+ * storing, [19] tile visits of the flat BFS, [20..22] kilo-cycles summed over
+ * them spent staging, searching and storing, [23..24] kilo-cycles the warps of
+ * the flood and of the repair flood spent waiting for a tile, end of the queue
+ * included (all of the last step's realizations). */
 cageo_status cageo_pipeline_stats(cageo_pipeline* p, int64_t* h_stats, int n);
 /* Tuning of the pipeline's kernels (no counterpart in the reference).  The
  * results never depend on it.  fill_rounds: sweep rounds a fill tile visit
  * may run before the tile queues itself again (1..1024; default 64).
- * fill_warps: warps per SM of the fill's lower-bound flood (16, 20 or 22;
+ * fill_warps: warps per SM of the fill's flood (16, 20 or 22;
  * more warps hide more latency, fewer leave more registers to each; default
  * 20).  The fill's tile shape is fixed at 32 x 32 cells, the warp width: a
  * warp owns a tile and holds its rows as 32-bit lane masks.  conv_tile:
