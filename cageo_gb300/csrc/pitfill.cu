@@ -986,9 +986,11 @@ static cageo_status launch_resolve(const Resolve& r, cudaStream_t s) {
   if (st) return st;
   Resolve args = r;
   void* params[] = {&args};
-  // No more blocks than a list of every cell would need.
+  // Blocks for lists of up to 1 cell in 128 (walls above their q are 1 in 600 on
+  // terrain; blocks take several turns on longer lists).  All of them have to
+  // find room on the GPU at once, beside what other streams run.
   const int64_t n = (int64_t)r.w.W * r.w.H;
-  const int grid = (int)std::min<int64_t>(blocks, (n + kResolveShare - 1) / kResolveShare);
+  const int grid = (int)std::min<int64_t>(blocks, (n + 128 * kResolveShare - 1) / (128 * kResolveShare));
   CAGEO_CUDA(cudaLaunchCooperativeKernel((const void*)fill_resolve_kernel, dim3(grid),
                                          dim3(kResolveThreads), params, 0, s));
   return CAGEO_OK;
