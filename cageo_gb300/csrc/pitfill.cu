@@ -533,12 +533,38 @@ struct Resolve {
   }
 };
 
+// Two blocks on an SM: a step's few cells leave most of a block waiting (batch
+// 8 at 8192^2: 27.1 ms; one block of 1024 28.1; four of 256 27.5, and slower on
+// long lists of few fronts).
+constexpr int kResolveThreads = 512;
+// Entries of the list a block takes at a time at most (walls; cells of reopened
+// components), and entries per block of the launch: with 1024 a block (one
+// on a grid of 512x512) the passes over the list took several turns each.
+constexpr unsigned int kResolveRun = 512, kReopenRun = 256, kResolveShare = 128;
+constexpr int kFrontCells = 1024, kFreshCells = 2048;
+
+// A block's front: cells whose level fell (or walls that have come to relay),
+// with that level; one buffer is read while the other fills.  Three counters
+// in turn, so a step needs one block barrier.
+struct Front {
+  uint32_t cell[2][kFrontCells];
+  float level[2][kFrontCells];
+  int n[3];
+  int full;  // an entry did not fit: its cell was marked kActive instead
+  // Cells to list.  They are listed many at a time: an addition to the list's
+  // length in every step made it three dependent L2 accesses instead of two.
+  uint32_t fresh[kFreshCells];
+  int nfresh;
+  unsigned int at;
+  unsigned int gen;  // grid barriers passed (thread 0)
+};
+
 // Grid barrier of the `nblocks` blocks of the resolution.  Returns whether any
 // thread passed true; *more = the entries listed by then (nothing is listed
 // between the last arrival, which takes the number, and the release); *ok =
 // false on an error (any block's) or a wait limit.
-__device__ bool any_of(const FillWork& w, unsigned int nblocks, bool mine, unsigned int* more,
-                       bool* ok) {
+__device__ bool any_of(const FillWork& w, Front& f, unsigned int nblocks, bool mine,
+                       unsigned int* more, bool* ok) {
   __shared__ unsigned int sh_any, sh_more, sh_ok;
   volatile unsigned int* vs = w.scal;
   const int block = __syncthreads_or(mine);
@@ -549,7 +575,9 @@ __device__ bool any_of(const FillWork& w, unsigned int nblocks, bool mine, unsig
       sh_any = block ? 1u : 0u;
       sh_more = vs[S_MORE];
     } else {
-      const unsigned int gen = vs[S_BAR_GEN];
+      // (The generation is counted, not read here: a read could be performed
+      // after the arrival, and after the release that it is to wait for.)
+      const unsigned int gen = f.gen++;
       // The count of the arrivals, and 65536 times that of those with a true.
       const unsigned int arrived = atomicAdd(&w.scal[S_BAR_COUNT], block ? 65537u : 1u);
       if ((arrived & 0xffffu) == nblocks - 1) {
@@ -584,31 +612,6 @@ __device__ bool any_of(const FillWork& w, unsigned int nblocks, bool mine, unsig
   __syncthreads();
   return any && *ok;
 }
-
-// Two blocks on an SM: a step's few cells leave most of a block waiting (batch
-// 8 at 8192^2: 27.1 ms; one block of 1024 28.1; four of 256 27.5, and slower on
-// long lists of few fronts).
-constexpr int kResolveThreads = 512;
-// Entries of the list a block takes at a time at most (walls; cells of reopened
-// components), and entries per block of the launch: with 1024 a block (one
-// on a grid of 512x512) the passes over the list took several turns each.
-constexpr unsigned int kResolveRun = 512, kReopenRun = 256, kResolveShare = 128;
-constexpr int kFrontCells = 1024, kFreshCells = 2048;
-
-// A block's front: cells whose level fell (or walls that have come to relay),
-// with that level; one buffer is read while the other fills.  Three counters
-// in turn, so a step needs one block barrier.
-struct Front {
-  uint32_t cell[2][kFrontCells];
-  float level[2][kFrontCells];
-  int n[3];
-  int full;  // an entry did not fit: its cell was marked kActive instead
-  // Cells to list.  They are listed many at a time: an addition to the list's
-  // length in every step made it three dependent L2 accesses instead of two.
-  uint32_t fresh[kFreshCells];
-  int nfresh;
-  unsigned int at;
-};
 
 // The whole block: lists the fresh cells from entry `end` + S_MORE on.
 __device__ void list_fresh(const Resolve& r, Front& f, unsigned int end) {
@@ -742,7 +745,7 @@ __device__ unsigned int relax(const Resolve& r, Front& f, const uint32_t* list, 
     }
     if (LOWER) list_fresh(r, f, nu0);
     __syncthreads();
-    again = any_of(w, nblocks, f.full != 0, more, ok);
+    again = any_of(w, f, nblocks, f.full != 0, more, ok);
   }
   return steps;
 }
@@ -759,6 +762,7 @@ __global__ void __launch_bounds__(kResolveThreads, 2) fill_resolve_kernel(Resolv
   if (blockIdx.x >= nblocks) return;
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t nthreads = (int64_t)nblocks * blockDim.x;
+  if (threadIdx.x == 0) front.gen = vs[S_BAR_GEN];  // (any_of fences before it arrives)
   const unsigned long long t0 = global_ns();
   int phases = 0;
   unsigned int more = 0;
@@ -795,7 +799,7 @@ __global__ void __launch_bounds__(kResolveThreads, 2) fill_resolve_kernel(Resolv
     if (wb != sb && qb != r.nodata) united &= uf_unite(w.label, c, b);
   }
   if (!united) atomicCAS((int*)(w.scal + S_ERR), 0, 6);
-  if (nu0 && any_of(w, nblocks, reopen, &more, &ok)) {
+  if (nu0 && any_of(w, front, nblocks, reopen, &more, &ok)) {
     for (int64_t j = tid; j < nu; j += nthreads) {
       const uint32_t c = __ldcg(w.cand + j);
       if (!(r.get(c) & kMember)) continue;
@@ -804,7 +808,7 @@ __global__ void __launch_bounds__(kResolveThreads, 2) fill_resolve_kernel(Resolv
       const float qc = r.q[c];
       if (r.level(c) <= qc && r.walled(c) > qc && r.wall(c, qc)) r.set(root, kReopened);
     }
-    any_of(w, nblocks, false, &more, &ok);
+    any_of(w, front, nblocks, false, &more, &ok);
     // The cells of reopened components restart at S -- or at what a settled
     // listed wall beside them offers, if that is less -- with the walls that A
     // left above their q confirmed, and are listed once more after the others
@@ -848,7 +852,7 @@ __global__ void __launch_bounds__(kResolveThreads, 2) fill_resolve_kernel(Resolv
       const unsigned int pos = warp_append(&w.scal[S_OPEN], open && apart);
       if (open && apart) __stcg(w.cand + nu + pos, c);
     }
-    any_of(w, nblocks, false, &more, &ok);
+    any_of(w, front, nblocks, false, &more, &ok);
     const unsigned int no = apart ? vs[S_OPEN] : nu;
     const uint32_t* open_list = apart ? w.cand + nu : w.cand;
     while (ok) {
@@ -872,7 +876,7 @@ __global__ void __launch_bounds__(kResolveThreads, 2) fill_resolve_kernel(Resolv
         atomicMin(&w.aux[__ldcg(w.label + c)], __float_as_uint(lv));
         some = true;
       }
-      if (!any_of(w, nblocks, some, &more, &ok)) break;
+      if (!any_of(w, front, nblocks, some, &more, &ok)) break;
       // Each phase confirms at least one cell of every component with a
       // pending one (the cell holding its minimum).
       if (++phases > (int)min(nu, 0x7fffff00u) + 8) {
@@ -884,7 +888,7 @@ __global__ void __launch_bounds__(kResolveThreads, 2) fill_resolve_kernel(Resolv
         const unsigned int m = __ldcg(w.aux + __ldcg(w.label + c));
         if (m != 0xffffffffu && qc <= __uint_as_float(m)) r.set(c, kConfirmed | kActive);
       }
-      any_of(w, nblocks, false, &more, &ok);
+      any_of(w, front, nblocks, false, &more, &ok);
     }
   }
   // The marks come off, and cells no outlet reached keep q.
