@@ -273,11 +273,13 @@ __device__ __forceinline__ void conv_line8(int L, f32x2 one, V v, Tap tap, f32x2
 // rows start on a 16-byte boundary.
 __host__ __device__ inline int sep_pad(int r) { return (r + 3) & ~3; }
 
-// Blocks per SM the registers are held to: 5 (at 8192^2, radius 15, 64 x 32
-// tiles: 0.58 ms; 4: 0.61), but 4 for radius 23, whose longer unrolled lines
-// would spill (16384^2: 3.14 ms; 5: 3.27).  128 or 192 threads, or 6 blocks,
-// are slower for both.  The lines are unrolled for these two radii (the
-// runtime loop takes 0.61 and 3.5 ms).
+// Blocks per SM the registers are held to: 5 (front at 8192^2, radius 15, 64 x
+// 32 tiles, before the epilogue's quads: 0.58 ms; 4: 0.61), but 4 for radius
+// 23, whose longer unrolled lines would spill (16384^2: 3.14 ms; 5: 3.27).
+// 128 or 192 threads, or 6 blocks, are slower for both.  The lines are unrolled
+// for these two radii (the runtime loop takes 0.61 and 3.5 ms).  With the quads:
+// 0.51 ms, of which the convolution alone is 0.42 and its packed products and
+// sums, at two a clock and SM, 0.26.
 template <class Epi, int LC, int TW, int TH>
 __global__ void __launch_bounds__(kSepThreads, LC == 47 ? 4 : 5)
 conv_sep_kernel(const float* __restrict__ in, int W, int H,

@@ -522,7 +522,7 @@ static void set_step(cageo_pipeline* p, int K) {
 
 // Realizations stacked per step where none was asked for.  A realization of a
 // small grid is a chain of ~15 launches that leave most of the GPU idle (330
-// us at 512^2, 20 of them stacked: 860 us), so as many are stacked as
+// us at 512^2, 20 of them stacked: 700 us), so as many are stacked as
 // make up kStackCells cells (about 32 bytes a cell: 2.1 GB).  Four at 4096^2:
 // 3.9 ms in one step, 4.5 in two (6.5 singly, measured with slower stages);
 // twice as many cells a step gain nothing there.
