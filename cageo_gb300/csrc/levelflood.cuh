@@ -294,7 +294,8 @@ __device__ __forceinline__ void level_visit(LevelSmem& s, const LevelArgs& a, co
   // flight with the rims and masks (a first visit copies levels it does not
   // use rather than wait for the tile's state).  The levels were last written
   // by whichever SM visited the tile before; taking it from the queue ended in
-  // a fence, which orders these loads after that visit's stores.
+  // a fence by lane 0 and a __syncwarp, which order every lane's loads after
+  // that visit's stores (so copies through L1 read no older level).
   if (full) {
     const float* qp = a.q + base;
     const float* wp = a.Wg + base;

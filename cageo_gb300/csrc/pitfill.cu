@@ -232,6 +232,7 @@ __device__ bool drain(const FillWork& w, int lane, int ntiles, bool b_slots, Vis
     int t = -1;
     if (lane == 0) t = tq_try_dequeue(q, &ticket);
     t = __shfl_sync(0xffffffffu, t, 0);
+    __syncwarp();  // lane 0's fence holds for the loads of all lanes (a shuffle orders no memory)
     if (t >= 0) {
       if (lane == 0 && idle_from >= 0) st.kidle += (unsigned int)((clock64() - idle_from) >> 10);
       idle_from = -1;

@@ -612,6 +612,7 @@ __global__ void __launch_bounds__(kFWarps * 32, 1) flat_relax_kernel(RouteWork w
       int t = -1;
       if (lane == 0) t = tq_try_dequeue(q, &ticket);
       t = __shfl_sync(0xffffffffu, t, 0);
+      __syncwarp();  // lane 0's fence holds for the loads of all lanes (a shuffle orders no memory)
       if (t >= 0) {
         flat_tile(w, t, lane, st);
         if (lane == 0) {

@@ -72,7 +72,8 @@ __device__ __forceinline__ void tq_enqueue(const TileQueue& q, bool want, int t)
   if (push) tq_store(q, pos + __popc(ball & ((1u << lane) - 1u)), t);
 }
 
-// Lane 0: take the next queued tile.  A warp takes a ticket (the next ring
+// Lane 0 (the other lanes follow after a __syncwarp, which hands them the order
+// that lane 0's fence makes): take the next queued tile.  A warp takes a ticket (the next ring
 // position) as soon as it is free and keeps it until the slot is filled --
 // possibly by a later push -- so no claim ever fails (looking whether the
 // ring holds an entry first would be one more L2 access a visit).  Returns
