@@ -14,7 +14,9 @@
 // The queue is drained when as many tiles have been finished as were ever
 // pushed: a tile is pushed by a warp that has not finished its own yet, so
 // reading `done` first and `tail` after it and finding them equal means that
-// no tile was queued or in process at the first read.  Warps add their
+// no tile was queued or in process at the first read (a fence lies between a
+// warp's pushes and its addition to `done`: a warp that saw the latter without
+// the former would leave with a ticket that a later push fills).  Warps add their
 // finished tiles to `done` only when they find no tile waiting, and a warp
 // pushes all the neighbours of a visit with one addition to `tail`: two
 // same-address atomics a visit, against five with a counter of pending tiles
@@ -108,6 +110,7 @@ __device__ __forceinline__ void tq_finish(const TileQueue& q, int t) {
 __device__ __forceinline__ bool tq_drained(const TileQueue& q, unsigned int* finished) {
   unsigned int d;
   if (*finished) {
+    __threadfence();  // the pushes of these tiles' visits before their end is counted
     d = atomicAdd(q.done, *finished) + *finished;
     *finished = 0;
   } else {

@@ -41,3 +41,19 @@ def test_levels_and_distances_across_tiles(cuda, oracle, W, H):
         e = api.pitfill(v.clone(), mode=api.FILL_EXACT)
         assert np.array_equal(bits(e.cpu().numpy()), bits(e_ref))
         assert np.array_equal(api.route_d8(e_dev).cpu().numpy(), d_ref)
+
+
+def test_many_short_drains(cuda, oracle):
+    """Grids of a few tiles, where most warps wait with a ticket while the last
+    tiles are pushed: every drain ends, with nothing left behind."""
+    import torch
+    from cageo_gb300 import api
+    for W, H in [(33, 64), (70, 70), (100, 40)]:
+        dem = _corridor(W, H, seed=W)
+        e_ref = oracle.pitfill_exact(dem)
+        d_ref = torch.from_numpy(oracle.flow_route(e_ref)).to(cuda)
+        e_dev = torch.from_numpy(e_ref).to(cuda)
+        v = torch.from_numpy(dem).to(cuda)
+        for _ in range(200):
+            assert torch.equal(api.pitfill(v, mode=api.FILL_EXACT), e_dev)
+            assert torch.equal(api.route_d8(e_dev), d_ref)
