@@ -99,9 +99,13 @@ __device__ __forceinline__ int tq_try_dequeue(const TileQueue& q, long long* tic
 // finished tile.
 __device__ __forceinline__ void tq_finish(const TileQueue& q, int t) {
   if (atomicCAS(&q.state[t], kBusy, kIdle) != kBusy) {
-    // Processing and queued again: only the owner changes that state.
+    // Processing and queued again: only the owner changes that state.  The
+    // fence keeps this store ahead of the entry, whose taker changes the state
+    // next: landing after that, it would leave the tile "queued" with no entry.
     ((volatile int*)q.state)[t] = kQueued;
-    tq_store(q, atomicAdd(q.tail, 1u), t);
+    const unsigned int pos = atomicAdd(q.tail, 1u);
+    __threadfence();
+    tq_store(q, pos, t);
   }
 }
 

@@ -57,3 +57,20 @@ def test_many_short_drains(cuda, oracle):
         for _ in range(200):
             assert torch.equal(api.pitfill(v, mode=api.FILL_EXACT), e_dev)
             assert torch.equal(api.route_d8(e_dev), d_ref)
+
+
+def test_tiles_queued_while_processed(cuda):
+    """One sweep round per visit: nearly every visit ends with its tile queued
+    again, by itself and by its neighbours."""
+    from cageo_gb300 import api
+    from cases import make_case
+    dem, streams = make_case(257, 131, seed=5, pits=400)
+    p = api.Pipeline(dem, streams, error_stddev=1.5, seed=4)
+    p.run(0, 200)
+    want = p.counts()
+    for warps in (16, 22):
+        p.reset_counts()
+        p.set_tuning(1, warps)
+        p.run(0, 200)
+        assert np.array_equal(p.counts(), want)
+    p.close()
