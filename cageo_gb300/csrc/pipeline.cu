@@ -52,14 +52,32 @@ cageo_status ws_infer(const float* params, const float* v, float* warm, float* d
 
 // Layout of the device scalars (cageo_pipeline::dscal).
 constexpr int kMaxStack = 64;               // realizations of a step
-constexpr int kFlags = 4;                   // their anomaly flags
+constexpr int kErrors = 1;                  // the run's first errors (keep_errors)
+constexpr int kFlags = 4;                   // the step's anomaly flags
 constexpr int kRedo = kFlags + kMaxStack;   // realizations to redo
 constexpr unsigned int kMaxRedo = 4096;
 
+// The error words of a step's fill, routing and tracing.
+struct StepErrors {
+  const unsigned int *fill, *route, *trace;
+};
+
+// One thread at the end of a step: the next step's start clears the stages'
+// error words, so the first step of a run that left any is kept, a byte per
+// stage, until the host reads it at the run's end.
+__device__ __forceinline__ void keep_errors(const StepErrors& e, uint32_t* kept) {
+  const uint32_t now = min(*e.fill, 255u) | min(*e.route, 255u) << 8 | min(*e.trace, 255u) << 16;
+  if (now && *kept == 0u) *kept = now;
+}
+
+__global__ void keep_errors_kernel(StepErrors e, uint32_t* kept) { keep_errors(e, kept); }
+
 // End of a step of `count` realizations: list the flagged ones (they were not
-// counted), clear their flags and advance the device realization counter.
+// counted), clear their flags, keep the stages' errors and advance the device
+// realization counter.
 __global__ void realization_end_kernel(uint32_t* real, int* anomaly, uint32_t* redo,
-                                       unsigned int* nredo, unsigned int count) {
+                                       unsigned int* nredo, unsigned int count, StepErrors errors,
+                                       uint32_t* kept) {
   for (unsigned int j = threadIdx.x; j < count; j += blockDim.x) {
     if (anomaly[j]) {
       const unsigned int k = atomicAdd(nredo, 1u);
@@ -68,7 +86,10 @@ __global__ void realization_end_kernel(uint32_t* real, int* anomaly, uint32_t* r
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0) *real += count;
+  if (threadIdx.x == 0) {
+    keep_errors(errors, kept);
+    *real += count;
+  }
 }
 
 // Order-independent 64-bit digest of a float grid: the wrapping sum over
@@ -135,9 +156,9 @@ struct cageo_pipeline {
   FillWork fw;
   RouteWork rw;
   TraceWork tw;
-  // device scalars: [0] realization counter, [1] -, [2] nredo, [3] the run's
-  // last realization (the one whose labels are kept), [4..] the anomaly flags
-  // of a step's slabs, then the redo list
+  // device scalars: [0] realization counter, [1] the run's first errors, [2]
+  // nredo, [3] the run's last realization (the one whose labels are kept),
+  // [4..] the anomaly flags of a step's slabs, then the redo list
   uint32_t* dscal = nullptr;
   FrontParams fp{};
   cudaGraph_t graph = nullptr;
@@ -251,6 +272,29 @@ cageo_status enqueue_trace_border(cageo_pipeline* p, const int* gate, bool every
                                every ? nullptr : p->dscal + 3, p->stream);
 }
 
+StepErrors step_errors(const FillWork& f, const RouteWork& r, const TraceWork& t) {
+  return StepErrors{fill_error_word(f), route_error_word(r), trace_error_word(t)};
+}
+
+// End of a step of `count` realizations in the given workspaces.
+cageo_status enqueue_end(cageo_pipeline* p, const StepErrors& e, int count) {
+  realization_end_kernel<<<1, 32, 0, p->stream>>>(p->dscal, (int*)p->dscal + kFlags,
+                                                  p->dscal + kRedo, p->dscal + 2,
+                                                  (unsigned int)count, e, p->dscal + kErrors);
+  CAGEO_CUDA(cudaGetLastError());
+  return CAGEO_OK;
+}
+
+// What keep_errors kept of a run.
+cageo_status kept_status(uint32_t kept) {
+  if (!kept) return CAGEO_OK;
+  const uint32_t fill = kept & 255u;
+  if (fill) set_error("pit filling: %s", fill_error_text(fill));
+  else if (kept >> 8 & 255u) set_error("flow routing: %s", route_error_text());
+  else set_error("flow tracing: %s", trace_error_text());
+  return CAGEO_ERR_NO_CONVERGENCE;
+}
+
 // Launch sequence of one realization on the fast path.  The realization
 // number is read from dscal[0] by the noise kernel.
 cageo_status enqueue_fast(cageo_pipeline* p) {
@@ -266,10 +310,7 @@ cageo_status enqueue_fast(cageo_pipeline* p) {
   if ((st = enqueue_fill(p))) return st;
   if ((st = enqueue_route(p))) return st;
   if ((st = enqueue_trace_border(p, (const int*)p->dscal + kFlags, false))) return st;
-  realization_end_kernel<<<1, 32, 0, s>>>(p->dscal, (int*)p->dscal + kFlags, p->dscal + kRedo,
-                                          p->dscal + 2, 1u);
-  CAGEO_CUDA(cudaGetLastError());
-  return CAGEO_OK;
+  return enqueue_end(p, step_errors(p->fw, p->rw, p->tw), 1);
 }
 
 // Launch sequence of one stacked step: p->step realizations from the device
@@ -317,10 +358,7 @@ cageo_status enqueue_step(cageo_pipeline* p) {
   if ((st = border_u32_from_state(p->twb, p->label, p->counts, (const int*)p->dscal + kFlags,
                                   trace_mode(p), p->dscal, p->dscal + 3, s)))
     return st;
-  realization_end_kernel<<<1, 32, 0, s>>>(p->dscal, (int*)p->dscal + kFlags, p->dscal + kRedo,
-                                          p->dscal + 2, (unsigned int)K);
-  CAGEO_CUDA(cudaGetLastError());
-  return CAGEO_OK;
+  return enqueue_end(p, step_errors(p->fwb, p->rwb, p->twb), K);
 }
 
 // Reference-order stage sequence for one realization (exact burning).
@@ -345,6 +383,8 @@ cageo_status run_stage_path(cageo_pipeline* p, uint32_t r) {
   if (st) return st;
   if ((st = enqueue_route(p))) return st;
   if ((st = enqueue_trace_border(p, nullptr, true))) return st;
+  keep_errors_kernel<<<1, 1, 0, s>>>(step_errors(p->fw, p->rw, p->tw), p->dscal + kErrors);
+  CAGEO_CUDA(cudaGetLastError());
   return CAGEO_OK;
 }
 
@@ -594,16 +634,9 @@ static cageo_status pipeline_run(cageo_pipeline* p, uint32_t first, int count) {
     K = 1;
   }
   const bool stacked = K > 1 && count >= K;
-  auto step_status = [&]() -> cageo_status {
-    CAGEO_CUDA(cudaStreamSynchronize(s));
-    cageo_status e;
-    if ((e = fill_check_status(p->fwb, fs)) || (e = route_check_status(p->rwb, rs))) return e;
-    return trace_check_status(p->twb, &jumps);
-  };
   if (stacked) {
     const int steps = count / K, tail = asked ? 0 : count - steps * K;
     if ((st = run_steps(p, K, steps))) return st;
-    if (tail && (st = step_status())) return st;
     if (tail) {
       set_step(p, tail);
       if ((st = enqueue_step(p))) return st;
@@ -644,15 +677,15 @@ static cageo_status pipeline_run(cageo_pipeline* p, uint32_t first, int count) {
     }
   }
   CAGEO_CUDA(cudaStreamSynchronize(s));
-  if (p->last_batched) {
-    if ((st = step_status())) return st;
-  } else {
-    if ((st = fill_check_status(p->fw, fs))) return st;
-    if ((st = route_check_status(p->rw, rs))) return st;
-    if ((st = trace_check_status(p->tw, &jumps))) return st;
-  }
-  uint32_t nredo = 0;
-  CAGEO_CUDA(cudaMemcpy(&nredo, p->dscal + 2, sizeof(uint32_t), cudaMemcpyDeviceToHost));
+  // The last step's status and statistics, then what any step kept.
+  const bool top = p->last_batched;
+  if ((st = fill_check_status(top ? p->fwb : p->fw, fs))) return st;
+  if ((st = route_check_status(top ? p->rwb : p->rw, rs))) return st;
+  if ((st = trace_check_status(top ? p->twb : p->tw, &jumps))) return st;
+  uint32_t ends[2];  // errors, realizations to redo
+  CAGEO_CUDA(cudaMemcpy(ends, p->dscal + kErrors, sizeof(ends), cudaMemcpyDeviceToHost));
+  if ((st = kept_status(ends[0]))) return st;
+  const uint32_t nredo = ends[1];
   if (nredo) {
     if (nredo > kMaxRedo) {
       set_error("more than 4096 realizations need the exact burning path in one run");
@@ -667,6 +700,8 @@ static cageo_status pipeline_run(cageo_pipeline* p, uint32_t first, int count) {
       if ((st = run_stage_path(p, r))) return st;
     CAGEO_CUDA(cudaStreamSynchronize(s));
     if ((st = fill_check_status(p->fw, fs))) return st;
+    CAGEO_CUDA(cudaMemcpy(ends, p->dscal + kErrors, sizeof(uint32_t), cudaMemcpyDeviceToHost));
+    if ((st = kept_status(ends[0]))) return st;
     p->last_batched = false;  // the last realization computed is the last redone
   }
   p->stats[0] = fs[0];
@@ -731,8 +766,7 @@ extern "C" cageo_status cageo_pipeline_profile(cageo_pipeline* p, uint32_t reali
     if ((st = border_u32_from_state(p->tw, p->label, p->counts, (const int*)p->dscal + kFlags,
                                     trace_mode(p), p->dscal, nullptr, s)))
       break;
-    realization_end_kernel<<<1, 32, 0, s>>>(p->dscal, (int*)p->dscal + kFlags, p->dscal + kRedo,
-                                            p->dscal + 2, 1u);
+    if ((st = enqueue_end(p, step_errors(p->fw, p->rw, p->tw), 1))) break;
     cudaEventRecord(ev[6], s);
     if (cudaStreamSynchronize(s) != cudaSuccess) {
       st = cuda_fail(cudaGetLastError(), "cudaStreamSynchronize");
@@ -1106,7 +1140,11 @@ extern "C" cageo_status cageo_pipeline_autotune(cageo_pipeline* p, uint32_t firs
       st = cuda_fail(cudaGetLastError(), "cudaEventSynchronize");
       break;
     }
-    if (st == CAGEO_OK) st = fill_check_status(p->fw, nullptr);
+    uint32_t kept = 0;
+    if (st == CAGEO_OK &&
+        cudaMemcpy(&kept, p->dscal + kErrors, sizeof(kept), cudaMemcpyDeviceToHost) != cudaSuccess)
+      st = cuda_fail(cudaGetLastError(), "cudaMemcpy");
+    if (st == CAGEO_OK) st = kept_status(kept);
     float ms = 0.0f;
     cudaEventElapsedTime(&ms, e0, e1);
     ms /= (float)trials;

@@ -1095,6 +1095,19 @@ cageo_status fill_accumulate_warm_stats(const FillWork& w, unsigned long long* a
   return CAGEO_OK;
 }
 
+const unsigned int* fill_error_word(const FillWork& w) { return w.scal + S_ERR; }
+
+const char* fill_error_text(unsigned int error) {
+  static const char* what[] = {"",
+                               "a grid-wide wait hit its limit",
+                               "a warp waited for a tile past its limit",
+                               "a tile's queue state kept changing",
+                               "the tile visits or relaxation rounds passed their limit",
+                               "the confirmation phases passed their limit",
+                               "the labels of the unsettled cells are not settled roots"};
+  return error < 7 ? what[error] : "unknown error";
+}
+
 cageo_status fill_check_status(const FillWork& w, int64_t* stats) {
   unsigned int h[S_SIZE];
   CAGEO_CUDA(cudaMemcpy(h, w.scal, sizeof(h), cudaMemcpyDeviceToHost));
@@ -1118,16 +1131,8 @@ cageo_status fill_check_status(const FillWork& w, int64_t* stats) {
     stats[16] = h[S_RESET];
   }
   if (h[S_ERR]) {
-    static const char* what[] = {"",
-                                 "a grid-wide wait hit its limit",
-                                 "a warp waited for a tile past its limit",
-                                 "a tile's queue state kept changing",
-                                 "the tile visits or relaxation rounds passed their limit",
-                                 "the confirmation phases passed their limit",
-                                 "the labels of the unsettled cells are not settled roots"};
-    const unsigned int e = h[S_ERR];
     set_error("pit filling: %s (tiles finished %u, phases %u, listed cells %u)",
-              e < 7 ? what[e] : "unknown error", h[S_DONE], h[S_PHASES], h[S_CAND]);
+              fill_error_text(h[S_ERR]), h[S_DONE], h[S_PHASES], h[S_CAND]);
     return CAGEO_ERR_NO_CONVERGENCE;
   }
   return CAGEO_OK;

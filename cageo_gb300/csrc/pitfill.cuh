@@ -85,6 +85,10 @@ unsigned int* fill_min_slot(const FillWork& w);
 constexpr int kFillStats = 17;
 constexpr int kFillScalars = 224;  // words of the scalar block
 cageo_status fill_check_status(const FillWork& w, int64_t* stats);
+// The device word that a fill leaves at 0 or at an error (cleared by the next
+// fill_begin), and what that error says.
+const unsigned int* fill_error_word(const FillWork& w);
+const char* fill_error_text(unsigned int error);
 // Adds the last warm-started exact fill's counters to acc (9 device
 // uint64: fills, fills that restarted cells, cells restarted, warm-flood
 // tile visits and sweep rounds, repair sweep rounds, warm and repair

@@ -736,6 +736,10 @@ cageo_status route_run(const float* filled, int8_t* dir, int* fd, const RouteWor
   return CAGEO_OK;
 }
 
+const unsigned int* route_error_word(const RouteWork& w) { return w.scal + R_ERR; }
+
+const char* route_error_text() { return "flat-surface relaxation hit a wait or pass limit"; }
+
 cageo_status route_check_status(const RouteWork& w, int64_t* stats) {
   unsigned int h[R_SIZE];
   CAGEO_CUDA(cudaMemcpy(h, w.scal, sizeof(h), cudaMemcpyDeviceToHost));
@@ -749,7 +753,7 @@ cageo_status route_check_status(const RouteWork& w, int64_t* stats) {
     stats[6] = h[R_KCYC_STORE];
   }
   if (h[R_ERR]) {
-    set_error("flow routing: flat-surface relaxation hit a wait or pass limit");
+    set_error("flow routing: %s", route_error_text());
     return CAGEO_ERR_NO_CONVERGENCE;
   }
   return CAGEO_OK;

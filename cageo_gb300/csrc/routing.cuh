@@ -34,6 +34,9 @@ cageo_status route_run(const float* filled, int8_t* dir, int* flatdist,
 // microseconds of the flat relaxation, flat tile visits, and kilo-cycles
 // summed over visits spent staging, searching, storing.
 cageo_status route_check_status(const RouteWork& w, int64_t* stats);
+// The device word that a routing leaves at 0 or at an error, and what it says.
+const unsigned int* route_error_word(const RouteWork& w);
+const char* route_error_text();
 
 struct TraceWork {
   int W = 0, H = 0, tiles_x = 0, tiles_y = 0;
@@ -56,6 +59,9 @@ TraceWork trace_carve(void* base, int W, int H);
 cageo_status trace_run(const int8_t* dir, const float* streams, const uint8_t* code, int* label,
                        const TraceWork& w, cudaStream_t s, int mode, bool write_labels);
 cageo_status trace_check_status(const TraceWork& w, int64_t* jumps);
+// The same for a tracing.
+const unsigned int* trace_error_word(const TraceWork& w);
+const char* trace_error_text();
 
 // count[i] += border(label) (stage API).
 cageo_status border_float(const int* label, float* count, int W, int H,

@@ -315,12 +315,16 @@ cageo_status trace_run(const int8_t* dir, const float* streams, const uint8_t* c
   return CAGEO_OK;
 }
 
+const unsigned int* trace_error_word(const TraceWork& w) { return w.scal + T_ERR; }
+
+const char* trace_error_text() { return "pointer jumping hit a wait or pass limit"; }
+
 cageo_status trace_check_status(const TraceWork& w, int64_t* jumps) {
   unsigned int h[T_SIZE];
   CAGEO_CUDA(cudaMemcpy(h, w.scal, sizeof(h), cudaMemcpyDeviceToHost));
   if (jumps) *jumps = h[T_JUMPS];
   if (h[T_ERR]) {
-    set_error("flow tracing: pointer jumping hit a wait or pass limit");
+    set_error("flow tracing: %s", trace_error_text());
     return CAGEO_ERR_NO_CONVERGENCE;
   }
   return CAGEO_OK;
