@@ -13,7 +13,8 @@
 // neighbour in N..NW order.  A flat cell has no lower neighbour, so such a
 // neighbour is at its own elevation, and adjacent flat cells are level with
 // each other: layers 1 need the elevations once (the first pass finds them,
-// with their directions), all later layers only the masks of flat cells.
+// with their directions), all later layers only the masks of flat cells.  (A
+// NaN cell is level with nothing and is left out of the masks.)
 // Layer numbers are breadth-first distances; they are computed tile by tile
 // (32x32) from three things only: the tile's mask of flat cells, its mask of
 // layer-1 cells, and the distances on the neighbouring tiles' rims, kept in a
@@ -238,7 +239,9 @@ __global__ void __launch_bounds__(256) d8_kernel(const float* __restrict__ dem,
         if (xborder || ys == 0 || ys == slab_h - 1) n = 9;
         if (!xin || yw + k >= H) n = 10;
       }
-      const unsigned int f = __ballot_sync(0xffffffffu, n == 8);
+      // (CPU rules: a NaN cell is flat, but level with nothing, so that no layer
+      // enters or leaves it; the GPU order compares elevations for layer 1 only.)
+      const unsigned int f = __ballot_sync(0xffffffffu, n == 8 && (GPU || b1 == b1));
       const unsigned int h = __ballot_sync(0xffffffffu, kPlain ? n < 8 : n < 8 || n == 9);
       code[k] = n;
       if (f) {  // (no neighbour is lower: <= is level)
