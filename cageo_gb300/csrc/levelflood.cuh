@@ -140,7 +140,8 @@ __device__ __forceinline__ unsigned int sweep_lines(float2* C, int lane, unsigne
 }
 
 // One lane's column of a tile: which cells never relay (dead: outside the
-// grid, NODATA, not passable), which of those are walls (interior and not
+// grid, NODATA, not passable; in the exact fill, outlets whose elevation is
+// NaN, no level to pass on), which of those are walls (interior and not
 // passable: they take a level once the flood is over), which are outlets
 // that relay.  q_at(y) is the raw elevation; a stack of realizations takes
 // each slab's borders and minimum.
@@ -160,7 +161,7 @@ __device__ __forceinline__ CellMasks cell_masks(const FillWork& w, const unsigne
     const bool in = xin && y0 + y < w.H;
     const float v = in ? q_at(y) : 0.0f;
     const bool outlet = xborder || ys == 0 || ys == slab_h - 1 || v == 0.0f;
-    const bool pas = !minslot || passable_quantized(v, minE);
+    const bool pas = minslot ? passable_quantized(v, minE) : !outlet || v == v;
     const unsigned int bit = 1u << y;
     if (!in || v == nodata) {
       m.dead |= bit;

@@ -46,3 +46,49 @@ def test_routing_through_nan_cells(cuda, oracle, W, H):
         gr, gfr = oracle.flow_route_gpu(dem, with_flatdist=True)
         assert np.array_equal(g.cpu().numpy(), gr)
         assert np.array_equal(gfd.cpu().numpy(), gfr)
+
+
+def _exact_fill(dem, nodata=-9999.0):
+    """The exact fill's levels by relaxation: a NaN elevation bounds no level
+    (the larger of it and a level is the level), and a NaN outlet passes none on."""
+    H, W = dem.shape
+    keep = (dem == nodata) | (dem == 0)
+    keep[0] = keep[-1] = keep[:, 0] = keep[:, -1] = True
+    w = np.where(keep, dem, np.float32(np.inf))
+    while True:
+        r = np.pad(np.where((dem == nodata) | np.isnan(w), np.float32(np.inf), w), 1,
+                   constant_values=np.inf)
+        m = np.full_like(w, np.inf)
+        for dy in range(3):
+            for dx in range(3):
+                if (dy, dx) != (1, 1):
+                    m = np.minimum(m, r[dy:dy + H, dx:dx + W])
+        n = np.where(keep, dem, np.minimum(w, np.fmax(dem, m)))
+        if np.array_equal(n, w, equal_nan=True):
+            return np.where(~keep & np.isinf(n), np.float32(99990000.0), n)
+        w = n
+
+
+@pytest.mark.parametrize("W,H", [(12, 9), (33, 32), (65, 70), (130, 97)])
+def test_exact_fill_with_nan_cells(cuda, W, H):
+    """NaN outlets (a border of them, as a frame without data leaves) pass no
+    level on from one neighbour to another; NaN cells inside do."""
+    import torch
+    from cageo_gb300 import api
+    for seed in range(4):
+        rng = np.random.default_rng(seed * 100 + W)
+        dem = rng.uniform(1.0, 9.0, (H, W)).astype(np.float32)
+        frame = np.zeros((H, W), bool)
+        frame[0] = frame[-1] = frame[:, 0] = frame[:, -1] = True
+        dem[frame & (rng.random((H, W)) < (0.9 if seed % 2 else 0.4))] = np.nan
+        dem[rng.random((H, W)) < 0.02] = np.nan
+        dem[rng.random((H, W)) < 0.01] = -9999.0
+        dem[0, 0] = 1.0
+        want = _exact_fill(dem)
+        v = torch.from_numpy(dem).to(cuda)
+        f = api.pitfill(v.clone(), mode=api.FILL_EXACT).cpu().numpy()
+        assert np.array_equal(f, want, equal_nan=True)
+        warm = torch.full_like(v, float("inf"))
+        f = api.pitfill_exact_warm(v, warm)
+        f = (f[0] if isinstance(f, tuple) else f).cpu().numpy()
+        assert np.array_equal(f, want, equal_nan=True)
