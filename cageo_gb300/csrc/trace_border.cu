@@ -335,10 +335,13 @@ cageo_status trace_check_status(const TraceWork& w, int64_t* jumps) {
 // tile's columns from 4 on (16-byte aligned).  LAKE, which neither is nor makes
 // a border, and cells outside the grid are staged as the least integer, so a
 // cell is a border exactly when the largest of the 3x3 cells around it
-// exceeds its own.
+// exceeds its own.  The labels below LAKE move up by one into the place it
+// leaves, so that the least integer, a label like any other, stays apart.
 constexpr int kBS = 40;
 constexpr int kNoLabel = (int)0x80000000;
-__device__ __forceinline__ int border_key(int label) { return label == kLake ? kNoLabel : label; }
+__device__ __forceinline__ int border_key(int label) {
+  return label == kLake ? kNoLabel : label + (label < kLake ? 1 : 0);
+}
 
 // Position around the tile of halo cell h (0..131): top and bottom rows with
 // the corners, then the sides.
