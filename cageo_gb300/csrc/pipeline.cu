@@ -568,9 +568,11 @@ static void set_step(cageo_pipeline* p, int K) {
 // twice as many cells a step gain nothing there.
 constexpr int64_t kStackCells = (int64_t)1 << 26;
 
+// Rows of a stack: launches over tiles of 32 rows have them in grid.y.
+constexpr int kStackRows = 65535 * 32;
+
 static int stack_of(const cageo_pipeline* p, int count) {
-  // (Launches over tiles have their rows in grid.y: 65535 at most.)
-  const int64_t fit = std::min<int64_t>({kMaxStack, kStackCells / p->N, 65535 * 32 / p->H});
+  const int64_t fit = std::min<int64_t>({kMaxStack, kStackCells / p->N, kStackRows / p->H});
   if (p->plain || fit < 2 || count < 2) return 1;
   const int steps = (int)((count + fit - 1) / fit);
   return (count + steps - 1) / steps;  // even steps
@@ -1182,6 +1184,7 @@ extern "C" cageo_status cageo_pipeline_set_batch(cageo_pipeline* p, int batch) {
   p->batch = 1;
   p->plain = batch == 1;
   if (batch == 1) return CAGEO_OK;
+  batch = std::min(batch, kStackRows / p->H);  // (at least 32: H <= 65535)
   const cageo_status st = ensure_stack(p, batch);
   if (st) return st;
   set_step(p, batch);

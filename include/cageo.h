@@ -333,8 +333,9 @@ cageo_status cageo_pipeline_run_filter(cageo_pipeline* p, uint32_t first_realiza
  * not with a learned warm start) and runs singly where the memory for a stack
  * (28 to 32 bytes per cell per realization, allocated by the first such run)
  * cannot be had.  batch = 1: one realization at a time, no stacks; frees them.
- * batch > 1: steps of that many whatever the grid, the rest of `count` singly;
- * batch <= 64, batch * cells < 2^31, CPU-compatible fill mode only. */
+ * batch > 1: steps of that many (at most 2097120 / height) whatever the grid,
+ * the rest of `count` singly; batch <= 64, batch * cells < 2^31, CPU-compatible
+ * fill mode only. */
 cageo_status cageo_pipeline_set_batch(cageo_pipeline* p, int batch);
 /* Border counts so far as float (the reference's CatchmentBorderType). */
 cageo_status cageo_pipeline_counts(cageo_pipeline* p, float* h_out);
