@@ -19,8 +19,8 @@
 // reference has no flag for it), --no-graphs, --fill cpu|exact (cpu: the
 // reference CPU path's semantics, the default; exact: its GPU path's exact
 // float fill, flat order and dead-end handling), --checkpoint FILE,
-// --resume FILE, --batch K (realizations per batched step; 1).  Output
-// files go to the
+// --resume FILE, --batch K (realizations per stacked step, 1: one at a time;
+// unset: small grids are stacked by themselves).  Output files go to the
 // working directory under the stem of -o (the reference keeps only the
 // stem).  This driver runs on the GPU only; --cpu
 // is refused rather than silently using another implementation.
@@ -39,8 +39,8 @@ struct Options {
   std::string dem = "dem10", stream = "streams", dem_path = "DEM", stream_path = "DEM";
   std::string filter = "Gaussian", output_file, output_option, checkpoint, resume, fill = "cpu";
   float range = 60.0f, mean = 0.0f, sd = 1.0f;
-  int iterations = 10, bevel = 2, batch = 1;
-  bool gpu = true, cpu = false, graphs = true, have_seed = false;
+  int iterations = 10, bevel = 2, batch = 0;
+  bool gpu = true, cpu = false, graphs = true, have_seed = false, have_batch = false;
   unsigned long long seed = 0;
 };
 
@@ -67,7 +67,8 @@ void usage() {
       "  --fill arg (=cpu)            cpu: CPU-path semantics; exact: GPU-path exact float fill\n"
       "  --checkpoint arg             Save counts + next realization here after each output\n"
       "  --resume arg                 Continue from a checkpoint (same grid and --seed)\n"
-      "  --batch arg (=1)             Realizations per batched step (CPU-path fill; same results)\n");
+      "  --batch arg                  Realizations per stacked step, 1: one at a time (above 1: CPU-path\n"
+      "                               fill; same results; default: chosen by the grid's size)\n");
 }
 
 bool parse_bool(const std::string& v) { return !(v == "0" || v == "false" || v == "off"); }
@@ -106,7 +107,7 @@ int parse(int argc, char** argv, Options* o) {
     else if (a == "--seed") { if (!next(&v)) return 1; o->seed = std::strtoull(v.c_str(), nullptr, 10); o->have_seed = true; }
     else if (a == "--bevel-radius") { if (!next(&v)) return 1; o->bevel = std::atoi(v.c_str()); }
     else if (a == "--no-graphs") { o->graphs = false; }
-    else if (a == "--batch") { if (!next(&v)) return 1; o->batch = std::atoi(v.c_str()); }
+    else if (a == "--batch") { if (!next(&v)) return 1; o->batch = std::atoi(v.c_str()); o->have_batch = true; }
     else if (a == "--fill") {
       if (!next(&o->fill)) return 1;
       if (o->fill != "cpu" && o->fill != "exact") {
@@ -213,7 +214,7 @@ int main(int argc, char** argv) {
   std::printf("Seed: %llu\n", (unsigned long long)cfg.seed);
   cageo_pipeline* p = nullptr;
   if (cageo_pipeline_create(&p, &cfg, dem.data(), streams.data())) return fail("pipeline");
-  if (o.batch != 1 && cageo_pipeline_set_batch(p, o.batch)) {
+  if (o.have_batch && cageo_pipeline_set_batch(p, o.batch)) {
     cageo_pipeline_destroy(p);
     return fail("batch");
   }
