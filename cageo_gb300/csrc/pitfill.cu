@@ -30,10 +30,12 @@
 //      change can leave.  A component without a cell of the kind just named
 //      is settled at A.  In the others the cells restart at S, those
 //      non-passable cells with A > q are confirmed (they certainly expand),
-//      and phases follow: relax; M = the component's least level among
-//      unconfirmed non-passable cells above their q; every such cell with
-//      q <= M is confirmed (no later change can take its level below M);
-//      until none is left.
+//      and the levels relax to an upper bound B.  Where B == A both are the
+//      answer.  The cells between A and B form components of their own, for
+//      which phases follow: M = the component's least level among unconfirmed
+//      non-passable cells above their q; every such cell with q <= M is
+//      confirmed (no later change can take its level below M); relax; until
+//      none is left.
 //
 // Steps 2 and 3 work on lists of cells (fill_resolve_kernel); the flood of
 // step 1 -- and the exact fill, which is that flood without walls -- is a
@@ -63,6 +65,9 @@ enum : int {
   S_CAND = 10,     // walls on the list of the resolution
   S_MORE = 22,     // cells listed by the resolution itself
   S_OPEN = 23,     // cells of the reopened components
+  S_UNSURE = 24,   // walls between the bounds A and B
+  S_FRONT = 25,    // other cells among the first S_UNSURE of the list
+  S_BEHIND = 26,   // such walls after those
   S_PASS = 11,     // floods and relaxations run so far in this fill
   S_PHASES = 12,
   S_PASSES_A = 13, // drains of the flood (1)
@@ -97,7 +102,8 @@ __device__ __forceinline__ unsigned long long global_ns() {
 }
 
 // Per-cell flag bits of the resolution.
-constexpr unsigned int kActive = 1, kConfirmed = 2, kMember = 4, kReopened = 8;
+constexpr unsigned int kActive = 1, kConfirmed = 2, kMember = 4, kReopened = 8, kUnsure = 16,
+                       kUnsureWall = 32;
 
 // The space that the flood's rims and masks share with the component labels
 // of the resolution: the labels are the larger part except on grids only a
@@ -640,11 +646,14 @@ __device__ __forceinline__ void front_push(const Resolve& r, Front& f, int buf, 
   }
 }
 
-// Relaxes from the active cells among the nl of a list until no level falls.
+// Relaxes from the active cells among the first nl of a list -- after that, what
+// a full buffer left among all na of it -- until no level falls.
 // LOWER: the list is cand; walls with S > q relay whatever their level, and a
 // neighbour that falls is listed (from entry nu0 on, *more of them so far);
-// otherwise the list holds the reopened components, confirmed walls above
-// their q relay, and only these cells can fall.
+// otherwise the list holds the reopened components or the cells between the
+// bounds, confirmed walls above their q relay, and only these cells can fall.
+// minima: the least pending levels (aux) of the first nl cells' components are
+// reset.
 //
 // The falls travel up to ~70 cells at 4096^2 (~170 at 8192^2) from where they
 // start, so what counts is the time of a step.  Each block follows the fronts
@@ -658,12 +667,14 @@ __device__ __forceinline__ void front_push(const Resolve& r, Front& f, int buf, 
 // consecutive entries, which lie in the same tiles.
 template <bool LOWER>
 __device__ unsigned int relax(const Resolve& r, Front& f, const uint32_t* list, unsigned int nl,
-                              unsigned int nblocks, unsigned int* more, bool* ok) {
+                              unsigned int na, unsigned int nblocks, bool minima,
+                              unsigned int* more, bool* ok) {
   const FillWork& w = r.w;
   const unsigned int nu0 = nl;
   unsigned int steps = 0;
-  for (bool again = true; again;) {
-    const unsigned int nu = LOWER ? nl + *more : nl;
+  bool again_all = false;
+  for (bool again = true; again; again_all = true) {
+    const unsigned int nu = LOWER ? nl + *more : again_all ? na : nl;
     const unsigned int run = min(LOWER ? kResolveRun : kReopenRun, (nu + nblocks - 1) / nblocks);
     if (threadIdx.x == 0) f.full = f.nfresh = 0;
     for (unsigned int base = blockIdx.x * run; base < nu; base += nblocks * run) {
@@ -678,8 +689,8 @@ __device__ unsigned int relax(const Resolve& r, Front& f, const uint32_t* list, 
         const unsigned int fl = r.get(c);
         if (LOWER) {
           if (j < nu0) w.label[c] = c;
-        } else if (__ldcg(w.label + c) == c) {
-          __stcg(w.aux + c, 0xffffffffu);  // the component's least pending level
+        } else if (minima && !again_all) {
+          __stcg(w.aux + __ldcg(w.label + c), 0xffffffffu);
         }
         if (!(fl & kActive)) continue;
         r.clear(c, kActive);
@@ -769,7 +780,7 @@ __global__ void __launch_bounds__(kResolveThreads, 2) fill_resolve_kernel(Resolv
   unsigned int more = 0;
   bool ok = true;
   if (nu0) {
-    const unsigned int steps = relax<true>(r, front, w.cand, nu0, nblocks, &more, &ok);
+    const unsigned int steps = relax<true>(r, front, w.cand, nu0, 0u, nblocks, false, &more, &ok);
     if (threadIdx.x == 0) atomicMax(&w.scal[S_STEPS], steps);
   }
   const unsigned long long t1 = global_ns();
@@ -813,15 +824,15 @@ __global__ void __launch_bounds__(kResolveThreads, 2) fill_resolve_kernel(Resolv
     // The cells of reopened components restart at S -- or at what a settled
     // listed wall beside them offers, if that is less -- with the walls that A
     // left above their q confirmed, and are listed once more after the others
-    // (where the list fills the array, it is used whole).  From here aux
-    // holds the components' least pending level.
+    // (where the list fills the array, it is used whole).  aux holds their A
+    // from here on.
     const bool apart = 2 * (uint64_t)nu <= (uint64_t)w.W * w.H;
     for (int64_t j = tid; j < nu && ok; j += nthreads) {
       const uint32_t c = __ldcg(w.cand + j);
       if (!(r.get(c) & kMember)) continue;
       const uint32_t root = __ldcg(w.label + c);
-      // Every label is a root: a cell labelled otherwise would take a
-      // minimum nothing resets.
+      // Every label is a root: a cell labelled otherwise would miss its
+      // component's mark.
       if (__ldcg(w.label + root) != root) atomicCAS((int*)(w.scal + S_ERR), 0, 6);
       const bool open = r.get(root) & kReopened;
       if (open) {
@@ -848,6 +859,7 @@ __global__ void __launch_bounds__(kResolveThreads, 2) fill_resolve_kernel(Resolv
         }
         const bool confirm = lv > qc && s > qc && r.wall(c, qc);
         if (confirm || start < s) r.set(c, (confirm ? kConfirmed : 0u) | kActive);
+        __stcg(w.aux + c, __float_as_uint(lv));
         __stcg(r.Wg + c, -start);
       }
       const unsigned int pos = warp_append(&w.scal[S_OPEN], open && apart);
@@ -855,41 +867,101 @@ __global__ void __launch_bounds__(kResolveThreads, 2) fill_resolve_kernel(Resolv
     }
     any_of(w, front, nblocks, false, &more, &ok);
     const unsigned int no = apart ? vs[S_OPEN] : nu;
-    const uint32_t* open_list = apart ? w.cand + nu : w.cand;
-    while (ok) {
-      relax<false>(r, front, open_list, no, nblocks, &more, &ok);
-      if (!ok) break;
-      // The unconfirmed walls above their q.
-      auto pending = [&](int64_t j, uint32_t& c, float& lv, float& qc) {
-        c = __ldcg(open_list + j);
+    uint32_t* list = apart ? w.cand + nu : w.cand;
+    if (ok) relax<false>(r, front, list, no, no, nblocks, false, &more, &ok);
+    // The upper bound B; the cells above A are labelled anew.
+    auto between = [&](uint32_t c) { return (r.get(c) & kUnsure) != 0; };
+    bool unsure = false;
+    for (int64_t j = tid; j < no && ok; j += nthreads) {
+      const uint32_t c = __ldcg(list + j);
+      const bool u = (r.get(c) & kMember) &&
+                     (apart || (r.get(__ldcg(w.label + c)) & kReopened)) && r.level(c) != r.walled(c);
+      const bool wall = u && r.wall(c, r.q[c]);
+      warp_append(&w.scal[S_UNSURE], wall);
+      if (!u) continue;
+      r.set(c, kUnsure | (wall ? kUnsureWall : 0u));
+      __stcg(w.label + c, c);
+      unsure |= wall;
+    }
+    if (any_of(w, front, nblocks, unsure, &more, &ok)) {
+      // The walls among them, which are all that the phases look at, move to the
+      // front of the list, in exchange for others (whose places are noted in
+      // aux, which is free now; at most half of the list each).
+      const unsigned int nq = vs[S_UNSURE];
+      uint32_t *places = w.aux, *behind = w.aux + (uint64_t)w.W * w.H / 2;
+      bool joined = true;
+      for (int64_t j = tid; j < no; j += nthreads) {
+        const uint32_t c = __ldcg(list + j);
         const unsigned int f = r.get(c);
-        qc = r.q[c];
-        lv = r.level(c);
-        if (!(f & kMember) || (f & kConfirmed)) return false;
-        if (!apart && !(r.get(__ldcg(w.label + c)) & kReopened)) return false;
-        return lv > qc && r.wall(c, qc);
-      };
-      bool some = false;
-      uint32_t c;
-      float lv, qc;
-      for (int64_t j = tid; j < no; j += nthreads) {
-        if (!pending(j, c, lv, qc) || lv == kInf) continue;
-        atomicMin(&w.aux[__ldcg(w.label + c)], __float_as_uint(lv));
-        some = true;
+        const bool u = f & kUnsureWall;
+        const unsigned int a = warp_append(&w.scal[S_FRONT], !u && j < nq);
+        const unsigned int b = warp_append(&w.scal[S_BEHIND], u && j >= nq);
+        if (!u && j < nq) __stcg(places + a, (uint32_t)j);
+        if (u && j >= nq) __stcg(behind + b, (uint32_t)j);
+        if (!(f & kUnsure)) continue;
+        const int cx = (int)(c % (uint32_t)w.W), cy = (int)(c / (uint32_t)w.W);
+#pragma unroll 1
+        for (int d = 0; d < 4; d++) {  // W, NW, N, NE
+          const int nx = cx + (d == 0 ? -1 : d - 2), ny = cy + (d == 0 ? 0 : -1);
+          if (nx < 0 || ny < 0 || nx >= w.W) continue;
+          const uint32_t n = (uint32_t)ny * (uint32_t)w.W + (uint32_t)nx;
+          if (between(n)) joined &= uf_unite(w.label, c, n);
+        }
       }
-      if (!any_of(w, front, nblocks, some, &more, &ok)) break;
-      // Each phase confirms at least one cell of every component with a
-      // pending one (the cell holding its minimum).
-      if (++phases > (int)min(nu, 0x7fffff00u) + 8) {
-        if (threadIdx.x == 0) atomicCAS((int*)(w.scal + S_ERR), 0, 5);
-        break;  // (in every block)
-      }
-      for (int64_t j = tid; j < no; j += nthreads) {
-        if (!pending(j, c, lv, qc)) continue;
-        const unsigned int m = __ldcg(w.aux + __ldcg(w.label + c));
-        if (m != 0xffffffffu && qc <= __uint_as_float(m)) r.set(c, kConfirmed | kActive);
+      if (!joined) atomicCAS((int*)(w.scal + S_ERR), 0, 6);
+      any_of(w, front, nblocks, false, &more, &ok);
+      const unsigned int moves = vs[S_FRONT];
+      for (int64_t k = tid; k < moves && ok; k += nthreads) {
+        const uint32_t a = __ldcg(places + k), b = __ldcg(behind + k);
+        const uint32_t ca = __ldcg(list + a), cb = __ldcg(list + b);
+        __stcg(list + a, cb);
+        __stcg(list + b, ca);
       }
       any_of(w, front, nblocks, false, &more, &ok);
+      // From here aux holds the components' least pending level (at their roots).
+      for (int64_t j = tid; j < nq && ok; j += nthreads) {
+        const uint32_t c = __ldcg(list + j), root = uf_root(w.label, c);
+        w.label[c] = root;
+        __stcg(w.aux + root, 0xffffffffu);
+      }
+      any_of(w, front, nblocks, false, &more, &ok);
+      while (ok) {
+        // The unconfirmed walls above their q.
+        auto pending = [&](int64_t j, uint32_t& c, float& lv, float& qc) {
+          c = __ldcg(list + j);
+          if (r.get(c) & kConfirmed) return false;
+          qc = r.q[c];
+          lv = r.level(c);
+          return lv > qc;
+        };
+        bool some = false;
+        uint32_t c;
+        float lv, qc;
+        for (int64_t j = tid; j < nq; j += nthreads) {
+          if (!pending(j, c, lv, qc) || lv == kInf) continue;
+          const uint32_t root = __ldcg(w.label + c);
+          // Every label is a root: a cell labelled otherwise would take a minimum
+          // nothing resets.
+          if (phases == 0 && __ldcg(w.label + root) != root)
+            atomicCAS((int*)(w.scal + S_ERR), 0, 6);
+          atomicMin(&w.aux[root], __float_as_uint(lv));
+          some = true;
+        }
+        if (!any_of(w, front, nblocks, some, &more, &ok)) break;
+        // Each phase confirms at least one cell of every component with a
+        // pending one (the cell holding its minimum).
+        if (++phases > (int)min(nq, 0x7fffff00u) + 8) {
+          if (threadIdx.x == 0) atomicCAS((int*)(w.scal + S_ERR), 0, 5);
+          break;  // (in every block)
+        }
+        for (int64_t j = tid; j < nq; j += nthreads) {
+          if (!pending(j, c, lv, qc)) continue;
+          const unsigned int m = __ldcg(w.aux + __ldcg(w.label + c));
+          if (m != 0xffffffffu && qc <= __uint_as_float(m)) r.set(c, kConfirmed | kActive);
+        }
+        any_of(w, front, nblocks, false, &more, &ok);
+        if (ok) relax<false>(r, front, list, nq, no, nblocks, true, &more, &ok);
+      }
     }
   }
   // The marks come off, and cells no outlet reached keep q.
