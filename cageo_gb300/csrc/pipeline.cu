@@ -57,17 +57,22 @@ constexpr int kFlags = 4;                   // the step's anomaly flags
 constexpr int kRedo = kFlags + kMaxStack;   // realizations to redo
 constexpr unsigned int kMaxRedo = 4096;
 
-// The error words of a step's fill, routing and tracing.
+// The error words of a step's fill, routing and tracing, and the word that says
+// whether the fill needs the wide resolution.
 struct StepErrors {
-  const unsigned int *fill, *route, *trace;
+  const unsigned int *fill, *route, *trace, *wide;
 };
+constexpr uint32_t kWideSeen = 1u << 24;  // in dscal[kErrors]
 
 // One thread at the end of a step: the next step's start clears the stages'
 // error words, so the first step of a run that left any is kept, a byte per
-// stage, until the host reads it at the run's end.
+// stage, until the host reads it at the run's end, and kWideSeen beside it.
 __device__ __forceinline__ void keep_errors(const StepErrors& e, uint32_t* kept) {
   const uint32_t now = min(*e.fill, 255u) | min(*e.route, 255u) << 8 | min(*e.trace, 255u) << 16;
-  if (now && *kept == 0u) *kept = now;
+  const bool wide = *e.wide != 0u;
+  if (!now && !wide) return;
+  const uint32_t was = *kept;
+  *kept = (was & (kWideSeen - 1u) ? was : was | now) | (wide ? kWideSeen : 0u);
 }
 
 __global__ void keep_errors_kernel(StepErrors e, uint32_t* kept) { keep_errors(e, kept); }
@@ -207,6 +212,15 @@ void drop_step_graph(cageo_pipeline* p) {
   p->graph_k = 0;
 }
 
+void drop_graph(cageo_pipeline* p) {
+  if (p->exec) cudaGraphExecDestroy(p->exec);
+  if (p->graph) cudaGraphDestroy(p->graph);
+  p->exec = nullptr;
+  p->graph = nullptr;
+  p->graph_ok = false;
+  drop_step_graph(p);
+}
+
 void free_stack(cageo_pipeline* p) {
   drop_step_graph(p);
   void* bufs[] = {p->qb, p->filledb, p->noiseb, p->fill_ws_b, p->slab_min, p->dirb,
@@ -273,7 +287,8 @@ cageo_status enqueue_trace_border(cageo_pipeline* p, const int* gate, bool every
 }
 
 StepErrors step_errors(const FillWork& f, const RouteWork& r, const TraceWork& t) {
-  return StepErrors{fill_error_word(f), route_error_word(r), trace_error_word(t)};
+  return StepErrors{fill_error_word(f), route_error_word(r), trace_error_word(t),
+                    fill_wide_word(f)};
 }
 
 // End of a step of `count` realizations in the given workspaces.
@@ -287,7 +302,7 @@ cageo_status enqueue_end(cageo_pipeline* p, const StepErrors& e, int count) {
 
 // What keep_errors kept of a run.
 cageo_status kept_status(uint32_t kept) {
-  if (!kept) return CAGEO_OK;
+  if (!(kept & (kWideSeen - 1u))) return CAGEO_OK;
   const uint32_t fill = kept & 255u;
   if (fill) set_error("pit filling: %s", fill_error_text(fill));
   else if (kept >> 8 & 255u) set_error("flow routing: %s", route_error_text());
@@ -361,6 +376,14 @@ cageo_status enqueue_step(cageo_pipeline* p) {
   return enqueue_end(p, step_errors(p->fwb, p->rwb, p->twb), K);
 }
 
+// The wide resolution is part of every fill as long as this lives.
+struct WithWide {
+  FillWork& w;
+  const bool was;
+  explicit WithWide(FillWork& fill) : w(fill), was(fill.wide) { w.wide = true; }
+  ~WithWide() { w.wide = was; }
+};
+
 // Reference-order stage sequence for one realization (exact burning).
 cageo_status run_stage_path(cageo_pipeline* p, uint32_t r) {
   cudaStream_t s = p->stream;
@@ -378,6 +401,7 @@ cageo_status run_stage_path(cageo_pipeline* p, uint32_t r) {
   if (!exact_mode(p) && (st = fill_quantize_min(p->q, p->fw, c.nodata_dem, s))) return st;
   // In exact mode no stage kernel has set the fill's seeds.
   p->fw.seeded = !exact_mode(p);
+  const WithWide wide(p->fw);
   st = enqueue_fill(p);
   p->fw.seeded = true;
   if (st) return st;
@@ -498,6 +522,7 @@ cageo_status create_common(cageo_pipeline** out, const cageo_pipeline_config* cf
   p->fp.W = W;
   p->fp.H = H;
   p->fw.seeded = true;
+  p->fw.undone = p->fp.anomaly;
   PCUDA(cudaStreamSynchronize(s));
 #undef PCUDA
   *out = p;
@@ -556,6 +581,8 @@ static void set_step(cageo_pipeline* p, int K) {
   p->fwb.slab_h = p->H;
   p->fwb.slab_min = p->slab_min;
   p->fwb.seeded = true;
+  p->fwb.wide = p->fw.wide;
+  p->fwb.undone = p->fw.undone;
   p->fwb.max_rounds = p->fw.max_rounds;
   p->fwb.flood_warps = p->fw.flood_warps;
 }
@@ -578,6 +605,37 @@ static int stack_of(const cageo_pipeline* p, int count) {
   return (count + steps - 1) / steps;  // even steps
 }
 
+// Steps start without the wide resolution, whose launch costs 5 us where it is
+// not needed (14 us beside other streams' kernels: it asks for room on all SMs).
+// A fill that needs it flags its step's realizations, which are then redone like
+// those of the burn check; from then on the steps include it.
+static void take_wide(cageo_pipeline* p) {
+  p->fw.wide = p->fwb.wide = true;
+  drop_graph(p);  // captured without it
+}
+
+// Waits for a first step (of K realizations) that is about to be captured;
+// whether it has to run again with the wide resolution.
+static cageo_status first_step_again(cageo_pipeline* p, uint32_t K, bool* again) {
+  *again = false;
+  if (exact_mode(p) || p->fw.wide) {
+    CAGEO_CUDA(cudaStreamSynchronize(p->stream));
+    return CAGEO_OK;
+  }
+  uint32_t scalars[3];  // (the copy to pageable memory waits, too)
+  CAGEO_CUDA(cudaMemcpyAsync(scalars, p->dscal, sizeof(scalars), cudaMemcpyDeviceToHost, p->stream));
+  CAGEO_CUDA(cudaStreamSynchronize(p->stream));
+  if (!(scalars[kErrors] & kWideSeen)) return CAGEO_OK;
+  take_wide(p);
+  // Not counted, flagged, listed last: as if it had not run.
+  scalars[0] -= K;
+  scalars[kErrors] &= kWideSeen - 1u;
+  scalars[2] -= K;
+  CAGEO_CUDA(cudaMemcpyAsync(p->dscal, scalars, sizeof(scalars), cudaMemcpyHostToDevice, p->stream));
+  *again = true;
+  return CAGEO_OK;
+}
+
 // `steps` stacked steps of K realizations, replaying a captured graph where
 // one is wanted: it is captured on first use, and again for another K once
 // that has been used by two runs in a row.
@@ -589,9 +647,11 @@ static cageo_status run_steps(cageo_pipeline* p, int K, int steps) {
   if (p->cfg.use_graphs && p->graph_k != K && (p->graph_k == 0 || p->last_k == K)) {
     drop_step_graph(p);
     // Warm-up outside capture, then capture one step.
-    if ((st = enqueue_step(p))) return st;
+    for (bool again = true; again;) {
+      if ((st = enqueue_step(p))) return st;
+      if ((st = first_step_again(p, (uint32_t)K, &again))) return st;
+    }
     b = 1;
-    CAGEO_CUDA(cudaStreamSynchronize(s));
     cudaGraph_t g = nullptr;
     if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
       cageo_status cst = enqueue_step(p);
@@ -615,8 +675,8 @@ static cageo_status run_steps(cageo_pipeline* p, int K, int steps) {
   return CAGEO_OK;
 }
 
-static cageo_status pipeline_run(cageo_pipeline* p, uint32_t first, int count) {
-  CAGEO_CHECK_ARG(p && count >= 0, "pipeline and count");
+// At most kMaxRedo realizations, of which any may have to be redone.
+static cageo_status run_part(cageo_pipeline* p, uint32_t first, int count) {
   cudaStream_t s = p->stream;
   cageo_status st;
   const uint32_t scalars[kRedo] = {first, 0, 0, first + (uint32_t)count - 1u};
@@ -649,9 +709,11 @@ static cageo_status pipeline_run(cageo_pipeline* p, uint32_t first, int count) {
   if (!stage_only && count > done && p->cfg.use_graphs && !p->graph_ok && !p->exec) {
     // Warm-up outside capture (kernel attributes, occupancy caches), then
     // capture one realization.
-    if ((st = enqueue_fast(p))) return st;
+    for (bool again = true; again;) {
+      if ((st = enqueue_fast(p))) return st;
+      if ((st = first_step_again(p, 1u, &again))) return st;
+    }
     done += 1;
-    CAGEO_CUDA(cudaStreamSynchronize(s));
     if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
       cageo_status cst = enqueue_fast(p);
       cudaGraph_t g = nullptr;
@@ -687,12 +749,9 @@ static cageo_status pipeline_run(cageo_pipeline* p, uint32_t first, int count) {
   uint32_t ends[2];  // errors, realizations to redo
   CAGEO_CUDA(cudaMemcpy(ends, p->dscal + kErrors, sizeof(ends), cudaMemcpyDeviceToHost));
   if ((st = kept_status(ends[0]))) return st;
+  if ((ends[0] & kWideSeen) && !p->fw.wide) take_wide(p);
   const uint32_t nredo = ends[1];
   if (nredo) {
-    if (nredo > kMaxRedo) {
-      set_error("more than 4096 realizations need the exact burning path in one run");
-      return CAGEO_ERR_NO_CONVERGENCE;
-    }
     std::vector<uint32_t> redo(nredo);
     CAGEO_CUDA(cudaMemcpy(redo.data(), p->dscal + kRedo, sizeof(uint32_t) * nredo,
                           cudaMemcpyDeviceToHost));
@@ -721,6 +780,21 @@ static cageo_status pipeline_run(cageo_pipeline* p, uint32_t first, int count) {
   return CAGEO_OK;
 }
 
+static cageo_status pipeline_run(cageo_pipeline* p, uint32_t first, int count) {
+  CAGEO_CHECK_ARG(p && count >= 0, "pipeline and count");
+  // (Whole steps of the batch asked for in every part but the last.)
+  const int part = (int)kMaxRedo / p->batch * p->batch;
+  for (int64_t redone = 0;;) {
+    const int n = std::min(count, part);
+    const cageo_status st = run_part(p, first, n);
+    if (st) return st;
+    p->stats[4] = redone += p->stats[4];
+    first += (uint32_t)n;
+    count -= n;
+    if (count == 0) return CAGEO_OK;
+  }
+}
+
 extern "C" cageo_status cageo_pipeline_run(cageo_pipeline* p, uint32_t first, int count) {
   return guarded("cageo_pipeline_run", [&] { return pipeline_run(p, first, count); });
 }
@@ -736,6 +810,7 @@ extern "C" cageo_status cageo_pipeline_profile(cageo_pipeline* p, uint32_t reali
   CAGEO_CHECK_ARG(p->cfg.nodata_dem != 0.0f, "profiling needs the fused path (NODATA != 0)");
   cudaStream_t s = p->stream;
   const cageo_pipeline_config& c = p->cfg;
+  const WithWide wide(p->fw);
   p->last_batched = false;
   cudaEvent_t ev[7], fm[4];
   for (auto& e : ev) CAGEO_CUDA(cudaEventCreate(&e));
@@ -823,13 +898,7 @@ static cageo_status pipeline_run_filter(cageo_pipeline* p, uint32_t first, int c
   p->cfg.error_mean = error_mean;
   p->cfg.error_stddev = error_stddev;
   p->radius = r;
-  // The captured graphs hold the old filter's launch shapes: drop them.
-  if (p->exec) cudaGraphExecDestroy(p->exec);
-  if (p->graph) cudaGraphDestroy(p->graph);
-  p->exec = nullptr;
-  p->graph = nullptr;
-  p->graph_ok = false;
-  drop_step_graph(p);
+  drop_graph(p);  // captured with the old filter's launch shapes
   p->cfg.use_graphs = 0;
   return pipeline_run(p, first, count);
 }
@@ -1051,15 +1120,6 @@ extern "C" int cageo_autotune_candidates(cageo_tuning* h_out, int n) {
   return kTuneCandidates;
 }
 
-static void drop_graph(cageo_pipeline* p) {
-  if (p->exec) cudaGraphExecDestroy(p->exec);
-  if (p->graph) cudaGraphDestroy(p->graph);
-  p->exec = nullptr;
-  p->graph = nullptr;
-  p->graph_ok = false;
-  drop_step_graph(p);
-}
-
 // Stacked steps run with the single fill's tuning.
 static void sync_step_tuning(cageo_pipeline* p) {
   if (p->step) set_step(p, p->step);
@@ -1104,6 +1164,7 @@ extern "C" cageo_status cageo_pipeline_autotune(cageo_pipeline* p, uint32_t firs
   CAGEO_CUDA(cudaEventCreate(&e0));
   CAGEO_CUDA(cudaEventCreate(&e1));
   cageo_status st = CAGEO_OK;
+  const WithWide wide(p->fw);
   p->last_batched = false;
   float best_ms = 0.0f;
   cageo_tuning best{p->fw.max_rounds, p->fw.flood_warps, p->conv_tile};

@@ -37,7 +37,9 @@
 //      confirmed (no later change can take its level below M); relax; until
 //      none is left.
 //
-// Steps 2 and 3 work on lists of cells (fill_resolve_kernel); the flood of
+// Steps 2 and 3 work on lists of cells (fill_resolve_kernel), or, where the
+// lower bound would take long that way, on tiles again
+// (fill_resolve_wide_kernel); the flood of
 // step 1 -- and the exact fill, which is that flood without walls -- is a
 // persistent cooperative kernel over 32x32 tiles (levelflood.cuh): one warp
 // owns a tile at a time and sweeps it until it is a fixed point for its
@@ -68,6 +70,7 @@ enum : int {
   S_UNSURE = 24,   // walls between the bounds A and B
   S_FRONT = 25,    // other cells among the first S_UNSURE of the list
   S_BEHIND = 26,   // such walls after those
+  S_WIDE = 27,     // 1: the lower bound is left to the wide resolution
   S_PASS = 11,     // floods and relaxations run so far in this fill
   S_PHASES = 12,
   S_PASSES_A = 13, // drains of the flood (1)
@@ -558,6 +561,7 @@ struct Front {
   float level[2][kFrontCells];
   int n[3];
   int full;  // an entry did not fit: its cell was marked kActive instead
+  int stop;  // a block has left the lower bound to the wide resolution
   // Cells to list.  They are listed many at a time: an addition to the list's
   // length in every step made it three dependent L2 accesses instead of two.
   uint32_t fresh[kFreshCells];
@@ -568,8 +572,9 @@ struct Front {
 
 // Grid barrier of the `nblocks` blocks of the resolution.  Returns whether any
 // thread passed true; *more = the entries listed by then (nothing is listed
-// between the last arrival, which takes the number, and the release); *ok =
-// false on an error (any block's) or a wait limit.
+// between the last arrival, which takes the number, and the release); f.stop =
+// whether the fill is left to the wide resolution; *ok = false on an error (any
+// block's) or a wait limit.
 __device__ bool any_of(const FillWork& w, Front& f, unsigned int nblocks, bool mine,
                        unsigned int* more, bool* ok) {
   __shared__ unsigned int sh_any, sh_more, sh_ok;
@@ -580,7 +585,7 @@ __device__ bool any_of(const FillWork& w, Front& f, unsigned int nblocks, bool m
     sh_ok = 1u;
     if (nblocks == 1) {
       sh_any = block ? 1u : 0u;
-      sh_more = vs[S_MORE];
+      sh_more = vs[S_MORE] | vs[S_WIDE] << 31;
     } else {
       // (The generation is counted, not read here: a read could be performed
       // after the arrival, and after the release that it is to wait for.)
@@ -590,7 +595,7 @@ __device__ bool any_of(const FillWork& w, Front& f, unsigned int nblocks, bool m
       if ((arrived & 0xffffu) == nblocks - 1) {
         vs[S_BAR_COUNT] = 0u;
         vs[S_RESULT] = block || arrived >> 16 ? 1u : 0u;
-        vs[S_MORE_AT] = vs[S_MORE];
+        vs[S_MORE_AT] = vs[S_MORE] | vs[S_WIDE] << 31;  // (S_MORE is below 2^31)
         __threadfence();
         atomicAdd(&w.scal[S_BAR_GEN], 1u);
       } else {
@@ -611,10 +616,11 @@ __device__ bool any_of(const FillWork& w, Front& f, unsigned int nblocks, bool m
       sh_more = vs[S_MORE_AT];
     }
     if (vs[S_ERR]) sh_ok = 0u;
+    f.stop = (int)(sh_more >> 31);
   }
   __syncthreads();
   const bool any = sh_any != 0u;
-  *more = sh_more;
+  *more = sh_more & 0x7fffffffu;
   *ok = sh_ok != 0u;
   __syncthreads();
   return any && *ok;
@@ -646,6 +652,75 @@ __device__ __forceinline__ void front_push(const Resolve& r, Front& f, int buf, 
   }
 }
 
+// The whole block: follows its front (buffer 0, f.n[0] entries) until no level
+// falls.  THREADS: the block's, 0: any number.  LOWER: `work` counts entries, and
+// 128 for each step (64 take ~0.5 us); past the budget, or where another block's
+// is spent, the rest is left to the wide resolution: returns whether it is.
+template <bool LOWER, int THREADS>
+__device__ __forceinline__ bool follow(const Resolve& r, Front& f, unsigned int nu0,
+                                       unsigned int budget, unsigned int& steps, unsigned int& work) {
+  const FillWork& w = r.w;
+  volatile unsigned int* vs = w.scal;
+  int buf = 0, cnt = 0;
+  bool stop = false;  // (thread 0's)
+  for (;;) {
+    // (A half full buffer is emptied; what does not fit a step is listed at once.)
+    if (__syncthreads_or(LOWER && threadIdx.x == 0 && (f.nfresh > kFreshCells / 2 || stop))) {
+      if (threadIdx.x == 0) f.stop = stop;
+      list_fresh(r, f, nu0);  // (a block barrier at least)
+      if (f.stop) return true;
+    }
+    const int nf = min(f.n[cnt], kFrontCells);
+    const int nxt = cnt == 2 ? 0 : cnt + 1;
+    if (threadIdx.x == 0) f.n[nxt == 2 ? 0 : nxt + 1] = 0;
+    if (nf == 0) return false;
+    if (++steps > (1u << 26)) {  // every step lowers a level: far beyond any path
+      if (threadIdx.x == 0) atomicCAS((int*)(w.scal + S_ERR), 0, 4);
+      return false;
+    }
+    if (LOWER) {
+      const unsigned int before = work;
+      work += 128u + (unsigned int)nf;
+      if (work > budget) {
+        if (threadIdx.x == 0) vs[S_WIDE] = 1u;
+        return true;
+      }
+      // (A look costs the block an L2 access.)
+      if (((work ^ before) & 8192u) && threadIdx.x == 0) stop = vs[S_WIDE] != 0u;
+    }
+    const int k = threadIdx.x & 7;
+    for (int e = threadIdx.x >> 3; e < nf; e += (THREADS ? THREADS : (int)blockDim.x) / 8) {
+      const uint32_t c = f.cell[buf][e];
+      const float lv = f.level[buf][e];
+      const int nx = (int)(c % (uint32_t)w.W) + d8_dx(k), ny = (int)(c / (uint32_t)w.W) + d8_dy(k);
+      if (nx < 0 || nx >= w.W || ny < 0 || ny >= w.H) continue;
+      const int64_t b = (int64_t)ny * w.W + nx;
+      const float qb = r.q[b], nv = fmaxf(qb, lv);
+      const unsigned int fl = LOWER ? 0u : r.get(b);  // (kConfirmed does not change meanwhile)
+      // (Outlets are at their elevation.)
+      if (!(nv < r.level(b)) || qb == r.nodata) continue;
+      const int mine = (int)(__float_as_uint(nv) | 0x80000000u);
+      const int prev = atomicMin(reinterpret_cast<int*>(r.Wg + b), mine);
+      if (LOWER) {
+        const bool first = prev >= 0;
+        const unsigned int at = warp_append((unsigned int*)&f.nfresh, first);
+        if (first) {
+          __stcg(w.aux + b, (unsigned int)prev);
+          __stcg(w.label + b, (uint32_t)b);
+          if (at < kFreshCells) f.fresh[at] = (uint32_t)b;
+          else __stcg(w.cand + nu0 + atomicAdd(&w.scal[S_MORE], 1u), (uint32_t)b);
+        }
+      }
+      if (prev <= mine) continue;
+      // A wall that falls was above its q, so LOWER lets it relay.
+      if (LOWER || !r.wall(b, qb) || ((fl & kConfirmed) && nv > qb))
+        front_push(r, f, buf ^ 1, nxt, (uint32_t)b, nv);
+    }
+    buf ^= 1;
+    cnt = nxt;
+  }
+}
+
 // Relaxes from the active cells among the first nl of a list -- after that, what
 // a full buffer left among all na of it -- until no level falls.
 // LOWER: the list is cand; walls with S > q relay whatever their level, and a
@@ -668,16 +743,16 @@ __device__ __forceinline__ void front_push(const Resolve& r, Front& f, int buf, 
 template <bool LOWER>
 __device__ unsigned int relax(const Resolve& r, Front& f, const uint32_t* list, unsigned int nl,
                               unsigned int na, unsigned int nblocks, bool minima,
-                              unsigned int* more, bool* ok) {
+                              unsigned int* more, bool* ok, unsigned int budget = 0) {
   const FillWork& w = r.w;
   const unsigned int nu0 = nl;
-  unsigned int steps = 0;
-  bool again_all = false;
+  unsigned int steps = 0, work = 0;
+  bool again_all = false, stop = false;
   for (bool again = true; again; again_all = true) {
     const unsigned int nu = LOWER ? nl + *more : again_all ? na : nl;
     const unsigned int run = min(LOWER ? kResolveRun : kReopenRun, (nu + nblocks - 1) / nblocks);
     if (threadIdx.x == 0) f.full = f.nfresh = 0;
-    for (unsigned int base = blockIdx.x * run; base < nu; base += nblocks * run) {
+    for (unsigned int base = blockIdx.x * run; base < nu && !stop; base += nblocks * run) {
       __syncthreads();
       if (threadIdx.x < 3) f.n[threadIdx.x] = 0;
       __syncthreads();
@@ -710,56 +785,23 @@ __device__ unsigned int relax(const Resolve& r, Front& f, const uint32_t* list, 
         }
         if (lowers) front_push(r, f, 0, 0, c, lv);
       }
-      int buf = 0, cnt = 0;
-      for (;;) {
-        // (A half full buffer is emptied; what does not fit a step is listed at once.)
-        if (__syncthreads_or(LOWER && threadIdx.x == 0 && f.nfresh > kFreshCells / 2))
-          list_fresh(r, f, nu0);
-        const int nf = min(f.n[cnt], kFrontCells);
-        const int nxt = cnt == 2 ? 0 : cnt + 1;
-        if (threadIdx.x == 0) f.n[nxt == 2 ? 0 : nxt + 1] = 0;
-        if (nf == 0) break;
-        if (++steps > (1u << 26)) {  // every step lowers a level: far beyond any path
-          if (threadIdx.x == 0) atomicCAS((int*)(w.scal + S_ERR), 0, 4);
-          break;
-        }
-        const int k = threadIdx.x & 7;
-        for (int e = threadIdx.x >> 3; e < nf; e += kResolveThreads / 8) {
-          const uint32_t c = f.cell[buf][e];
-          const float lv = f.level[buf][e];
-          const int nx = (int)(c % (uint32_t)w.W) + d8_dx(k), ny = (int)(c / (uint32_t)w.W) + d8_dy(k);
-          if (nx < 0 || nx >= w.W || ny < 0 || ny >= w.H) continue;
-          const int64_t b = (int64_t)ny * w.W + nx;
-          const float qb = r.q[b], nv = fmaxf(qb, lv);
-          const unsigned int fl = LOWER ? 0u : r.get(b);  // (kConfirmed does not change meanwhile)
-          // (Outlets are at their elevation.)
-          if (!(nv < r.level(b)) || qb == r.nodata) continue;
-          const int mine = (int)(__float_as_uint(nv) | 0x80000000u);
-          const int prev = atomicMin(reinterpret_cast<int*>(r.Wg + b), mine);
-          if (LOWER) {
-            const bool first = prev >= 0;
-            const unsigned int at = warp_append((unsigned int*)&f.nfresh, first);
-            if (first) {
-              __stcg(w.aux + b, (unsigned int)prev);
-              __stcg(w.label + b, (uint32_t)b);
-              if (at < kFreshCells) f.fresh[at] = (uint32_t)b;
-              else __stcg(w.cand + nu0 + atomicAdd(&w.scal[S_MORE], 1u), (uint32_t)b);
-            }
-          }
-          if (prev <= mine) continue;
-          // A wall that falls was above its q, so LOWER lets it relay.
-          if (LOWER || !r.wall(b, qb) || ((fl & kConfirmed) && nv > qb))
-            front_push(r, f, buf ^ 1, nxt, (uint32_t)b, nv);
-        }
-        buf ^= 1;
-        cnt = nxt;
-      }
+      stop = follow<LOWER, kResolveThreads>(r, f, nu0, budget, steps, work);
     }
     if (LOWER) list_fresh(r, f, nu0);
     __syncthreads();
     again = any_of(w, f, nblocks, f.full != 0, more, ok);
+    if (LOWER && f.stop) again = false;  // (in every block)
   }
   return steps;
+}
+
+// Work (follow()) that a block may spend on the lower bound: about the time that
+// the wide resolution's floods take, 0.3 ms and 45 ns per 1000 cells, so at worst
+// a fill takes twice as long as by the better way.  Terrain with streams stays far
+// below it: the longest front takes 157 steps of at most 2986 at 8192^2, 425 of
+// 11178 on 16384^2 cells with lakes, 178 of 508 on 2016x3073 with lakes.
+__device__ __forceinline__ unsigned int wide_budget(const FillWork& w) {
+  return 32768u + (unsigned int)((int64_t)w.W * w.H / 192);
 }
 
 // Steps 2 and 3, and the cells no outlet reaches.  A cooperative launch; only
@@ -780,8 +822,15 @@ __global__ void __launch_bounds__(kResolveThreads, 2) fill_resolve_kernel(Resolv
   unsigned int more = 0;
   bool ok = true;
   if (nu0) {
-    const unsigned int steps = relax<true>(r, front, w.cand, nu0, 0u, nblocks, false, &more, &ok);
+    const unsigned int steps =
+        relax<true>(r, front, w.cand, nu0, 0u, nblocks, false, &more, &ok, wide_budget(w));
     if (threadIdx.x == 0) atomicMax(&w.scal[S_STEPS], steps);
+    if (front.stop) {
+      if (tid == 0) vs[S_US_B] = (unsigned int)((global_ns() - t0) / 1000);
+      if (w.undone && !w.wide)
+        for (int64_t k = tid; k < w.H / r.slab_h; k += nthreads) w.undone[k] = 1;
+      return;
+    }
   }
   const unsigned long long t1 = global_ns();
   const unsigned int nu = ok ? nu0 + more : 0u;
@@ -988,6 +1037,396 @@ __global__ void __launch_bounds__(kResolveThreads, 2) fill_resolve_kernel(Resolv
   }
 }
 
+// ---- wide resolution ---------------------------------------------------------
+// Terrain without streams has lakes whose level the walls under water decide
+// far and wide: the falls of the lower bound then reach most cells, many times
+// over, and following them cell by cell takes longer than any flood.  The
+// resolution above gives up such a fill (S_WIDE), and this kernel, which leaves
+// at once otherwise, takes it from there: both bounds by floods over tiles
+// (levelflood.cuh), the cells between them listed tile by tile, and phases that
+// look at the walls still pending only, with every SM (the resolution above has
+// blocks for the list it starts from).  Whole fills, in ms, by the lists alone
+// and so: rough ground of 512^2 cells 38 and 13, of 2048^2 824 and 106; hills of
+// 2048^2 804 and 257, of 5000x3001 147 and 26; a bowl of 1024^2 11.9 and 1.9.
+// Bound by the phases: 0.05 to 0.3 ms each, of which there are up to 2000, and
+// in them by the fronts of lakes that drain one after another.
+//
+// The floods use the tiles' rims and masks, in the space of the labels; mdead
+// holds the cells that do not relay in the present flood, mclean the walls that
+// the walled flood left above their q (up), of which the second flood's start
+// keeps those not confirmed.
+
+// Levels of tile t's rim, from this lane's column: level(y), or +inf where dead.
+template <class Level, class Elev>
+__device__ __forceinline__ void wide_rim(const FillWork& w, int t, int lane, unsigned int dead,
+                                         Level level, Elev elev) {
+  uint2* rim = w.rim + (size_t)t * kRimCells;
+  for (int y = 0; y < kTile; y++) {
+    const bool d = (dead >> y) & 1u;
+    const float v = d ? kInf : level(y);
+    const uint2 e = make_uint2(__float_as_uint(v), d || v == elev(y) ? kRimFinal : 0u);
+    if (y == 0) rim[kTop * kTile + lane] = e;
+    if (y == kTile - 1) rim[kBottom * kTile + lane] = e;
+    if (lane == 0) rim[kLeft * kTile + y] = e;
+    if (lane == kTile - 1) rim[kRight * kTile + y] = e;
+  }
+}
+
+// Start of the lower bound's flood: the levels so far without their marks (they
+// are no lower than the bound), S of every cell in aux.
+__device__ __forceinline__ void wide_start_lower(const LevelArgs& a, int t, int lane) {
+  const FillWork& w = a.w;
+  const int x = (t % w.tiles_x) * kTile + lane, y0 = (t / w.tiles_x) * kTile;
+  const int64_t base = (int64_t)y0 * w.W + x;
+  const CellMasks m =
+      cell_masks(w, a.minslot, a.nodata, x, y0, [&](int y) { return a.q[base + (int64_t)y * w.W]; });
+  const unsigned int never = m.dead & ~m.wall;
+  unsigned int up = 0;
+  for (int y = 0; y < kTile; y++) {
+    if ((never >> y) & 1u) continue;
+    const int64_t i = base + (int64_t)y * w.W;
+    const float v = a.Wg[i];
+    float s = v;
+    if (__float_as_int(v) < 0) {  // listed: S is in aux
+      s = __uint_as_float(w.aux[i]);
+      a.Wg[i] = fabsf(v);
+    } else {
+      w.aux[i] = __float_as_uint(v);
+    }
+    if (((m.wall >> y) & 1u) && s > a.q[i]) up |= 1u << y;
+  }
+  const unsigned int dead = m.dead & ~up;
+  w.mdead[t * kTile + lane] = dead;
+  w.mwall[t * kTile + lane] = m.wall;
+  w.mclean[t * kTile + lane] = up;
+  wide_rim(w, t, lane, dead, [&](int y) { return __ldcg(a.Wg + base + (int64_t)y * w.W); },
+           [&](int y) { return a.q[base + (int64_t)y * w.W]; });
+  if (lane == 0) {
+    w.tvis[t] = kVisited | kUnsettled;
+    w.tseed[t] = 1;
+  }
+}
+
+// Start of the upper bound's flood: levels at S, A in aux, the walls that A
+// left above their q confirmed.  Only tiles with A != S can change.
+__device__ __forceinline__ void wide_start_upper(const LevelArgs& a, int t, int lane) {
+  const FillWork& w = a.w;
+  const int x = (t % w.tiles_x) * kTile + lane, y0 = (t / w.tiles_x) * kTile;
+  const int64_t base = (int64_t)y0 * w.W + x;
+  const unsigned int wall = w.mwall[t * kTile + lane], up = w.mclean[t * kTile + lane];
+  const unsigned int all = w.mdead[t * kTile + lane] | up, never = all & ~wall;
+  unsigned int confirmed = 0;
+  bool fell = false;
+  for (int y = 0; y < kTile; y++) {
+    if (x >= w.W || y0 + y >= w.H) break;
+    const int64_t i = base + (int64_t)y * w.W;
+    bool sure = false;
+    if (!((never >> y) & 1u)) {
+      const float v = __ldcg(a.Wg + i), s = __uint_as_float(w.aux[i]);
+      if (v != s) {
+        a.Wg[i] = s;
+        w.aux[i] = __float_as_uint(v);
+        fell = true;
+      }
+      sure = ((up >> y) & 1u) && v > a.q[i];
+    }
+    if (sure) confirmed |= 1u << y;
+    w.flags[i] = sure ? kConfirmed : 0;
+  }
+  const unsigned int dead = all & ~confirmed;
+  w.mdead[t * kTile + lane] = dead;
+  w.mclean[t * kTile + lane] = up & ~confirmed;
+  wide_rim(w, t, lane, dead, [&](int y) { return __ldcg(a.Wg + base + (int64_t)y * w.W); },
+           [&](int y) { return a.q[base + (int64_t)y * w.W]; });
+  fell = __any_sync(0xffffffffu, fell);
+  if (lane == 0) {
+    w.tvis[t] = kVisited | kUnsettled;
+    w.tseed[t] = fell;
+  }
+}
+
+// Upper bound of the walls not confirmed: they do not relay.
+__device__ __forceinline__ void wide_walls(const Resolve& r, int t, int lane) {
+  const FillWork& w = r.w;
+  const int x = (t % w.tiles_x) * kTile + lane, y0 = (t / w.tiles_x) * kTile;
+  for (unsigned int m = w.mclean[t * kTile + lane]; m; m &= m - 1) {
+    const int y = y0 + __ffs(m) - 1;
+    const int64_t i = (int64_t)y * w.W + x;
+    const float minE = ordered_to_float(r.minslot[y / r.slab_h]);
+    float least = kInf;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {  // a wall is interior: all 8 are in its slab
+      const int64_t n = i + (int64_t)d8_dy(k) * w.W + d8_dx(k);
+      if (relays(r.q[n], minE, r.nodata) || (r.get(n) & kConfirmed))
+        least = fminf(least, __ldcg(r.Wg + n));
+    }
+    const float v = fmaxf(r.q[i], least);
+    if (v < __ldcg(r.Wg + i)) __stcg(r.Wg + i, v);
+  }
+}
+
+// The cells of tile t where the bounds differ are flagged, the walls not
+// confirmed among them counted.
+__device__ __forceinline__ void wide_between(const Resolve& r, int t, int lane) {
+  const FillWork& w = r.w;
+  const int x = (t % w.tiles_x) * kTile + lane, y0 = (t / w.tiles_x) * kTile;
+  const unsigned int never = w.mdead[t * kTile + lane] & ~w.mwall[t * kTile + lane];
+  const unsigned int open = w.mclean[t * kTile + lane];
+  unsigned int walls = 0;
+  for (int y = 0; y < kTile && x < w.W && y0 + y < w.H; y++) {
+    if ((never >> y) & 1u) continue;
+    const int64_t i = (int64_t)(y0 + y) * w.W + x;
+    if (__ldcg(r.Wg + i) == r.walled(i)) continue;
+    const bool is_wall = (open >> y) & 1u;
+    w.flags[i] |= kUnsure | (is_wall ? kUnsureWall : 0u);  // (this lane's byte)
+    walls += is_wall;
+  }
+  walls = __reduce_add_sync(0xffffffffu, walls);
+  if (lane == 0 && walls) atomicAdd(&w.scal[S_UNSURE], walls);
+}
+
+// Those cells listed: such walls from the list's start, others from nq on, row by row.
+__device__ __forceinline__ void wide_list(const Resolve& r, int t, int lane, unsigned int nq) {
+  const FillWork& w = r.w;
+  const int x = (t % w.tiles_x) * kTile + lane, y0 = (t / w.tiles_x) * kTile;
+  unsigned int any = 0, wall = 0;
+  for (int y = 0; y < kTile && x < w.W && y0 + y < w.H; y++) {
+    const unsigned int f = __ldcg(w.flags + (int64_t)(y0 + y) * w.W + x);
+    if (f & kUnsure) any |= 1u << y;
+    if (f & kUnsureWall) wall |= 1u << y;
+  }
+  const unsigned int all = __reduce_add_sync(0xffffffffu, (unsigned int)__popc(any));
+  if (!all) return;
+  const unsigned int walls = __reduce_add_sync(0xffffffffu, (unsigned int)__popc(wall));
+  unsigned int at = 0, other = 0;
+  if (lane == 0) {
+    at = atomicAdd(&w.scal[S_FRONT], walls);
+    other = nq + atomicAdd(&w.scal[S_BEHIND], all - walls);
+  }
+  at = __shfl_sync(0xffffffffu, at, 0);
+  other = __shfl_sync(0xffffffffu, other, 0);
+  for (int y = 0; y < kTile; y++) {
+    const bool u = (any >> y) & 1u, is_wall = (wall >> y) & 1u;
+    const unsigned int bw = __ballot_sync(0xffffffffu, is_wall);
+    const unsigned int bo = __ballot_sync(0xffffffffu, u && !is_wall);
+    const unsigned int below = (1u << lane) - 1u;
+    if (u) {
+      const int64_t i = (int64_t)(y0 + y) * w.W + x;
+      __stcg(w.cand + (is_wall ? at + __popc(bw & below) : other + __popc(bo & below)), (uint32_t)i);
+      __stcg(w.label + i, (uint32_t)i);
+      __stcg(r.Wg + i, -__ldcg(r.Wg + i));  // marked
+    }
+    at += __popc(bw);
+    other += __popc(bo);
+  }
+}
+
+// The whole block: follows what did not fit a front (cells marked kActive).  The
+// block looks through its share of the flags; *again = whether any did not fit.
+__device__ void wide_rest(const Resolve& r, Front& f, unsigned int& steps) {
+  const FillWork& w = r.w;
+  const int64_t words = ((int64_t)w.W * w.H + 15) / 16;  // (the flags' space is a multiple of 256)
+  const int64_t share = (words + gridDim.x - 1) / gridDim.x;
+  const int64_t b0 = share * blockIdx.x, b1 = min(b0 + share, words);
+  unsigned int work = 0;
+  for (int64_t base = b0; base < b1; base += blockDim.x) {
+    __syncthreads();
+    if (threadIdx.x < 3) f.n[threadIdx.x] = 0;
+    __syncthreads();
+    if (base + threadIdx.x < b1) {
+      const int64_t c16 = (base + threadIdx.x) * 16;
+      const uint4 v = __ldcg(reinterpret_cast<const uint4*>(w.flags + c16));
+      const unsigned int f4[4] = {v.x, v.y, v.z, v.w};
+      static_assert(kActive == 1, "the low bit of each flag byte");
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        for (unsigned int m = f4[k] & 0x01010101u; m; m &= m - 1) {
+          const int64_t c = c16 + 4 * k + ((__ffs(m) - 1) >> 3);
+          r.clear(c, kActive);
+          __threadfence();  // a fall after the read below marks the cell again
+          // (Of a wall just confirmed: its component's minimum is used up.)
+          if (r.get(c) & kUnsureWall) __stcg(w.aux + __ldcg(w.label + c), 0xffffffffu);
+          front_push(r, f, 0, 0, (uint32_t)c, r.level(c));
+        }
+    }
+    follow<false, 0>(r, f, 0u, 0u, steps, work);
+  }
+}
+
+// The phases over the nq walls at the list's start, all levels marked.
+// Returns their number.
+__device__ int wide_phases(const Resolve& r, Front& f, unsigned int nq, bool* ok) {
+  const FillWork& w = r.w;
+  const unsigned int nblocks = gridDim.x;
+  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const unsigned int gwarp = blockIdx.x * warps + (threadIdx.x >> 5), nwarps = nblocks * warps;
+  unsigned int more = 0, steps = 0, work = 0;
+  int phases = 0;
+  // A warp's entries: groups of 32 at a stride, so that each warp has a part of
+  // every lake.  Those still pending are kept at the front of its own places.
+  auto place = [&](unsigned int k) { return ((k >> 5) * nwarps + gwarp) * 32u + (k & 31u); };
+  const unsigned int groups = (nq + 31u) / 32u;
+  unsigned int len = groups > gwarp ? (groups - gwarp + nwarps - 1) / nwarps * 32u : 0u;
+  if (len && place(len - 1) >= nq) len -= place(len - 1) - (nq - 1);
+  // fn(c) for each entry; it stays if that is true.
+  auto sift = [&](auto fn) {
+    unsigned int out = 0;
+    for (unsigned int k0 = 0; k0 < len; k0 += 32) {
+      const bool in = k0 + lane < len;
+      const uint32_t c = in ? __ldcg(w.cand + place(k0 + lane)) : 0u;
+      const bool keep = in && fn(c);
+      const unsigned int ball = __ballot_sync(0xffffffffu, keep);
+      const unsigned int to = out + __popc(ball & ((1u << lane) - 1u));
+      if (keep && to != k0 + lane) __stcg(w.cand + place(to), c);
+      out += __popc(ball);
+    }
+    __syncwarp();
+    len = out;
+  };
+  while (*ok) {
+    // The least level of each component's pending walls (above their q).
+    __syncthreads();
+    if (threadIdx.x < 3) f.n[threadIdx.x] = 0;
+    if (threadIdx.x == 0) f.full = f.nfresh = 0;
+    bool some = false;
+    sift([&](uint32_t c) {
+      const float lv = r.level(c);
+      if (!(lv > r.q[c])) return false;  // for good: levels only fall
+      if (lv < kInf) {
+        const uint32_t root = __ldcg(w.label + c);
+        // Every label is a root: a cell labelled otherwise would take a minimum
+        // nothing resets.
+        if (phases == 0 && __ldcg(w.label + root) != root) atomicCAS((int*)(w.scal + S_ERR), 0, 6);
+        if (__float_as_uint(lv) < __ldcg(w.aux + root)) atomicMin(&w.aux[root], __float_as_uint(lv));
+        some = true;
+      }
+      return true;
+    });
+    if (!any_of(w, f, nblocks, some, &more, ok)) break;
+    // Each phase confirms at least one cell of every component with a pending
+    // one (the cell holding its minimum).
+    if (++phases > (int)min(nq, 0x7fffff00u) + 8) {
+      if (threadIdx.x == 0) atomicCAS((int*)(w.scal + S_ERR), 0, 5);
+      break;  // (in every block)
+    }
+    sift([&](uint32_t c) {
+      const unsigned int m = __ldcg(w.aux + __ldcg(w.label + c));
+      if (m == 0xffffffffu || !(r.q[c] <= __uint_as_float(m))) return true;
+      r.set(c, kConfirmed);
+      const float lv = r.level(c);
+      if (lv < kInf) front_push(r, f, 0, 0, c, lv);
+      return false;
+    });
+    any_of(w, f, nblocks, false, &more, ok);
+    if (!*ok) break;
+    // The minima that were used are reset: the cell that holds one is among
+    // those just confirmed.
+    for (int e = threadIdx.x; e < min(f.n[0], kFrontCells); e += blockDim.x)
+      __stcg(w.aux + __ldcg(w.label + f.cell[0][e]), 0xffffffffu);
+    follow<false, 0>(r, f, 0u, 0u, steps, work);
+    for (;;) {
+      __syncthreads();
+      const bool full = f.full != 0;
+      if (!any_of(w, f, nblocks, full, &more, ok)) break;
+      if (threadIdx.x == 0) f.full = 0;
+      wide_rest(r, f, steps);
+    }
+  }
+  return phases;
+}
+
+template <int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 1)
+fill_resolve_wide_kernel(LevelArgs a, Resolve r, int flood_warps) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const FillWork& w = a.w;
+  volatile unsigned int* vs = w.scal;
+  if (!vs[S_WIDE] || vs[S_ERR]) return;  // (final before the launch)
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const int gwarp = blockIdx.x * warps + warp, nwarps = gridDim.x * warps;
+  const int ntiles = w.tiles_x * w.tiles_y;
+  GridSync gs{w.scal + S_BAR_COUNT, w.scal + S_BAR_GEN, (int*)(w.scal + S_ERR)};
+  LevelSmem& s = reinterpret_cast<LevelSmem*>(smraw)[warp];
+  const unsigned long long t0 = global_ns();
+  // A flood from the levels and masks that `start` leaves in every tile.
+  auto flood = [&](auto start) -> bool {
+    for (int t = gwarp; t < ntiles; t += nwarps) start(t);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      vs[S_HEAD] = 0u;  // (the queue is empty, abandoned tickets aside)
+      vs[S_TAIL] = 0u;
+      vs[S_DONE] = 0u;
+    }
+    if (!grid_barrier(gs, gridDim.x)) return false;
+    if (!seed_queue(w, gs, gwarp, nwarps, lane, ntiles)) return false;
+    if (warp < flood_warps)
+      drain(w, lane, ntiles, false, [&](int t, VisitStats& st) {
+        level_visit<false>(s, a, fill_queue(w), t, lane, st);
+      });
+    // (A failure is in the error word.)
+    return grid_barrier(gs, gridDim.x) && !__syncthreads_or(vs[S_ERR] != 0u);
+  };
+  if (!flood([&](int t) { wide_start_lower(a, t, lane); })) return;
+  const unsigned long long t1 = global_ns();
+  if (!flood([&](int t) { wide_start_upper(a, t, lane); })) return;
+  for (int t = gwarp; t < ntiles; t += nwarps) wide_walls(r, t, lane);
+  if (!grid_barrier(gs, gridDim.x)) return;
+  for (int t = gwarp; t < ntiles; t += nwarps) wide_between(r, t, lane);
+  if (!grid_barrier(gs, gridDim.x)) return;
+  // (No mask is read from here on: the labels take their space.)
+  const unsigned int nq = vs[S_UNSURE];
+  int phases = 0;
+  if (nq) {
+    for (int t = gwarp; t < ntiles; t += nwarps) wide_list(r, t, lane, nq);
+    if (!grid_barrier(gs, gridDim.x)) return;
+    const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
+    const int64_t no = (int64_t)nq + vs[S_BEHIND];
+    bool joined = true;
+    for (int64_t j = tid; j < 4 * no; j += nthreads) {  // four threads a cell: W, NW, N, NE
+      const int d = (int)(j & 3);
+      const uint32_t c = __ldcg(w.cand + (j >> 2));
+      const int cx = (int)(c % (uint32_t)w.W), cy = (int)(c / (uint32_t)w.W);
+      const int nx = cx + (d == 0 ? -1 : d - 2), ny = cy + (d == 0 ? 0 : -1);
+      if (nx < 0 || ny < 0 || nx >= w.W) continue;
+      const uint32_t n = (uint32_t)ny * (uint32_t)w.W + (uint32_t)nx;
+      if (r.get(n) & kUnsure) joined &= uf_unite(w.label, c, n);
+    }
+    if (!joined) atomicCAS((int*)(w.scal + S_ERR), 0, 6);
+    if (!grid_barrier(gs, gridDim.x)) return;
+    // From here aux holds the components' least pending level (at their roots).
+    for (int64_t j = tid; j < nq; j += nthreads) {
+      const uint32_t c = __ldcg(w.cand + j), root = uf_root(w.label, c);
+      w.label[c] = root;
+      __stcg(w.aux + root, 0xffffffffu);
+    }
+    if (!grid_barrier(gs, gridDim.x)) return;
+    Front& front = *reinterpret_cast<Front*>(smraw);
+    if (threadIdx.x == 0) front.gen = vs[S_BAR_GEN];  // (any_of fences before it arrives)
+    __syncthreads();
+    bool ok = true;
+    phases = wide_phases(r, front, nq, &ok);
+    if (!ok) return;
+  }
+  // The marks come off, and cells no outlet reached keep q.
+  for (int t = gwarp; t < ntiles; t += nwarps) {
+    const int x = (t % w.tiles_x) * kTile + lane, y0 = (t / w.tiles_x) * kTile;
+    for (int y = y0; y < min(y0 + kTile, w.H) && x < w.W; y++) {
+      const int64_t i = (int64_t)y * w.W + x;
+      const float qv = r.q[i], v = __ldcg(r.Wg + i), lv = fabsf(v);
+      if (qv == r.nodata) continue;
+      const float n = lv == kInf ? qv : lv;
+      if (__float_as_uint(n) != __float_as_uint(v)) r.Wg[i] = n;
+    }
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    const unsigned long long t2 = global_ns();
+    vs[S_PASS] = vs[S_PASS] + 4u + (unsigned int)phases;
+    vs[S_PHASES] = (unsigned int)phases;
+    vs[S_US_B] = vs[S_US_B] + (unsigned int)((t1 - t0) / 1000);
+    vs[S_US_P] = (unsigned int)((t2 - t1) / 1000);
+  }
+}
+
 __global__ void quantize_min_kernel(float* __restrict__ d, int W, int H, float nodata,
                                     unsigned int* minslot, uint8_t* __restrict__ tseed,
                                     int tiles_x) {
@@ -1073,6 +1512,30 @@ static cageo_status launch_resolve(const Resolve& r, cudaStream_t s) {
   return CAGEO_OK;
 }
 
+// The wide resolution: a block per SM, of which a small grid's floods use as many
+// warps as the flood would.
+static cageo_status launch_resolve_wide(const LevelArgs& a, const Resolve& r, cudaStream_t s) {
+  constexpr int kWarps = 20;
+  constexpr size_t kSmem = sizeof(LevelSmem) * kWarps;
+  static_assert(kSmem >= sizeof(Front), "the front lies in the tiles' space");
+  auto fn = fill_resolve_wide_kernel<kWarps>;
+  static PerDevice resident;
+  int blocks = 0;
+  cageo_status st = per_device(resident, &blocks, [&](int dev, int* v) -> cageo_status {
+    CAGEO_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
+    return resident_blocks((const void*)fn, kWarps * 32, kSmem, dev, v);
+  });
+  if (st) return st;
+  int grid, per;
+  flood_shape(a.w.tiles_x * a.w.tiles_y, blocks, kWarps, &grid, &per);
+  LevelArgs la = a;
+  Resolve lr = r;
+  void* params[] = {&la, &lr, &per};
+  CAGEO_CUDA(cudaLaunchCooperativeKernel((const void*)fn, dim3(grid), dim3(kWarps * 32), params,
+                                         kSmem, s));
+  return CAGEO_OK;
+}
+
 cageo_status fill_begin(const FillWork& w, cudaStream_t s) {
   const int ntiles = w.tiles_x * w.tiles_y;
   // 8 rim words (16 bytes each) per thread, but no more blocks than fill the GPU.
@@ -1085,12 +1548,19 @@ cageo_status fill_begin(const FillWork& w, cudaStream_t s) {
 
 static unsigned warp_per_tile_blocks(size_t nt) { return (unsigned)((nt + 7) / 8); }
 
+static LevelArgs walled_args(const float* q, float* filled, const FillWork& w, float nodata) {
+  return LevelArgs{q, filled, w, nodata, w.slab_min ? w.slab_min : w.scal + S_MIN, 0, 0};
+}
+
+static Resolve resolve_args(const LevelArgs& a) {
+  return Resolve{a.q, a.Wg, a.w, a.nodata, a.minslot, a.w.slab_h ? a.w.slab_h : a.w.H};
+}
+
 cageo_status fill_run(const float* q, float* filled, const FillWork& w, float nodata,
                       cudaStream_t s) {
   const unsigned tblocks = warp_per_tile_blocks((size_t)w.tiles_x * w.tiles_y);
   if (!w.seeded) fill_seed_kernel<<<tblocks, 256, 0, s>>>(q, w);
-  const unsigned int* minslot = w.slab_min ? w.slab_min : w.scal + S_MIN;
-  LevelArgs a{q, filled, w, nodata, minslot, 0, 0};
+  const LevelArgs a = walled_args(q, filled, w, nodata);
   if (w.marks) CAGEO_CUDA(cudaEventRecord(w.marks[0], s));
   cageo_status st = launch_level<false>(a, s);
   if (st) return st;
@@ -1098,8 +1568,9 @@ cageo_status fill_run(const float* q, float* filled, const FillWork& w, float no
   fill_walls_kernel<<<tblocks, 256, 0, s>>>(a);
   CAGEO_CUDA(cudaGetLastError());
   if (w.marks) CAGEO_CUDA(cudaEventRecord(w.marks[2], s));
-  st = launch_resolve(Resolve{q, filled, w, nodata, minslot, w.slab_h ? w.slab_h : w.H}, s);
-  if (st) return st;
+  const Resolve r = resolve_args(a);
+  if ((st = launch_resolve(r, s))) return st;
+  if (w.wide && (st = launch_resolve_wide(a, r, s))) return st;
   if (w.marks) CAGEO_CUDA(cudaEventRecord(w.marks[3], s));
   return CAGEO_OK;
 }
@@ -1180,9 +1651,9 @@ const char* fill_error_text(unsigned int error) {
   return error < 7 ? what[error] : "unknown error";
 }
 
-cageo_status fill_check_status(const FillWork& w, int64_t* stats) {
-  unsigned int h[S_SIZE];
-  CAGEO_CUDA(cudaMemcpy(h, w.scal, sizeof(h), cudaMemcpyDeviceToHost));
+const unsigned int* fill_wide_word(const FillWork& w) { return w.scal + S_WIDE; }
+
+static cageo_status check_scalars(const unsigned int (&h)[S_SIZE], int64_t* stats) {
   if (stats) {
     stats[0] = h[S_PASS];
     stats[1] = h[S_PHASES];
@@ -1208,6 +1679,27 @@ cageo_status fill_check_status(const FillWork& w, int64_t* stats) {
     return CAGEO_ERR_NO_CONVERGENCE;
   }
   return CAGEO_OK;
+}
+
+cageo_status fill_check_status(const FillWork& w, int64_t* stats) {
+  unsigned int h[S_SIZE];
+  CAGEO_CUDA(cudaMemcpy(h, w.scal, sizeof(h), cudaMemcpyDeviceToHost));
+  return check_scalars(h, stats);
+}
+
+cageo_status fill_finish(const float* q, float* filled, const FillWork& w, float nodata,
+                         int64_t* stats, cudaStream_t s) {
+  unsigned int h[S_SIZE];
+  CAGEO_CUDA(cudaStreamSynchronize(s));
+  CAGEO_CUDA(cudaMemcpy(h, w.scal, sizeof(h), cudaMemcpyDeviceToHost));
+  if (h[S_WIDE] && !h[S_ERR]) {
+    const LevelArgs a = walled_args(q, filled, w, nodata);
+    const cageo_status st = launch_resolve_wide(a, resolve_args(a), s);
+    if (st) return st;
+    CAGEO_CUDA(cudaStreamSynchronize(s));
+    CAGEO_CUDA(cudaMemcpy(h, w.scal, sizeof(h), cudaMemcpyDeviceToHost));
+  }
+  return check_scalars(h, stats);
 }
 
 }  // namespace cageo
@@ -1254,6 +1746,7 @@ extern "C" cageo_status cageo_pitfill(float* d_dem, float* d_filled, int W, int 
     if ((st = fill_quantize_min(d_dem, w, nodata_dem, stream))) return st;
     w.seeded = true;
     if ((st = fill_run(d_dem, d_filled, w, nodata_dem, stream))) return st;
+    return fill_finish(d_dem, d_filled, w, nodata_dem, nullptr, stream);
   }
   CAGEO_CUDA(cudaStreamSynchronize(stream));
   return fill_check_status(w, nullptr);

@@ -38,6 +38,12 @@ struct FillWork {
   // minE).  slab_h = 0: one realization, minimum in the scalar block.
   int slab_h = 0;
   const unsigned int* slab_min = nullptr;
+  // The lower bound of the resolution has a budget (see pitfill.cu).  A fill that
+  // would exceed it is left to the wide resolution: fill_run launches that, too,
+  // if `wide`; if not, such a fill is left unfinished, with undone[k] (not null)
+  // set for each slab k, and fill_finish or another fill_run finishes it.
+  bool wide = false;
+  int* undone = nullptr;
   // The fused front (or fill_quantize_min) has set the tile seeds; otherwise
   // the fill finds them itself.
   bool seeded = false;
@@ -85,6 +91,13 @@ unsigned int* fill_min_slot(const FillWork& w);
 constexpr int kFillStats = 17;
 constexpr int kFillScalars = 224;  // words of the scalar block
 cageo_status fill_check_status(const FillWork& w, int64_t* stats);
+// After a fill_run without `wide`, with the same arguments: waits for it, finishes
+// it if it was left unfinished, and checks its status like fill_check_status.
+cageo_status fill_finish(const float* q, float* filled, const FillWork& w, float nodata,
+                         int64_t* stats, cudaStream_t s);
+// The device word that is not 0 after a fill that took, or needs, the wide
+// resolution.
+const unsigned int* fill_wide_word(const FillWork& w);
 // The device word that a fill leaves at 0 or at an error (cleared by the next
 // fill_begin), and what that error says.
 const unsigned int* fill_error_word(const FillWork& w);

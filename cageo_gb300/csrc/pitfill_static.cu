@@ -78,6 +78,7 @@ extern "C" cageo_status cageo_pitfill_static(float* d_dem, float* d_filled, int 
     if ((st = fill_quantize_min(d_dem, w, nodata_dem, stream))) return st;
     w.seeded = true;
     if ((st = fill_run(d_dem, d_filled, w, nodata_dem, stream))) return st;
+    return fill_finish(d_dem, d_filled, w, nodata_dem, nullptr, stream);
   }
   CAGEO_CUDA(cudaStreamSynchronize(stream));
   return fill_check_status(w, nullptr);

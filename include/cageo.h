@@ -378,11 +378,13 @@ cageo_status cageo_pipeline_graph_kernels(cageo_pipeline* p, int64_t* h_count);
 cageo_status cageo_pipeline_profile(cageo_pipeline* p, uint32_t realization,
                                     float* h_ms, int n);
 /* Counters of the last run: [0] fill work-queue drains, [1] confirmation
- * phases, [2] flat-BFS passes, [3] trace jumps, [4] burn re-runs, [5] drains
+ * phases, [2] flat-BFS passes, [3] trace jumps, [4] realizations redone
+ * (burn check; fills that a step was not prepared for), [5] drains
  * of the flood, [6] most steps of a front in the resolution (drains of the
  * repair flood with a warm start), [7..9] microseconds of the flood, of the
  * resolution's lower bound (of the repair flood) and of the rest of the
- * resolution, [10..11] tile visits and sweep rounds of the flood, [12..13]
+ * resolution, [10..11] tile visits and sweep rounds of the flood (those of a
+ * wide resolution included), [12..13]
  * cells listed by the resolution and 0 (visits and rounds of the repair
  * flood), [14] flat cells, [15] microseconds of the flat BFS, [16..18]
  * kilo-cycles summed over the fill's tile visits spent staging, sweeping and
