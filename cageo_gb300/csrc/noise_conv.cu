@@ -69,9 +69,10 @@ __global__ void noise_kernel(float* __restrict__ out, int64_t n, uint32_t k0,
 // Output tile of a block (columns x rows), 256 threads.  A wider or taller
 // tile stages less halo per output but leaves fewer blocks per SM, and the
 // column pass (items of 8 rows x 2 columns over the tile's width plus the
-// halo) and the row pass (8 outputs per item) fill the 256 threads
-// differently for each shape and radius: at radius 15, 64 x 32 gives the
-// column pass 188 items, 96 x 32 gives it 252.  The cageo_convolve stage
+// halo, 4 rows at other radii than 15 and 23) and the row pass (8 or 4 outputs
+// per item, of two rows) fill the 256 threads differently for each shape and
+// radius: at radius 15, 64 x 32 gives the column pass 188 items, 96 x 32 gives
+// it 252.  The cageo_convolve stage
 // uses the first shape; the fused front takes the pipeline's choice.
 struct SepTile {
   int tw, th;
@@ -241,29 +242,48 @@ __device__ __forceinline__ f32x2 muladd2_rn(f32x2 acc, f32x2 w, f32x2 t, f32x2 o
   return p;
 }
 
-// 8 outputs along a line for two neighbouring lines at once: acc[j] = sum_t
-// v(j + t) * tap(t), t ascending, each sum starting at 0.  The window of 8
-// pairs is a ring of registers: tap t + u of a group of 8 finds output j's
-// value at (j + u) % 8 and replaces entry u.  LC > 0: the tap count is a
-// compile-time constant; LC = 0: runtime count L.
-template <int LC, class V, class Tap>
-__device__ __forceinline__ void conv_line8(int L, f32x2 one, V v, Tap tap, f32x2 (&acc)[8]) {
-  f32x2 win[8];
+// N outputs (8 or 4) along a line for two neighbouring lines at once: acc[j] =
+// sum_t v(j + t) * tap(t), t ascending, each sum starting at 0.  The window of N
+// pairs is a ring of registers: tap t + u of a group of N finds output j's
+// value at (j + u) % N and replaces entry u.  LC > 0: the tap count is a
+// compile-time constant; LC = 0: runtime count L, groups of 8 taps without a
+// test in between, so that their loads are in flight together.  (With a test
+// at every tap, and N = 8, which leaves half of a block's threads without an
+// item of the rows, a block spent most of its time on load latency: radius 64,
+// 3001x401 cells, 210 us against 114; radius 30, 1500x733 cells, 34 against
+// 28.5, 4096^2 cells 303 against 268.  N = 8 without the tests spills.)
+template <int LC, int N, class V, class Tap>
+__device__ __forceinline__ void conv_line(int L, f32x2 one, V v, Tap tap, f32x2 (&acc)[N]) {
+  f32x2 win[N];
 #pragma unroll
-  for (int j = 0; j < 8; j++) {
+  for (int j = 0; j < N; j++) {
     win[j] = v(j);
     acc[j] = 0;
   }
   const int n = LC > 0 ? LC : L;
+  auto step = [&](int t, int u) {
+    const f32x2 w = tap(t);
+#pragma unroll
+    for (int j = 0; j < N; j++) acc[j] = muladd2_rn(acc[j], win[(j + u) & (N - 1)], w, one);
+  };
+  int t = 0;
+  if (LC == 0) {
+#pragma unroll 1
+    for (; t + 8 < n; t += 8) {
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        step(t + u, u);
+        win[u & (N - 1)] = v(t + u + N);
+      }
+    }
+  }
 #pragma unroll(LC > 0 ? (LC + 7) / 8 : 1)
-  for (int t = 0; t < n; t += 8) {
+  for (; t < n; t += 8) {
 #pragma unroll
     for (int u = 0; u < 8; u++) {
       if (t + u < n) {
-        const f32x2 w = tap(t + u);
-#pragma unroll
-        for (int j = 0; j < 8; j++) acc[j] = muladd2_rn(acc[j], win[(j + u) & 7], w, one);
-        if (t + u + 1 < n) win[u] = v(t + u + 8);
+        step(t + u, u);
+        if (t + u + 1 < n) win[u & (N - 1)] = v(t + u + N);
       }
     }
   }
@@ -277,14 +297,15 @@ __host__ __device__ inline int sep_pad(int r) { return (r + 3) & ~3; }
 // 32 tiles, before the epilogue's quads: 0.58 ms; 4: 0.61), but 4 for radius
 // 23, whose longer unrolled lines would spill (16384^2: 3.14 ms; 5: 3.27).
 // 128 or 192 threads, or 6 blocks, are slower for both.  The lines are unrolled
-// for these two radii (the runtime loop takes 0.61 and 3.5 ms).  With the quads:
+// for these two radii (a runtime loop took 0.61 and 3.5 ms).  With the quads:
 // 0.51 ms, of which the convolution alone is 0.42 and its packed products and
 // sums, at two a clock and SM, 0.26.
 template <class Epi, int LC, int TW, int TH>
 __global__ void __launch_bounds__(kSepThreads, LC == 47 ? 4 : 5)
 conv_sep_kernel(const float* __restrict__ in, int W, int H,
                 const float* __restrict__ taps, int r, float one, Epi epi) {
-  static_assert(TW % 8 == 0 && TH % 8 == 0, "items are 8 outputs wide / 8 rows tall");
+  constexpr int N = LC > 0 ? 8 : 4;  // outputs of an item (see conv_line)
+  static_assert(TW % 8 == 0 && TH % 8 == 0, "whole items");
   extern __shared__ __align__(16) unsigned char smraw[];
   const int L = 2 * r + 1, rp = sep_pad(r);
   const int IW = TW + 2 * rp, IH = TH + 2 * r, TS = IW + 1;
@@ -332,40 +353,40 @@ conv_sep_kernel(const float* __restrict__ in, int W, int H,
   }
   cp_async_wait();
   __syncthreads();
-  // Column pass: tmp[y][ix] = sum_t in[y+t][ix] * taps[t]; an item is 8 rows
+  // Column pass: tmp[y][ix] = sum_t in[y+t][ix] * taps[t]; an item is N rows
   // of two adjacent columns.  The results are kept as pairs of rows, which is
   // what the row pass multiplies; its row stride is odd, so 16 row pairs are
   // read without bank conflicts.
   const int p0 = (rp - r) >> 1, np = ((rp + TW + r + 1) >> 1) - p0;
-  for (int item = threadIdx.x; item < np * (TH / 8); item += kSepThreads) {
+  for (int item = threadIdx.x; item < np * (TH / N); item += kSepThreads) {
     const int g = item / np, ix = 2 * (p0 + item - g * np);
-    const float* base = s_in + (8 * g) * IW + ix;
-    f32x2 acc[8];
-    conv_line8<LC>(L, one2,
-                   [&](int k) { return *reinterpret_cast<const f32x2*>(base + k * IW); },
-                   [&](int t) { return s_taps[t]; }, acc);
+    const float* base = s_in + (N * g) * IW + ix;
+    f32x2 acc[N];
+    conv_line<LC, N>(L, one2,
+                     [&](int k) { return *reinterpret_cast<const f32x2*>(base + k * IW); },
+                     [&](int t) { return s_taps[t]; }, acc);
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
+    for (int j = 0; j < N / 2; j++) {
       float a0, a1, b0, b1;
       unpack2(acc[2 * j], a0, a1);
       unpack2(acc[2 * j + 1], b0, b1);
-      f32x2* o = s_tmp + (4 * g + j) * TS + ix;
+      f32x2* o = s_tmp + (N / 2 * g + j) * TS + ix;
       o[0] = pack2(a0, b0);
       o[1] = pack2(a1, b1);
     }
   }
   __syncthreads();
-  // Row pass: an item is 8 consecutive outputs of two rows.
+  // Row pass: an item is N consecutive outputs of two rows.
   constexpr int OS = TW + 4;
   float* s_out = s_in;
-  for (int item = threadIdx.x; item < (TH / 2) * (TW / 8); item += kSepThreads) {
+  for (int item = threadIdx.x; item < (TH / 2) * (TW / N); item += kSepThreads) {
     const int g = item / (TH / 2), j = item - g * (TH / 2);
-    const f32x2* base = s_tmp + j * TS + 8 * g + (rp - r);
-    f32x2 acc[8];
-    conv_line8<LC>(L, one2, [&](int k) { return base[k]; }, [&](int t) { return s_taps[t]; }, acc);
-    float* o = s_out + 2 * j * OS + 8 * g;
+    const f32x2* base = s_tmp + j * TS + N * g + (rp - r);
+    f32x2 acc[N];
+    conv_line<LC, N>(L, one2, [&](int k) { return base[k]; }, [&](int t) { return s_taps[t]; }, acc);
+    float* o = s_out + 2 * j * OS + N * g;
 #pragma unroll
-    for (int k = 0; k < 8; k++) unpack2(acc[k], o[k], o[OS + k]);
+    for (int k = 0; k < N; k++) unpack2(acc[k], o[k], o[OS + k]);
   }
   __syncthreads();
   tile_out<TW, TH>(s_out, OS, x0, y0, W, H, epi);
