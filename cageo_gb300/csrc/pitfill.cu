@@ -678,15 +678,15 @@ __device__ __forceinline__ bool follow(const Resolve& r, Front& f, unsigned int 
       if (threadIdx.x == 0) atomicCAS((int*)(w.scal + S_ERR), 0, 4);
       return false;
     }
-    if (LOWER) {
+    if (LOWER && threadIdx.x == 0) {
       const unsigned int before = work;
       work += 128u + (unsigned int)nf;
       if (work > budget) {
-        if (threadIdx.x == 0) vs[S_WIDE] = 1u;
-        return true;
+        vs[S_WIDE] = 1u;
+        stop = true;
+      } else if ((work ^ before) & 8192u) {  // (a look costs the block an L2 access)
+        stop = vs[S_WIDE] != 0u;
       }
-      // (A look costs the block an L2 access.)
-      if (((work ^ before) & 8192u) && threadIdx.x == 0) stop = vs[S_WIDE] != 0u;
     }
     const int k = threadIdx.x & 7;
     for (int e = threadIdx.x >> 3; e < nf; e += (THREADS ? THREADS : (int)blockDim.x) / 8) {
