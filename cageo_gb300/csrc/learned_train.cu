@@ -292,6 +292,89 @@ train_conv1_kernel(const float* __restrict__ in, const float* __restrict__ w,
   }
 }
 
+// ---- grids a few cells wide ------------------------------------------------------
+// The same sums with one cell and COUT channels a thread, in the same order: the
+// tiles above are 32 columns wide whatever the grid is.
+template <int COUT, bool FLIP>
+__global__ void __launch_bounds__(kTrainThreads)
+train_conv_narrow_kernel(const float* __restrict__ in, int cin, const float* __restrict__ w,
+                         const float* __restrict__ bias, const float* __restrict__ mask,
+                         float* __restrict__ out, int W, int H, int B, int relu) {
+  extern __shared__ __align__(16) float smem[];  // [ci][t][co]
+  for (int k = threadIdx.x; k < COUT * cin * 9; k += kTrainThreads) {
+    const int t = k % 9, p = k / 9;  // FLIP: [ci][co][8 - t], otherwise [co][ci][t]
+    const int ci = FLIP ? p / COUT : p % cin, co = FLIP ? p % COUT : p / cin;
+    smem[(ci * 9 + (FLIP ? 8 - t : t)) * COUT + co] = bf16_round(w[k]);
+  }
+  __syncthreads();
+  const int64_t n = (int64_t)W * H, i = (int64_t)blockIdx.x * kTrainThreads + threadIdx.x;
+  if (i >= n * B) return;
+  const int b = (int)(i / n);
+  const int64_t c = i - (int64_t)b * n;
+  const int x = (int)(c % W), y = (int)(c / W);
+  float acc[COUT];
+#pragma unroll
+  for (int co = 0; co < COUT; co++) acc[co] = bias ? bf16_round(bias[co]) : 0.0f;
+  for (int ci = 0; ci < cin; ci++) {
+    const float* plane = in + ((int64_t)b * cin + ci) * n;
+#pragma unroll
+    for (int t = 0; t < 9; t++) {
+      const int xx = x + t % 3 - 1, yy = y + t / 3 - 1;
+      if (xx < 0 || yy < 0 || xx >= W || yy >= H) continue;
+      const float a = plane[(int64_t)yy * W + xx];
+#pragma unroll
+      for (int co = 0; co < COUT; co++) acc[co] = fmaf(smem[(ci * 9 + t) * COUT + co], a, acc[co]);
+    }
+  }
+  const int64_t o = (int64_t)b * COUT * n + c;
+#pragma unroll
+  for (int co = 0; co < COUT; co++) {
+    float v = relu ? fmaxf(acc[co], 0.0f) : acc[co];
+    if (mask && !(mask[o + co * n] > 0.0f)) v = 0.0f;
+    out[o + co * n] = v;
+  }
+}
+
+// Weight gradients of such grids: a block per output channel and input channel.
+__global__ void __launch_bounds__(256)
+train_wgrad_narrow_kernel(const float* __restrict__ dz, int cout, const float* __restrict__ a,
+                          int cin, float* __restrict__ gw, float* __restrict__ gb, int W, int H,
+                          int B) {
+  const int co = blockIdx.x / cin, ci = blockIdx.x % cin;
+  const int64_t n = (int64_t)W * H;
+  float s[10] = {};
+  for (int64_t i = threadIdx.x; i < n * B; i += 256) {
+    const int b = (int)(i / n);
+    const int64_t c = i - (int64_t)b * n;
+    const float g = dz[((int64_t)b * cout + co) * n + c];
+    if (g == 0.0f) continue;
+    const float* p = a + ((int64_t)b * cin + ci) * n;
+    const int x = (int)(c % W), y = (int)(c / W);
+#pragma unroll
+    for (int t = 0; t < 9; t++) {
+      const int xx = x + t % 3 - 1, yy = y + t / 3 - 1;
+      if (xx < 0 || yy < 0 || xx >= W || yy >= H) continue;
+      s[t] = fmaf(g, p[(int64_t)yy * W + xx], s[t]);
+    }
+    s[9] += g;
+  }
+  __shared__ float red[8][10];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int t = 0; t < 10; t++) {
+    float v = s[t];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) red[warp][t] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x < 10) {
+    float v = 0.0f;
+    for (int k = 0; k < 8; k++) v += red[k][threadIdx.x];
+    if (threadIdx.x < 9) gw[(co * cin + ci) * 9 + threadIdx.x] += v;
+    else if (ci == 0) gb[co] += v;
+  }
+}
+
 // ---- weight gradients ---------------------------------------------------------
 // gw[co][ci][t] += sum_b sum_cell dz[b][co](y,x) * a[b][ci](y+dy, x+dx) and
 // gb[co] += sum dz[b][co].
@@ -607,6 +690,15 @@ cageo_status train_sms(int* sms) {
 
 struct Shape {
   int W, H, B, sms;
+  int64_t cells() const { return (int64_t)W * H * B; }
+  // Grids whose rows fill little of a tile's.  Forward, 16 x 12x20000: tiles 5.9
+  // ms, a cell a thread 3.9; 64 x 3x400: 0.52 and 0.13; from 14 columns on tiles.
+  bool narrow() const { return W <= 12; }
+  // The weight gradients' blocks are as many as their sums have room for, 289
+  // cells each, which few columns spread over many tiles; a block per channel pair
+  // walks all cells alone.  A backward pass of 2 x 3x400: 0.35 ms by tiles, 0.11 by
+  // pairs; of 16 x 4x300 0.32 and 0.36; of 64 x 3x400 0.71 and 1.23.
+  bool narrow_sums() const { return W <= 24 && cells() * W <= 65536; }
   bool aligned(std::initializer_list<const void*> ptrs) const {
     uintptr_t m = W & 3 ? 1 : 0;
     for (const void* p : ptrs) m |= (uintptr_t)p & 15u;
@@ -617,6 +709,12 @@ struct Shape {
 template <bool FLIP>
 void conv32(const Shape& g, const float* in, int cin, const float* w, const float* bias,
             const float* mask, float* out, int relu, cudaStream_t s) {
+  if (g.narrow()) {
+    train_conv_narrow_kernel<32, FLIP><<<(unsigned)((g.cells() + kTrainThreads - 1) / kTrainThreads),
+                                         kTrainThreads, 32 * cin * 9 * sizeof(float), s>>>(
+        in, cin, w, bias, mask, out, g.W, g.H, g.B, relu);
+    return;
+  }
   const int64_t tiles = TrainTiles(g.W, g.H, g.B, kConvRows).count;
   train_conv32_kernel<FLIP><<<(unsigned)std::min<int64_t>(tiles, 3 * g.sms), kTrainThreads,
                               conv32_smem(cin), s>>>(in, cin, w, bias, mask, out, g.W, g.H, g.B,
@@ -628,8 +726,13 @@ template <int COUT, int TCO, int CIG, int PXS, int ROWS>
 void wgrad(const Shape& g, const float* dz, const float* a, float* gw, float* gb, float* part,
            cudaStream_t s) {
   using K = Wgrad<COUT, TCO, CIG, PXS, ROWS>;
+  if (g.narrow_sums()) {
+    train_wgrad_narrow_kernel<<<COUT * K::kCin, 256, 0, s>>>(dz, COUT, a, K::kCin, gw, gb, g.W, g.H,
+                                                             g.B);
+    return;
+  }
   const int64_t tiles = TrainTiles(g.W, g.H, g.B, ROWS).count;
-  const int64_t room = 32 * (int64_t)g.W * g.H * g.B / K::kSums;
+  const int64_t room = 32 * g.cells() / K::kSums;
   const int per = std::min(3, 220 * 1024 / K::kSmem);  // resident blocks per SM
   const int blocks = (int)std::max<int64_t>(1, std::min({tiles, room, (int64_t)per * g.sms}));
   train_wgrad_kernel<COUT, TCO, CIG, PXS, ROWS><<<blocks, kTrainThreads, K::kSmem, s>>>(
@@ -655,9 +758,15 @@ extern "C" cageo_status cageo_ws_forward(const float* d_params, const float* d_f
   if (st) return st;
   conv32<false>(g, d_feat, 4, d_params + kOffW1, d_params + kOffB1, nullptr, d_a1, 1, stream);
   conv32<false>(g, d_a1, 32, d_params + kOffW2, d_params + kOffB2, nullptr, d_a2, 1, stream);
-  const int64_t tiles = TrainTiles(W, H, B, kConvRows).count;
-  train_conv1_kernel<<<(unsigned)std::min<int64_t>(tiles, 7 * g.sms), kTrainThreads, 0, stream>>>(
-      d_a2, d_params + kOffW3, d_params + kOffB3, d_out, W, H, B);
+  if (g.narrow()) {
+    train_conv_narrow_kernel<1, false><<<(unsigned)((g.cells() + kTrainThreads - 1) / kTrainThreads),
+                                         kTrainThreads, 32 * 9 * sizeof(float), stream>>>(
+        d_a2, 32, d_params + kOffW3, d_params + kOffB3, nullptr, d_out, W, H, B, 0);
+  } else {
+    const int64_t tiles = TrainTiles(W, H, B, kConvRows).count;
+    train_conv1_kernel<<<(unsigned)std::min<int64_t>(tiles, 7 * g.sms), kTrainThreads, 0, stream>>>(
+        d_a2, d_params + kOffW3, d_params + kOffB3, d_out, W, H, B);
+  }
   CAGEO_CUDA(cudaGetLastError());
   return CAGEO_OK;
 }
