@@ -338,9 +338,8 @@ def ws_backward(params, feat, a1, a2, dout, grad, tmp1=None, tmp2=None, wflip=No
     B, _, H, W = feat.shape
     tmp1 = torch.empty_like(a1) if tmp1 is None else tmp1
     tmp2 = torch.empty_like(a1) if tmp2 is None else tmp2
-    wflip = torch.empty(9216, dtype=torch.float32, device=feat.device) if wflip is None else wflip
     _check(lib().cageo_ws_backward(_ptr(params), _ptr(feat), _ptr(a1), _ptr(a2), _ptr(dout), W, H,
-                                   B, _ptr(grad), _ptr(tmp1), _ptr(tmp2), _ptr(wflip), _stream()))
+                                   B, _ptr(grad), _ptr(tmp1), _ptr(tmp2), _ptr(tmp1 if wflip is None else wflip), _stream()))
     return grad
 
 
@@ -459,7 +458,7 @@ class Pipeline:
 
     def autotune(self, first, trials=3):
         """Pick the tuning (the fill's sweep rounds per tile visit and warps
-        per SM of its lower-bound flood, then the front's convolution tile)
+        per SM of its flood, then the front's convolution tile)
         by timing every candidate; resets the counts.  Returns (chosen
         tuning, [(candidate, ms per realization)]); a convolution tile that
         does not apply has 0 ms."""

@@ -5,10 +5,10 @@
 // will flood it.  Cells predicted dry start the fill at their own elevation,
 // the others at +inf; the fill then relaxes down from that start
 // (fill_run_exact with a warm surface).  A start below the answer anywhere
-// leaves a wrong, lower surface, so the pipeline verifies every warm-started
-// realization by its tracing (every cell must drain to an outlet) and
-// repairs the cells that do not drain (see pipeline.cu): the counts stay
-// bit-identical to the plain exact fill.
+// would leave a wrong, lower surface, so the fill verifies every warm start: a
+// level counts only where a chain of relays from an outlet supports it, and the
+// other cells restart from +inf and are flooded again (fill_unsupported_kernel
+// in pitfill.cu).  The counts stay bit-identical to the plain exact fill's.
 //
 // Network: features (4 channels) -> conv 3x3, 32 channels, ReLU -> conv 3x3,
 // 32 channels, ReLU -> conv 3x3, 1 channel (predicted depth, metres).  Zero

@@ -591,8 +591,10 @@ static void set_step(cageo_pipeline* p, int K) {
 // small grid is a chain of ~15 launches that leave most of the GPU idle (330
 // us at 512^2, 20 of them stacked: 700 us), so as many are stacked as
 // make up kStackCells cells (about 32 bytes a cell: 2.1 GB).  Four at 4096^2:
-// 3.9 ms in one step, 4.5 in two (6.5 singly, measured with slower stages);
-// twice as many cells a step gain nothing there.
+// 3.9 ms in one step, 4.5 in two (6.5 singly, measured with slower stages).
+// The limit is one of memory: larger grids gain from stacks, too (8192^2: 3.82 ms a
+// realization singly, 3.43 in steps of 4, 3.31 of 16), but at 1.9 GB each a program
+// has to ask for those (cageo_pipeline_set_batch).
 constexpr int64_t kStackCells = (int64_t)1 << 26;
 
 // Rows of a stack: launches over tiles of 32 rows have them in grid.y.
@@ -1100,7 +1102,7 @@ extern "C" cageo_status cageo_pipeline_reset_counts(cageo_pipeline* p) {
 }
 
 // Candidate settings of the autotuner: sweep rounds per fill tile visit x
-// warps per SM of the fill's lower-bound flood (with the first convolution
+// warps per SM of the fill's flood (with the first convolution
 // tile), then the other convolution tiles with the fill setting chosen
 // among those (fill fields 0).  The front and the fill are separate stages,
 // so tuning them one after the other finds the best of the product.

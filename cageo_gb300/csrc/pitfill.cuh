@@ -13,7 +13,7 @@ struct FillWork {
   int W = 0, H = 0;
   int tiles_x = 0, tiles_y = 0;
   uint8_t* flags = nullptr;      // W*H: cell flags of the resolution
-  int* queued = nullptr;         // ntiles: tile state in the work queue (idle, queued, processing, re-queued, done)
+  int* queued = nullptr;         // ntiles: tile state in the work queue (tilequeue.cuh)
   int* lists = nullptr;          // 2 * ntiles + kRingSlack: the work queue's ring
   uint8_t* tseed = nullptr;      // ntiles: tile holds an outlet (or a cell to repair)
   uint8_t* tvis = nullptr;       // ntiles: tile state of the flood (levelflood.cuh)
@@ -23,13 +23,14 @@ struct FillWork {
   // The flood (levelflood.cuh), in the space of the labels: per tile the rim
   // entries (4 sides x 32: level bits, flags), and 32 column masks each (lane
   // = column, bit = row) of the cells that are clean, that never relay in
-  // the flood, and that are walls (interior and not passable).
+  // the flood, and that are walls (interior and not passable).  (The wide
+  // resolution keeps other cells in the first two.)
   uint2* rim = nullptr;
   uint32_t *mclean = nullptr, *mdead = nullptr, *mwall = nullptr;
   unsigned int* scal = nullptr;  // scalar block (see pitfill.cu)
   int max_rounds = 64;           // sweep rounds per tile visit before the tile re-queues itself
   int flood_warps = 20;          // warps per block (per SM) of the flood: 16, 20 or 22
-  // Stacked realizations (CPU-compatible fill only): the grid holds
+  // Stacked realizations (cold starts of either fill): the grid holds
   // H / slab_h realizations of slab_h rows each, one above the other.
   // Every slab's first and last rows are its border (outlets), so no flood
   // value crosses from one slab to another: a cell that is not on a border

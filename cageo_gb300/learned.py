@@ -100,7 +100,6 @@ def train(steps=2000, batch=16, crop=128, lr=2e-3, seed=0, source=None, log=prin
     loss = torch.zeros(1, device=dev)
     tmp1 = torch.empty((batch, 32, crop, crop), device=dev)
     tmp2 = torch.empty_like(tmp1)
-    wflip = torch.empty(9216, device=dev)
     rng = np.random.default_rng(seed)
     H, W = src.shape
     hist = []
@@ -117,7 +116,7 @@ def train(steps=2000, batch=16, crop=128, lr=2e-3, seed=0, source=None, log=prin
         loss.zero_()
         api.ws_mse(out, tb, dy, loss, margin=3)
         grad.zero_()
-        api.ws_backward(params, fb, a1, a2, dy, grad, tmp1, tmp2, wflip)
+        api.ws_backward(params, fb, a1, a2, dy, grad, tmp1, tmp2)
         step_lr = lr * (0.05 ** (step / steps))  # exponential decay to 5 %
         api.ws_adam(params, grad, m1, m2, step_lr, step)
         if step % 50 == 0 or step == 1:

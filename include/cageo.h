@@ -260,7 +260,8 @@ cageo_status cageo_ws_forward(const float* d_params, const float* d_feat, int W,
                               cudaStream_t stream);
 /* Backward pass: adds the gradient of the loss (given d_dout = dL/d out)
  * with respect to every parameter into d_grad.  d_tmp1, d_tmp2:
- * [B][32][H][W] scratch; d_wflip: 9216 floats of scratch. */
+ * [B][32][H][W] scratch; d_wflip: not null; nothing is read or written there
+ * (it once held 9216 floats of flipped weights). */
 cageo_status cageo_ws_backward(const float* d_params, const float* d_feat, const float* d_a1,
                                const float* d_a2, const float* d_dout, int W, int H, int B,
                                float* d_grad, float* d_tmp1, float* d_tmp2, float* d_wflip,
